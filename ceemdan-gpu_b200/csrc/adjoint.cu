@@ -12,7 +12,7 @@
 // and these kernels apply the transposed maps in reverse order, one launch per step of one
 // iteration over all realizations.  The spline matrix restricted to its interior rows is
 // symmetric, so the transposed solve is the forward's canonical partitioned solve with a new
-// right-hand side (cta_tridiag).  Every kernel is deterministic (no atomics; fixed summation
+// right-hand side (cta_spline_tridiag).  Every kernel is deterministic (no atomics; fixed summation
 // orders), and the arithmetic order is the CPU oracle's (oracle/ceemdan_oracle.cpp,
 // env_adjoint, sift_adjoint, vjp).
 #include "canon.cuh"
@@ -262,7 +262,7 @@ k_adj_solve(const unsigned char* slot, TapeLayout L, int cap, const double* sys,
     const Slot v = view(slot, L);
     const int sp = blockIdx.x;
     if (!updated(v, L.nr, sp % L.nr)) return;
-    cta_tridiag(knots(v, sp, cap), sys + (size_t)sp * 4 * cap, cap, z + (size_t)sp * cap,
+    cta_spline_tridiag(knots(v, sp, cap), sys + (size_t)sp * 4 * cap, cap, z + (size_t)sp * cap,
                 ws + (size_t)sp * ws_stride);
 }
 

@@ -226,7 +226,9 @@ __global__ void k_tridiag_batched(int n, const double* l, const double* m, const
 // (l, m, u, r) at sys, solution to x, workspace ws of >= 0.75*n + 16 doubles; every thread of
 // the CTA calls it.
 __device__ void cta_tridiag(int n, const double* sys, int plane, double* x, double* ws);
-// cta_tridiag's solve for nsys systems at once, one level per launch (sift_kernels.cu)
+// the same solve of a spline system (pivots in pivot_inv's range)
+__device__ void cta_spline_tridiag(int n, const double* sys, int plane, double* x, double* ws);
+// cta_spline_tridiag's solve for nsys systems at once, one level per launch (sift_kernels.cu)
 cudaError_t psolve_launch(int nsys, int max_rows, const int* nrows, const double* sys, int plane,
                           double* x, double* ws, size_t ws_stride, cudaStream_t st,
                           int* launches, const int32_t* kx);

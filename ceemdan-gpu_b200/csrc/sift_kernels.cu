@@ -275,18 +275,18 @@ struct ChunkEnds {
 // End relations of a chunk of `len` rows: top-down elimination gives the last row
 // x_b = gb + ab*xL + bb*xR, bottom-up elimination the first row x_a = ga + aa*xL + ba*xR.
 // The two sweeps are independent chains and run interleaved.
-template <class RowFn>
+template <class Pivot = SplinePivot, class RowFn>
 __device__ __forceinline__ ChunkEnds chunk_ends(int len, const RowFn& row) {
     const Row wa = row(0), wb = row(len - 1);
-    double iw = 1.0 / wa.m;
+    double iw = Pivot::inv(wa.m);
     double cp = wa.u * iw, gp = wa.r * iw, ap = -wa.l * iw;
-    double iv = 1.0 / wb.m;
+    double iv = Pivot::inv(wb.m);
     double cq = wb.l * iv, gq = wb.r * iv, bq = -wb.u * iv;
     for (int k = 1; k < len; ++k) {
         const Row w = row(k);
         const Row v = row(len - 1 - k);
-        iw = 1.0 / fma(-w.l, cp, w.m);
-        iv = 1.0 / fma(-v.u, cq, v.m);
+        iw = Pivot::inv(fma(-w.l, cp, w.m));
+        iv = Pivot::inv(fma(-v.u, cq, v.m));
         cp = w.u * iw;
         gp = fma(-w.l, gp, w.r) * iw;
         ap = (-w.l * ap) * iw;
@@ -307,7 +307,7 @@ __device__ __forceinline__ ChunkEnds chunk_ends(int len, const RowFn& row) {
 // Interior of a chunk of `len` rows once its separator values xl, xr are known: coupling
 // terms move to the right-hand side, then canonical Thomas; x_k written to out[k*stride].
 // kCoupled = false is the plain canonical Thomas (no coupling terms at all).
-template <bool kCoupled = true, class RowFn, class Out>
+template <bool kCoupled = true, class Pivot = SplinePivot, class RowFn, class Out>
 __device__ __forceinline__ void chunk_interior(int len, const RowFn& row, double xl, double xr,
                                                Out out, int stride) {
     double cp[kChunk], gp[kChunk];
@@ -319,11 +319,11 @@ __device__ __forceinline__ void chunk_interior(int len, const RowFn& row, double
             if (kCoupled && k == 0) ri = fma(-w.l, xl, ri);
             if (kCoupled && k == len - 1) ri = fma(-w.u, xr, ri);
             if (k == 0) {
-                const double iw = 1.0 / w.m;
+                const double iw = Pivot::inv(w.m);
                 cp[0] = w.u * iw;
                 gp[0] = ri * iw;
             } else {
-                const double iw = pivot_rcp(w, cp[k - 1]);
+                const double iw = Pivot::inv(fma(-w.l, cp[k - 1], w.m));
                 cp[k] = w.u * iw;
                 gp[k] = fma(-w.l, gp[k - 1], ri) * iw;
             }
@@ -340,9 +340,9 @@ __device__ __forceinline__ void chunk_interior(int len, const RowFn& row, double
 }
 
 // Canonical Thomas on n <= kChunk rows (base case), x written with stride.
-template <class RowFn>
+template <class Pivot = SplinePivot, class RowFn>
 __device__ __forceinline__ void thomas_small(int n, const RowFn& row, double* x, int stride) {
-    chunk_interior<false>(n, row, 0.0, 0.0, x, stride);
+    chunk_interior<false, Pivot>(n, row, 0.0, 0.0, x, stride);
 }
 
 }  // namespace
@@ -698,9 +698,9 @@ __device__ __forceinline__ ChunkEnds chunk_ends_slab(const int32_t* x, const dou
                                                      int len) {
     auto row = [&](int k) { return spline_row(x[k], x[k + 1], x[k + 2], s[k], s[k + 1]); };
     const Row wa = row(0), wb = row(len - 1);
-    double iw = 1.0 / wa.m;
+    double iw = pivot_inv(wa.m);
     double cp = wa.u * iw, gp = wa.r * iw, ap = -wa.l * iw;
-    double iv = 1.0 / wb.m;
+    double iv = pivot_inv(wb.m);
     double cq = wb.l * iv, gq = wb.r * iv, bq = -wb.u * iv;
     Row wn = wa, vn = wb;
     if (len > 1) {
@@ -713,8 +713,8 @@ __device__ __forceinline__ ChunkEnds chunk_ends_slab(const int32_t* x, const dou
             wn = row(k + 1);
             vn = row(len - 2 - k);
         }
-        iw = 1.0 / fma(-w.l, cp, w.m);
-        iv = 1.0 / fma(-v.u, cq, v.m);
+        iw = pivot_inv(fma(-w.l, cp, w.m));
+        iv = pivot_inv(fma(-v.u, cq, v.m));
         cp = w.u * iw;
         gp = fma(-w.l, gp, w.r) * iw;
         ap = (-w.l * ap) * iw;
@@ -956,10 +956,10 @@ __device__ __forceinline__ void chunk_interior_slab(int len, const int32_t* x, c
         if (k == len - 1) ri = fma(-w.u, xr, ri);
         double iw;
         if (k == 0) {
-            iw = 1.0 / w.m;
+            iw = pivot_inv(w.m);
             gp = ri * iw;
         } else {
-            iw = pivot_rcp(w, cp);
+            iw = pivot_inv(fma(-w.l, cp, w.m));
             gp = fma(-w.l, gp, ri) * iw;
         }
         cp = w.u * iw;
@@ -1114,6 +1114,7 @@ struct GlobalRowFn {
 // In-CTA canonical partitioned solve of an explicit system stored at sys (4 planes of
 // `plane` doubles: l, m, u, r), solution to x.  ws: workspace for the deeper levels
 // (<= 0.75*n + 16 doubles).  All threads of the CTA must call it.
+template <class Pivot>
 __device__ void cta_partitioned(int n, const double* sys, int plane, double* x, double* ws) {
     int sizes[8];
     int depth = 0;
@@ -1145,7 +1146,7 @@ __device__ void cta_partitioned(int n, const double* sys, int plane, double* x, 
             const int first = q * kChunk;
             const int len = (q < P) ? kChunk - 1 : nk - first;
             GlobalRowFn fn{L, L + pl, L + 2 * pl, L + 3 * pl, first};
-            const ChunkEnds ce = chunk_ends(len, fn);
+            const ChunkEnds ce = chunk_ends<Pivot>(len, fn);
             ends[6 * q + 0] = ce.ga;
             ends[6 * q + 1] = ce.aa;
             ends[6 * q + 2] = ce.ba;
@@ -1177,7 +1178,7 @@ __device__ void cta_partitioned(int n, const double* sys, int plane, double* x, 
         const int pl = (depth == 0) ? plane : nb;
         const double* L = lv[depth];
         GlobalRowFn fn{L, L + pl, L + 2 * pl, L + 3 * pl, 0};
-        thomas_small(nb, fn, xv[depth], 1);
+        thomas_small<Pivot>(nb, fn, xv[depth], 1);
     }
     __syncthreads();
     for (int k = depth - 1; k >= 0; --k) {
@@ -1193,7 +1194,7 @@ __device__ void cta_partitioned(int n, const double* sys, int plane, double* x, 
             GlobalRowFn fn{L, L + pl, L + 2 * pl, L + 3 * pl, first};
             const double xl = (q > 0) ? Xs[q - 1] : 0.0;
             const double xr = (q < P) ? Xs[q] : 0.0;
-            chunk_interior(len, fn, xl, xr, xo + first, 1);
+            chunk_interior<true, Pivot>(len, fn, xl, xr, xo + first, 1);
             if (q < P) xo[first + kChunk - 1] = xr;
         }
         __syncthreads();
@@ -1203,7 +1204,10 @@ __device__ void cta_partitioned(int n, const double* sys, int plane, double* x, 
 }  // namespace
 
 __device__ void cta_tridiag(int n, const double* sys, int plane, double* x, double* ws) {
-    cta_partitioned(n, sys, plane, x, ws);
+    cta_partitioned<AnyPivot>(n, sys, plane, x, ws);
+}
+__device__ void cta_spline_tridiag(int n, const double* sys, int plane, double* x, double* ws) {
+    cta_partitioned<SplinePivot>(n, sys, plane, x, ws);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1559,7 +1563,7 @@ __device__ __forceinline__ void reduced_solve_one(unsigned char* dyn_smem, const
         L3[3 * Q + p] = w.r;
     }
     __syncthreads();
-    cta_partitioned(Q, L3, Q, x3, ws3);
+    cta_partitioned<SplinePivot>(Q, L3, Q, x3, ws3);
     for (int p0 = 0; p0 < P; p0 += kRedPass) {
         __syncthreads();
         if (P > kRedPass) stage_level2(st, rc, pl, o, p0, P);  // else: still staged from pass one
@@ -1914,7 +1918,7 @@ k_tridiag_batched(int n, const double* l, const double* m, const double* u, cons
         S[3 * n + i] = r[b * n + i];
     }
     __syncthreads();
-    cta_partitioned(n, S, n, x + b * n, ws + b * ws_stride);
+    cta_partitioned<AnyPivot>(n, S, n, x + b * n, ws + b * ws_stride);
 }
 
 // =======================================================================================
@@ -2245,7 +2249,7 @@ __device__ __noinline__ void small_spline(const SmallSmem& S, int n, int K) {
             L3[3 * Q + p] = w.r;
         }
         __syncthreads();
-        cta_partitioned(Q, L3, Q, x3, ws3);
+        cta_partitioned<SplinePivot>(Q, L3, Q, x3, ws3);
         for (int q = threadIdx.x; q <= Q; q += kSmallThreads) {
             const int first = q * kChunk;
             const int len = (q < Q) ? kChunk - 1 : P - first;
