@@ -257,7 +257,7 @@ k_adj_rows(const unsigned char* slot, TapeLayout L, int cap, const int32_t* kx, 
 
 // Transposed spline solve: one CTA per spline, the canonical partitioned solve.
 __global__ void __launch_bounds__(kAdjThreads)
-k_adj_solve(const unsigned char* slot, TapeLayout L, int cap, const double* sys, double* z,
+k_adj_solve(const unsigned char* slot, TapeLayout L, int cap, double* sys, double* z,
             double* ws, size_t ws_stride) {
     const Slot v = view(slot, L);
     const int sp = blockIdx.x;

@@ -7,7 +7,7 @@
 // stages; one iteration of the loop is
 //   k_stage_end, k_stage_stats, k_stage_begin, k_commit_plan   (channels whose stage finished
 //                                                               move to their next stage)
-//   k_extrema ... k_criterion                                  (one sift iteration of every
+//   k_tile_knots, k_spline_solve, k_tile_sift                  (one sift iteration of every
 //                                                               channel whose stage runs)
 // so channels never wait for each other: a channel that finishes a stage starts the next one
 // at the next iteration, in the same launches as the others.  G iterations are captured once
@@ -15,8 +15,7 @@
 // the other runs) and replayed until every channel has finished; the host never launches
 // single kernels inside the loop.  The persistent grid sizes are chosen by a small autotuner
 // that times the first replays of the wave with each candidate (the candidates compute the
-// same results: only the assignment of tiles and splines to CTAs and the tile kernels'
-// register budgets differ) and keeps the fastest for later waves and calls of the same shape.
+// same results: only the assignment of tiles to CTAs differs) and keeps the fastest for later waves and calls of the same shape.
 //
 // Channels that do not fit the device memory together are processed in waves, longest first.
 #include <cuda_runtime.h>
@@ -44,44 +43,15 @@ struct BatchChannel {
     const double* noise = nullptr;  // [nr*n] N(0,1) noise; null = cuRAND with `seed`
 };
 
-// Launch shapes of one wave: persistent grid sizes (in multiples of the resident CTAs of the
-// whole GPU) and the register budgets of the tile kernels.  Every choice computes the same
-// results: only the assignment of tiles and splines to CTAs and the registers differ.
-struct TuneConfig {
-    int tile_mult;    // k_extrema / k_eval: 1, 2 or 4 waves of resident CTAs
-    int split_mult;   // k_chunk_reduce / k_segments: 1 or 2
-    int extrema_b;    // k_extrema with its second register budget
-    int eval_b;       // k_eval with its second register budget
-    bool operator<(const TuneConfig& o) const {
-        return std::tie(tile_mult, split_mult, extrema_b, eval_b) <
-               std::tie(o.tile_mult, o.split_mult, o.extrema_b, o.eval_b);
-    }
-    bool operator==(const TuneConfig& o) const { return !(*this < o) && !(o < *this); }
-};
-
-constexpr TuneConfig kDefaultConfig = {1, 1, 0, 0};
-
-// kernels of one loop iteration: four transitions and eight sift kernels
-constexpr int kLoopKernels = 12;
-
-// Tuned configurations by shape: channels, realizations, total samples (log2 bucket).
-std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int>, TuneConfig> g_tuned;
-
-std::tuple<int, int, int> shape_key(const std::vector<BatchChannel>& ch, size_t nr) {
-    size_t tot = 0;
-    for (const auto& c : ch) tot += c.n;
-    int lg = 0;
-    while (((size_t)1 << (lg + 1)) <= tot) ++lg;
-    return std::make_tuple((int)ch.size(), (int)nr, lg);
-}
+// transition kernels of one loop iteration
+constexpr int kTransKernels = 4;
 
 // Device bytes of one channel in a wave (sift state, noise modes, knots, records).
 size_t channel_bytes(size_t n, size_t nr, size_t nimf) {
     const size_t rn = nr * n;
     const size_t tiles = nr * ((n + kTileSamples - 1) / kTileSamples);
     const size_t planes = (nimf + 6) * rn * 8;          // h x2, menv, W, H0, MODE, E
-    const size_t knots = tiles * kTileCap * (2 * 12 + 2 * 32);  // kx, ky, records (x2)
+    const size_t knots = tiles * 1028 * (2 * 12 + 2 * 32);  // (a bound of the tiles' workspaces)
     const size_t rec = nr * (n / 2 / kChunk + 64) * 8 * 2 * 17;  // chunk records, X, workspace
     return planes + knots + rec + tiles * 1024;
 }
@@ -134,30 +104,6 @@ ceemdan_status capture(Wave& w, cudaStream_t st, long first, cudaGraphExec_t* ou
     return CEEMDAN_OK;
 }
 
-void apply_config(SiftEngine& eng, const TuneConfig& t) {
-    const int sms = sm_count();
-    int per = 0;
-    eng.extrema_b = t.extrema_b != 0;
-    eng.eval_b = t.eval_b != 0;
-    if (eng.extrema_b)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_extrema_t<kExtremaBlocksB, true>,
-                                                      kThreads, 0);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_extrema_t<kExtremaBlocksA, true>,
-                                                      kThreads, 0);
-    eng.tile_grid = std::max(1, std::min(eng.a.ntot, t.tile_mult * std::max(1, per) * sms));
-    if (eng.eval_b)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_eval_t<kEvalBlocksB>, kThreads, 0);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_eval_t<kEvalBlocksA>, kThreads, 0);
-    eng.eval_grid = std::max(1, std::min(eng.a.ntot, t.tile_mult * std::max(1, per) * sms));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_chunk_reduce, 128, 0);
-    eng.reduce_grid = t.split_mult * std::max(1, per) * sms;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_segments, 64, 0);
-    eng.segments_grid = t.split_mult * std::max(1, per) * sms;
-    cudaGetLastError();
-}
-
 ceemdan_status run_wave(const std::vector<BatchChannel>& ch, size_t nr, size_t nimf,
                         size_t max_iter, double nstd, const ceemdan_options& o,
                         cudaStream_t st, int32_t* h_iters, size_t* peak_bytes) {
@@ -175,7 +121,7 @@ ceemdan_status run_wave(const std::vector<BatchChannel>& ch, size_t nr, size_t n
     }
     CKS(eng.init(ws, specs, o));
     const Chan& lastc = eng.hchan.back();
-    const size_t S = (size_t)lastc.samp0 + (((size_t)lastc.nr * lastc.n + 31) & ~(size_t)31);
+    const size_t S = (size_t)lastc.samp0 + (((size_t)lastc.nr * row_ld(lastc.n) + 31) & ~(size_t)31);
     BatchArgs& b = w.b;
     b.nimf = (int)nimf;
     b.M = M;
@@ -251,132 +197,20 @@ ceemdan_status run_wave(const std::vector<BatchChannel>& ch, size_t nr, size_t n
     eng.group = w.G;
     if (o.h_kernel_ms) CKS(eng.enable_timing(o.h_kernel_ms));
 
-    // autotune (first wave of a shape) or reuse
-    const auto key = shape_key(ch, nr);
-    TuneConfig cfg = kDefaultConfig;
-    bool tuned = false;
-    {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        auto it = g_tuned.find(key);
-        if (it != g_tuned.end()) {
-            cfg = it->second;
-            tuned = true;
-        }
-    }
-    const char* tune_env = std::getenv("CEEMDAN_BATCH_TUNE");
-    if (tune_env && tune_env[0] == '0') tuned = true;
-
     int* hs = eng.hstate;  // two slots of (finished, err, -, -)
     cudaEvent_t done_ev[2] = {eng.group_ev[0], eng.group_ev[1]};
-    cudaEvent_t t0 = nullptr, t1 = nullptr;
-    CK(cudaEventCreate(&t0));
-    CK(cudaEventCreate(&t1));
-    struct EvGuard {
-        cudaEvent_t a, b;
-        ~EvGuard() {
-            cudaEventDestroy(a);
-            cudaEventDestroy(b);
-        }
-    } evg{t0, t1};
-
     long launched = 0;  // iterations launched
-    // executable graphs of every configuration built so far (the tuner compares several)
-    std::map<TuneConfig, std::pair<cudaGraphExec_t, cudaGraphExec_t>> built;
-    struct BuiltGuard {
-        std::map<TuneConfig, std::pair<cudaGraphExec_t, cudaGraphExec_t>>& m;
-        Wave& w;
-        ~BuiltGuard() {
-            cudaStreamSynchronize(w.st);
-            for (auto& kv : m) {
-                if (kv.second.first && kv.second.first != w.exec[0])
-                    cudaGraphExecDestroy(kv.second.first);
-                if (kv.second.second && kv.second.second != w.exec[1])
-                    cudaGraphExecDestroy(kv.second.second);
-            }
-        }
-    } bg{built, w};
-    auto use = [&](const TuneConfig& t) -> ceemdan_status {
-        auto it = built.find(t);
-        if (it == built.end()) {
-            apply_config(eng, t);
-            std::pair<cudaGraphExec_t, cudaGraphExec_t> ex{nullptr, nullptr};
-            CKS(capture(w, st, 0, &ex.first));
-            const ceemdan_status s2 = capture(w, st, (long)w.G, &ex.second);
-            if (s2 != CEEMDAN_OK) {
-                cudaGraphExecDestroy(ex.first);
-                return s2;
-            }
-            it = built.emplace(t, ex).first;
-        }
-        w.exec[0] = it->second.first;
-        w.exec[1] = it->second.second;
-        return CEEMDAN_OK;
-    };
+    CKS(capture(w, st, 0, &w.exec[0]));
+    CKS(capture(w, st, (long)w.G, &w.exec[1]));
     auto replay = [&](int slot) -> ceemdan_status {
         CK(cudaGraphLaunch(w.exec[slot], st));
         launched += w.G;
-        g_launches += (uint64_t)w.G * kLoopKernels;
+        g_launches += (uint64_t)w.G * (kTransKernels + eng.sift_kernels());
         CK(cudaMemcpyAsync(hs + 4 * slot, b.finished, sizeof(int), cudaMemcpyDeviceToHost, st));
         CK(cudaEventRecord(done_ev[slot], st));
         return CEEMDAN_OK;
     };
-    // one timed replay of configuration t (synchronous; its events harvested)
     auto cancelled = [&]() -> bool { return o.h_cancel && *o.h_cancel; };
-    auto timed_replay = [&](const TuneConfig& t, float* ms) -> ceemdan_status {
-        if (cancelled()) {
-            cudaStreamSynchronize(st);
-            g_last_error = "cancelled by the host cancel word";
-            return CEEMDAN_ERR_CANCELLED;
-        }
-        CKS(use(t));
-        CK(cudaEventRecord(t0, st));
-        CKS(replay(0));
-        CK(cudaEventRecord(t1, st));
-        CK(cudaEventSynchronize(t1));
-        eng.harvest_timing(0, w.G);
-        float m = 0.f;
-        CK(cudaEventElapsedTime(&m, t0, t1));
-        *ms += m;
-        return CEEMDAN_OK;
-    };
-
-    if (!tuned) {
-        // coordinate descent over the four choices: each challenger against the best so far,
-        // timed in the order best, challenger, challenger, best on the wave's own iterations
-        // (the work drifts slowly as the stages advance; the symmetric order cancels that)
-        const TuneConfig axes[][3] = {
-            {{2, 1, 0, 0}, {4, 1, 0, 0}, {0, 0, 0, 0}},
-            {{0, 2, 0, 0}, {0, 0, 0, 0}, {0, 0, 0, 0}},
-            {{0, 0, 1, 0}, {0, 0, 0, 0}, {0, 0, 0, 0}},
-            {{0, 0, 0, 1}, {0, 0, 0, 0}, {0, 0, 0, 0}}};
-        TuneConfig best = kDefaultConfig;
-        float dummy = 0.f;
-        CKS(timed_replay(best, &dummy));  // warm
-        for (int ax = 0; ax < 4; ++ax) {
-            for (int v = 0; v < 3; ++v) {
-                const TuneConfig& d = axes[ax][v];
-                if (d.tile_mult == 0 && d.split_mult == 0 && d.extrema_b == 0 && d.eval_b == 0)
-                    continue;
-                TuneConfig c = best;
-                if (ax == 0) c.tile_mult = d.tile_mult;
-                if (ax == 1) c.split_mult = d.split_mult;
-                if (ax == 2) c.extrema_b = d.extrema_b;
-                if (ax == 3) c.eval_b = d.eval_b;
-                if (c == best) continue;
-                CKS(timed_replay(c, &dummy));  // warm the challenger's graphs
-                float tb = 0.f, tc = 0.f;
-                CKS(timed_replay(best, &tb));
-                CKS(timed_replay(c, &tc));
-                CKS(timed_replay(c, &tc));
-                CKS(timed_replay(best, &tb));
-                if (tc < 0.99f * tb) best = c;
-            }
-        }
-        cfg = best;
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        g_tuned[key] = cfg;
-    }
-    CKS(use(cfg));
     int slot = 0;
     // double-buffered loop: replay slot s^1 is queued before the host waits for slot s
     CKS(replay(slot));

@@ -107,13 +107,21 @@ CEEMDAN_HD Row identity_row() {
 // has RN(1/x) = 2^-(k+1) (1 + 2^-52), selected.  No branch: two independent sweeps interleave
 // where the general reciprocal's range branch makes them run one after the other (measured on
 // a B200, two reciprocal-and-fma chains side by side: 162 cycles a step with 1.0/x, 71 so).
-CEEMDAN_HD double pivot_inv(double x) {
+// rcp_raw is the reciprocal without that selection, for x known to have another significand.
+CEEMDAN_HD double rcp_raw(double x) {
 #ifdef __CUDA_ARCH__
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double e = fma(-x, y, 1.0);
     y = fma(y, fma(e, e, e), y);
-    const double q = fma(fma(-x, y, 1.0), y, y);
+    return fma(fma(-x, y, 1.0), y, y);
+#else
+    return 1.0 / x;
+#endif
+}
+CEEMDAN_HD double pivot_inv(double x) {
+#ifdef __CUDA_ARCH__
+    const double q = rcp_raw(x);
     const int hi = __double2hiint(x);
     const bool ones = __double2loint(x) == -1 && (hi | (int)0xfff00000) == -1;
     return ones ? __hiloint2double(0x7fd00000 - (hi & 0x7ff00000), 1) : q;

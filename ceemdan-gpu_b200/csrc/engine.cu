@@ -348,7 +348,7 @@ ceemdan_status decompose_impl(size_t nr, size_t n, size_t nimf, size_t max_iter,
     for (size_t i = 0; i + 1 < nimf && state_in; ++i)
         if (o.h_iters_out) o.h_iters_out[i] = 0;
     for (size_t i = 0; i + 1 < nimf && !state_in; ++i) {
-        CK(cudaMemcpyAsync(eng.h[0], w, rn * sizeof(double), cudaMemcpyDeviceToDevice, st));
+        CKS(eng.rows_in(eng.h[0], w, nr, st));
         int it = 0;
         CKS(eng.run_stage(E + i * rn, o.noise_sift_cap, st, &it, o.h_cancel));
         if (o.h_iters_out) o.h_iters_out[i] = it;
@@ -362,16 +362,14 @@ ceemdan_status decompose_impl(size_t nr, size_t n, size_t nimf, size_t max_iter,
     // the carries the noise phase leaves (mean envelope, sifting fraction): restored from the
     // given state, or exported with the modes
     if (state_in) {
-        CK(cudaMemcpyAsync(eng.a.menv, o.d_noise_state_in + nimf * rn, rn * sizeof(double),
-                           cudaMemcpyDeviceToDevice, st));
+        CKS(eng.rows_in(eng.a.menv, o.d_noise_state_in + nimf * rn, nr, st));
         CK(cudaMemcpyAsync(eng.a.frac, o.d_noise_state_in + (nimf + 1) * rn, nr * sizeof(double),
                            cudaMemcpyDeviceToDevice, st));
     }
     if (o.d_noise_state_out) {
         CK(cudaMemcpyAsync(o.d_noise_state_out, E, nimf * rn * sizeof(double),
                            cudaMemcpyDeviceToDevice, st));
-        CK(cudaMemcpyAsync(o.d_noise_state_out + nimf * rn, eng.a.menv, rn * sizeof(double),
-                           cudaMemcpyDeviceToDevice, st));
+        CKS(eng.rows_out(o.d_noise_state_out + nimf * rn, eng.a.menv, nr, st));
         CK(cudaMemcpyAsync(o.d_noise_state_out + (nimf + 1) * rn, eng.a.frac,
                            nr * sizeof(double), cudaMemcpyDeviceToDevice, st));
     }
@@ -435,11 +433,8 @@ ceemdan_status decompose_impl(size_t nr, size_t n, size_t nimf, size_t max_iter,
             rc = CEEMDAN_ERR_CUDA;
             break;
         }
-        if (cudaMemcpyAsync(eng.h[0], h0, rn * sizeof(double), cudaMemcpyDeviceToDevice, st) !=
-            cudaSuccess) {
-            rc = CEEMDAN_ERR_CUDA;
-            break;
-        }
+        rc = eng.rows_in(eng.h[0], h0, nr, st);
+        if (rc != CEEMDAN_OK) break;
         if (tape && cudaMemcpyAsync(tape->stats + 2 * i, stat, 2 * sizeof(double),
                                     cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
             rc = CEEMDAN_ERR_CUDA;
@@ -447,10 +442,8 @@ ceemdan_status decompose_impl(size_t nr, size_t n, size_t nimf, size_t max_iter,
         }
         if (tape && tape->checkpointed) {
             double* c = tape->ck + i * tape->ck_stride();
-            if (cudaMemcpyAsync(c, eng.h[0], rn * sizeof(double), cudaMemcpyDeviceToDevice, st) !=
-                    cudaSuccess ||
-                cudaMemcpyAsync(c + rn, eng.a.menv, rn * sizeof(double),
-                                cudaMemcpyDeviceToDevice, st) != cudaSuccess ||
+            if (eng.rows_out(c, eng.h[0], nr, st) != CEEMDAN_OK ||
+                eng.rows_out(c + rn, eng.a.menv, nr, st) != CEEMDAN_OK ||
                 cudaMemcpyAsync(c + 2 * rn, eng.a.frac, nr * sizeof(double),
                                 cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
                 rc = CEEMDAN_ERR_CUDA;
@@ -645,11 +638,9 @@ ceemdan_status backward_impl(const ceemdan_tape& T, const double* g, double* gy,
                 SiftEngine& E = rows == nb ? reng : reng2;
                 double* rm = rows == nb ? rmode : rmode2;
                 const double* c = T.ck + (size_t)i * T.ck_stride();
-                const size_t off = (size_t)r0 * T.n, bn = (size_t)rows * T.n;
-                CK(cudaMemcpyAsync(E.h[0], c + off, bn * sizeof(double), cudaMemcpyDeviceToDevice,
-                                   st));
-                CK(cudaMemcpyAsync(E.a.menv, c + rn + off, bn * sizeof(double),
-                                   cudaMemcpyDeviceToDevice, st));
+                const size_t off = (size_t)r0 * T.n;
+                CKS(E.rows_in(E.h[0], c + off, (size_t)rows, st));
+                CKS(E.rows_in(E.a.menv, c + rn + off, (size_t)rows, st));
                 CK(cudaMemcpyAsync(E.a.frac, c + 2 * rn + r0, rows * sizeof(double),
                                    cudaMemcpyDeviceToDevice, st));
                 one.nr = (size_t)rows;
@@ -1032,7 +1023,7 @@ ceemdan_status ceemdan_envelopes_f64(size_t nr, size_t n, const double* d_h, dou
     CKS(eng.init(ws, (int)nr, (int)n, o));
     CKS(eng.reset_carries(st));
     CK(cudaMemsetAsync(eng.a.mark, 0xff, sizeof(int) * nr, st));
-    CK(cudaMemcpyAsync(eng.h[0], d_h, nr * n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    CKS(eng.rows_in(eng.h[0], d_h, nr, st));
     eng.a.dbg_upper = d_upper;
     eng.a.dbg_lower = d_lower;
     CKS(eng.launch_iteration(0, st));
@@ -1061,11 +1052,11 @@ ceemdan_status ceemdan_extrema_f64(size_t nr, size_t n, const double* d_h, int32
     CKS(eng.init(ws, (int)nr, (int)n, o));
     CKS(eng.reset_carries(st));
     CK(cudaMemsetAsync(eng.a.mark, 0xff, sizeof(int) * nr, st));
-    CK(cudaMemcpyAsync(eng.h[0], d_h, nr * n * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    CKS(eng.rows_in(eng.h[0], d_h, nr, st));
     SiftArgs& a = eng.a;
     const dim3 grid_tiles((unsigned)eng.ntiles, (unsigned)nr);
-    k_extrema_t<kExtremaBlocksA, false><<<eng.tile_grid, kThreads, 0, st>>>(a);
-    k_scan_boundary<<<eng.scan_grid, kThreads, 0, st>>>(a);
+    k_tile_knots<<<eng.knots_grid, kTileThreads, tile_knots_smem(), st>>>(a);
+    k_spline_solve<<<eng.solve_grid, kSolveThreads, kSolveSmem, st>>>(a);
     k_gather_knots<<<grid_tiles, kThreads, 0, st>>>(a, 0, d_kx_max, d_ky_max);
     k_gather_knots<<<grid_tiles, kThreads, 0, st>>>(a, 1, d_kx_min, d_ky_min);
     CK(cudaGetLastError());

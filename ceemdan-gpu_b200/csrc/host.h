@@ -39,6 +39,14 @@ extern std::atomic<uint64_t> g_launches;        // kernels launched by the libra
 
 constexpr int kThreads = 256;
 
+// The tile kernels run as persistent CTAs over the active tiles.  kEnv: the envelopes of one
+// iteration to dbg_upper / dbg_lower, no update and no stop test.  kDense: shared memory for
+// kSiftDense entries (three CTAs per SM) or kSiftSparse (four).
+__global__ void k_tile_knots(const __grid_constant__ SiftArgs a);
+template <bool kDense, bool kEnv>
+__global__ void k_tile_sift(const __grid_constant__ SiftArgs a);
+__global__ void k_spline_solve(const __grid_constant__ SiftArgs a);
+
 const double* rcp_tables();
 int sm_count();
 cudaMemPool_t engine_pool();
@@ -175,16 +183,13 @@ struct SiftEngine {
     int nr = 0, n = 0, ntiles = 0;  // channel 0
     cudaEvent_t group_ev[2] = {nullptr, nullptr};
     int group = 4;
-    size_t red_smem = 0;
-    // persistent grids: resident CTAs x SMs (the separator kernels), or the work itself
-    int reduce_grid = 0, segments_grid = 0, red_grid = 0, tile_grid = 0, eval_grid = 0,
-        scan_grid = 0;
+    // persistent grids of the tile kernels, one CTA per spline
+    int knots_grid = 0, dense_grid = 0, sift_grid = 0, solve_grid = 0;
     double* kernel_ms = nullptr;           // host accumulators (optional)
     std::vector<cudaEvent_t> ev;           // [group][kinds][2] when timing
     ceemdan_tape* tape = nullptr;          // taped forward: the stage being recorded
     size_t tape_stage = 0;
     bool plan_by_caller = false;           // the batched loop computes the plan (k_commit_plan)
-    bool extrema_b = false, eval_b = false;  // the tile kernels' second register budgets
 
     ceemdan_status init(Workspace& ws, int nr_, int n_, const ceemdan_options& o) {
         return init(ws, std::vector<ChanSpec>{{n_, nr_}}, o);
@@ -213,7 +218,7 @@ struct SiftEngine {
             rows += ch.nr;
             tiles += (long long)ch.nr * ch.ntiles;
             // every channel's block of rows starts 256-byte aligned (16-byte sample pairs)
-            samp += ((long long)ch.nr * ch.n + 31) & ~31LL;
+            samp += ((long long)ch.nr * row_ld(ch.n) + 31) & ~31LL;
             rec += (long long)ch.nr * ch.rec_stride;
             red += (long long)ch.nr * red_stride_of(ch.rec_stride);
         }
@@ -228,13 +233,11 @@ struct SiftEngine {
         a.ntiles1 = ntiles;
         a.nr1 = nr;
         a.rs1 = hchan[0].rec_stride;
-        a.par = -1;
         a.nrows = (int)rows;
         a.nchan = nchan;
         a.ntot = (int)tiles;
         a.rec_total = rec;
         a.red_total = red;
-        a.rec_plane = (size_t)2 * (size_t)rec;
         a.spin_limit = o.spin_limit > 0 ? o.spin_limit : (1 << 22);
         a.sd = o.sd;
         a.sd2 = o.sd2;
@@ -242,7 +245,6 @@ struct SiftEngine {
         sx_bounds(o.sd2, &a.sd2_hi, &a.sd2_lo);
         a.tol = o.tol;
         const size_t R = (size_t)rows, T = (size_t)tiles, S = (size_t)samp;
-        const size_t kn = T * kTileCap;  // per-tile knot slots
         CKS(ws.alloc_n(&h[0], S));
         CKS(ws.alloc_n(&h[1], S));
         a.h[0] = h[0];
@@ -254,22 +256,29 @@ struct SiftEngine {
         CKS(ws.alloc_n(&a.cnt, R));
         CKS(ws.alloc_n(&a.any, R));
         CKS(ws.alloc_n(&a.kcount, 2 * R));
+        CKS(ws.alloc_n(&a.par, R));
+        CKS(ws.alloc_n(&a.acc, R));
+        CKS(ws.alloc_n(&a.acc_wide, 2 * R));
+        // counts of rows of up to 2^17 - 1 tiles fit one word (CEEMDAN_SPLIT_COUNT=1: never)
+        a.count_bits = 17;
+        if (const char* e = std::getenv("CEEMDAN_SPLIT_COUNT"))
+            if (e[0] == '1') a.count_bits = 0;
+        CKS(ws.alloc_n(&a.cmax, 2 * R));
         CKS(ws.alloc_n(&a.tile_cnt, 2 * T));
-        CKS(ws.alloc_n(&a.tile_off, 2 * (T + R)));
-        CKS(ws.alloc_n(&a.sep_off, 2 * (T + R)));
-        CKS(ws.alloc_n(&a.pcount, 2 * R));
-        CKS(ws.alloc_n(&a.gcount, 2 * R));
-        CKS(ws.alloc_n(&a.gsum, 2 * R + 1));
         CKS(ws.alloc_n(&a.plan, 2 * (size_t)nchan + 2));
         CKS(ws.alloc_n(&a.bitmap, 2 * T * (kTileSamples / 32)));
-        CKS(ws.alloc_n(&a.nbr, 2 * T * 2));
-        CKS(ws.alloc_n(&a.kx_max, kn));
-        CKS(ws.alloc_n(&a.kx_min, kn));
-        CKS(ws.alloc_n(&a.ky_max, kn));
-        CKS(ws.alloc_n(&a.ky_min, kn));
-        for (int e = 0; e < 2; ++e) CKS(ws.alloc_n(&a.seg[e], 4 * kn));
-        CKS(ws.alloc_n(&a.rec, 10 * a.rec_plane));
-        CKS(ws.alloc_n(&a.xsep, 2 * (size_t)rec));
+        CKS(ws.alloc_n(&a.scan, T));
+        CKS(ws.alloc_n(&a.hdr, 2 * T));
+        CKS(ws.alloc_n(&a.edge, 2 * T));
+        CKS(ws.alloc_n(&a.rows, 2 * T * kRowSlots * 4));
+        CKS(ws.alloc_n(&a.sep_off, 2 * (T + R)));
+        CKS(ws.alloc_n(&a.tile_rank, 2 * (T + R)));
+        CKS(ws.alloc_n(&a.tile_list, 2 * (T + R)));
+        CKS(ws.alloc_n(&a.yend, 2 * R * 2));
+        CKS(ws.alloc_n(&a.end_x, 2 * R * 2 * kEndKnots));
+        CKS(ws.alloc_n(&a.end_y, 2 * R * 2 * kEndKnots));
+        // (k_tile_sift copies a whole tile's slots from a tile's first separator on)
+        CKS(ws.alloc_n(&a.xsep, 2 * (size_t)rec + kRowSlots));
         CKS(ws.alloc_n(&a.red, 2 * (size_t)red));
         double* rcp = nullptr;
         CKS(ws.alloc_n(&rcp, 2 * (size_t)(kRcpMax + 1)));
@@ -298,27 +307,30 @@ struct SiftEngine {
         } else {
             group = rn >= (size_t)(1 << 22) ? 4 : (rn >= (size_t)(1 << 18) ? 8 : 32);
         }
-        int dev = 0, sms = 0, per = 0;
-        CK(cudaGetDevice(&dev));
-        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_chunk_reduce, 128, 0));
-        reduce_grid = std::max(1, per) * sms;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_segments, 64, 0));
-        segments_grid = std::max(1, per) * sms;
-        red_smem = reduced_solve_smem(&a.red_qcap);
-        // the bound, not this call's size: concurrent calls of other sizes set the same value
-        CK(cudaFuncSetAttribute(k_reduced_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kRedSmemMax));
-        // one CTA per tile / spline when every channel sifts (the whole work in one wave of
-        // launches); the batched engine caps these at a few waves of resident CTAs
-        tile_grid = (int)std::max<size_t>(1, T);
-        eval_grid = tile_grid;
-        // the tile kernels' second register budgets (the batched engine's tuner chooses them;
-        // CEEMDAN_TILE_BUDGET=B selects them for the one-channel engine)
-        if (const char* e = std::getenv("CEEMDAN_TILE_BUDGET"))
-            if (e[0] == 'B') extrema_b = eval_b = true;
-        red_grid = (int)std::max<size_t>(1, 2 * R);
-        scan_grid = (int)std::max<size_t>(1, (2 * R + 7) / 8);
+        a.solve_wcap = (kSolveSmem - kSolveStage) / (int)sizeof(double);
+        CK(cudaFuncSetAttribute(k_spline_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                kSolveSmem));
+        for (auto k : {k_tile_sift<false, false>, k_tile_sift<false, true>})
+            CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)tile_sift_smem(false)));
+        for (auto k : {k_tile_sift<true, false>, k_tile_sift<true, true>})
+            CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)tile_sift_smem(true)));
+        CK(cudaFuncSetAttribute(k_tile_knots, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)tile_knots_smem()));
+        // persistent CTAs, as many as the GPU holds at once
+        auto grid = [&](const void* k, size_t smem) {
+            int per = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kTileThreads, smem);
+            return std::max(1, (int)std::min<size_t>(T, (size_t)std::max(1, per) * sm_count()));
+        };
+        knots_grid = grid((const void*)k_tile_knots, tile_knots_smem());
+        dense_grid = grid((const void*)k_tile_sift<true, false>, tile_sift_smem(true));
+        sift_grid = grid((const void*)k_tile_sift<false, false>, tile_sift_smem(false));
+        CK(cudaGetLastError());
+        // as many tiles as the dense form holds at once: one launch does for all rows
+        a.sift_split = (size_t)dense_grid < T ? 1 : 0;
+        solve_grid = (int)std::max<size_t>(1, 2 * R);
         return CEEMDAN_OK;
     }
 
@@ -329,8 +341,14 @@ struct SiftEngine {
         for (cudaEvent_t e : ev) cudaEventDestroy(e);
     }
 
-    // kinds timed per iteration (the on-chip stage kernel is timed per launch)
-    static constexpr int kIterKinds = CEEMDAN_K_SIFT_SMALL;
+    // kernels of one sift iteration
+    int sift_kernels() const { return a.sift_split ? 4 : 3; }
+
+    // kinds timed per iteration (the on-chip stage kernel is timed per launch): the three
+    // kernels of an iteration report under the kinds of their main steps
+    static constexpr int kIterKinds = 3;
+    static constexpr int kIterKind[kIterKinds] = {CEEMDAN_K_EXTREMA, CEEMDAN_K_REDUCED_SOLVE,
+                                                  CEEMDAN_K_EVAL};
 
     ceemdan_status enable_timing(double* ms) {
         kernel_ms = ms;
@@ -351,26 +369,49 @@ struct SiftEngine {
             for (int k = 0; k < kIterKinds; ++k) {
                 float ms = 0.f;
                 if (cudaEventElapsedTime(&ms, event(it, k, 0), event(it, k, 1)) == cudaSuccess)
-                    kernel_ms[k] += ms;
+                    kernel_ms[kIterKind[k]] += ms;
             }
         }
+    }
+
+    // Rows of the engine's planes (row_ld(n) apart) from and to contiguous rows of n samples, rows
+    // r0 .. r0 + rows - 1 of channel 0.
+    ceemdan_status rows_in(double* plane, const double* src, size_t rows, cudaStream_t st) {
+        const size_t w = sizeof(double) * (size_t)n;
+        if (row_ld(n) == n)
+            CK(cudaMemcpyAsync(plane, src, w * rows, cudaMemcpyDeviceToDevice, st));
+        else
+            CK(cudaMemcpy2DAsync(plane, sizeof(double) * row_ld(n), src, w, w, rows,
+                                 cudaMemcpyDeviceToDevice, st));
+        return CEEMDAN_OK;
+    }
+    ceemdan_status rows_out(double* dst, const double* plane, size_t rows, cudaStream_t st) {
+        const size_t w = sizeof(double) * (size_t)n;
+        if (row_ld(n) == n)
+            CK(cudaMemcpyAsync(dst, plane, w * rows, cudaMemcpyDeviceToDevice, st));
+        else
+            CK(cudaMemcpy2DAsync(dst, w, plane, sizeof(double) * row_ld(n), w, rows,
+                                 cudaMemcpyDeviceToDevice, st));
+        return CEEMDAN_OK;
     }
 
     // Zero the whole-call carries: mean envelope and sifting fraction accumulator, and the
     // channels' states.
     ceemdan_status reset_carries(cudaStream_t st) {
         const Chan& last = hchan.back();
-        const size_t S = (size_t)last.samp0 + (size_t)last.nr * last.n;
+        const size_t S = (size_t)last.samp0 + (size_t)last.nr * row_ld(last.n);
         CK(cudaMemsetAsync(a.menv, 0, sizeof(double) * S, st));
         CK(cudaMemsetAsync(a.frac, 0, sizeof(double) * a.nrows, st));
         CK(cudaMemsetAsync(a.cnt, 0, sizeof(unsigned) * a.nrows, st));
         CK(cudaMemsetAsync(a.any, 0, sizeof(int) * a.nrows, st));
+        CK(cudaMemsetAsync(a.par, 0, sizeof(int) * a.nrows, st));
+        CK(cudaMemsetAsync(a.acc, 0, sizeof(*a.acc) * a.nrows, st));
+        CK(cudaMemsetAsync(a.acc_wide, 0, sizeof(*a.acc_wide) * 2 * a.nrows, st));
         CK(cudaMemsetAsync(cs, 0, sizeof(ChanState) * a.nchan, st));
         return CEEMDAN_OK;
     }
 
-    // Launch one sift iteration of every channel whose stage runs (channel c reads
-    // h[iter_c%2], writes h[(iter_c+1)%2]).
+    // Launch one sift iteration of every channel whose stage runs.
     ceemdan_status launch_iteration(long j, cudaStream_t st) {
         unsigned char* slot = nullptr;
         if (tape) {
@@ -381,9 +422,6 @@ struct SiftEngine {
             }
         }
         a.tape_mark = slot ? reinterpret_cast<signed char*>(slot + tape->L.off_mark) : nullptr;
-        // one channel driven from the host: iteration j of the stage reads h[j%2] (the device
-        // counter equals j until the stage has finished, and then the kernels return at once)
-        a.par = (a.nchan == 1 && !plan_by_caller) ? (int)(j & 1) : -1;
         const bool timed = kernel_ms != nullptr;
         const int ti = (int)(j % (2 * group));
         // inside a stream capture an event record becomes a graph node only as an external
@@ -399,37 +437,12 @@ struct SiftEngine {
             k_plan<<<1, 1024, 0, st>>>(a);
             ++g_launches;
         }
-        mark_ev(CEEMDAN_K_EXTREMA, 0);
-        // a grid that covers every tile runs one tile per CTA (no persistent loop)
-        const bool loop = tile_grid < a.ntot;
-        if (extrema_b && loop)
-            k_extrema_t<kExtremaBlocksB, true><<<tile_grid, kThreads, 0, st>>>(a);
-        else if (extrema_b)
-            k_extrema_t<kExtremaBlocksB, false><<<tile_grid, kThreads, 0, st>>>(a);
-        else if (loop)
-            k_extrema_t<kExtremaBlocksA, true><<<tile_grid, kThreads, 0, st>>>(a);
-        else
-            k_extrema_t<kExtremaBlocksA, false><<<tile_grid, kThreads, 0, st>>>(a);
-        mark_ev(CEEMDAN_K_EXTREMA, 1);
-        mark_ev(CEEMDAN_K_BOUNDARY, 0);
-        k_scan_boundary<<<scan_grid, kThreads, 0, st>>>(a);
-        mark_ev(CEEMDAN_K_BOUNDARY, 1);
-        mark_ev(CEEMDAN_K_CHUNK_REDUCE, 0);
-        k_group_scan<<<1, 1024, 0, st>>>(a);
-        k_chunk_reduce<<<reduce_grid, 128, 0, st>>>(a);
-        mark_ev(CEEMDAN_K_CHUNK_REDUCE, 1);
-        mark_ev(CEEMDAN_K_REDUCED_SOLVE, 0);
-        k_reduced_solve<<<red_grid, kRedThreads, red_smem, st>>>(a);
-        mark_ev(CEEMDAN_K_REDUCED_SOLVE, 1);
-        mark_ev(CEEMDAN_K_SEGMENTS, 0);
-        k_segments<<<segments_grid, 64, 0, st>>>(a);
-        mark_ev(CEEMDAN_K_SEGMENTS, 1);
-        mark_ev(CEEMDAN_K_EVAL, 0);
-        if (eval_b)
-            k_eval_t<kEvalBlocksB><<<eval_grid, kThreads, 0, st>>>(a);
-        else
-            k_eval_t<kEvalBlocksA><<<eval_grid, kThreads, 0, st>>>(a);
-        mark_ev(CEEMDAN_K_EVAL, 1);
+        mark_ev(0, 0);
+        k_tile_knots<<<knots_grid, kTileThreads, tile_knots_smem(), st>>>(a);
+        mark_ev(0, 1);
+        mark_ev(1, 0);
+        k_spline_solve<<<solve_grid, kSolveThreads, kSolveSmem, st>>>(a);
+        mark_ev(1, 1);
         if (slot) {
             const size_t pieces = tape->L.off_kc / 16;  // 16-byte pieces of the bitmaps
             const unsigned g = (unsigned)std::min<size_t>((pieces + kThreads - 1) / kThreads,
@@ -437,10 +450,19 @@ struct SiftEngine {
             k_tape_record<<<g, kThreads, 0, st>>>(a, tape->L, slot);
             ++g_launches;
         }
-        mark_ev(CEEMDAN_K_CRITERION, 0);
-        if (!a.dbg_upper) k_criterion<<<std::min(a.nchan, 4 * sm_count()), kThreads, 0, st>>>(a);
-        mark_ev(CEEMDAN_K_CRITERION, 1);
-        g_launches += a.dbg_upper ? 7 : 8;
+        mark_ev(2, 0);
+        if (a.dbg_upper) {
+            k_tile_sift<true, true><<<dense_grid, kTileThreads, tile_sift_smem(true), st>>>(a);
+            if (a.sift_split)
+                k_tile_sift<false, true><<<sift_grid, kTileThreads, tile_sift_smem(false), st>>>(a);
+        } else {
+            k_tile_sift<true, false><<<dense_grid, kTileThreads, tile_sift_smem(true), st>>>(a);
+            if (a.sift_split)
+                k_tile_sift<false, false><<<sift_grid, kTileThreads, tile_sift_smem(false), st>>>(
+                    a);
+        }
+        mark_ev(2, 1);
+        g_launches += sift_kernels();
         CK(cudaGetLastError());
         return CEEMDAN_OK;
     }
@@ -484,7 +506,7 @@ struct SiftEngine {
         CKS(ws.alloc_n(&sa.pair_mark, (size_t)nr));
         CKS(ws.alloc_n(&sa.arrive, 1));
         CKS(ws.alloc_n(&sa.nfin, (size_t)std::max(1, max_cap)));
-        CKS(ws.alloc_n(&sa.up, (size_t)nr * n));
+        CKS(ws.alloc_n(&sa.up, (size_t)nr * row_ld(n)));
         // device copy of a taped stage's block table (blocks of kTapeBlockSlots slots)
         CKS(ws.alloc_n(&tblocks_dev, (size_t)(std::max(1, max_cap) + kTapeBlockSlots - 1) /
                                          kTapeBlockSlots));

@@ -8,8 +8,13 @@
 namespace ceemdan {
 
 constexpr int kTileSamples = 2048;  // samples per extrema / evaluation tile
-constexpr int kTileCap = 1028;      // knot slots per tile and envelope (max 1025 knots)
+constexpr int kRowSlots = 66;       // separator rows per tile and envelope (at most 65)
+constexpr int kEndKnots = 6;        // knots kept of a sparse end tile (at most 5)
 constexpr int kRcpMax = 4096;       // reciprocal tables cover knot spacings 1..kRcpMax
+
+// Stride of a row of n samples in the engine's own planes (h, mean envelope): a multiple of four
+// samples, so that every thread's groups of four are 32-byte aligned whatever n is.
+__host__ __device__ inline int row_ld(int n) { return (n + 3) & ~3; }
 
 // Static description of one channel (device array, read-only while the channel sifts): nr
 // realizations ("rows") of n samples.  Rows of all channels are numbered globally (channel c
@@ -36,29 +41,53 @@ struct ChanState {
     int err;               // device error word (0 = none)
     int cap;               // sift cap of the current stage
     int stage;             // batched engine: current stage (2*(num_imfs-1) = all done)
-    int pad[3];
+    int pad;
+    // rows counted in the current iteration, and in the high word those of them that have finished
+    // (back to 0 at its end)
+    unsigned long long rows;
     double* mode_out;      // modes of the current stage (row r of the channel at r*n)
     unsigned long long knots;  // knots summed over executed iterations (both envelopes)
     unsigned long long iters;  // executed iterations, all stages
+};
+
+// What the rest of its spline needs of one tile (k_tile_knots -> k_spline_solve): the two knots
+// at either end (the same knot twice when there is only one) and the end relations of the tile's
+// first and last chunk on the side of the tile's first and last separator.
+struct TileHdr {
+    double y0, y1, ya, yb;
+    double ga, aa, ba, gb, ab, bb;
+    int x0, x1, xa, xb;
+};
+// The knots just outside a tile (position, value, spline value) and the index of the tile's first
+// separator in its spline (k_spline_solve -> k_tile_sift).
+struct TileEdge {
+    double py, pc, ny, nc;
+    int px, nx, sep0, pad;
+};
+
+// Threads per CTA of the tile kernels: a thread holds 16 consecutive samples.
+constexpr int kTileThreads = 128;
+
+// Knots of a tile (maxima in the low half words, minima in the high ones): before each warp's
+// samples, and in all.
+struct TileScan {
+    int before[kTileThreads / 32], total, pad[3];
 };
 
 // Everything one sift iteration touches (device pointers unless noted).
 struct SiftArgs {
     int nrows, nchan;      // rows and channels
     // channel 0's geometry as launch parameters (used when nchan == 1, so that the kernels
-    // need no load of the channel table), and the parity of the iteration when the host knows
-    // it (one channel, host-driven iterations; -1: read the channel's iteration counter)
+    // need no load of the channel table)
     int n1, ntiles1, nr1, rs1;
-    int par;
     // one channel re-run for a known number of iterations (a block of the realizations of a
     // recorded stage): the stage ends after `forced` iterations whatever the block's own
     // lock-step test says; 0: the stop test decides
     int forced;
     int ntot;              // tiles over all rows
-    int red_qcap;          // level-3 rows whose workspace fits the reduced solve's shared memory
+    int solve_wcap;        // doubles of k_spline_solve's shared memory after the staged rows
     long long rec_total;   // record slots of one envelope (sum of the rows' rec_stride)
     long long red_total;   // reduced-workspace doubles of one envelope
-    size_t rec_plane;      // stride between record fields (2*rec_total)
     int spin_limit;        // cap of in-kernel waits (reserved: no kernel waits today)
     double sd, sd2, tol;
     // margins of the division-free sx tests (sx_bounds): sx > t is true when |U+L| > |U-L|*t_hi
@@ -71,40 +100,45 @@ struct SiftArgs {
     // channels that sift in this iteration (done == 0).  With one channel the kernels read the
     // channel's done word instead.
     int* plan;
-    int* gcount;           // [2*nrows] warp groups of each active spline, active-spline order
-    double* h[2];          // sift state ping / pong: iteration j of a stage reads h[j%2]
-    double* menv;          // mean envelope, persists for the whole decomposition
-    int* mark;             // [nrows] -1 none, 0 export, 1 subtract
+    double* h[2];          // sift state: row g's current h is in plane par[g], the other one
+                           //   takes its next value
+    int* par;              // [nrows]
+    double* menv;          // mean envelope (rows as h), persists for the whole decomposition
+    int* mark;             // [nrows] last iteration's decision: -1 none yet, 0 finished (the mode is
+                           //   h, the next iteration repeats this one), 1 subtract
     int* finish;
     double* frac;          // sifting fraction accumulator, persists
-    unsigned* cnt;
+    unsigned* cnt;         // [nrows] counts of a finished row's last iteration, for its repetition
     int* any;
+    // a row's counts of the current iteration (count_tile; back to 0 at its end): [nrows], or for
+    // rows whose tile count has more than count_bits bits [nrows][2]
+    unsigned long long *acc, *acc_wide;
+    int count_bits;
     int* kcount;           // [2*nrows] maxima counts, minima counts (by spline)
+    int* cmax;             // [2*nrows] knots of a spline's densest tile
+    int sift_split;        // k_tile_sift runs as two launches (dense and sparse rows), else one
     int* tile_cnt;         // [2*ntot] knots found in each tile
-    int* tile_off;         // [2*(ntot+nrows)] exclusive prefix of tile_cnt (global knot index)
-    int* sep_off;          // [2*(ntot+nrows)] exclusive prefix of the separators per tile
-    int* pcount;           // [2*nrows] separators per spline
-    int* gsum;             // [2*nrows+1] exclusive prefix of gcount (active-spline order)
     unsigned* bitmap;      // [2][ntot][64] knot flags of each tile (word j/32, bit j%32)
-    long long* nbr;        // [2][ntot][2] address of the knot before / after each tile
-                           //   (-1 if none)
-    // knots, tile-local: knot i of global tile gt at gt*kTileCap + (i - tile_off[t])
-    int32_t *kx_max, *kx_min;
-    double *ky_max, *ky_min;
-    // record {a = y, b, c, d} of the segment starting at each knot (same slots, 4 doubles
-    // each, 32-byte aligned)
-    double* seg[2];
+    TileScan* scan;        // [ntot]
+    TileHdr* hdr;          // [2*ntot]
+    TileEdge* edge;        // [2*ntot]
+    double* rows;          // [2*ntot][kRowSlots][4] rows (l, m, u, r) of the separator system
+    // tables of splines with more tiles than k_spline_solve's shared memory holds
+    // [2*(ntot+nrows)]: separators before each tile, tiles with knots before it, those tiles
+    int *sep_off, *tile_rank, *tile_list;
+    double* yend;          // [2*nrows][2] values of a spline's two end knots
+    // knots of a spline's first and last tile when they are fewer than six [2*nrows][2][kEndKnots]
+    int* end_x;
+    double* end_y;
     const double* rcp_h;   // [kRcpMax+1] RN(1/h)
     const double* rcp_3h;  // [kRcpMax+1] RN(1/(3h))
-    double* rec;           // 10 planes of chunk records: 6 end relations of the chunk left of
-                           //   each separator, then the separator's own row (l, m, u, r)
     double* xsep;          // [2*rec_total] spline values at the separators
     double* red;           // [2*red_total] reduced-solve workspace
     double* dbg_upper;     // optional envelope outputs (stage-level entry point, one channel)
     double* dbg_lower;
     // taped forward only (one channel; null otherwise): end-rule flags of each spline [2*nr]
-    // written by k_scan_boundary (bit 0: the left end value was replaced by the extrapolation,
-    // bit 1: the right one), and the tape slot's mark array [nr] that k_criterion fills
+    // written by k_spline_solve (bit 0: the left end value was replaced by the extrapolation,
+    // bit 1: the right one), and the tape slot's mark array [nr] that k_tile_sift fills
     unsigned char* bflags;
     signed char* tape_mark;
 };
@@ -188,23 +222,14 @@ struct SmallArgs {
 };
 constexpr int kTapeBlockSlots = 32;  // tape slots per allocation block
 
-// The tile kernels come in two register budgets (minimum resident CTAs per SM, the
-// __launch_bounds__ of each variant); the batched engine's autotuner picks one, the results
-// are the same.  A is the default.
-constexpr int kExtremaBlocksA = 6, kExtremaBlocksB = 4;
-constexpr int kEvalBlocksA = 5, kEvalBlocksB = 4;
-template <int kMinBlocks, bool kLoop>
-__global__ void k_extrema_t(SiftArgs a);
-template <int kMinBlocks>
-__global__ void k_eval_t(SiftArgs a);
-__global__ void k_scan_boundary(SiftArgs a);
 __global__ void k_gather_knots(SiftArgs a, int e, int32_t* kx, double* ky);
-__global__ void k_chunk_reduce(SiftArgs a);
-__global__ void k_group_scan(SiftArgs a);
-__global__ void k_reduced_solve(SiftArgs a);
-__global__ void k_segments(SiftArgs a);
+// Shared-memory entries of k_tile_sift.  Dense: both envelopes of a tile of up to about 1860 knots
+// at once (white noise has 1370, sifted a thousand times 1490), one after the other above.
+// Sparse: up to about 1260 knots a tile, every stage after the first of white noise.
+constexpr int kSiftDense = 1984, kSiftSparse = 1344;
+size_t tile_sift_smem(bool dense);
+size_t tile_knots_smem();
 
-__global__ void k_criterion(SiftArgs a);
 __global__ void k_export_final(SiftArgs a, int c);
 __global__ void k_plan(SiftArgs a);
 __global__ void k_begin_stage(SiftArgs a, int c, int cap, double* mode_out);
@@ -223,11 +248,11 @@ __global__ void k_tridiag_batched(int n, const double* l, const double* m, const
                                   const double* r, double* x, double* sys, double* ws,
                                   size_t ws_stride);
 // In-CTA canonical partitioned solve (sift_kernels.cu): system in 4 planes of `plane` doubles
-// (l, m, u, r) at sys, solution to x, workspace ws of >= 0.75*n + 16 doubles; every thread of
+// (l, m, u, r) at sys (u is overwritten), solution to x, workspace ws of >= 0.75*n + 16 doubles; every thread of
 // the CTA calls it.
-__device__ void cta_tridiag(int n, const double* sys, int plane, double* x, double* ws);
+__device__ void cta_tridiag(int n, double* sys, int plane, double* x, double* ws);
 // the same solve of a spline system (pivots in pivot_inv's range)
-__device__ void cta_spline_tridiag(int n, const double* sys, int plane, double* x, double* ws);
+__device__ void cta_spline_tridiag(int n, double* sys, int plane, double* x, double* ws);
 // cta_spline_tridiag's solve for nsys systems at once, one level per launch (sift_kernels.cu)
 cudaError_t psolve_launch(int nsys, int max_rows, const int* nrows, const double* sys, int plane,
                           double* x, double* ws, size_t ws_stride, cudaStream_t st,
@@ -242,7 +267,7 @@ __global__ void k_adj_segsums(const unsigned char* slot, TapeLayout L, int n, in
                               const int32_t* kx, const double* eb, double* S);
 __global__ void k_adj_rows(const unsigned char* slot, TapeLayout L, int cap, const int32_t* kx,
                            const double* S, double* yb, double* sys, int* nrows);
-__global__ void k_adj_solve(const unsigned char* slot, TapeLayout L, int cap, const double* sys,
+__global__ void k_adj_solve(const unsigned char* slot, TapeLayout L, int cap, double* sys,
                             double* z, double* ws, size_t ws_stride);
 __global__ void k_adj_rhs(const unsigned char* slot, TapeLayout L, int cap, const int32_t* kx,
                           const double* yb, const double* z, double* y2);
@@ -262,13 +287,12 @@ __global__ void k_adj_out(int stage, const double* g, const double* hs, const do
 size_t small_sift_smem(int n);
 __global__ void k_sift_small(SiftArgs a, SmallArgs sa);
 
-// dynamic shared memory of the reduced solve
-size_t reduced_solve_smem(int* qcap);
-constexpr int kRedThreads = 128;  // threads per CTA of k_reduced_solve
-// Upper bound of reduced_solve_smem(): the function attribute is always set to this value, so
-// that decompositions of different sizes running concurrently agree on it.  70 KB keeps three
-// CTAs per SM (measured best); level-3 systems beyond what fits use global memory.
-constexpr size_t kRedSmemMax = (size_t)70 * 1024;
+// k_spline_solve: threads per CTA, chunks swept per pass over the staged rows, dynamic shared
+// memory (the stage of 87,080 bytes and the level-3 workspace; two CTAs per SM).
+constexpr int kSolveThreads = 256;
+constexpr int kSolveChunks = 128;
+constexpr int kSolveStage = 87080;
+constexpr int kSolveSmem = 111600;
 
 // stage kernels (stage_kernels.cu)
 __global__ void k_canon_mean(const double* v, size_t n, size_t stride, double* acc,

@@ -1,27 +1,23 @@
 // Sifting kernels of the ICEEMDAN engine (sm_100a, FP64).
 //
 // One sift iteration over all realizations of a stage is:
-//   k_extrema        deferred update h -= m (or mode export) + strict-extrema flags +
-//                    warp-ballot compaction into per-tile knot storage, knot bitmaps
-//                    (find_extrema_shfl_* :93-148, select_extrema_* :151-207,
-//                     updateRealizations :528-544 of the previous iteration)
-//   k_scan_boundary  per-spline scan of the tile knot counts (CUB scan :1582-1604), separator
-//                    offsets, neighbour-knot addresses and the end-knot extrapolation
-//                    (setBoundaryMax/Min :210-291)
-//   k_group_scan     prefix over the splines of their 32-separator warp groups
-//   k_chunk_reduce   end relations of the tile-aligned chunks of the canonical partitioned
-//                    spline solve and the separator rows (tridiagonal_setup :311-343)
-//   k_reduced_solve  per-spline separator solve (levels >= 2), one CTA per spline
-//                    (with the chunk kernels: cusparseDgtsv2_nopivot :1622-1641)
-//   k_segments       chunk interiors -> spline values -> segment coefficients, one record per
-//                    segment (spline_coefficients :383-401)
-//   k_eval           envelopes, mean envelope, sx statistics
-//                    (interpolate :404-439, averageUppperLower :442-454, produceSX :457-467,
-//                     thresholdJudge :470-492)
-//   k_criterion      sifting fraction carry + stop test + break test
-//                    (meanD/multiplyD on sx :1851, siftingCriterion :495-525,
-//                     checkBreak :547-580)
-// Line numbers refer to the reference's cudaICEEMDAN.cu.
+//   k_tile_knots     strict extrema of every tile (find_extrema_shfl_* :93-148,
+//                    select_extrema_* :151-207), the knots' slopes and the end relations of the
+//                    chunks of the canonical partitioned spline solve (tridiagonal_setup
+//                    :311-343); knot bitmaps and the rows of the separator system are written
+//   k_spline_solve   per spline: scan of the tile counts (CUB scan :1582-1604), end-knot
+//                    extrapolation where it spans tiles (setBoundaryMax/Min :210-291), the
+//                    separator system (with the tile kernels: cusparseDgtsv2_nopivot :1622-1641)
+//   k_tile_sift      chunk interiors and segment coefficients (spline_coefficients :383-401),
+//                    envelopes, mean envelope, sx statistics (interpolate :404-439,
+//                    averageUppperLower :442-454, produceSX :457-467, thresholdJudge :470-492),
+//                    the update h -= m (updateRealizations :528-544), and after a row's last
+//                    tile its stop test (meanD/multiplyD on sx :1851, siftingCriterion :495-525,
+//                    checkBreak :547-580)
+// Knots, slopes and coefficients live in shared memory only; both tile kernels rebuild a tile's
+// knots from its samples and bitmap.  An iteration moves 8 N bytes in k_tile_knots and 24 N in
+// k_tile_sift (h, next h, mean envelope) plus N/2 of bitmaps and about 6 bytes per knot of
+// separator rows.  Line numbers refer to the reference's cudaICEEMDAN.cu.
 #include <cuda/atomic>
 #include <cuda_runtime.h>
 
@@ -35,27 +31,13 @@ namespace ceemdan {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kPerThread = kTileSamples / kThreads;  // samples per thread in a tile
-constexpr int kWords = kPerThread * (kThreads / 32); // ballot words per tile (64)
-
-__device__ __forceinline__ int pad17(int j) { return j + (j >> 4); }
-
-
-// Asynchronous global -> shared copies (cp.async): the whole staging window is in flight at
-// once instead of one round trip per loop iteration.
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::); }
+constexpr int kPerThread = kTileSamples / kTileThreads;  // samples per thread in a tile
+constexpr int kTileWarps = kTileThreads / 32;
+constexpr int kWarpSamples = 32 * kPerThread;
+// a thread's samples in the knot bitmaps
+using TileBits = unsigned short;
+static_assert(8 * sizeof(TileBits) == kPerThread, "one bit per sample");
+constexpr int kWords = kTileSamples / 32;            // bitmap words per tile (64)
 
 // ---------------------------------------------------------------------------------------
 // Geometry of the ragged multi-channel layout (kernels.h: Chan, SiftArgs).
@@ -64,7 +46,7 @@ struct Geo {
     int c, r, g;       // channel, realization within the channel, global row
     int n, ntiles;     // samples and tiles of the row
     int tile0;         // first global tile of the row
-    size_t base;       // first sample of the row
+    size_t base;       // first sample of the row in the padded planes (h, mean envelope)
 };
 
 __device__ __forceinline__ Geo geo(const SiftArgs& a, int c, int r) {
@@ -76,7 +58,7 @@ __device__ __forceinline__ Geo geo(const SiftArgs& a, int c, int r) {
         q.n = a.n1;
         q.ntiles = a.ntiles1;
         q.tile0 = r * a.ntiles1;
-        q.base = (size_t)r * (size_t)a.n1;
+        q.base = (size_t)r * (size_t)row_ld(a.n1);
         return q;
     }
     const Chan* ch = a.chan + c;
@@ -86,7 +68,7 @@ __device__ __forceinline__ Geo geo(const SiftArgs& a, int c, int r) {
     q.ntiles = __ldg(&ch->ntiles);
     q.g = __ldg(&ch->row0) + r;
     q.tile0 = __ldg(&ch->tile0) + r * q.ntiles;
-    q.base = (size_t)__ldg(&ch->samp0) + (size_t)r * (size_t)q.n;
+    q.base = (size_t)__ldg(&ch->samp0) + (size_t)r * (size_t)row_ld(q.n);
     return q;
 }
 
@@ -150,8 +132,6 @@ __device__ __forceinline__ size_t oix(const SiftArgs& a, int e, const Geo& q) {
 __device__ __forceinline__ int spline_id(const SiftArgs& a, int e, const Geo& q) {
     return e * a.nrows + q.g;
 }
-// first knot slot of global tile gt in the tile-local knot arrays
-__device__ __forceinline__ size_t tile_base(int gt) { return (size_t)gt * kTileCap; }
 // record / separator-value offset and reduced-workspace offset of row q's spline e
 __device__ __forceinline__ size_t rec_base(const SiftArgs& a, int e, const Geo& q) {
     if (a.nchan == 1) return (size_t)e * (size_t)a.rec_total + (size_t)q.r * (size_t)a.rs1;
@@ -167,102 +147,14 @@ __device__ __forceinline__ size_t red_base(const SiftArgs& a, int e, const Geo& 
            (size_t)q.r * (size_t)red_stride_of(__ldg(&ch->rec_stride));
 }
 
-// Global address of knot i of a spline whose tile offsets are off[0..ntiles] and whose first
-// tile is tile0: the tile is found by walking from tile `t` (a tile at or before the one
-// holding knot i when walking forward, at or after it when backward) -- one or two steps for
-// the end knots and the neighbours of a tile.
-__device__ __forceinline__ size_t knot_addr_fwd(const int* off, int tile0, int t, int i) {
-    while (off[t + 1] <= i) ++t;
-    return tile_base(tile0 + t) + (size_t)(i - off[t]);
-}
-__device__ __forceinline__ size_t knot_addr_bwd(const int* off, int tile0, int t, int i) {
-    while (off[t] > i) --t;
-    return tile_base(tile0 + t) + (size_t)(i - off[t]);
-}
-
-// ---------------------------------------------------------------------------------------
-// Exact divisions of the spline arithmetic, warp-wide.  Each lane forms div_rcp's quotient from
-// a tabled reciprocal (Markstein's correction, correctly rounded in its range); lanes outside
-// that range (tiny or huge operands, spacings beyond the table) take the division, under a
-// vote of the whole warp so that the division is skipped when no lane needs it -- as a plain
-// branch the compiler evaluates it unconditionally.  Every lane of the warp must call these
-// together (warp-uniform control flow); `active` = false lanes compute nothing meaningful.
-// ---------------------------------------------------------------------------------------
+// Exact division by a tabled reciprocal: div_rcp's quotient (Markstein's correction, correctly
+// rounded in its range); `slow` marks operands outside that range, which take the division.
 __device__ __forceinline__ double rcp_fast(double a, double d, double y, bool& slow) {
     const double q0 = a * y;
     const double r = fma(-q0, d, a);
     const double q1 = fma(r, y, q0);
     slow = !(fabs(a) > 0x1p-960) || !(fabs(q1) < 0x1p+1000);
     return q1;
-}
-
-// Fast parts alone, for loops that collect the lanes needing the division over all their
-// iterations and take it once after the loop (one vote instead of one per iteration).  The
-// results equal the divisions' whenever `slow` comes back false.
-__device__ __forceinline__ double slope_fast(const SiftArgs& a, int32_t x0, int32_t x1, double y0,
-                                             double y1, bool& slow) {
-    const int h = x1 - x0;
-    const bool tab = h >= 1 && h <= kRcpMax;
-    const double q = rcp_fast(y1 - y0, (double)h, __ldg(a.rcp_h + (tab ? h : 1)), slow);
-    slow = slow || !tab;
-    return q;
-}
-
-__device__ __forceinline__ void seg_coeffs_fast(const SiftArgs& a, int32_t x0, int32_t x1,
-                                                double slope, double c0, double c1, double& b,
-                                                double& d, bool& slow) {
-    const int hi = x1 - x0;
-    const bool tab = hi >= 1 && hi <= kRcpMax;
-    const double h = (double)hi;
-    bool slow_b, slow_d;
-    const double qb = rcp_fast(h * fma(2.0, c0, c1), 3.0, kRcp3, slow_b);
-    d = rcp_fast(c1 - c0, 3.0 * h, __ldg(a.rcp_3h + (tab ? hi : 1)), slow_d);
-    b = slope - qb;
-    slow = slow_b || slow_d || !tab;
-}
-
-// The same coefficients by the divisions themselves (the fallback of seg_coeffs_fast).
-__device__ __forceinline__ void seg_coeffs_div(int32_t x0, int32_t x1, double slope, double c0,
-                                               double c1, double& b, double& d) {
-    const double h = (double)(x1 - x0);
-    b = slope - (h * fma(2.0, c0, c1)) / 3.0;
-    d = (c1 - c0) / (3.0 * h);
-}
-
-// (y1 - y0) / (x1 - x0), the same quotient as seg_slope.
-__device__ __forceinline__ double slope_warp(const SiftArgs& a, int32_t x0, int32_t x1, double y0,
-                                             double y1, bool active) {
-    const int h = x1 - x0;
-    const bool tab = h >= 1 && h <= kRcpMax;
-    const double dy = y1 - y0;
-    bool slow;
-    double q = rcp_fast(dy, (double)h, __ldg(a.rcp_h + (tab ? h : 1)), slow);
-    slow = active && (slow || !tab);
-    if (__any_sync(0xffffffffu, slow)) {
-        if (slow) q = dy / (double)h;
-    }
-    return q;
-}
-
-// Segment coefficients b and d (seg_coeffs) from the segment's slope and spline values.
-__device__ __forceinline__ void seg_coeffs_warp(const SiftArgs& a, int32_t x0, int32_t x1,
-                                                double slope, double c0, double c1, double& b,
-                                                double& d, bool active) {
-    const int hi = x1 - x0;
-    const bool tab = hi >= 1 && hi <= kRcpMax;
-    const double h = (double)hi;
-    const double hq = h * fma(2.0, c0, c1);
-    const double dc = c1 - c0;
-    bool slow_b, slow_d;
-    double qb = rcp_fast(hq, 3.0, kRcp3, slow_b);
-    d = rcp_fast(dc, 3.0 * h, __ldg(a.rcp_3h + (tab ? hi : 1)), slow_d);
-    slow_b = active && slow_b;
-    slow_d = active && (slow_d || !tab);
-    if (__any_sync(0xffffffffu, slow_b || slow_d)) {
-        if (slow_b) qb = hq / 3.0;
-        if (slow_d) d = dc / (3.0 * h);
-    }
-    b = slope - qb;
 }
 
 // ---------------------------------------------------------------------------------------
@@ -274,25 +166,35 @@ struct ChunkEnds {
 
 // End relations of a chunk of `len` rows: top-down elimination gives the last row
 // x_b = gb + ab*xL + bb*xR, bottom-up elimination the first row x_a = ga + aa*xL + ba*xR.
-// The two sweeps are independent chains and run interleaved.
-template <class Pivot = SplinePivot, class RowFn>
-__device__ __forceinline__ ChunkEnds chunk_ends(int len, const RowFn& row) {
+// The two sweeps are independent chains and run interleaved.  The pivot reciprocals of the
+// top-down sweep are those of the interior's sweep: row k's goes to iw_out(k), where
+// chunk_interior_iw takes it from.  (Loops stay rolled: a CTA passes here once, and unrolled
+// sweeps spent most of their time fetching instructions, up to 1000 cycles a row.)
+template <class Pivot = SplinePivot, class RowFn, class IwOut>
+__device__ __forceinline__ ChunkEnds chunk_ends(int len, const RowFn& row, const IwOut& iw_out) {
     const Row wa = row(0), wb = row(len - 1);
     double iw = Pivot::inv(wa.m);
-    double cp = wa.u * iw, gp = wa.r * iw, ap = -wa.l * iw;
     double iv = Pivot::inv(wb.m);
+    double cp = wa.u * iw, gp = wa.r * iw, ap = -wa.l * iw;
     double cq = wb.l * iv, gq = wb.r * iv, bq = -wb.u * iv;
+    iw_out(0) = iw;
+    Row w = len > 1 ? row(1) : wa, v = len > 1 ? row(len - 2) : wb;
+#pragma unroll 1
     for (int k = 1; k < len; ++k) {
-        const Row w = row(k);
-        const Row v = row(len - 1 - k);
-        iw = Pivot::inv(fma(-w.l, cp, w.m));
-        iv = Pivot::inv(fma(-v.u, cq, v.m));
-        cp = w.u * iw;
-        gp = fma(-w.l, gp, w.r) * iw;
-        ap = (-w.l * ap) * iw;
-        cq = v.l * iv;
-        gq = fma(-v.u, gq, v.r) * iv;
-        bq = (-v.u * bq) * iv;
+        const Row wc = w, vc = v;
+        if (k + 1 < len) {  // the next rows load while this row's reciprocals form
+            w = row(k + 1);
+            v = row(len - 2 - k);
+        }
+        iw = Pivot::inv(fma(-wc.l, cp, wc.m));
+        iv = Pivot::inv(fma(-vc.u, cq, vc.m));
+        cp = wc.u * iw;
+        gp = fma(-wc.l, gp, wc.r) * iw;
+        ap = (-wc.l * ap) * iw;
+        cq = vc.l * iv;
+        gq = fma(-vc.u, gq, vc.r) * iv;
+        bq = (-vc.u * bq) * iv;
+        iw_out(k) = iw;
     }
     ChunkEnds e;
     e.gb = gp;
@@ -303,6 +205,101 @@ __device__ __forceinline__ ChunkEnds chunk_ends(int len, const RowFn& row) {
     e.aa = -wa.l * iv;
     return e;
 }
+
+// Interior of a chunk whose end relations chunk_ends formed: coupling terms to the right-hand
+// side, then canonical Thomas with the reciprocals left in x(k); x(k) receives the solution,
+// fac(k) the factors meanwhile (fac(k) may be row k's own u or a slot of it that rows after k do
+// not read).
+template <class RowFn, class X, class Fac>
+__device__ __forceinline__ void chunk_interior_iw(int len, const RowFn& row, double xl, double xr,
+                                                  const X& x, const Fac& fac) {
+    Row w = row(0);
+    double iw = x(0), gp = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < len; ++k) {
+        const Row wc = w;
+        const double ic = iw;
+        if (k + 1 < len) {
+            w = row(k + 1);
+            iw = x(k + 1);
+        }
+        double ri = wc.r;
+        if (k == 0) ri = fma(-wc.l, xl, ri);
+        if (k == len - 1) ri = fma(-wc.u, xr, ri);
+        gp = k == 0 ? ri * ic : fma(-wc.l, gp, ri) * ic;
+        fac(k) = wc.u * ic;
+        x(k) = gp;
+    }
+    double xv = gp;
+#pragma unroll 1
+    for (int k = len - 2; k >= 0; --k) {
+        xv = fma(-fac(k), xv, x(k));
+        x(k) = xv;
+    }
+}
+
+// Canonical Thomas on n <= kChunk rows, solution to x(k), factors to fac(k) meanwhile.
+template <class Pivot = SplinePivot, class RowFn, class X, class Fac>
+__device__ __forceinline__ void thomas_rolled(int n, const RowFn& row, const X& x,
+                                              const Fac& fac) {
+    Row w = row(0);
+    double cp = 0.0, gp = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) {
+        const Row wc = w;
+        if (k + 1 < n) w = row(k + 1);
+        const double iw = Pivot::inv(k == 0 ? wc.m : fma(-wc.l, cp, wc.m));
+        gp = k == 0 ? wc.r * iw : fma(-wc.l, gp, wc.r) * iw;
+        cp = wc.u * iw;
+        fac(k) = cp;
+        x(k) = gp;
+    }
+    double xv = gp;
+#pragma unroll 1
+    for (int k = n - 2; k >= 0; --k) {
+        xv = fma(-fac(k), xv, x(k));
+        x(k) = xv;
+    }
+}
+
+// chunk_interior_iw without stored reciprocals (the same values, formed again).
+template <class RowFn, class X, class Fac>
+__device__ __forceinline__ void chunk_interior_rolled(int len, const RowFn& row, double xl,
+                                                      double xr, const X& x, const Fac& fac) {
+    Row w = row(0);
+    double cp = 0.0, gp = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < len; ++k) {
+        const Row wc = w;
+        if (k + 1 < len) w = row(k + 1);
+        double ri = wc.r;
+        if (k == 0) ri = fma(-wc.l, xl, ri);
+        if (k == len - 1) ri = fma(-wc.u, xr, ri);
+        const double iw = pivot_inv(k == 0 ? wc.m : fma(-wc.l, cp, wc.m));
+        gp = k == 0 ? ri * iw : fma(-wc.l, gp, ri) * iw;
+        cp = wc.u * iw;
+        fac(k) = cp;
+        x(k) = gp;
+    }
+    double xv = gp;
+#pragma unroll 1
+    for (int k = len - 2; k >= 0; --k) {
+        xv = fma(-fac(k), xv, x(k));
+        x(k) = xv;
+    }
+}
+
+// Consecutive doubles as a row-indexed destination; NoIw drops what it is given.
+struct Slots {
+    double* p;
+    __device__ __forceinline__ double& operator()(int k) const { return p[k]; }
+};
+struct NoIw {
+    struct Sink {
+        __device__ __forceinline__ void operator=(double) const {}
+    };
+    __device__ __forceinline__ Sink operator()(int) const { return Sink(); }
+};
 
 // Interior of a chunk of `len` rows once its separator values xl, xr are known: coupling
 // terms move to the right-hand side, then canonical Thomas; x_k written to out[k*stride].
@@ -345,755 +342,539 @@ __device__ __forceinline__ void thomas_small(int n, const RowFn& row, double* x,
     chunk_interior<false, Pivot>(n, row, 0.0, 0.0, x, stride);
 }
 
-}  // namespace
+// Rows of a tile, knots of a spline: the padded position of in-tile knot m in the shared-memory
+// knot arrays, one pad slot after every 16 knots, so that the chunk sweeps (lane p walks the
+// knots of chunk p, 16 knots after lane p-1's) read different banks.
+__device__ __forceinline__ int kq(int m) { return m + (m >> 4); }
 
-// =======================================================================================
-// k_extrema
-// =======================================================================================
-template <int kMinBlocks, bool kLoop>
-__global__ void __launch_bounds__(kThreads, kMinBlocks)
-k_extrema_t(SiftArgs a) {
-    __shared__ __align__(16) double sh[kTileSamples + 4];  // sh[2 + j] = sample n0 + j
-    __shared__ __align__(16) double sm[kTileSamples];      // mean envelope of the tile
-    __shared__ int s_cnt[2][kWords];
-    __shared__ int s_off[2][kWords];
-    __shared__ __align__(16) double s_halo[4];  // h at n0-1 and n0+2048, then the mean there
+// Entry of k_tile_sift's arrays where the segment of a sample with r knots before it in the tile
+// starts: the knot before the tile at 0, in-tile knot m at 2 + kq(m).
+__device__ __forceinline__ int seg_at(int r) { return r + ((r + 15) >> 4); }
 
-    const int total = active_tiles(a);
-    // kLoop: persistent CTAs, active tiles v, v + gridDim.x, ... (CTA-uniform loop); else the
-    // grid covers every tile, one per CTA
-    for (int v = blockIdx.x; v < total; v += gridDim.x) {
-    int tile;
-    const Geo q = tile_geo(a, v, tile);
-    const int n = q.n;
-    const int n0 = tile * kTileSamples;
-    const size_t base = q.base;
-    const ChanState& cst = a.cs[q.c];
-    const int it = a.par >= 0 ? a.par : cst.iter;
-    const int mk = a.mark[q.g];
-    const double* __restrict__ hin = a.h[it & 1] + base;
-    double* __restrict__ hout = a.h[(it + 1) & 1] + base;
-    const double* __restrict__ me = a.menv + base;
-    double* __restrict__ mo = mk == 0 ? cst.mode_out + (size_t)q.r * n : nullptr;
+// separators of a tile with c knots (local 0, 16, 32, ... and the last one)
+__device__ __forceinline__ int tile_seps(int c) { return c > 0 ? (c + kChunk - 2) / kChunk + 1 : 0; }
 
-    // Deferred update of the previous iteration (h -= m, or mode export).  The tile of h (and
-    // of the mean envelope when it is subtracted) is copied to shared memory with cp.async,
-    // all copies in flight at once; registers hold nothing while they land.  Even n: the tile
-    // moves as 16-byte pieces (sample pairs), piece k*256 + t by thread t, so every warp
-    // instruction covers 512 contiguous bytes (n even keeps every piece 16-byte aligned and
-    // inside the row; every row starts at an even sample of the channel's block, and blocks
-    // start 256-byte aligned).
-    const bool even = (n & 1) == 0;
-    if (even) {
-#pragma unroll
-        for (int k = 0; k < kPerThread / 2; ++k) {
-            const int j = 2 * (k * kThreads + threadIdx.x);
-            const int s = n0 + j;
-            if (s < n) {
-                cp_async16(&sh[2 + j], hin + s);
-                if (mk == 1) cp_async16(&sm[j], me + s);
-            }
+// Four doubles to a 32-byte aligned address, as one access.
+__device__ __forceinline__ void store4(double* p, const double* v) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]),
+                 "d"(v[2]), "d"(v[3])
+                 : "memory");
+}
+
+// Asynchronous global -> shared copies.
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+// all but the newest group
+__device__ __forceinline__ void cp_async_wait_but_one() {
+    asm volatile("cp.async.wait_group 1;\n" ::);
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::); }
+
+// The tile kernels run as persistent CTAs: CTA b works on the b-th of gridDim.x contiguous ranges
+// of the active tiles, and copies the next tile's samples to shared memory while it computes on
+// the current one.  TileIter walks the range; mark and par are the row's (loaded once a row).
+struct TileIter {
+    int v, end;  // active tile, end of the range
+    int tile, mark, par;
+    // averageUppperLower: the mean envelope keeps its previous value unless both envelopes have
+    // more than 3 knots
+    bool mean;
+    int need;  // shared-memory entries of k_tile_sift the row's tiles need at most
+    Geo q;
+    __device__ __forceinline__ void row(const SiftArgs& a) {
+        q = tile_geo(a, v, tile);
+        mark = a.mark[q.g];
+        par = a.par[q.g];
+        mean = min(a.kcount[q.g], a.kcount[a.nrows + q.g]) > 3;
+        need = seg_at(a.cmax[q.g] + 1) + seg_at(a.cmax[a.nrows + q.g] + 1) + 2;
+    }
+    __device__ __forceinline__ explicit TileIter(const SiftArgs& a) {
+        const int total = active_tiles(a);
+        v = (int)((long long)total * blockIdx.x / gridDim.x);
+        end = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
+        tile = mark = par = need = 0;
+        mean = false;
+        if (v < end) row(a);
+    }
+    __device__ __forceinline__ bool more() const { return v < end; }
+    __device__ __forceinline__ void next(const SiftArgs& a) {
+        ++v;
+        if (++tile == q.ntiles && v < end) row(a);
+    }
+    // past the rest of the row while it does not satisfy pred
+    template <class Pred>
+    __device__ __forceinline__ void to_row(const SiftArgs& a, Pred pred) {
+        while (v < end && !pred(*this)) {
+            v += q.ntiles - tile;
+            if (v < end) row(a);
         }
+    }
+};
+
+// The samples of a tile in shared memory, 16-byte piece u at stage_piece(u): a warp copies its
+// own samples coalesced (pieces l, l + 32, ...), then thread t reads its consecutive pieces without
+// bank conflicts.  Every warp stages and reads only its own pieces.
+__device__ __forceinline__ int stage_piece(int u) { return u ^ ((u >> 3) & 7); }
+
+__device__ __forceinline__ void stage_tile(double2* st, const double* h, int m, int tid) {
+    const int u0 = (tid & ~31) * (kPerThread / 2) + (tid & 31);
+    if (m == kTileSamples) {
+#pragma unroll
+        for (int g = 0; g < kPerThread / 2; ++g) cp_async16(st + stage_piece(u0 + 32 * g), h + 2 * (u0 + 32 * g));
     } else {
+        const int m4 = (m + 3) & ~3;  // rows are padded to a multiple of four samples
 #pragma unroll
-        for (int k = 0; k < kPerThread; ++k) {
-            const int j = k * kThreads + threadIdx.x;
-            const int s = n0 + j;
-            if (s < n) {
-                cp_async8(&sh[2 + j], hin + s);
-                if (mk == 1) cp_async8(&sm[j], me + s);
-            }
-        }
+        for (int g = 0; g < kPerThread / 2; ++g)
+            if (2 * (u0 + 32 * g) < m4)
+                cp_async16(st + stage_piece(u0 + 32 * g), h + 2 * (u0 + 32 * g));
     }
-    if (threadIdx.x < 2) {  // halo samples n0-1 and n0+kTileSamples, with the tile's copies
-        const int s = threadIdx.x == 0 ? n0 - 1 : n0 + kTileSamples;
-        if (s >= 0 && s < n) {
-            cp_async8(&s_halo[threadIdx.x], hin + s);
-            if (mk == 1) cp_async8(&s_halo[2 + threadIdx.x], me + s);
-        }
-    }
-    cp_async_wait_all();
-    // each thread updates the samples it copied (no other thread reads them before the barrier)
-    if (even) {
+}
+// sample j of the tile
+__device__ __forceinline__ double staged(const double2* st, int j) {
+    return reinterpret_cast<const double*>(st + stage_piece(j >> 1))[j & 1];
+}
+// the thread's samples (zeros past the row)
+__device__ __forceinline__ void unstage_tile(double* h, const double2* st, int m, int tid) {
 #pragma unroll
-        for (int k = 0; k < kPerThread / 2; ++k) {
-            const int j = 2 * (k * kThreads + threadIdx.x);
-            const int s = n0 + j;
-            double2 val = make_double2(0.0, 0.0);
-            if (s < n) {
-                const double2 hv = *reinterpret_cast<const double2*>(&sh[2 + j]);
-                val = hv;
-                if (mk == 1) {
-                    const double2 mv = *reinterpret_cast<const double2*>(&sm[j]);
-                    val.x = hv.x - mv.x;
-                    val.y = hv.y - mv.y;
-                }
-                *reinterpret_cast<double2*>(hout + s) = val;
-                if (mk == 0) *reinterpret_cast<double2*>(mo + s) = hv;
-            }
-            *reinterpret_cast<double2*>(&sh[2 + j]) = val;
-        }
-    } else {
+    for (int g = 0; g < kPerThread / 2; ++g) {
+        const double2 w = st[stage_piece(kPerThread / 2 * tid + g)];
+        h[2 * g] = w.x;
+        h[2 * g + 1] = w.y;
+    }
+    if (m < kTileSamples) {
 #pragma unroll
-        for (int k = 0; k < kPerThread; ++k) {
-            const int j = k * kThreads + threadIdx.x;
-            const int s = n0 + j;
-            double val = 0.0;
-            if (s < n) {
-                const double hv = sh[2 + j];
-                val = (mk == 1) ? hv - sm[j] : hv;
-                hout[s] = val;
-                if (mk == 0) mo[s] = hv;
-            }
-            sh[2 + j] = val;
-        }
-    }
-    if (threadIdx.x < 2) {  // the halo this thread copied
-        const int s = threadIdx.x == 0 ? n0 - 1 : n0 + kTileSamples;
-        double val = 0.0;
-        if (s >= 0 && s < n) {
-            const double hv = s_halo[threadIdx.x];
-            val = (mk == 1) ? hv - s_halo[2 + threadIdx.x] : hv;
-        }
-        sh[threadIdx.x == 0 ? 1 : 2 + kTileSamples] = val;
-    }
-    __syncthreads();
-
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const size_t bw0 = tix(a, 0, q, tile) * kWords;
-    const size_t bw1 = tix(a, 1, q, tile) * kWords;
-    unsigned bmax[kPerThread], bmin[kPerThread];
-#pragma unroll
-    for (int k = 0; k < kPerThread; ++k) {
-        const int j = k * kThreads + threadIdx.x;  // local sample
-        const int s = n0 + j;
-        bool fmax = false, fmin = false;
-        if (s < n) {
-            if (s == 0 || s == n - 1) {
-                fmax = fmin = true;
-            } else {
-                const double x = sh[2 + j], xl = sh[1 + j], xr = sh[3 + j];
-                fmax = x > xl && x > xr;
-                fmin = x < xl && x < xr;
-            }
-        }
-        bmax[k] = __ballot_sync(0xffffffffu, fmax);
-        bmin[k] = __ballot_sync(0xffffffffu, fmin);
-        if (lane == 0) {
-            const int w = k * (kThreads / 32) + warp;
-            s_cnt[0][w] = __popc(bmax[k]);
-            s_cnt[1][w] = __popc(bmin[k]);
-            a.bitmap[bw0 + w] = bmax[k];
-            a.bitmap[bw1 + w] = bmin[k];
-        }
-    }
-    __syncthreads();
-
-    // Exclusive scan of the 64 word counts per envelope: warp 0 -> maxima, warp 1 -> minima;
-    // the total is the tile's knot count.
-    static_assert(kWords == 64, "scan assumes 64 words");
-    if (warp < 2) {
-        const int e = warp;
-        const int c0 = s_cnt[e][2 * lane], c1 = s_cnt[e][2 * lane + 1];
-        int incl = c0 + c1;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        const int excl = incl - (c0 + c1);
-        s_off[e][2 * lane] = excl;
-        s_off[e][2 * lane + 1] = excl + c0;
-        if (lane == 31) a.tile_cnt[tix(a, e, q, tile)] = incl;
-    }
-    __syncthreads();
-
-    const unsigned lt = (1u << lane) - 1u;
-    const size_t kb = tile_base(q.tile0 + tile);
-#pragma unroll
-    for (int k = 0; k < kPerThread; ++k) {
-        const int j = k * kThreads + threadIdx.x;
-        const int s = n0 + j;
-        const int w = k * (kThreads / 32) + warp;
-        if (bmax[k] & (1u << lane)) {
-            const int pos = s_off[0][w] + __popc(bmax[k] & lt);
-            a.kx_max[kb + pos] = s;
-            a.ky_max[kb + pos] = sh[2 + j];
-        }
-        if (bmin[k] & (1u << lane)) {
-            const int pos = s_off[1][w] + __popc(bmin[k] & lt);
-            a.kx_min[kb + pos] = s;
-            a.ky_min[kb + pos] = sh[2 + j];
-        }
-    }
-    if (!kLoop) break;
-    __syncthreads();  // shared memory is reused by the CTA's next tile
+        for (int i = 0; i < kPerThread; ++i)
+            if (kPerThread * tid + i >= m) h[i] = 0.0;
     }
 }
 
-// The register budgets the autotuner chooses between (resident CTAs per SM), persistent or one
-// tile per CTA; same results.
-template __global__ void k_extrema_t<kExtremaBlocksA, true>(SiftArgs a);
-template __global__ void k_extrema_t<kExtremaBlocksB, true>(SiftArgs a);
-template __global__ void k_extrema_t<kExtremaBlocksA, false>(SiftArgs a);
-template __global__ void k_extrema_t<kExtremaBlocksB, false>(SiftArgs a);
-
-// =======================================================================================
-// k_scan_boundary: one warp per spline (envelope, realization): exclusive scan of the tile
-// knot counts into the offset row, the knot count, and the end-knot extrapolation.
-// =======================================================================================
-__global__ void __launch_bounds__(kThreads)
-k_scan_boundary(SiftArgs a) {
-    const int lane = threadIdx.x & 31;
-    const int ra = active_rows(a);
-    const int wpb = kThreads / 32;
-    // one warp per active spline (warp-uniform loop)
-    for (int v = blockIdx.x * wpb + (threadIdx.x >> 5); v < 2 * ra; v += gridDim.x * wpb) {
-    int e;
-    const Geo q = spline_geo(a, v, ra, e);
-    const int id = spline_id(a, e, q);
-    const int ntiles = q.ntiles;
-    const int* cnt = a.tile_cnt + tix(a, e, q, 0);
-    int* off = a.tile_off + oix(a, e, q);
-    int carry = 0;
-    for (int t0 = 0; t0 < ntiles; t0 += 32) {
-        const int t = t0 + lane;
-        const int c = t < ntiles ? cnt[t] : 0;
-        int incl = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += u;
-        }
-        if (t < ntiles) off[t] = carry + incl - c;
-        carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    const int K = carry;
-    if (lane == 0) {
-        off[ntiles] = K;
-        a.kcount[id] = K;
-    }
-    // separators per tile (local 0, 16, 32, ... and the last knot), exclusive scan
-    int* soff = a.sep_off + oix(a, e, q);
-    int scarry = 0;
-    for (int t0 = 0; t0 < ntiles; t0 += 32) {
-        const int t = t0 + lane;
-        const int c = t < ntiles ? cnt[t] : 0;
-        const int ns = c > 0 ? (c + kChunk - 2) / kChunk + 1 : 0;
-        int incl = ns;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += u;
-        }
-        if (t < ntiles) soff[t] = scarry + incl - ns;
-        scarry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) {
-        soff[ntiles] = scarry;
-        a.pcount[id] = scarry;
-        a.gcount[v] = (scarry + 31) >> 5;  // warp groups of k_chunk_reduce / k_segments
-    }
-    // address of the knot just before each tile (last knot of the nearest non-empty tile
-    // before it) and just after it (first knot of the nearest non-empty tile after it)
-    long long* nb = a.nbr + tix(a, e, q, 0) * 2;
-    int last = -1;  // nearest non-empty tile before the current chunk
-    for (int t0 = 0; t0 < ntiles; t0 += 32) {
-        const int t = t0 + lane;
-        const int c = t < ntiles ? cnt[t] : 0;
-        int w = c > 0 ? t : -1;  // inclusive max-scan of non-empty tile indices
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w = max(w, u);
-        }
-        int before = __shfl_up_sync(0xffffffffu, w, 1);
-        if (lane == 0) before = -1;
-        before = max(before, last);
-        if (t < ntiles)
-            nb[2 * t] = before >= 0
-                            ? (long long)(tile_base(q.tile0 + before) + cnt[before] - 1)
-                            : -1;
-        last = max(last, __shfl_sync(0xffffffffu, w, 31));
-    }
-    int first = 0x7fffffff;  // nearest non-empty tile after the current chunk
-    for (int t0 = ((ntiles - 1) / 32) * 32; t0 >= 0; t0 -= 32) {
-        const int t = t0 + lane;
-        const int c = t < ntiles ? cnt[t] : 0;
-        int w = c > 0 ? t : 0x7fffffff;  // inclusive min-scan from the right
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_down_sync(0xffffffffu, w, o);
-            if (lane + o < 32) w = min(w, u);
-        }
-        int after = __shfl_down_sync(0xffffffffu, w, 1);
-        if (lane == 31) after = 0x7fffffff;
-        after = min(after, first);
-        if (t < ntiles)
-            nb[2 * t + 1] = after < ntiles ? (long long)tile_base(q.tile0 + after) : -1;
-        first = min(first, __shfl_sync(0xffffffffu, w, 0));
-    }
-    __syncwarp();
-    if (lane == 0 && K - 1 > 4) {
-        int32_t* kx = e == 0 ? a.kx_max : a.kx_min;
-        double* ky = e == 0 ? a.ky_max : a.ky_min;
-        const int L = K - 1;
-        const int tl = ntiles - 1;
-        const size_t p0 = knot_addr_fwd(off, q.tile0, 0, 0),
-                     p1 = knot_addr_fwd(off, q.tile0, 0, 1),
-                     p2 = knot_addr_fwd(off, q.tile0, 0, 2);
-        const size_t q0 = knot_addr_bwd(off, q.tile0, tl, L - 2),
-                     q1 = knot_addr_bwd(off, q.tile0, tl, L - 1),
-                     q2 = knot_addr_bwd(off, q.tile0, tl, L);
-        const double y0 = boundary_left(e, kx[p0], kx[p1], kx[p2], ky[p0], ky[p1], ky[p2]);
-        const double yL = boundary_right(e, kx[q0], kx[q1], kx[q2], ky[q0], ky[q1], ky[q2]);
-        // a replaced end value differs from the old one in its bits (t > y or t < y)
-        if (a.bflags)
-            a.bflags[id] = (unsigned char)(
-                (__double_as_longlong(y0) != __double_as_longlong(ky[p0]) ? 1 : 0) |
-                (__double_as_longlong(yL) != __double_as_longlong(ky[q2]) ? 2 : 0));
-        ky[p0] = y0;
-        ky[q2] = yL;
-    } else if (lane == 0 && a.bflags) {
-        a.bflags[id] = 0;
-    }
-    __syncwarp();
-    }
+// The quotient a / d by the division itself, kept out of line of the fast path (a plain
+// division in a branch is evaluated unconditionally by the compiler).
+__device__ __forceinline__ double div_cold(double a, double d) {
+    double q;
+    asm volatile("div.rn.f64 %0, %1, %2;" : "=d"(q) : "d"(a), "d"(d));
+    return q;
 }
 
-// Compacted copy of the knots of envelope e (stage-level entry point, one channel): row r's
-// knots to kx/ky[r*n + i].
-__global__ void k_gather_knots(SiftArgs a, int e, int32_t* kx, double* ky) {
-    const int tile = blockIdx.x;
-    const Geo q = geo(a, 0, blockIdx.y);
-    const int* off = a.tile_off + oix(a, e, q);
-    const int o = off[tile], c = off[tile + 1] - o;
-    const size_t src = tile_base(q.tile0 + tile);
-    const int32_t* sx = e == 0 ? a.kx_max : a.kx_min;
-    const double* sy = e == 0 ? a.ky_max : a.ky_min;
-    for (int j = threadIdx.x; j < c; j += blockDim.x) {
-        kx[q.base + o + j] = sx[src + j];
-        ky[q.base + o + j] = sy[src + j];
-    }
+// a / d for an integer-valued d in [1, 2^40], from its reciprocal (Markstein's correction as in
+// div_rcp; operands outside its range take the division).  The reciprocal is pivot_inv's without
+// the check for the all-ones significand, which an integer below 2^52 does not have; measured
+// against a table of 1/d in global memory it saves the load and its bounds.
+__device__ __forceinline__ double div_int(double a, double d) {
+    bool slow;
+    double q = rcp_fast(a, d, rcp_raw(d), slow);
+    if (slow) q = div_cold(a, d);
+    return q;
 }
 
-// =======================================================================================
-// Tile-aligned first level of the canonical spline solve.  In each tile, the knots at local
-// index 0, 16, 32, ... and the tile's last knot are separators; chunk k of a tile holds the
-// knots strictly between its separators k-1 and k and has global chunk index sep_off[t] + k
-// (the chunk left of separator sep_off[t] + k; the chunk left of local 0 is empty).
-// =======================================================================================
-namespace {
+// seg_coeffs' b and d from the segment's length, slope and spline values.
+__device__ __forceinline__ void seg_coeffs_int(double h, double slope, double c0, double c1,
+                                               double& b, double& d) {
+    const double hq = h * fma(2.0, c0, c1);
+    bool slow;
+    double qb = rcp_fast(hq, 3.0, kRcp3, slow);
+    if (slow) qb = div_cold(hq, 3.0);
+    d = div_int(c1 - c0, 3.0 * h);
+    b = slope - qb;
+}
 
-__device__ __forceinline__ int sep_local(int k, int cnt) { return min(k * kChunk, cnt - 1); }
+// Pivots of one chunk inverted by rcp_raw, with one look for the all-ones significand at the end
+// (low word -1; once in 2^32 pivots the caller repeats the chunk with pivot_inv).
+struct RawPivot {
+    bool ones = false;
+    __device__ __forceinline__ double inv(double x) {
+        ones |= __double2loint(x) == -1;
+        return rcp_raw(x);
+    }
+};
+struct CheckedPivot {
+    bool ones = false;
+    __device__ __forceinline__ double inv(double x) { return pivot_inv(x); }
+};
 
-}  // namespace
-
-// End relations of a chunk of len >= 1 rows from a slab: x[0] is the knot before row 0,
-// rows 0..len-1 are knots 1..len, knot len+1 closes the last row, s[i] is the slope of
-// segment i -> i+1.  The operations and their order are those of chunk_ends; the next rows
-// of both sweeps are loaded ahead of the reciprocal chain.
-__device__ __forceinline__ ChunkEnds chunk_ends_slab(const int32_t* x, const double* s,
-                                                     int len) {
-    auto row = [&](int k) { return spline_row(x[k], x[k + 1], x[k + 2], s[k], s[k + 1]); };
-    const Row wa = row(0), wb = row(len - 1);
-    double iw = pivot_inv(wa.m);
-    double cp = wa.u * iw, gp = wa.r * iw, ap = -wa.l * iw;
-    double iv = pivot_inv(wb.m);
-    double cq = wb.l * iv, gq = wb.r * iv, bq = -wb.u * iv;
-    Row wn = wa, vn = wb;
+// End relations (chunk_ends: same operations, same order) of the chunk whose knots 0..len+1 sit
+// in the padded arrays x, s from the chunk's base on (s[i]: slope of segment i -> i+1).  Each
+// sweep loads one new knot and slope per row, a row ahead of its use.
+template <class Pivot, class XT>
+__device__ __forceinline__ ChunkEnds chunk_ends_sweep(Pivot& pv, const XT* x, const double* s,
+                                                      int len) {
+    int xt = x[2], xb = x[len - 1];
+    // top-down row 0 and bottom-up row len-1
+    double lt = (double)(x[1] - x[0]), ut = (double)(xt - x[1]);
+    double ub = (double)(x[kq(len + 1)] - x[len]), lb = (double)(x[len] - xb);
+    double st = s[1], sb = s[len - 1];
+    const double wr0 = 3.0 * (st - s[0]), vr0 = 3.0 * (s[len] - sb);
+    const double lf = lt, ul = ub;
+    double un = 0.0, lp = 0.0, sn = 0.0, sp = 0.0;  // the next row's
     if (len > 1) {
-        wn = row(1);
-        vn = row(len - 2);
+        const int xn = x[kq(3)], xp = x[len - 2];
+        un = (double)(xn - xt);
+        xt = xn;
+        lp = (double)(xb - xp);
+        xb = xp;
+        sn = s[2];
+        sp = s[len - 2];
     }
+    double iw = pv.inv(2.0 * (lt + ut));
+    double iv = pv.inv(2.0 * (lb + ub));
+    double cp = ut * iw, gp = wr0 * iw, ap = -lt * iw;
+    double cq = lb * iv, gq = vr0 * iv, bq = -ub * iv;
+#pragma unroll 2
     for (int k = 1; k < len; ++k) {
-        const Row w = wn, v = vn;
+        lt = ut;
+        ut = un;
+        ub = lb;
+        lb = lp;
+        const double wr = 3.0 * (sn - st), vr = 3.0 * (sb - sp);
+        st = sn;
+        sb = sp;
         if (k + 1 < len) {
-            wn = row(k + 1);
-            vn = row(len - 2 - k);
+            const int xn = x[kq(k + 3)], xp = x[len - 2 - k];
+            un = (double)(xn - xt);
+            xt = xn;
+            lp = (double)(xb - xp);
+            xb = xp;
+            sn = s[k + 2];
+            sp = s[len - 2 - k];
         }
-        iw = pivot_inv(fma(-w.l, cp, w.m));
-        iv = pivot_inv(fma(-v.u, cq, v.m));
-        cp = w.u * iw;
-        gp = fma(-w.l, gp, w.r) * iw;
-        ap = (-w.l * ap) * iw;
-        cq = v.l * iv;
-        gq = fma(-v.u, gq, v.r) * iv;
-        bq = (-v.u * bq) * iv;
+        iw = pv.inv(fma(-lt, cp, 2.0 * (lt + ut)));
+        iv = pv.inv(fma(-ub, cq, 2.0 * (lb + ub)));
+        cp = ut * iw;
+        gp = fma(-lt, gp, wr) * iw;
+        ap = (-lt * ap) * iw;
+        cq = lb * iv;
+        gq = fma(-ub, gq, vr) * iv;
+        bq = (-ub * bq) * iv;
     }
     ChunkEnds e;
     e.gb = gp;
     e.ab = ap;
-    e.bb = -wb.u * iw;
+    e.bb = -ul * iw;
     e.ga = gq;
     e.ba = bq;
-    e.aa = -wa.l * iv;
+    e.aa = -lf * iv;
+    return e;
+}
+template <class XT>
+__device__ __noinline__ void chunk_ends_checked(ChunkEnds& e, const XT* x, const double* s,
+                                                int len) {
+    CheckedPivot pv;
+    e = chunk_ends_sweep(pv, x, s, len);
+}
+template <class XT>
+__device__ __forceinline__ ChunkEnds chunk_ends_knots(const XT* x, const double* s, int len) {
+    RawPivot pv;
+    ChunkEnds e = chunk_ends_sweep(pv, x, s, len);
+    if (pv.ones) {
+        ChunkEnds c;
+        chunk_ends_checked(c, x, s, len);
+        e = c;
+    }
     return e;
 }
 
-// k_group_scan: one CTA of 1024 threads.  gsum[v] = exclusive prefix over the active splines
-// (k_scan_boundary's order) of gcount[v] = ceil(pcount / 32), the warp groups of 32 separators
-// that k_chunk_reduce and k_segments hand to their warps; gsum[2*ra] is the total.
-__global__ void __launch_bounds__(1024)
-k_group_scan(SiftArgs a) {
-    __shared__ int s_warp[32];
-    const int m = 2 * active_rows(a);
-    const int per = (m + 1023) / 1024;
-    const int i0 = threadIdx.x * per;
-    int sum = 0;
-    for (int i = i0; i < min(i0 + per, m); ++i) sum += a.gcount[i];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int incl = sum;
+// Inclusive prefix of v over the warp's lanes.
+__device__ __forceinline__ int warp_scan(int v, int lane) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
+        const int t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += t;
     }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        int w = s_warp[lane];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += v;
-        }
-        s_warp[lane] = w;  // inclusive over warps
-    }
-    __syncthreads();
-    int run = (warp > 0 ? s_warp[warp - 1] : 0) + incl - sum;
-    for (int i = i0; i < min(i0 + per, m); ++i) {
-        a.gsum[i] = run;
-        run += a.gcount[i];
-    }
-    if (threadIdx.x == 1023) a.gsum[m] = s_warp[31];
+    return v;
 }
 
-// Active spline of warp group gw: the last of the m active splines whose group prefix is <= gw
-// (warp-uniform).
-__device__ __forceinline__ int group_spline(const SiftArgs& a, int gw, int m) {
-    int lo = 0, hi = m - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(a.gsum + mid) <= gw) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
+// The chunk a thread sweeps, given the separators of the tile's two envelopes: the chunks of
+// envelope 0, then envelope 1, on consecutive threads (at most 128).  k: the separator closing
+// the chunk.
+__device__ __forceinline__ bool sweep_lane(int tid, int ns0, int ns1, int& e, int& k) {
+    const int m0 = max(ns0 - 1, 0), m1 = max(ns1 - 1, 0);
+    e = tid >= m0 ? 1 : 0;
+    k = tid - (e ? m0 : 0) + 1;
+    return tid < m0 + m1;
 }
 
-constexpr int kSlab = kChunk + 1;  // knots of one chunk: the one before it .. its separator
-constexpr int kReduceWarps = 4;
-constexpr int kSegWarps = 2;
-
-// The chunk of a lane: separator p of spline (e, r) (lanes past the spline's last separator
-// take the last one).  Its tile is the last tile whose separator offset is <= p (tiles without
-// knots own no separators); js is the separator's local knot, jb the knot before the chunk's
-// first row (js for the empty chunk left of local knot 0), len the chunk's rows.
-struct ChunkLane {
-    int t, k, off0, cnt, js, jb, len;
-    size_t tb;
+// Shared memory of k_tile_knots: per envelope the knots' positions within the tile and the slopes
+// of the segments starting at them (padded positions kq), and the tile's samples.  41.5 KB: five
+// CTAs per SM.
+constexpr int kKnotCap = kTileSamples / 2 + 1 + (kTileSamples / 2 + 1) / kChunk + 1;
+struct KnotSmem {
+    double s[2][kKnotCap];
+    double ex[2][3][kRowSlots];       // first-row end relations of chunk k
+    double2 stage[kTileSamples / 2];  // the samples
+    double halo[kTileWarps][2];       // each warp's neighbours
+    double yend[2][2];                // the row's end values
+    short x[2][kKnotCap];
 };
 
-__device__ __forceinline__ ChunkLane locate_chunk(const SiftArgs& a, int e, const Geo& q, int p) {
-    const size_t o1 = oix(a, e, q);
-    const int* soff = a.sep_off + o1;
-    int lo = 0, hi = q.ntiles - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(soff + mid) <= p) lo = mid;
-        else hi = mid - 1;
-    }
-    ChunkLane c;
-    c.t = lo;
-    c.k = p - __ldg(soff + lo);
-    const int* off = a.tile_off + o1;
-    c.off0 = __ldg(off + lo);
-    c.cnt = __ldg(off + lo + 1) - c.off0;
-    c.tb = tile_base(q.tile0 + lo);
-    c.js = sep_local(c.k, c.cnt);
-    c.jb = c.k > 0 ? sep_local(c.k - 1, c.cnt) : c.js;
-    c.len = c.js - c.jb - 1;
-    return c;
-}
+}  // namespace
 
-// Copy each lane's knots first .. first+c-1 into its slab (positions 0..c-1), then replace the
-// knot values by the slopes of the slab's c-1 segments.  Warp-collective; sx/sy are the warp's
-// slabs (lane l at l*kSlab).  The warp's knots form a few contiguous runs (one per tile
-// touched), so the copies go as flattened positions f = 0..total-1, 32 consecutive ones per
-// step (coalesced), all in flight together (cp.async); tab (>= 32*kSlab entries) and gs (32)
-// are warp scratch mapping f to (lane, position).  The slopes are then computed by each lane
-// in its own slab, with one vote for the exact-division fallback after the loop.
-__device__ __forceinline__ void stage_slabs(const SiftArgs& a, const int32_t* kx, const double* ky,
-                                            int c, size_t first, int32_t* sx, double* sy,
-                                            int lane, unsigned short* tab, long long* gs) {
-    int incl = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    const int excl = incl - c;
-    for (int i = 0; i < c; ++i) tab[excl + i] = (unsigned short)((lane << 5) | i);
-    gs[lane] = (long long)first;
-    __syncwarp();
-    for (int f = lane; f < total; f += 32) {
-        const unsigned t = tab[f];
-        const int ow = (int)(t >> 5), i = (int)(t & 31u);
-        const size_t src = (size_t)gs[ow] + i;
-        cp_async4(&sx[ow * kSlab + i], kx + src);
-        cp_async8(&sy[ow * kSlab + i], ky + src);
-    }
+size_t tile_knots_smem() { return sizeof(KnotSmem); }
+
+// =======================================================================================
+// k_tile_knots: one CTA per 2048-sample tile, both envelopes; thread t holds samples 16t..16t+15.
+// Strict extrema from the signs of neighbour differences, eight to a byte of the knot bitmaps; the
+// knots compacted into shared memory; the segment slopes; the end relations of the chunks between
+// separators (one thread per chunk) and from them the rows of the separator system inside the
+// tile.  What the tile's first and last separators need from other tiles goes into the tile's
+// header for k_spline_solve.  Issue bound: eight samples to a thread take half the instructions
+// of one sample to a lane (signs shared between neighbours, one scan step per thread).
+// =======================================================================================
+__global__ void __launch_bounds__(kTileThreads, 5)
+k_tile_knots(const __grid_constant__ SiftArgs a) {
+    extern __shared__ __align__(16) unsigned char dyn_smem[];
+    KnotSmem& S = *reinterpret_cast<KnotSmem*>(dyn_smem);
+    __shared__ int s_w[kTileWarps];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    TileIter it(a);
+    auto live = [](const TileIter& t) { return t.mark != 0; };  // else: repeats (k_tile_sift)
+    auto prefetch = [&]() {
+        if (!it.more()) return;
+        const int n0 = it.tile * kTileSamples, left = it.q.n - n0;
+        const double* h = a.h[it.par] + it.q.base + n0;
+        stage_tile(S.stage, h, min(kTileSamples, left), tid);
+        const int j = warp * kWarpSamples;  // the neighbours of the warp's samples
+        if (lane == 0 && n0 + j > 0 && j <= left) cp_async8(&S.halo[warp][0], h + j - 1);
+        if (lane == 31 && j + kWarpSamples < left)
+            cp_async8(&S.halo[warp][1], h + j + kWarpSamples);
+    };
+    it.to_row(a, live);
+    prefetch();
+    while (it.more()) {
+    const Geo q = it.q;
+    const int tile = it.tile;
+    const int n0 = tile * kTileSamples;
+    const int left = q.n - n0;               // samples of the row from the tile on
+    const int m = min(kTileSamples, left);   // samples of the tile
+    const int j0 = kPerThread * tid;
     cp_async_wait_all();
     __syncwarp();
-    int32_t* x = sx + lane * kSlab;
-    double* y = sy + lane * kSlab;
-    unsigned slow_i = 0u;
-    for (int i = 0; i + 1 < c; ++i) {  // slope i reads knots i, i+1, then replaces knot i
-        bool slow;
-        const double sl = slope_fast(a, x[i], x[i + 1], y[i], y[i + 1], slow);
-        if (slow) slow_i |= 1u << i;
-        y[i] = sl;
-    }
-    if (__any_sync(0xffffffffu, slow_i != 0u)) {
-        for (int i = 0; i + 1 < c; ++i)
-            if (slow_i >> i & 1u)
-                y[i] = (ky[first + i + 1] - ky[first + i]) / (double)(x[i + 1] - x[i]);
-    }
-    __syncwarp();
-}
-
-// k_chunk_reduce: one thread per separator p of a spline; each warp takes groups of 32
-// separators of one spline (k_group_scan) until all are done.  The thread writes the
-// separator's own row and the end relations of the chunk left of it (identity for an empty
-// chunk).  Each warp first
-// copies the knots of its 32 chunks -- a few contiguous runs, one per tile touched -- with
-// coalesced loads into per-lane slabs of shared memory (stride 17: no bank conflicts when
-// every lane reads the same slab position), replaces the knot values by the segment slopes,
-// then every lane sweeps its own slab.
-__global__ void __launch_bounds__(kReduceWarps * 32)
-k_chunk_reduce(SiftArgs a) {
-    __shared__ int32_t slab_x[kReduceWarps][32 * kSlab];
-    __shared__ double slab_y[kReduceWarps][32 * kSlab];
-    __shared__ unsigned short slab_tab[kReduceWarps][32 * kSlab];
-    __shared__ long long slab_gs[kReduceWarps][32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ra = active_rows(a);
-    const int groups = a.gsum[2 * ra];
-    for (int gw = blockIdx.x * kReduceWarps + warp; gw < groups;
-         gw += gridDim.x * kReduceWarps) {  // warp-uniform
-    const int vs = group_spline(a, gw, 2 * ra);
-    int e;
-    const Geo q = spline_geo(a, vs, ra, e);
-    const int se = spline_id(a, e, q);
-    const int P = a.pcount[se];
-    const int p0 = (gw - __ldg(a.gsum + vs)) * 32;
-    const int p = p0 + lane;
-    const bool live = p < P;
-    const ChunkLane ch = locate_chunk(a, e, q, live ? p : P - 1);
-    const int K = a.kcount[se];
-    const int32_t* kx = e == 0 ? a.kx_max : a.kx_min;
-    const double* ky = e == 0 ? a.ky_max : a.ky_min;
-    const int js = ch.js, len = ch.len;
-    const size_t tb = ch.tb;
-    int32_t* sx = slab_x[warp];
-    double* sy = slab_y[warp];
-    stage_slabs(a, kx, ky, (live && len > 0) ? len + 2 : 0, tb + ch.jb, sx, sy, lane,
-                slab_tab[warp], slab_gs[warp]);
-
-    // separator row; its neighbours may lie in other tiles.  Computed by every lane (lanes past
-    // the last separator repeat the last one) so that the slopes' votes see the whole warp.
-    const bool ident = ch.off0 + js == 0 || ch.off0 + js == K - 1;
-    const long long* nb = a.nbr + tix(a, e, q, ch.t) * 2;
-    size_t im = js > 0 ? tb + js - 1 : (size_t)nb[0];
-    size_t ip = js < ch.cnt - 1 ? tb + js + 1 : (size_t)nb[1];
-    if (ident) im = ip = tb + js;  // end knots: identity row, no neighbours needed
-    const int32_t xm = kx[im], xs = kx[tb + js], xp = kx[ip];
-    const double ym = ky[im], ys = ky[tb + js], yp = ky[ip];
-    const double sm = slope_warp(a, xm, xs, ym, ys, !ident);
-    const double sp = slope_warp(a, xs, xp, ys, yp, !ident);
-    if (live) {
-    const Row sr = ident ? identity_row() : spline_row(xm, xs, xp, sm, sp);
-
-    const size_t o = rec_base(a, e, q) + p;
-    double* rc = a.rec;
-    const size_t pl = a.rec_plane;
-    rc[6 * pl + o] = sr.l;
-    rc[7 * pl + o] = sr.m;
-    rc[8 * pl + o] = sr.u;
-    rc[9 * pl + o] = sr.r;
-
-    ChunkEnds ce;
-    if (len > 0) {
-        ce = chunk_ends_slab(sx + lane * kSlab, sy + lane * kSlab, len);
-    } else {
-        ce.ga = 0.0; ce.aa = 0.0; ce.ba = 1.0;
-        ce.gb = 0.0; ce.ab = 1.0; ce.bb = 0.0;
-    }
-    rc[0 * pl + o] = ce.ga;
-    rc[1 * pl + o] = ce.aa;
-    rc[2 * pl + o] = ce.ba;
-    rc[3 * pl + o] = ce.gb;
-    rc[4 * pl + o] = ce.ab;
-    rc[5 * pl + o] = ce.bb;
-    }
-    __syncwarp();  // the slabs are reused by the warp's next group
-    }
-}
-
-// chunk_interior on a slab: row k (k = 0..len-1) is slab knot k+1; the spline values of slab
-// knots 1..len are written to cv[1..len], cpw[1..len] holds the Thomas factors meanwhile.  The
-// same operations in the same order as chunk_interior<true>.
-__device__ __forceinline__ void chunk_interior_slab(int len, const int32_t* x, const double* s,
-                                                    double xl, double xr, double* cpw,
-                                                    double* cv) {
-    double cp = 0.0, gp = 0.0;
-    for (int k = 0; k < len; ++k) {
-        const Row w = spline_row(x[k], x[k + 1], x[k + 2], s[k], s[k + 1]);
-        double ri = w.r;
-        if (k == 0) ri = fma(-w.l, xl, ri);
-        if (k == len - 1) ri = fma(-w.u, xr, ri);
-        double iw;
-        if (k == 0) {
-            iw = pivot_inv(w.m);
-            gp = ri * iw;
-        } else {
-            iw = pivot_inv(fma(-w.l, cp, w.m));
-            gp = fma(-w.l, gp, ri) * iw;
+    unsigned b0, b1;
+    {
+        double h[kPerThread + 1];
+        unstage_tile(h, S.stage, m, tid);
+        double nb = 0.0;
+        if (lane == 0) nb = S.halo[warp][0];
+        if (lane == 31) nb = S.halo[warp][1];
+        h[kPerThread] = __shfl_down_sync(0xffffffffu, h[0], 1);
+        if (lane == 31) h[kPerThread] = nb;
+        unsigned rise = 0u, fall = 0u;  // bit i: h[i] < h[i+1], h[i] > h[i+1]
+#pragma unroll
+        for (int i = 0; i < kPerThread; ++i) {
+            if (h[i] < h[i + 1]) rise |= 1u << i;
+            if (h[i] > h[i + 1]) fall |= 1u << i;
         }
-        cp = w.u * iw;
-        cpw[k + 1] = cp;
-        cv[k + 1] = gp;
+        unsigned before = (rise >> (kPerThread - 1)) | (fall >> (kPerThread - 1)) << 1;
+        before = __shfl_up_sync(0xffffffffu, before, 1);
+        if (lane == 0) before = (nb < h[0] ? 1u : 0u) | (nb > h[0] ? 2u : 0u);
+        b0 = ((rise << 1) | (before & 1u)) & fall;
+        b1 = ((fall << 1) | (before >> 1)) & rise;
     }
-    double xv = gp;
-    for (int k = len - 2; k >= 0; --k) {
-        xv = fma(-cpw[k + 1], xv, cv[k + 1]);
-        cv[k + 1] = xv;
+    b0 &= (1u << kPerThread) - 1u;
+    b1 &= (1u << kPerThread) - 1u;
+    // both end samples of the row are knots of both envelopes; none past the row
+    if (n0 + j0 == 0) {
+        b0 |= 1u;
+        b1 |= 1u;
     }
-}
-
-// k_segments: the spline coefficients of every segment (spline_coefficients), one thread per
-// separator p, warps taking groups of 32 separators as in k_chunk_reduce.  The lane's chunk spans knots jb..js: their spline values
-// are the separator values X[p-1], X[p] at the ends and the chunk interior between, and the
-// lane writes b, c, d of the segments starting at knots jb..js-1 at those knots' slots.  The
-// lane of the empty chunk left of a tile's first knot writes the segment that crosses into
-// the tile (from the last knot of the previous non-empty tile).
-__global__ void __launch_bounds__(kSegWarps * 32)
-k_segments(SiftArgs a) {
-    __shared__ __align__(16) int32_t slab_x[kSegWarps][32 * kSlab];  // later: copy-out table
-    __shared__ double slab_s[kSegWarps][32 * kSlab];  // knot values -> slopes -> b
-    __shared__ double slab_c[kSegWarps][32 * kSlab];  // spline values
-    __shared__ double slab_d[kSegWarps][32 * kSlab];  // Thomas factors -> d
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ra = active_rows(a);
-    const int groups = a.gsum[2 * ra];
-    for (int gw = blockIdx.x * kSegWarps + warp; gw < groups;
-         gw += gridDim.x * kSegWarps) {  // warp-uniform
-    const int vs = group_spline(a, gw, 2 * ra);
-    int e;
-    const Geo q = spline_geo(a, vs, ra, e);
-    const int se = spline_id(a, e, q);
-    const int P = a.pcount[se];
-    const int p0 = (gw - __ldg(a.gsum + vs)) * 32;
-    const int p = p0 + lane;
-    const bool live = p < P;
-    const ChunkLane ch = locate_chunk(a, e, q, live ? p : P - 1);
-    const int32_t* kx = e == 0 ? a.kx_max : a.kx_min;
-    const double* ky = e == 0 ? a.ky_max : a.ky_min;
-    const double* X = a.xsep + rec_base(a, e, q);
-    const int c = (live && ch.k > 0) ? ch.js - ch.jb + 1 : 0;  // slab knots (>= 2 if any)
-    int32_t* sx = slab_x[warp];
-    double* ss = slab_s[warp];
-    // the Thomas-factor and spline-value slabs are free until the interior solve: they hold
-    // the staging's position table meanwhile
-    stage_slabs(a, kx, ky, c, ch.tb + ch.jb, sx, ss, lane,
-                reinterpret_cast<unsigned short*>(slab_d[warp]),
-                reinterpret_cast<long long*>(slab_c[warp]));
-    const int32_t* x = sx + lane * kSlab;
-    double* s = ss + lane * kSlab;
-    double* cv = slab_c[warp] + lane * kSlab;
-    double* dv = slab_d[warp] + lane * kSlab;
-    if (c > 0) {
-        const double xl = X[p - 1], xr = X[p];
-        cv[0] = xl;
-        cv[c - 1] = xr;
-        if (ch.len > 0) chunk_interior_slab(ch.len, x, s, xl, xr, dv, cv);
+    const int e1 = left - 1 - j0;  // bit of sample n-1
+    if (e1 < kPerThread) {
+        const unsigned in = e1 > 0 ? (1u << e1) - 1u : 0u, end = e1 >= 0 ? 1u << e1 : 0u;
+        b0 = (b0 & in) | end;
+        b1 = (b1 & in) | end;
     }
-    // coefficients of slab segments i = 0..c-2 (loop trip count uniform over the warp)
-    // (segments whose quotients need the divisions are marked and redone after the loop, their
-    // slope recomputed from the knots in global memory: s[i] then holds b)
-    unsigned slow_seg = 0u;
-    for (int i = 0; i < kChunk; ++i) {
-        if (i < c - 1) {
-            double b, d;
-            bool slow;
-            seg_coeffs_fast(a, x[i], x[i + 1], s[i], cv[i], cv[i + 1], b, d, slow);
-            if (slow) slow_seg |= 1u << i;
-            s[i] = b;
-            dv[i] = d;
-        }
+    reinterpret_cast<TileBits*>(a.bitmap + tix(a, 0, q, tile) * kWords)[tid] = (TileBits)b0;
+    reinterpret_cast<TileBits*>(a.bitmap + tix(a, 1, q, tile) * kWords)[tid] = (TileBits)b1;
+    // knots before the thread (both envelopes in one word): the warp's scan, and the other warps'
+    // totals; k_tile_sift takes the warps' prefixes from the tile's TileScan
+    const int own = __popc(b0) | __popc(b1) << 16;
+    const int incl = warp_scan(own, lane);
+    if (lane == 31) s_w[warp] = incl;
+    __syncthreads();
+    int wb = 0, tot = 0;
+#pragma unroll
+    for (int i = 0; i < kTileWarps; ++i) {
+        if (i < warp) wb += s_w[i];
+        tot += s_w[i];
     }
-    if (__any_sync(0xffffffffu, slow_seg != 0u)) {
-        for (int i = 0; i < kChunk; ++i) {
-            if (slow_seg >> i & 1u) {
-                const size_t src = ch.tb + ch.jb + i;
-                const double slope = (ky[src + 1] - ky[src]) / (double)(x[i + 1] - x[i]);
-                seg_coeffs_div(x[i], x[i + 1], slope, cv[i], cv[i + 1], s[i], dv[i]);
+    if (lane == 0) {
+        TileScan& sc = a.scan[q.tile0 + tile];
+        sc.before[warp] = wb;
+        if (warp == 0) sc.total = tot;
+    }
+    const int c0 = tot & 0xffff, c1 = tot >> 16;
+    {
+        const int ex = wb + incl - own;
+        int p0 = ex & 0xffff, p1 = ex >> 16;
+        const unsigned any = __reduce_or_sync(0xffffffffu, b0 | b1);
+#pragma unroll
+        for (int i0 = 0; i0 < kPerThread; i0 += 4) {
+            if (!(any >> i0 & 15u)) continue;  // no knots at these samples in the whole warp
+#pragma unroll
+            for (int i = i0; i < i0 + 4; ++i) {
+                if (b0 >> i & 1u) S.x[0][kq(p0++)] = (short)(j0 + i);
+                if (b1 >> i & 1u) S.x[1][kq(p1++)] = (short)(j0 + i);
             }
         }
     }
-    // the segment crossing into the tile: last knot of the previous non-empty tile -> local 0
+    __syncthreads();
+    // End rule (setBoundaryMax/Min): applied here when the tile's own knots decide it (six or
+    // more), else by k_spline_solve from the knots of several tiles.
+    const bool first = tile == 0, last = tile == q.ntiles - 1;
+    if (first || last) {
+        if (tid < 64 && lane < 2) {
+            const int e = tid >> 5, c = e ? c1 : c0, side = lane;
+            const int sp = spline_id(a, e, q);
+            const short* x = S.x[e];
+            auto y = [&](int i) { return staged(S.stage, x[kq(i)]); };
+            if (side == 0 ? first : last) {
+                double v0 = side == 0 ? y(0) : y(c - 1);
+                if (c >= 6) {
+                    v0 = side == 0
+                             ? boundary_left(e, x[0], x[1], x[2], y(0), y(1), y(2))
+                             : boundary_right(e, x[kq(c - 3)], x[kq(c - 2)], x[kq(c - 1)],
+                                              y(c - 3), y(c - 2), y(c - 1));
+                } else {
+                    for (int i = 0; i < c; ++i) {
+                        a.end_x[(size_t)(2 * sp + side) * kEndKnots + i] = n0 + x[kq(i)];
+                        a.end_y[(size_t)(2 * sp + side) * kEndKnots + i] = y(i);
+                    }
+                }
+                a.yend[2 * sp + side] = S.yend[e][side] = v0;
+            }
+        }
+        __syncthreads();
+    }
     {
-        const bool act = live && ch.k == 0 && ch.off0 > 0;
-        const long long* nb = a.nbr + tix(a, e, q, ch.t) * 2;
-        const size_t im = act ? (size_t)nb[0] : ch.tb;
-        const int32_t x0 = kx[im], x1 = kx[ch.tb];
-        const double y0 = ky[im], y1 = ky[ch.tb];
-        const double c0 = act ? X[p - 1] : 0.0, c1 = act ? X[p] : 0.0;
-        const double sl = slope_warp(a, x0, x1, y0, y1, act);
-        double b, d;
-        seg_coeffs_warp(a, x0, x1, sl, c0, c1, b, d, act);
-        if (act) {
-            double2* rec = reinterpret_cast<double2*>(a.seg[e] + 4 * im);
-            rec[0] = make_double2(y0, b);
-            rec[1] = make_double2(c0, d);
+        constexpr int kHalf = kTileThreads / 2;  // threads per envelope
+        const int e = tid / kHalf;
+        const int c = e ? c1 : c0;
+        const short* x = S.x[e];
+        // value of knot i (at padded position p)
+        auto y = [&](int i, int p) {
+            double v = staged(S.stage, x[p]);
+            if (first && i == 0) v = S.yend[e][0];
+            if (last && i == c - 1) v = S.yend[e][1];
+            return v;
+        };
+        // 16 knots on, the padded positions advance by 17; the segments at the row's ends take
+        // the end values
+        for (int i = tid % kHalf, p0 = kq(i), p1 = kq(i + 1); i + 1 < c;
+             i += kHalf, p0 += kq(kHalf), p1 += kq(kHalf)) {
+            const int x0 = x[p0], x1 = x[p1];
+            S.s[e][p0] = div_int(staged(S.stage, x1) - staged(S.stage, x0), (double)(x1 - x0));
+        }
+        for (int side = 0; side < 2; ++side) {
+            const int i = side == 0 ? 0 : c - 2;  // written by the same thread above
+            if ((side == 0 ? first : last) && c > 1 && tid % kHalf == i % kHalf)
+                S.s[e][kq(i)] = div_int(y(i + 1, kq(i + 1)) - y(i, kq(i)),
+                                        (double)(x[kq(i + 1)] - x[kq(i)]));
+        }
+        if (tid % kHalf == kHalf - 1) {
+            if (c > 0) {
+                TileHdr& hd = a.hdr[tix(a, e, q, tile)];
+                const int i1 = c > 1 ? 1 : 0, pb = kq(c - 1), ia = c > 1 ? c - 2 : 0, pa = kq(ia);
+                hd.x0 = n0 + x[0];
+                hd.x1 = n0 + x[i1];
+                hd.xa = n0 + x[pa];
+                hd.xb = n0 + x[pb];
+                hd.y0 = y(0, 0);
+                hd.y1 = y(i1, i1);
+                hd.ya = y(ia, pa);
+                hd.yb = y(c - 1, pb);
+            }
+            a.tile_cnt[tix(a, e, q, tile)] = c;
         }
     }
-    // copy-out of the slab segments, coalesced: lane l's segments i = 0..c-2 -> the records
-    // {y, b, c, d} of slots tb+jb+i.  The knot-position slab is free now and holds the
-    // (lane, position) table of the m = c-1 segments per lane.
-    __syncwarp();
-    const int m = c > 0 ? c - 1 : 0;
-    int incl = m;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
+    __syncthreads();
+    // the samples are done with: the next tile's land during the sweeps
+    it.next(a);
+    it.to_row(a, live);
+    prefetch();
+    int e, k;
+    const bool act = sweep_lane(tid, tile_seps(c0), tile_seps(c1), e, k);
+    const int c = e ? c1 : c0;
+    const int js = min(k * kChunk, c - 1);  // the separator's knot
+    ChunkEnds ce;
+    if (act) {
+        const int jb = (k - 1) * kChunk;
+        const int len = js - jb - 1;
+        if (len > 0) {
+            ce = chunk_ends_knots(S.x[e] + kq(jb), S.s[e] + kq(jb), len);
+        } else {
+            ce.ga = 0.0; ce.aa = 0.0; ce.ba = 1.0;
+            ce.gb = 0.0; ce.ab = 1.0; ce.bb = 0.0;
+        }
+        S.ex[e][0][k] = ce.ga;
+        S.ex[e][1][k] = ce.aa;
+        S.ex[e][2][k] = ce.ba;
     }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    unsigned short* tab = reinterpret_cast<unsigned short*>(slab_x[warp]);
-    long long* gs = reinterpret_cast<long long*>(slab_x[warp] + 16 * kSlab);  // after tab
-    for (int i = 0; i < m; ++i) tab[incl - m + i] = (unsigned short)((lane << 5) | i);
-    gs[lane] = (long long)(ch.tb + ch.jb);
-    __syncwarp();
-    double* out = a.seg[e];
-    for (int f = lane; f < total; f += 32) {
-        const unsigned t = tab[f];
-        const int ow = (int)(t >> 5), i = (int)(t & 31u);
-        const size_t dst = (size_t)gs[ow] + i;
-        const int q = ow * kSlab + i;
-        double2* rec = reinterpret_cast<double2*>(out + 4 * dst);
-        rec[0] = make_double2(__ldg(ky + dst), ss[q]);
-        rec[1] = make_double2(slab_c[warp][q], slab_d[warp][q]);
+    __syncthreads();
+    if (act) {
+        TileHdr& hd = a.hdr[tix(a, e, q, tile)];
+        if (k == 1) {
+            hd.ga = ce.ga;
+            hd.aa = ce.aa;
+            hd.ba = ce.ba;
+        }
+        if (js == c - 1) {
+            hd.gb = ce.gb;
+            hd.ab = ce.ab;
+            hd.bb = ce.bb;
+        } else {
+            const int im = kq(js - 1), i0 = kq(js), ip = kq(js + 1);
+            const Row sr = spline_row(S.x[e][im], S.x[e][i0], S.x[e][ip], S.s[e][im], S.s[e][i0]);
+            const Row o = reduced_row(sr, ce.gb, ce.ab, ce.bb, S.ex[e][0][k + 1],
+                                      S.ex[e][1][k + 1], S.ex[e][2][k + 1]);
+            const double w[4] = {o.l, o.m, o.u, o.r};
+            store4(a.rows + (tix(a, e, q, tile) * kRowSlots + k) * 4, w);
+        }
     }
-    __syncwarp();  // the slabs are reused by the warp's next group
+    // (the next tile's first barrier separates these reads of s, x and ex from its writes)
+    }
+}
+
+// Compacted copy of the knots of envelope e (stage-level entry point, one channel): row r's
+// knots to kx/ky[r*n + i], from the bitmaps, the samples and the end values.
+__global__ void __launch_bounds__(kThreads)
+k_gather_knots(SiftArgs a, int e, int32_t* kx, double* ky) {
+    __shared__ int2 s_wo[kWords];
+    __shared__ int s_before;
+    const int tile = blockIdx.x;
+    const Geo q = geo(a, 0, blockIdx.y);
+    if (threadIdx.x == 0) s_before = 0;
+    __syncthreads();
+    int before = 0;
+    for (int t = threadIdx.x; t < tile; t += kThreads) before += a.tile_cnt[tix(a, e, q, t)];
+    if (before) atomicAdd(&s_before, before);
+    const unsigned* bm = a.bitmap + tix(a, e, q, tile) * kWords;
+    if (threadIdx.x < kWords) {
+        int w = 0;
+        for (int i = 0; i < (int)threadIdx.x; ++i) w += __popc(bm[i]);
+        s_wo[threadIdx.x] = make_int2((int)bm[threadIdx.x], w);
+    }
+    __syncthreads();
+    const int sp = spline_id(a, e, q);
+    const double* h = a.h[a.par[q.g]] + q.base;
+    for (int j = threadIdx.x; j < kTileSamples; j += kThreads) {
+        const int2 wo = s_wo[j >> 5];
+        if (!((unsigned)wo.x >> (j & 31) & 1u)) continue;
+        const size_t o =
+            (size_t)q.r * q.n + s_before + wo.y + __popc((unsigned)wo.x & ((1u << (j & 31)) - 1u));
+        const int s = tile * kTileSamples + j;
+        kx[o] = s;
+        ky[o] = s == 0 ? a.yend[2 * sp] : (s == q.n - 1 ? a.yend[2 * sp + 1] : h[s]);
     }
 }
 
 // =======================================================================================
-// k_reduced_solve: levels >= 2 of the partitioned solve (the system on the separators of
-// the tile-aligned first level), one CTA per spline system.
+// canonical partitioned solve of explicit systems
 // =======================================================================================
 namespace {
 
@@ -1112,41 +893,50 @@ struct GlobalRowFn {
 };
 
 // In-CTA canonical partitioned solve of an explicit system stored at sys (4 planes of
-// `plane` doubles: l, m, u, r), solution to x.  ws: workspace for the deeper levels
-// (<= 0.75*n + 16 doubles).  All threads of the CTA must call it.
+// `plane` doubles: l, m, u, r; the u plane is overwritten), solution to x.  ws: workspace for the
+// deeper levels (<= 0.75*n + 16 doubles).  All threads of the CTA must call it.
+struct PartLevel {
+    double *L, *x;  // rows (4 planes of pl doubles), solution
+    int n, pl;
+};
+// level k of a system of n rows: its size, and where its rows and solution start in the workspace
+// (all levels' rows, then all levels' solutions, then the end relations)
+__device__ __forceinline__ PartLevel part_level(int k, int depth, int n, double* sys, int plane,
+                                                double* x, double* ws) {
+    if (k == 0) return PartLevel{sys, x, n, plane};
+    int rows = 0, sols = 0, size = n, mine = 0, mrow = 0, msol = 0;
+    for (int i = 1; i <= depth; ++i) {
+        size = (size - 1) / kChunk;
+        if (i == k) {
+            mine = size;
+            mrow = rows;
+            msol = sols;
+        }
+        rows += 4 * size;
+        sols += size;
+    }
+    return PartLevel{ws + mrow, ws + rows + msol, mine, mine};
+}
+
 template <class Pivot>
-__device__ void cta_partitioned(int n, const double* sys, int plane, double* x, double* ws) {
-    int sizes[8];
-    int depth = 0;
-    sizes[0] = n;
-    while (sizes[depth] > kChunk && depth < 7) {
-        sizes[depth + 1] = (sizes[depth] - 1) / kChunk;
-        ++depth;
+__device__ void cta_partitioned(int n, double* sys, int plane, double* x, double* ws) {
+    int depth = 0, all = 0;  // all: rows and solutions of the levels below the first
+    for (int size = n; size > kChunk && depth < 7; ++depth) {
+        size = (size - 1) / kChunk;
+        all += 5 * size;
     }
-    const double* lv[8];
-    double* xv[8];
-    int off = 0;
-    lv[0] = sys;
-    for (int k = 1; k <= depth; ++k) {
-        lv[k] = ws + off;
-        off += 4 * sizes[k];
-    }
-    xv[0] = x;
-    for (int k = 1; k <= depth; ++k) {
-        xv[k] = ws + off;
-        off += sizes[k];
-    }
-    double* ends = ws + off;  // 6 * (chunks of the widest level)
+    double* ends = ws + all;  // 6 * (chunks of the widest level)
+#pragma unroll 1
     for (int k = 0; k < depth; ++k) {
-        const int nk = sizes[k];
-        const int P = sizes[k + 1];
-        const int pl = (k == 0) ? plane : nk;
-        const double* L = lv[k];
+        const PartLevel v = part_level(k, depth, n, sys, plane, x, ws);
+        const PartLevel o = part_level(k + 1, depth, n, sys, plane, x, ws);
+        const int P = o.n, pl = v.pl;
+        const double* L = v.L;
         for (int q = threadIdx.x; q <= P; q += blockDim.x) {
             const int first = q * kChunk;
-            const int len = (q < P) ? kChunk - 1 : nk - first;
+            const int len = (q < P) ? kChunk - 1 : v.n - first;
             GlobalRowFn fn{L, L + pl, L + 2 * pl, L + 3 * pl, first};
-            const ChunkEnds ce = chunk_ends<Pivot>(len, fn);
+            const ChunkEnds ce = chunk_ends<Pivot>(len, fn, Slots{v.x + first});
             ends[6 * q + 0] = ce.ga;
             ends[6 * q + 1] = ce.aa;
             ends[6 * q + 2] = ce.ba;
@@ -1155,7 +945,7 @@ __device__ void cta_partitioned(int n, const double* sys, int plane, double* x, 
             ends[6 * q + 5] = ce.bb;
         }
         __syncthreads();
-        double* R = const_cast<double*>(lv[k + 1]);
+        double* R = o.L;
         for (int p = threadIdx.x; p < P; p += blockDim.x) {
             const int s = p * kChunk + kChunk - 1;
             Row sr;
@@ -1163,39 +953,36 @@ __device__ void cta_partitioned(int n, const double* sys, int plane, double* x, 
             sr.m = L[pl + s];
             sr.u = L[2 * pl + s];
             sr.r = L[3 * pl + s];
-            const Row o = reduced_row(sr, ends[6 * p + 3], ends[6 * p + 4], ends[6 * p + 5],
+            const Row w = reduced_row(sr, ends[6 * p + 3], ends[6 * p + 4], ends[6 * p + 5],
                                       ends[6 * (p + 1) + 0], ends[6 * (p + 1) + 1],
                                       ends[6 * (p + 1) + 2]);
-            R[p] = o.l;
-            R[P + p] = o.m;
-            R[2 * P + p] = o.u;
-            R[3 * P + p] = o.r;
+            R[p] = w.l;
+            R[P + p] = w.m;
+            R[2 * P + p] = w.u;
+            R[3 * P + p] = w.r;
         }
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        const int nb = sizes[depth];
-        const int pl = (depth == 0) ? plane : nb;
-        const double* L = lv[depth];
-        GlobalRowFn fn{L, L + pl, L + 2 * pl, L + 3 * pl, 0};
-        thomas_small<Pivot>(nb, fn, xv[depth], 1);
+        const PartLevel v = part_level(depth, depth, n, sys, plane, x, ws);
+        GlobalRowFn fn{v.L, v.L + v.pl, v.L + 2 * v.pl, v.L + 3 * v.pl, 0};
+        thomas_rolled<Pivot>(v.n, fn, Slots{v.x}, Slots{v.L + 2 * v.pl});
     }
     __syncthreads();
+#pragma unroll 1
     for (int k = depth - 1; k >= 0; --k) {
-        const int nk = sizes[k];
-        const int P = sizes[k + 1];
-        const int pl = (k == 0) ? plane : nk;
-        const double* L = lv[k];
-        const double* Xs = xv[k + 1];
-        double* xo = xv[k];
+        const PartLevel v = part_level(k, depth, n, sys, plane, x, ws);
+        const PartLevel o = part_level(k + 1, depth, n, sys, plane, x, ws);
+        const int P = o.n, pl = v.pl;
+        double* L = v.L;
         for (int q = threadIdx.x; q <= P; q += blockDim.x) {
             const int first = q * kChunk;
-            const int len = (q < P) ? kChunk - 1 : nk - first;
+            const int len = (q < P) ? kChunk - 1 : v.n - first;
             GlobalRowFn fn{L, L + pl, L + 2 * pl, L + 3 * pl, first};
-            const double xl = (q > 0) ? Xs[q - 1] : 0.0;
-            const double xr = (q < P) ? Xs[q] : 0.0;
-            chunk_interior<true, Pivot>(len, fn, xl, xr, xo + first, 1);
-            if (q < P) xo[first + kChunk - 1] = xr;
+            const double xl = (q > 0) ? o.x[q - 1] : 0.0;
+            const double xr = (q < P) ? o.x[q] : 0.0;
+            chunk_interior_iw(len, fn, xl, xr, Slots{v.x + first}, Slots{L + 2 * pl + first});
+            if (q < P) v.x[first + kChunk - 1] = xr;
         }
         __syncthreads();
     }
@@ -1203,10 +990,10 @@ __device__ void cta_partitioned(int n, const double* sys, int plane, double* x, 
 
 }  // namespace
 
-__device__ void cta_tridiag(int n, const double* sys, int plane, double* x, double* ws) {
+__device__ void cta_tridiag(int n, double* sys, int plane, double* x, double* ws) {
     cta_partitioned<AnyPivot>(n, sys, plane, x, ws);
 }
-__device__ void cta_spline_tridiag(int n, const double* sys, int plane, double* x, double* ws) {
+__device__ void cta_spline_tridiag(int n, double* sys, int plane, double* x, double* ws) {
     cta_partitioned<SplinePivot>(n, sys, plane, x, ws);
 }
 
@@ -1295,8 +1082,9 @@ k_psolve_ends(int k, const int* nrows, const double* sys, int plane, double* ws,
     const int len = (q < P) ? kChunk - 1 : nk - first;
     const ChunkEnds ce =
         (k == 0 && kx) ? chunk_ends(len, KnotSysRows{kx + (size_t)plane * sidx, L + 3 * pl, n,
-                                                     first})
-                       : chunk_ends(len, GlobalRowFn{L, L + pl, L + 2 * pl, L + 3 * pl, first});
+                                                     first}, NoIw())
+                       : chunk_ends(len, GlobalRowFn{L, L + pl, L + 2 * pl, L + 3 * pl, first},
+                                    NoIw());
     double* ends = w + v.ends;
     ends[6 * q + 0] = ce.ga;
     ends[6 * q + 1] = ce.aa;
@@ -1422,19 +1210,28 @@ cudaError_t psolve_launch(int nsys, int max_rows, const int* nrows, const double
 
 namespace {
 
-constexpr int kRedPass = kRedThreads * kChunk;                // level-2 rows per pass
-constexpr int kRedSlots = kRedPass + (kRedPass >> 4) + 1;    // padded
+constexpr int kSolvePass = kSolveChunks * kChunk;                 // level-2 rows per pass
+constexpr int kSolveSlots = kSolvePass + (kSolvePass >> 4) + 1;  // padded
+constexpr int kTabTiles = 256;  // rows of up to this many tiles keep their tables in shared memory
 
 // Level-2 rows staged in shared memory (4 padded planes).
 struct RedStage {
-    double l[kRedSlots], m[kRedSlots], u[kRedSlots], r[kRedSlots];
+    double l[kSolveSlots], m[kSolveSlots], u[kSolveSlots], r[kSolveSlots];
+    double x[kSolveSlots];  // reciprocal pivots, then the solution
 };
+struct StageSlots {
+    double* p;
+    int first;
+    __device__ __forceinline__ double& operator()(int k) const { return p[kq(first + k)]; }
+};
+
+static_assert(sizeof(RedStage) == kSolveStage, "the host sizes the workspace after it");
 
 struct StageRowFn {
     const RedStage* st;
     int first;  // local row of chunk row 0
     __device__ __forceinline__ Row operator()(int k) const {
-        const int j = pad17(first + k);
+        const int j = kq(first + k);
         Row w;
         w.l = st->l[j];
         w.m = st->m[j];
@@ -1444,41 +1241,46 @@ struct StageRowFn {
     }
 };
 
-// Level-2 row p (separator p of the level-1 partition) from the chunk records; chunk p is the
-// chunk left of separator p, chunk p+1 the one right of it (chunk P, after the last knot,
-// is empty: x_{s+1} = x_{s_next}).
-__device__ __forceinline__ Row level2_row(const double* rc, size_t pl, size_t o, int p, int P) {
-    Row sr;
-    sr.l = rc[6 * pl + o + p];
-    sr.m = rc[7 * pl + o + p];
-    sr.u = rc[8 * pl + o + p];
-    sr.r = rc[9 * pl + o + p];
-    double ga = 0.0, aa = 0.0, ba = 1.0;
-    if (p + 1 < P) {
-        ga = rc[0 * pl + o + p + 1];
-        aa = rc[1 * pl + o + p + 1];
-        ba = rc[2 * pl + o + p + 1];
+// Rows of a spline's separator system, in their tiles' slots: separator p is separator
+// p - soff[t] of tile t, the last tile with soff[t] <= p.
+struct SepRows {
+    const double* rows;  // the spline's first tile's slots
+    const int* soff;
+    int ntiles;
+    __device__ __forceinline__ Row operator()(int p) const {
+        int lo = 0, hi = ntiles - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (soff[mid] <= p) lo = mid;
+            else hi = mid - 1;
+        }
+        const double2* s = reinterpret_cast<const double2*>(
+            rows + ((size_t)lo * kRowSlots + (size_t)(p - soff[lo])) * 4);
+        const double2 a = s[0], b = s[1];
+        Row w;
+        w.l = a.x;
+        w.m = a.y;
+        w.u = b.x;
+        w.r = b.y;
+        return w;
     }
-    return reduced_row(sr, rc[3 * pl + o + p], rc[4 * pl + o + p], rc[5 * pl + o + p], ga, aa, ba);
-}
+};
 
-__device__ __forceinline__ void stage_level2(RedStage& st, const double* rc, size_t pl, size_t o,
-                                             int p0,
-                                             int P) {
-    const int rows = min(kRedPass, P - p0);
-    constexpr int kB = 4;  // rows per thread whose record loads are in flight together
-    for (int j0 = threadIdx.x; j0 < rows; j0 += kB * kRedThreads) {
+__device__ __forceinline__ void stage_level2(RedStage& st, const SepRows& src, int p0, int P) {
+    const int rows = min(kSolvePass, P - p0);
+    constexpr int kB = 4;  // rows per thread whose loads are in flight together
+    for (int j0 = threadIdx.x; j0 < rows; j0 += kB * kSolveThreads) {
         Row w[kB];
 #pragma unroll
         for (int t = 0; t < kB; ++t) {
-            const int j = j0 + t * kRedThreads;
-            if (j < rows) w[t] = level2_row(rc, pl, o, p0 + j, P);
+            const int j = j0 + t * kSolveThreads;
+            if (j < rows) w[t] = src(p0 + j);
         }
 #pragma unroll
         for (int t = 0; t < kB; ++t) {
-            const int j = j0 + t * kRedThreads;
+            const int j = j0 + t * kSolveThreads;
             if (j < rows) {
-                const int q = pad17(j);
+                const int q = kq(j);
                 st.l[q] = w[t].l;
                 st.m[q] = w[t].m;
                 st.u[q] = w[t].u;
@@ -1488,50 +1290,47 @@ __device__ __forceinline__ void stage_level2(RedStage& st, const double* rc, siz
     }
 }
 
-}  // namespace
-
-// Dynamic shared memory of k_reduced_solve: the level-2 stage plus a level-3 workspace for up
-// to *qcap level-3 rows (16*Q + 74 doubles for Q rows), within kRedSmemMax.  Splines with more
-// level-3 rows use the global workspace.
-size_t reduced_solve_smem(int* qcap) {
-    const size_t base = sizeof(RedStage);
-    const long avail = (long)(kRedSmemMax - base) / (long)sizeof(double) - 74;
-    *qcap = avail > 0 ? (int)(avail / 16) : 0;
-    return base + sizeof(double) * (16 * (size_t)*qcap + 74);
-}
-
-namespace {
-
-// The reduced solve of one spline system (level-2 size P, records at rc + o of planes pl,
-// separator values to X, global level-3 workspace wg).  Every thread of the CTA calls it.
-__device__ __forceinline__ void reduced_solve_one(unsigned char* dyn_smem, const double* rc,
-                                               size_t pl, size_t o, int P, double* X,
-                                               int red_qcap, double* wg) {
+// The separator system of one spline (P rows), solution to X.  wg: global workspace, used when
+// the level-3 system does not fit the wcap doubles of shared memory after the stage.  Every
+// thread of the CTA calls it.
+__device__ __forceinline__ void solve_separators(unsigned char* dyn_smem, int wcap,
+                                                 const SepRows& src, int P, double* X,
+                                                 double* wg) {
     RedStage& st = *reinterpret_cast<RedStage*>(dyn_smem);
     if (P <= kChunk) {
-        stage_level2(st, rc, pl, o, 0, P);
+        stage_level2(st, src, 0, P);
         __syncthreads();
-        if (threadIdx.x == 0) thomas_small(P, StageRowFn{&st, 0}, X, 1);
+        if (threadIdx.x == 0)
+            thomas_rolled(P, StageRowFn{&st, 0}, Slots{X}, StageSlots{st.u, 0});
         return;
     }
     const int Q = (P - 1) / kChunk;  // level-3 size
-    // level-3 workspace: shared memory after the stage, or the global reduced workspace
-    double* w3 = Q <= red_qcap ? reinterpret_cast<double*>(dyn_smem + sizeof(RedStage)) : wg;
-    double* ends = w3;                       // 6 * (Q+1)
-    double* sep = ends + 6 * (size_t)(Q + 1);  // 4 * (Q+1)
-    double* L3 = sep + 4 * (size_t)(Q + 1);    // 4 * Q
-    double* x3 = L3 + 4 * (size_t)Q;           // Q
-    double* ws3 = x3 + Q;                     // deeper levels
-    for (int p0 = 0; p0 < P; p0 += kRedPass) {
+    const bool one = P <= kSolvePass;
+    // End relations and separator rows outlive the passes over the stage.  One pass: the level-3
+    // workspace follows the stage.  More: the stage is filled again for the second sweep, so its
+    // x plane (the reciprocals would not last) holds them with what follows the stage, and the
+    // rest of the level-3 workspace takes the staged rows' place in between.
+    const bool fits = one ? 16 * (size_t)Q + 74 <= (size_t)wcap
+                          : 10 * (size_t)(Q + 1) <= (size_t)wcap + kSolveSlots &&
+                                6 * (size_t)Q + 64 <= 4 * (size_t)kSolveSlots;
+    double* ends = !fits ? wg
+                         : (one ? reinterpret_cast<double*>(dyn_smem + sizeof(RedStage)) : st.x);
+    double* sep = ends + 6 * (size_t)(Q + 1);
+    double* L3 = (fits && !one) ? reinterpret_cast<double*>(dyn_smem) : sep + 4 * (size_t)(Q + 1);
+    double* x3 = L3 + 4 * (size_t)Q;
+    double* ws3 = x3 + Q;  // deeper levels
+    for (int p0 = 0; p0 < P; p0 += kSolvePass) {
         __syncthreads();
-        stage_level2(st, rc, pl, o, p0, P);
+        stage_level2(st, src, p0, P);
         __syncthreads();
         const int q = p0 / kChunk + threadIdx.x;
-        if (q <= Q) {
+        if (threadIdx.x < kSolveChunks && q <= Q) {
             const int first = q * kChunk;
             const int len = (q < Q) ? kChunk - 1 : P - first;
             const StageRowFn fn{&st, first - p0};
-            const ChunkEnds ce = chunk_ends(len, fn);
+            // one pass: the reciprocals stay in the stage
+            const ChunkEnds ce = one ? chunk_ends(len, fn, StageSlots{st.x, first})
+                                     : chunk_ends(len, fn, NoIw());
             ends[6 * q + 0] = ce.ga;
             ends[6 * q + 1] = ce.aa;
             ends[6 * q + 2] = ce.ba;
@@ -1548,7 +1347,7 @@ __device__ __forceinline__ void reduced_solve_one(unsigned char* dyn_smem, const
         }
     }
     __syncthreads();
-    for (int p = threadIdx.x; p < Q; p += kRedThreads) {
+    for (int p = threadIdx.x; p < Q; p += kSolveThreads) {
         Row s2;
         s2.l = sep[4 * p + 0];
         s2.m = sep[4 * p + 1];
@@ -1564,247 +1363,759 @@ __device__ __forceinline__ void reduced_solve_one(unsigned char* dyn_smem, const
     }
     __syncthreads();
     cta_partitioned<SplinePivot>(Q, L3, Q, x3, ws3);
-    for (int p0 = 0; p0 < P; p0 += kRedPass) {
+    double* xq = x3;
+    if (fits && !one) {  // the stage is filled again: the level-3 solution moves out of it
+        xq = ends;
+        for (int p = threadIdx.x; p < Q; p += kSolveThreads) xq[p] = x3[p];
+    }
+    for (int p0 = 0; p0 < P; p0 += kSolvePass) {
         __syncthreads();
-        if (P > kRedPass) stage_level2(st, rc, pl, o, p0, P);  // else: still staged from pass one
+        if (!one) stage_level2(st, src, p0, P);  // else: still staged from pass one
         __syncthreads();
         const int q = p0 / kChunk + threadIdx.x;
-        if (q <= Q) {
+        if (threadIdx.x < kSolveChunks && q <= Q) {
             const int first = q * kChunk;
             const int len = (q < Q) ? kChunk - 1 : P - first;
-            const double xl = (q > 0) ? x3[q - 1] : 0.0;
-            const double xr = (q < Q) ? x3[q] : 0.0;
-            chunk_interior(len, StageRowFn{&st, first - p0}, xl, xr, X + first, 1);
-            if (q < Q) X[first + kChunk - 1] = xr;
+            const double xl = (q > 0) ? xq[q - 1] : 0.0;
+            const double xr = (q < Q) ? xq[q] : 0.0;
+            const StageRowFn fn{&st, first - p0};
+            const StageSlots fac{st.u, first - p0};
+            if (one) {
+                chunk_interior_iw(len, fn, xl, xr, StageSlots{st.x, first}, fac);
+                if (q < Q) st.x[kq(first + kChunk - 1)] = xr;
+            } else {
+                chunk_interior_rolled(len, fn, xl, xr, StageSlots{st.r, first - p0}, fac);
+                if (q < Q) st.r[kq(first + kChunk - 1 - p0)] = xr;
+            }
+        }
+        __syncthreads();
+        const double* sol = one ? st.x : st.r;
+        for (int j = threadIdx.x; j < min(kSolvePass, P - p0); j += kSolveThreads)
+            X[p0 + j] = sol[kq(j)];
+    }
+}
+
+// The end rule of a spline whose first (side 0) or last (side 1) tile holds fewer than six
+// knots: the three end knots come from the tiles' headers, the tile's chunk is eliminated again
+// with the new end value.  ne: the tiles with knots, in order (NE of them); hd: the spline's
+// headers; cnt: the tiles' knot counts.
+__device__ __noinline__ void end_rule_sparse(const SiftArgs& a, int e, int sp, int side,
+                                             const int* ne, int NE, const int* cnt, TileHdr* hd) {
+    const int te = ne[side == 0 ? 0 : NE - 1];
+    TileHdr& h0 = hd[te];
+    const int c = cnt[te];
+    int x[5];
+    double y[5];
+    for (int i = 0; i < c && i < 5; ++i) {
+        x[i] = a.end_x[(size_t)(2 * sp + side) * kEndKnots + i];
+        y[i] = a.end_y[(size_t)(2 * sp + side) * kEndKnots + i];
+    }
+    int ex[3];
+    double ey[3];  // the three knots from the end inwards
+    int got = 0;
+    for (; got < 3 && got < c; ++got) {
+        const int i = side == 0 ? got : c - 1 - got;
+        ex[got] = x[i];
+        ey[got] = y[i];
+    }
+    for (int r = 1; got < 3 && r < NE; ++r) {
+        const int t = ne[side == 0 ? r : NE - 1 - r];
+        const TileHdr& h = hd[t];
+        ex[got] = side == 0 ? h.x0 : h.xb;
+        ey[got] = side == 0 ? h.y0 : h.yb;
+        ++got;
+        if (got < 3 && cnt[t] > 1) {
+            ex[got] = side == 0 ? h.x1 : h.xa;
+            ey[got] = side == 0 ? h.y1 : h.ya;
+            ++got;
         }
     }
+    const double v = side == 0 ? boundary_left(e, ex[0], ex[1], ex[2], ey[0], ey[1], ey[2])
+                               : boundary_right(e, ex[2], ex[1], ex[0], ey[2], ey[1], ey[0]);
+    a.yend[2 * sp + side] = v;
+    if (side == 0) {
+        h0.y0 = v;
+        if (c == 1) h0.yb = v;
+        if (c == 2) h0.ya = v;
+    } else {
+        h0.yb = v;
+        if (c == 1) h0.y0 = v;
+        if (c == 2) h0.y1 = v;
+    }
+    if (c < 3) return;  // no rows between the tile's separators
+    y[side == 0 ? 0 : c - 1] = v;
+    double s[4];
+    for (int i = 0; i + 1 < c; ++i) s[i] = seg_slope(x[i], x[i + 1], y[i], y[i + 1]);
+    const ChunkEnds ce = chunk_ends_knots(x, s, c - 2);
+    h0.ga = ce.ga;
+    h0.aa = ce.aa;
+    h0.ba = ce.ba;
+    h0.gb = ce.gb;
+    h0.ab = ce.ab;
+    h0.bb = ce.bb;
 }
 
 }  // namespace
 
-// k_reduced_solve: one CTA of kRedThreads per active spline system (maxima splines first,
-// then minima); the grid covers every spline of the engine, CTAs past the active ones exit.
-__global__ void __launch_bounds__(kRedThreads)
-k_reduced_solve(SiftArgs a) {
+// =======================================================================================
+// k_spline_solve: one CTA per spline (envelope, realization): prefix sums over its tiles (knots,
+// separators, tiles with knots), the end rule where one tile could not decide it, the rows of the
+// separators at the tiles' edges, the separator system (levels >= 2 of the canonical partitioned
+// solve), and for every tile the knots just outside it with their spline values.  The system's
+// rows are staged once when they fit a pass (2048 rows).  Latency bound: two CTAs per SM with
+// the level-3 system in shared memory.
+// =======================================================================================
+__global__ void __launch_bounds__(kSolveThreads, 2)
+k_spline_solve(const __grid_constant__ SiftArgs a) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
+    __shared__ int s_tab[3][kTabTiles + 1];
+    __shared__ int s_scan[kSolveThreads / 32], s_k[kSolveThreads / 32], s_m[kSolveThreads / 32];
     const int ra = active_rows(a);
     const int vs = blockIdx.x;
     if (vs >= 2 * ra) return;
     int e;
-    const Geo gq = spline_geo(a, vs, ra, e);
-    const int re = spline_id(a, e, gq);
-    const size_t o = rec_base(a, e, gq);
-    reduced_solve_one(dyn_smem, a.rec, a.rec_plane, o, a.pcount[re], a.xsep + o, a.red_qcap,
-                      a.red + red_base(a, e, gq));
-}
-
-// =======================================================================================
-// k_eval: envelopes + mean envelope + sx statistics over one tile of samples, both envelopes
-// at once.  Thread t handles local samples k*256 + t, so warp accesses to samples and bitmap
-// words are contiguous.  The segment of sample s is (#knots at positions < s) - 1, a popc
-// rank in the tile's knot bitmap: the word of a warp's 32 samples and the knot count before it
-// come by shuffle.  The segment's record {a, b, c, d} (k_segments) and start position are
-// read from its start knot's slot, the previous tile's last knot for the samples before the
-// tile's first knot.
-// =======================================================================================
-template <int kMinBlocks>
-__global__ void __launch_bounds__(kThreads, kMinBlocks)
-k_eval_t(SiftArgs a) {
-    __shared__ int s_red[kThreads / 32];
-    __shared__ int s_any[kThreads / 32];
-    const int total = active_tiles(a);
-    // persistent CTAs: active tiles v, v + gridDim.x, ... (CTA-uniform loop)
-    for (int vt = blockIdx.x; vt < total; vt += gridDim.x) {
-    int tile;
-    const Geo gq = tile_geo(a, vt, tile);
-    const int n = gq.n;
-    const int n0 = tile * kTileSamples;
-    const size_t base = gq.base;
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const unsigned lt = (1u << lane) - 1u;
-    const size_t tb = tile_base(gq.tile0 + tile);
-    // Per envelope: the slot of the knot before the tile, and for k = 0..7 (held by lane k)
-    // this warp's bitmap word k*8 + warp with the count of the tile's knots before it.
-    size_t pv[2];
-    unsigned wk[2];
-    int pk[2];
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        const int off0 = __ldg(a.tile_off + oix(a, e, gq) + tile);
-        pv[e] = off0 > 0 ? (size_t)__ldg(a.nbr + tix(a, e, gq, tile) * 2) : tb;
-        const unsigned* bm = a.bitmap + tix(a, e, gq, tile) * kWords;
-        const unsigned b0 = __ldg(bm + 2 * lane), b1 = __ldg(bm + 2 * lane + 1);
-        const int pair = __popc(b0) + __popc(b1);
-        int incl = pair;
+    const Geo q = spline_geo(a, vs, ra, e);
+    if (a.mark[q.g] == 0) return;  // the row repeats its last iteration (k_tile_sift)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int sp = spline_id(a, e, q);
+    const int ntiles = q.ntiles;
+    const size_t te0 = tix(a, e, q, 0);
+    const int* cnt = a.tile_cnt + te0;
+    TileHdr* hd = a.hdr + te0;
+    double* rows = a.rows + te0 * (size_t)(kRowSlots * 4);
+    const bool small = ntiles <= kTabTiles;
+    const size_t o1 = oix(a, e, q);
+    int* soff = small ? s_tab[0] : a.sep_off + o1;    // separators before each tile
+    int* rank = small ? s_tab[1] : a.tile_rank + o1;  // tiles with knots before each tile
+    int* ne = small ? s_tab[2] : a.tile_list + o1;    // the tiles with knots
+    int P = 0, NE = 0, K = 0, cm = 0;
+    for (int t0 = 0; t0 < ntiles; t0 += kSolveThreads) {
+        const int t = t0 + tid;
+        const int c = t < ntiles ? cnt[t] : 0;
+        const int own = tile_seps(c) | (c > 0 ? 0x10000 : 0);  // both sums stay below 2^16
+        int incl = own;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
+            const int u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
         }
-        // lane k < 8 takes word k*8 + warp from lane (k*8 + warp) / 2
-        const int src = (lane & 7) * 4 + (warp >> 1);
-        const unsigned a0 = __shfl_sync(0xffffffffu, b0, src);
-        const unsigned a1 = __shfl_sync(0xffffffffu, b1, src);
-        const int ex = __shfl_sync(0xffffffffu, incl - pair, src);
-        const bool odd = (warp & 1) != 0;
-        wk[e] = odd ? a1 : a0;
-        pk[e] = ex + (odd ? __popc(a0) : 0);
-    }
-    // envelope e at local sample k*256 + threadIdx.x
-    auto env_at = [&](int e, int k) {
-        const unsigned word = __shfl_sync(0xffffffffu, wk[e], k);
-        const int sl = __shfl_sync(0xffffffffu, pk[e], k) + __popc(word & lt) - 1;
-        const size_t q = sl >= 0 ? tb + (size_t)sl : pv[e];
-        const double2* rp = reinterpret_cast<const double2*>(a.seg[e] + 4 * q);
-        const double2 yb = __ldg(rp), cd = __ldg(rp + 1);
-        const int32_t x = __ldg((e == 0 ? a.kx_max : a.kx_min) + q);
-        const int s = n0 + k * kThreads + threadIdx.x;
-        return seg_eval(yb.x, yb.y, cd.x, cd.y, (double)(s - x));
-    };
-    // averageUppperLower: the mean envelope keeps its previous value unless both envelopes
-    // have more than 3 knots
-    const bool write_mean = a.kcount[gq.g] > 3 && a.kcount[a.nrows + gq.g] > 3;
-    int cnt = 0, any = 0;
-    // sx > t is decided without the division where the products give a margin (sx_bounds);
-    // undecided samples are redone exactly after the loop
-    unsigned undecided = 0u;
-#pragma unroll
-    for (int k = 0; k < kPerThread; ++k) {
-        const int s = n0 + k * kThreads + threadIdx.x;
-        const bool live = s < n;
-        const double u = env_at(0, k);
-        const double v = env_at(1, k);
-        if (live) {
-            if (write_mean) a.menv[base + s] = (u + v) / 2.0;
-            if (a.dbg_upper) {
-                a.dbg_upper[base + s] = u;
-                a.dbg_lower[base + s] = v;
-            }
+        const int kw = __reduce_add_sync(0xffffffffu, c);
+        const int mw = __reduce_max_sync(0xffffffffu, c);
+        if (lane == 31) {
+            s_scan[warp] = incl;
+            s_k[warp] = kw;
+            s_m[warp] = mw;
         }
-        const double p = fabs(u + v), q = fabs(u - v);
-        const bool inr = q > 0x1p-800 && q < 0x1p+800;
-        const bool any_t = p > q * a.sd2_hi, any_f = p < q * a.sd2_lo;
-        const bool cnt_t = p > q * a.sd_hi, cnt_f = p < q * a.sd_lo;
-        any |= (live && inr && any_t) ? 1 : 0;
-        cnt += (live && inr && cnt_t) ? 1 : 0;
-        if (live && !(inr && (any_t || any_f) && (cnt_t || cnt_f))) undecided |= 1u << k;
-    }
-    if (__any_sync(0xffffffffu, undecided != 0u)) {
+        __syncthreads();
+        int before = 0, all = 0;
 #pragma unroll
-        for (int k = 0; k < kPerThread; ++k) {
-            const double u = env_at(0, k);  // every lane: env_at shuffles
-            const double v = env_at(1, k);
-            if (!(undecided >> k & 1u)) continue;
-            const double p = fabs(u + v), q = fabs(u - v);
-            const bool inr = q > 0x1p-800 && q < 0x1p+800;
-            if (!(inr && (p > q * a.sd2_hi || p < q * a.sd2_lo)))
-                any |= sx_value_greater(u, v, a.sd2) ? 1 : 0;
-            if (!(inr && (p > q * a.sd_hi || p < q * a.sd_lo)))
-                cnt += sx_value_greater(u, v, a.sd) ? 1 : 0;
+        for (int w = 0; w < kSolveThreads / 32; ++w) {
+            if (w < warp) before += s_scan[w];
+            all += s_scan[w];
+            K += s_k[w];
+            cm = max(cm, s_m[w]);
         }
+        const int ex = before + incl - own;
+        if (t < ntiles) {
+            soff[t] = P + (ex & 0xffff);
+            rank[t] = NE + (ex >> 16);
+            if (c > 0) ne[NE + (ex >> 16)] = t;
+        }
+        P += all & 0xffff;
+        NE += all >> 16;
+        __syncthreads();  // s_scan and s_k are reused
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        any |= __shfl_xor_sync(0xffffffffu, any, o);
-    }
-    if (lane == 0) {
-        s_red[warp] = cnt;
-        s_any[warp] = any;
+    if (tid == 0) {
+        soff[ntiles] = P;
+        a.kcount[sp] = K;
+        a.cmax[sp] = cm;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int c = 0, y = 0;
-        for (int w = 0; w < kThreads / 32; ++w) {
-            c += s_red[w];
-            y |= s_any[w];
+    // the first tile holds sample 0 and the last one sample n-1, so both have knots
+    if (K > 5) {
+        const bool l = cnt[0] < 6, r = cnt[ntiles - 1] < 6;
+        if (l || r) {
+            if (tid == 0 && l) end_rule_sparse(a, e, sp, 0, ne, NE, cnt, hd);
+            if (tid == 32 && r) end_rule_sparse(a, e, sp, 1, ne, NE, cnt, hd);
+            __syncthreads();
         }
-        if (c) atomicAdd(&a.cnt[gq.g], (unsigned)c);
-        if (y) atomicOr(&a.any[gq.g], 1);
     }
-    __syncthreads();  // s_red / s_any are reused by the CTA's next tile
+    if (a.bflags && tid == 0) {
+        // a replaced end value differs from the sample in its bits (t > y or t < y)
+        const double* h = a.h[a.par[q.g]] + q.base;
+        a.bflags[sp] = (unsigned char)(
+            (__double_as_longlong(a.yend[2 * sp]) != __double_as_longlong(h[0]) ? 1 : 0) |
+            (__double_as_longlong(a.yend[2 * sp + 1]) != __double_as_longlong(h[q.n - 1]) ? 2
+                                                                                          : 0));
+    }
+    // rows of the first and last separator of every tile with knots
+    for (int i = tid; i < NE; i += kSolveThreads) {
+        const int t = ne[i], c = cnt[t];
+        const TileHdr h = hd[t];
+        TileHdr hp, hn;
+        if (i > 0) hp = hd[ne[i - 1]];
+        if (i + 1 < NE) hn = hd[ne[i + 1]];
+        double2* row = reinterpret_cast<double2*>(rows + (size_t)t * (kRowSlots * 4));
+        Row sr = identity_row();
+        if (i > 0 && (c > 1 || i + 1 < NE)) {
+            const int xp = c > 1 ? h.x1 : hn.x0;
+            const double yp = c > 1 ? h.y1 : hn.y0;
+            sr = spline_row(hp.xb, h.x0, xp, seg_slope(hp.xb, h.x0, hp.yb, h.y0),
+                            seg_slope(h.x0, xp, h.y0, yp));
+        }
+        Row o = c > 1 ? reduced_row(sr, 0.0, 1.0, 0.0, h.ga, h.aa, h.ba)
+                      : reduced_row(sr, 0.0, 1.0, 0.0, 0.0, 0.0, 1.0);
+        row[0] = make_double2(o.l, o.m);
+        row[1] = make_double2(o.u, o.r);
+        if (c > 1) {
+            sr = identity_row();
+            if (i + 1 < NE)
+                sr = spline_row(h.xa, h.xb, hn.x0, seg_slope(h.xa, h.xb, h.ya, h.yb),
+                                seg_slope(h.xb, hn.x0, h.yb, hn.y0));
+            o = reduced_row(sr, h.gb, h.ab, h.bb, 0.0, 0.0, 1.0);
+            const int k = tile_seps(c) - 1;
+            row[2 * k] = make_double2(o.l, o.m);
+            row[2 * k + 1] = make_double2(o.u, o.r);
+        }
+    }
+    __syncthreads();
+    double* X = a.xsep + rec_base(a, e, q);
+    solve_separators(dyn_smem, a.solve_wcap, SepRows{rows, soff, ntiles}, P, X,
+                     a.red + red_base(a, e, q));
+    __syncthreads();
+    // the knots just before and after every tile
+    TileEdge* ed = a.edge + te0;
+    for (int t = tid; t < ntiles; t += kSolveThreads) {
+        const int s0 = soff[t], s1 = soff[t + 1], r = rank[t];
+        TileEdge w;
+        w.sep0 = s0;
+        w.pad = 0;
+        w.px = w.nx = 0;
+        w.py = w.pc = w.ny = w.nc = 0.0;
+        if (r > 0) {
+            const TileHdr& h = hd[ne[r - 1]];
+            w.px = h.xb;
+            w.py = h.yb;
+            w.pc = X[s0 - 1];
+        }
+        const int rn = r + (s1 > s0 ? 1 : 0);
+        if (rn < NE) {
+            const TileHdr& h = hd[ne[rn]];
+            w.nx = h.x0;
+            w.ny = h.y0;
+            w.nc = X[s1];
+        }
+        ed[t] = w;
     }
 }
 
-// The register budgets the autotuner chooses between; same results.  (A one-tile-per-CTA
-// form, as k_extrema has, spills at budget A and was measured slower.)
-template __global__ void k_eval_t<kEvalBlocksA>(SiftArgs a);
-template __global__ void k_eval_t<kEvalBlocksB>(SiftArgs a);
+// =======================================================================================
+// k_tile_sift: one CTA per tile: the spline values of the tile's knots (chunk interiors, one
+// thread per chunk), the segment coefficients in shared memory, both envelopes at every sample,
+// the mean envelope, the sx statistics, and the sample's next value h - m written to the other h
+// plane.  The stop decision comes after a row's last tile (criterion below); it either takes the
+// new plane as the row's h (mark 1) or keeps the old one (mark 0, the realization has finished:
+// its mode is h).  A row marked 0 repeats its iteration: h, knots and envelopes are the same, so
+// the next launch only exports the mode and counts the iteration; the new plane is already what
+// that iteration's update gives.  The knots of both envelopes fit the shared-memory arrays at
+// white-noise density (about 1440 a tile); denser tiles take one envelope after the other.
+// =======================================================================================
+namespace {
 
-// =======================================================================================
-// k_criterion: one CTA per channel (persistent over the channels), over the channel's
-// realizations; channels whose stage has finished are skipped.
-// =======================================================================================
-__global__ void __launch_bounds__(kThreads)
-k_criterion(SiftArgs a) {
-    __shared__ int s_all[kThreads / 32];
-    __shared__ unsigned long long s_knots[kThreads / 32];
-    for (int c = blockIdx.x; c < a.nchan; c += gridDim.x) {
-    ChanState& cst = a.cs[c];
-    if (cst.done) continue;  // CTA-uniform
-    const Chan* ch = a.chan + c;
-    const int nr = __ldg(&ch->nr), row0 = __ldg(&ch->row0);
-    const double inv_n = 1.0 / (double)__ldg(&ch->n);
-    const int j = cst.iter;
-    const int cap = cst.cap;
-    int all = 1;
-    unsigned long long knots = 0;
-    for (int r = threadIdx.x; r < nr; r += blockDim.x) {
-        const int g = row0 + r;
-        const unsigned cn = a.cnt[g];
-        const int any = a.any[g];
-        a.cnt[g] = 0u;
-        a.any[g] = 0;
-        const int kmax = a.kcount[g], kmin = a.kcount[a.nrows + g];
-        knots += (unsigned long long)(kmax + kmin);
-        const double fr = (a.frac[g] + (double)cn) * inv_n;
-        a.frac[g] = fr;
-        const bool crit = fr > a.tol || (any != 0 && (kmax + kmin) > 6);
-        int fin = a.finish[g];
-        int mark;
-        if (crit) {
-            mark = 1;
-            if (fin == 0 && j == cap - 1) {
-                mark = 0;
-                fin = 1;
-            }
-        } else {
-            if (fin == 0) {
-                mark = 0;
-                fin = 1;
-            } else {
-                mark = 1;
-            }
-        }
-        a.mark[g] = mark;
-        if (a.tape_mark) a.tape_mark[r] = (signed char)mark;
-        a.finish[g] = fin;
-        all &= fin;
+// The row's stop decision after an iteration (sifting fraction carry, siftingCriterion,
+// checkBreak), by one thread once all its tiles are counted (cn samples with sx > sd, any: some
+// sx > sd2); the channel's last row closes the channel's iteration.
+__device__ __noinline__ void row_criterion(const SiftArgs& a, const Geo& q, ChanState& cst,
+                                           unsigned cn, int any) {
+    const int g = q.g;
+    const int nr = a.nchan == 1 ? a.nr1 : __ldg(&a.chan[q.c].nr);
+    const double inv_n = 1.0 / (double)q.n;
+    const int j = cst.iter, cap = cst.cap;
+    const int kk = a.kcount[g] + a.kcount[a.nrows + g];
+    const double fr = (a.frac[g] + (double)cn) * inv_n;
+    a.frac[g] = fr;
+    const bool crit = fr > a.tol || (any != 0 && kk > 6);
+    int fin = a.finish[g];
+    int mark = 1;
+    if (fin == 0 && (!crit || j == cap - 1)) {
+        mark = 0;
+        fin = 1;
     }
-    all = __all_sync(0xffffffffu, all);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) knots += __shfl_xor_sync(0xffffffffu, knots, o);
-    if ((threadIdx.x & 31) == 0) {
-        s_all[threadIdx.x >> 5] = all;
-        s_knots[threadIdx.x >> 5] = knots;
+    a.mark[g] = mark;
+    a.finish[g] = fin;
+    if (a.tape_mark) a.tape_mark[q.r] = (signed char)mark;
+    if (mark == 1) {
+        a.par[g] ^= 1;
+    } else {  // the row's repeated iteration has the same counts
+        a.cnt[g] = cn;
+        a.any[g] = any;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int d = 1;
-        unsigned long long kt = 0;
-        for (int w = 0; w < kThreads / 32; ++w) {
-            d &= s_all[w];
-            kt += s_knots[w];
-        }
+    atomicAdd(&cst.knots, (unsigned long long)kk);
+    // rows counted (low word) and finished (high word); the thread that completes the count
+    // knows both from the one sum
+    const unsigned long long add = 1ull | (unsigned long long)fin << 32;
+    const unsigned long long sum = atomicAdd(&cst.rows, add) + add;
+    if ((unsigned)sum == (unsigned)nr) {
+        cst.rows = 0ull;
         cst.iter = j + 1;
-        cst.knots += kt;
         cst.iters += 1ull;
-        if (a.forced > 0 ? j + 1 >= a.forced : d != 0) cst.done = 1;
-    }
-    __syncthreads();  // s_all / s_knots are reused for the CTA's next channel
+        if (a.forced > 0 ? j + 1 >= a.forced : (int)(sum >> 32) == nr) cst.done = 1;
     }
 }
+
+// Adds a tile's counts to its row's: one 64-bit sum of tiles, tiles with some sx > sd2, and
+// samples with sx > sd, so that the thread that completes the row has them all from its own
+// addition, without a fence between counts and ticket (a fence here waits for the tile's stores:
+// about a microsecond of every CTA).  Rows of 2^17 tiles and more (2^28 samples) do not fit one
+// word: they are counted in separate words, ordered by fences.  Returns true to the thread that
+// completes the row.
+__device__ __forceinline__ bool count_tile(const SiftArgs& a, const Geo& q, unsigned& cn,
+                                           int& any) {
+    const int bits = 32 - __clz(q.ntiles);
+    if (bits <= a.count_bits) {
+        const int s1 = bits + 12, s2 = s1 + bits;
+        const unsigned long long add = (unsigned long long)cn | (unsigned long long)any << s1 |
+                                       1ull << s2;
+        const unsigned long long sum = atomicAdd(&a.acc[q.g], add) + add;
+        if ((int)(sum >> s2) != q.ntiles) return false;
+        a.acc[q.g] = 0ull;
+        cn = (unsigned)(sum & ((1ull << s1) - 1ull));
+        any = (sum >> s1 & ((1ull << bits) - 1ull)) != 0ull ? 1 : 0;
+        return true;
+    }
+    unsigned* w = reinterpret_cast<unsigned*>(a.acc_wide + 2 * (size_t)q.g);
+    if (cn) atomicAdd(w, cn);
+    if (any) atomicOr(w + 1, 1u);
+    __threadfence();
+    if (atomicAdd(w + 2, 1u) != (unsigned)q.ntiles - 1u) return false;
+    __threadfence();
+    cn = atomicExch(w, 0u);
+    any = (int)atomicExch(w + 1, 0u);
+    w[2] = 0u;
+    return true;
+}
+
+// chunk_interior (same operations, same order) of the chunk whose knots 0..len+1 sit in the
+// padded arrays from the chunk's base on: s slopes, d segment lengths on entry; c receives the
+// spline values of knots 1..len, d[k] the factor of row k meanwhile.
+template <class Pivot>
+__device__ __forceinline__ void chunk_interior_sweep(Pivot& pv, const double* s, double* c,
+                                                     double* d, int len, double xl, double xr) {
+    // row k: lengths d[k], d[k+1], slopes s[k], s[k+1]; row 0 takes xl, row len-1 takes xr
+    double l = d[0], u = d[1], sn = s[1];
+    double ri = fma(-l, xl, 3.0 * (sn - s[0]));
+    if (len == 1) ri = fma(-u, xr, ri);
+    double iw = pv.inv(2.0 * (l + u));
+    double cp = u * iw, gp = ri * iw;
+    d[0] = cp;
+#pragma unroll 2
+    for (int k = 1; k < len; ++k) {
+        c[k] = gp;
+        const double sv = sn;
+        l = u;
+        u = d[k + 1];
+        sn = s[k + 1];
+        ri = 3.0 * (sn - sv);
+        if (k == len - 1) ri = fma(-u, xr, ri);
+        iw = pv.inv(fma(-l, cp, 2.0 * (l + u)));
+        gp = fma(-l, gp, ri) * iw;
+        cp = u * iw;
+        d[k] = cp;
+    }
+    c[len] = gp;
+    double xv = gp;
+#pragma unroll 4
+    for (int k = len - 2; k >= 0; --k) {
+        xv = fma(-d[k], xv, c[k + 1]);
+        c[k + 1] = xv;
+    }
+}
+// The factors of row k take the place of segment k's length, which rows after k do not read; the
+// rare repetition with checked pivots finds the lengths in the knots' positions.
+__device__ __noinline__ void chunk_interior_checked(const short* x, const double* s, double* c,
+                                                    double* d, int len, double xl, double xr) {
+    for (int i = 0; i <= len; ++i) d[i] = (double)(x[kq(i + 1)] - x[i]);
+    CheckedPivot pv;
+    chunk_interior_sweep(pv, s, c, d, len, xl, xr);
+}
+__device__ __forceinline__ void chunk_interior_knots(const short* x, const double* s, double* c,
+                                                     double* d, int len, double xl, double xr) {
+    RawPivot pv;
+    chunk_interior_sweep(pv, s, c, d, len, xl, xr);
+    if (pv.ones) chunk_interior_checked(x, s, c, d, len, xl, xr);
+}
+
+// Shared memory of k_tile_sift: kCap entries each for the knots' positions and segments (seg_at;
+// envelope 1 after envelope 0; the knot after the tile where in-tile knot `count` would be), the
+// tile's samples, and small pieces.  d holds the segment lengths until the sweeps.
+template <int kCap>
+struct SiftSmem {
+    double b[kCap], c[kCap], d[kCap];
+    double2 stage[kTileSamples / 2];  // the samples
+    TileEdge edge[2][2];              // this and the next tile's edges (envelopes 0, 1)
+    unsigned bits[2][2][kWords];      // and bitmaps
+    TileScan scan[2];                 // and knot counts
+    double xs[2][kRowSlots];          // the tile's separator values
+    short x[kCap];
+};
+
+}  // namespace
+
+size_t tile_sift_smem(bool dense) {
+    return dense ? sizeof(SiftSmem<kSiftDense>) : sizeof(SiftSmem<kSiftSparse>);
+}
+
+template <bool kDense, bool kEnv>
+__global__ void __launch_bounds__(kTileThreads, kDense ? 3 : 4)
+k_tile_sift(const __grid_constant__ SiftArgs a) {
+    constexpr int kCap = kDense ? kSiftDense : kSiftSparse;
+    extern __shared__ __align__(16) unsigned char dyn_smem[];
+    SiftSmem<kCap>& S = *reinterpret_cast<SiftSmem<kCap>*>(dyn_smem);
+    __shared__ int s_w[kTileWarps];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    TileIter it(a);
+    // the rows of this launch
+    auto mine = [&](const TileIter& t) {
+        return a.sift_split == 0 || (t.need > kSiftSparse) == kDense;
+    };
+    int buf = 0;
+    auto prefetch = [&](int to) {
+        if (!it.more()) return;
+        const int n0 = it.tile * kTileSamples;
+        stage_tile(S.stage, a.h[it.par] + it.q.base + n0, min(kTileSamples, it.q.n - n0), tid);
+        const int e = (tid >> 5) & 1;
+        const size_t te = tix(a, e, it.q, it.tile);
+        if (tid < 64 && lane < kWords / 4)
+            cp_async16(&S.bits[to][e][4 * lane], a.bitmap + te * kWords + 4 * lane);
+        if (tid < 64 && lane >= 16 && lane < 16 + (int)sizeof(TileEdge) / 16)
+            cp_async16(reinterpret_cast<char*>(&S.edge[to][e]) + 16 * (lane - 16),
+                       reinterpret_cast<const char*>(a.edge + te) + 16 * (lane - 16));
+        if (tid >= 24 && tid < 24 + (int)sizeof(TileScan) / 16)
+            cp_async16(reinterpret_cast<char*>(&S.scan[to]) + 16 * (tid - 24),
+                       reinterpret_cast<const char*>(a.scan + it.q.tile0 + it.tile) +
+                           16 * (tid - 24));
+    };
+    it.to_row(a, mine);
+    prefetch(0);
+    while (it.more()) {
+    const Geo q = it.q;
+    const int tile = it.tile;
+    const bool repeat = it.mark == 0, write_mean = it.mean;
+    ChanState& cst = a.cs[q.c];
+    const int n0 = tile * kTileSamples;
+    const int m = min(kTileSamples, q.n - n0);  // samples of the tile
+    const double* __restrict__ hin = a.h[it.par] + q.base + n0;
+    double* __restrict__ hout = a.h[it.par ^ 1] + q.base + n0;
+    const int j0 = kPerThread * tid;
+    const int lim = m - j0;  // the thread's samples in the row
+    cp_async_wait_all();
+    __syncthreads();  // also: the CTA's last tile is done with shared memory
+    unsigned cnt = 0u;  // samples with sx > sd
+    int any = 0;        // some sx > sd2
+    // once a warp is done with its staged samples the next tile's take their place
+    auto advance = [&]() {
+        __syncwarp();
+        it.next(a);
+        it.to_row(a, mine);
+        buf ^= 1;
+        prefetch(buf);
+    };
+    if (repeat) {
+        // repeated iteration of a finished row: its mode is h
+        double* mo = cst.mode_out + (size_t)q.r * q.n + n0;
+        const int w0 = warp * kWarpSamples;
+        for (int j = w0 + lane; j < min(m, w0 + kWarpSamples); j += 32) mo[j] = staged(S.stage, j);
+        advance();
+    } else {
+    const TileEdge* ed0 = &S.edge[buf][0];
+    const TileEdge* ed1 = &S.edge[buf][1];
+    // the tile's separator values land while its knots are compacted
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const double* X = a.xsep + rec_base(a, e, q) + (e ? ed1 : ed0)->sep0;
+        if (tid < kRowSlots) cp_async8(&S.xs[e][tid], X + tid);
+    }
+    const unsigned b0 = reinterpret_cast<const TileBits*>(S.bits[buf][0])[tid];
+    const unsigned b1 = reinterpret_cast<const TileBits*>(S.bits[buf][1])[tid];
+    const int tot = S.scan[buf].total;
+    const int own = __popc(b0) | __popc(b1) << 16;
+    const int ex = S.scan[buf].before[warp] + warp_scan(own, lane) - own;
+    const bool first = tile == 0, last = tile == q.ntiles - 1;
+    const int c0 = tot & 0xffff, c1 = tot >> 16;
+    // (only the densest tiles of the dense launch; the sparse launch's rows all fit)
+    const bool two = kDense && seg_at(c0 + 1) + seg_at(c1 + 1) + 2 > kCap;
+    const int base1 = two ? 0 : seg_at(c0 + 1) + 1;
+    // knots before the thread's first sample (sample 0 of the row lies in the first segment)
+    const bool origin = first && tid == 0;
+    const int rA0 = origin ? 1 : ex & 0xffff, rA1 = origin ? 1 : ex >> 16;
+    // position and value of knot r of envelope e (r = 0 before the tile, 1 .. count in it,
+    // count + 1 after it) at entry p
+    auto knot_x = [&](int e, int r, int p) -> int {
+        const TileEdge* ed = e ? ed1 : ed0;
+        if (r == 0) return ed->px - n0;
+        if (r > (e ? c1 : c0)) return ed->nx - n0;
+        return S.x[p];
+    };
+    auto knot_y = [&](int e, int r, int x) -> double {
+        const TileEdge* ed = e ? ed1 : ed0;
+        const int c = e ? c1 : c0;
+        if (r == 0) return ed->py;
+        if (r > c) return ed->ny;
+        if (first && r == 1) return a.yend[2 * (e * a.nrows + q.g)];
+        if (last && r == c) return a.yend[2 * (e * a.nrows + q.g) + 1];
+        return staged(S.stage, x);
+    };
+    // envelope e at the thread's sample i, one at a time (the paths that are not the common one);
+    // values from h itself: other warps may have refilled the stage
+    auto env_one = [&](int e, int i) -> double {
+        const unsigned b = (e ? b1 : b0) & ((1u << i) - 1u);
+        int r = (e ? ex >> 16 : ex & 0xffff) + __popc(b);
+        if (first && j0 + i == 0) r = 1;
+        const int p = (e ? base1 : 0) + seg_at(r);
+        const int x = knot_x(e, r, p);
+        double y;
+        if (r == 0) y = (e ? ed1 : ed0)->py;
+        else if (first && r == 1) y = a.yend[2 * (e * a.nrows + q.g)];
+        else y = hin[x];
+        return seg_eval(y, S.b[p], S.c[p], S.d[p], (double)(j0 + i - x));
+    };
+    double yu = 0.0, yv = 0.0;  // values of the knots the thread's first segments start at
+    int xu = 0, xv = 0;         // and their positions
+    for (int pass = 0; pass < (two ? 2 : 1); ++pass) {
+        if (pass) {  // the upper envelope waits in the tile's part of the output plane
+            double* up = kEnv ? a.dbg_upper + (size_t)q.r * q.n + n0 : hout;
+            for (int i = 0; i < kPerThread && i < lim; ++i) up[j0 + i] = env_one(0, i);
+            __syncthreads();
+        }
+        {
+            const unsigned w0 = two && pass ? 0u : b0, w1 = two && !pass ? 0u : b1;
+            const unsigned wb = __reduce_or_sync(0xffffffffu, w0 | w1);
+            int p0 = ex & 0xffff, p1 = ex >> 16;
+#pragma unroll
+            for (int i0 = 0; i0 < kPerThread; i0 += 4) {
+                if (!(wb >> i0 & 15u)) continue;  // no knots at these samples in the whole warp
+#pragma unroll
+                for (int i = i0; i < i0 + 4; ++i) {
+                    if (w0 >> i & 1u) S.x[2 + kq(p0++)] = (short)(j0 + i);
+                    if (w1 >> i & 1u) S.x[base1 + 2 + kq(p1++)] = (short)(j0 + i);
+                }
+            }
+        }
+        constexpr int kHalf = kTileThreads / 2;  // threads per envelope
+        const int eh = two ? pass : tid / kHalf, th = two ? tid : tid % kHalf;
+        const int wh = two ? kTileThreads : kHalf;
+        const int ch = eh ? c1 : c0, bh = eh ? base1 : 0;
+        __syncthreads();
+        if (!two) {
+            xu = knot_x(0, rA0, seg_at(rA0));
+            yu = knot_y(0, rA0, xu);
+            xv = knot_x(1, rA1, base1 + seg_at(rA1));
+            yv = knot_y(1, rA1, xv);
+        }
+        // slopes and lengths; segment r starts at seg_at(r) (r = 0: it enters the tile,
+        // r = count: it leaves)
+        const int r0 = first ? 1 : 0, r1 = last ? ch - 1 : ch;
+        const int step = kq(wh);  // seg_at advances by 17 for 16 segments
+        // the segments with a knot outside the tile or at an end of the row: the first and last
+        const bool outer = th >= wh - 2;
+        const int ro = th == wh - 1 ? r0 : r1, io = bh + seg_at(ro), io1 = bh + seg_at(ro + 1);
+        for (int r = r0 + 1 + th, i0 = bh + seg_at(r), i1 = bh + seg_at(r + 1); r < r1;
+             r += wh, i0 += step, i1 += step) {
+            const int x0 = S.x[i0], x1 = S.x[i1];
+            const double len = (double)(x1 - x0);
+            S.b[i0] = div_int(staged(S.stage, x1) - staged(S.stage, x0), len);
+            S.d[i0] = len;
+        }
+        double lo = 0.0;
+        if (outer) {
+            const int x0 = knot_x(eh, ro, io), x1 = knot_x(eh, ro + 1, io1);
+            lo = (double)(x1 - x0);
+            S.b[io] = div_int(knot_y(eh, ro + 1, x1) - knot_y(eh, ro, x0), lo);
+            S.d[io] = lo;
+        }
+        if (!pass) cp_async_wait_all();  // the separator values
+        __syncthreads();
+        {
+            const int ns0 = two && pass ? 0 : tile_seps(c0);
+            const int ns1 = two && !pass ? 0 : tile_seps(c1);
+            int e, k;
+            if (sweep_lane(tid, ns0, ns1, e, k)) {
+                const double xl = S.xs[e][k - 1], xr = S.xs[e][k];
+                const int jb = (k - 1) * kChunk, js = min(k * kChunk, (e ? c1 : c0) - 1);
+                const int base = (e ? base1 : 0) + 2, i = base + kq(jb);
+                if (js - jb > 1)
+                    chunk_interior_knots(S.x + i, S.b + i, S.c + i, S.d + i, js - jb - 1, xl,
+                                         xr);
+                S.c[base + kq(js)] = xr;
+                if (k == 1) S.c[base] = xl;
+            }
+            const TileEdge* ed = eh ? ed1 : ed0;
+            if (th == wh - 1) S.c[bh] = ed->pc;
+            if (th == wh - 2) S.c[bh + 2 + kq(ch)] = ed->nc;
+            if (th == wh - 3 && ch == 1) S.c[bh + 2] = S.xs[eh][0];
+        }
+        __syncthreads();
+        for (int r = r0 + 1 + th, i0 = bh + seg_at(r), i1 = bh + seg_at(r + 1); r < r1;
+             r += wh, i0 += step, i1 += step) {
+            double b, d;
+            seg_coeffs_int((double)(S.x[i1] - S.x[i0]), S.b[i0], S.c[i0], S.c[i1], b, d);
+            S.b[i0] = b;
+            S.d[i0] = d;
+        }
+        // (one of the two threads when the first segment is the last)
+        if (outer && (r0 != r1 || th == wh - 1)) {
+            double b, d;
+            seg_coeffs_int(lo, S.b[io], S.c[io], S.c[io1], b, d);
+            S.b[io] = b;
+            S.d[io] = d;
+        }
+        __syncthreads();
+    }
+    // kEnv: the envelopes themselves go to the caller's arrays in place of the next h and the
+    // mean envelope (contiguous rows, aligned to 32 bytes or not)
+    const size_t o = kEnv ? (size_t)q.r * q.n + n0 + j0 : q.base + n0 + j0;
+    double* __restrict__ me = (kEnv ? a.dbg_lower : a.menv) + o;
+    hout = kEnv ? a.dbg_upper + o : hout + j0;
+    const bool wide = !kEnv || (((size_t)a.dbg_upper | (size_t)a.dbg_lower) & 31) == 0 &&
+                                   (q.n & 3) == 0;
+    bool redo = false;
+    // (the warp's samples all in the row: warp-uniform)
+    const bool common = !two && (kEnv || write_mean) && wide && m - warp * kWarpSamples >= kWarpSamples;
+    if (common) {
+        // Both envelopes along the thread's samples: a segment's coefficients are loaded when the
+        // samples pass its first knot (whose value is that sample's).  sx > t is decided by the
+        // signs of p - q t for bounds t around the threshold (sx_bounds; one fma rounds to zero or
+        // to the exact sign, over- and underflow included); a thread with an undecided sample
+        // or a NaN redoes its samples with the division.
+        int ru = rA0, rv = rA1;
+        int pu = seg_at(ru), pv = base1 + seg_at(rv);
+        double bu = S.b[pu], cu = S.c[pu], du = S.d[pu], tu = (double)(j0 - xu);
+        double bv = S.b[pv], cv = S.c[pv], dv = S.d[pv], tv = (double)(j0 - xv);
+        const unsigned f0 = origin ? b0 & ~1u : b0, f1 = origin ? b1 & ~1u : b1;
+        const unsigned wf = __reduce_or_sync(0xffffffffu, f0 | f1);
+        int und = 0, amax = 0;
+        // four samples at a time: without a knot among them in the whole warp one set of
+        // coefficients serves all four, and nothing splits the block's instruction stream
+#pragma unroll 1
+        for (int i0 = 0; i0 < kPerThread; i0 += 4) {
+            const double2 ha = S.stage[stage_piece(kPerThread / 2 * tid + i0 / 2)];
+            const double2 hb = S.stage[stage_piece(kPerThread / 2 * tid + i0 / 2 + 1)];
+            const double h[4] = {ha.x, ha.y, hb.x, hb.y};
+            double eu[4], ev[4];
+            if (!(wf >> i0 & 15u)) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    eu[i] = seg_eval(yu, bu, cu, du, tu + (double)i);
+                    ev[i] = seg_eval(yv, bv, cv, dv, tv + (double)i);
+                }
+                tu += 4.0;
+                tv += 4.0;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    eu[i] = seg_eval(yu, bu, cu, du, tu);
+                    ev[i] = seg_eval(yv, bv, cv, dv, tv);
+                    tu += 1.0;
+                    tv += 1.0;
+                    if (f0 >> (i0 + i) & 1u) {
+                        ++ru;
+                        pu = seg_at(ru);
+                        yu = h[i];
+                        bu = S.b[pu];
+                        cu = S.c[pu];
+                        du = S.d[pu];
+                        tu = 1.0;
+                    }
+                    if (f1 >> (i0 + i) & 1u) {
+                        ++rv;
+                        pv = base1 + seg_at(rv);
+                        yv = h[i];
+                        bv = S.b[pv];
+                        cv = S.c[pv];
+                        dv = S.d[pv];
+                        tv = 1.0;
+                    }
+                }
+            }
+            if (kEnv) {
+                store4(hout + i0, eu);
+                store4(me + i0, ev);
+                continue;
+            }
+            double mv[4], hn[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const double s = eu[i] + ev[i], p = fabs(s), w = fabs(eu[i] - ev[i]);
+                mv[i] = s / 2.0;
+                hn[i] = h[i] - mv[i];
+                const int s1 = __double2hiint(fma(-a.sd_hi, w, p));
+                const int s0 = __double2hiint(fma(-a.sd_lo, w, p));
+                const int t1 = __double2hiint(fma(-a.sd2_hi, w, p));
+                const int t0 = __double2hiint(fma(-a.sd2_lo, w, p));
+                und |= ((s1 - 1) & ~s0) | ((t1 - 1) & ~t0);  // sign bit: neither bound decides
+                cnt += 1u - ((unsigned)s0 >> 31);  // (when decided, not below means above)
+                amax = max(amax, t1);
+            }
+            store4(hout + i0, hn);
+            store4(me + i0, mv);
+        }
+        any = amax > 0 ? 1 : 0;
+        redo = und < 0 || amax > 0x7ff00000;  // (a NaN)
+    }
+    if (!common || (redo && !kEnv)) {
+        cnt = 0u;
+        any = 0;
+#pragma unroll 1
+        for (int i = 0; i < kPerThread && i < lim; ++i) {
+            const double u = two ? hout[i] : env_one(0, i);
+            const double v = env_one(1, i);
+            if (kEnv) {
+                hout[i] = u;
+                me[i] = v;
+                continue;
+            }
+            if (!common) {
+                double mv = (u + v) / 2.0;
+                if (write_mean) me[i] = mv;
+                else mv = me[i];
+                hout[i] = hin[j0 + i] - mv;
+            }
+            any |= sx_greater(u, v, a.sd2) ? 1 : 0;
+            cnt += sx_greater(u, v, a.sd) ? 1 : 0;
+        }
+    }
+    advance();
+    }
+    if (!kEnv) {
+        // the counts of the warps, then the row's
+        any = __any_sync(0xffffffffu, any != 0) ? 1 : 0;
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if (lane == 0) s_w[warp] = (int)(cnt | (unsigned)any << 30);
+        __syncthreads();
+        if (tid == 0) {
+            unsigned t = 0u;
+            int y = 0;
+#pragma unroll
+            for (int w = 0; w < kTileWarps; ++w) {
+                t += (unsigned)s_w[w] & 0x3fffffffu;
+                y |= s_w[w] >> 30;
+            }
+            if (count_tile(a, q, t, y)) {
+                if (repeat) {
+                    t = a.cnt[q.g];
+                    y = a.any[q.g];
+                }
+                row_criterion(a, q, cst, t, y);
+            }
+        }
+    }
+    }
+}
+
+template __global__ void k_tile_sift<true, false>(const __grid_constant__ SiftArgs a);
+template __global__ void k_tile_sift<false, false>(const __grid_constant__ SiftArgs a);
+template __global__ void k_tile_sift<true, true>(const __grid_constant__ SiftArgs a);
+template __global__ void k_tile_sift<false, true>(const __grid_constant__ SiftArgs a);
 
 // Mode export of channel c's realizations that finished in the last executed iteration
 // (blockIdx.y = realization).
@@ -1812,7 +2123,7 @@ __global__ void k_export_final(SiftArgs a, int c) {
     const Geo q = geo(a, c, blockIdx.y);
     if (a.mark[q.g] != 0) return;
     const ChanState& cst = a.cs[c];
-    const double* h = a.h[cst.iter & 1] + q.base;
+    const double* h = a.h[a.par[q.g]] + q.base;
     double* mo = cst.mode_out + (size_t)q.r * q.n;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < q.n; s += gridDim.x * blockDim.x)
         mo[s] = h[s];
@@ -1826,6 +2137,9 @@ __global__ void k_begin_stage(SiftArgs a, int c, int cap, double* mode_out) {
     for (int r = threadIdx.x; r < nr; r += blockDim.x) {
         a.mark[row0 + r] = -1;
         a.finish[row0 + r] = 0;
+        a.par[row0 + r] = 0;
+        a.cnt[row0 + r] = 0u;
+        a.any[row0 + r] = 0;
     }
     if (threadIdx.x == 0) {
         ChanState& cst = a.cs[c];
@@ -1938,6 +2252,8 @@ k_tridiag_batched(int n, const double* l, const double* m, const double* u, cons
 // =======================================================================================
 namespace {
 
+__device__ __forceinline__ int sep_local(int k, int cnt) { return min(k * kChunk, cnt - 1); }
+
 struct SmallSmem {
     double *H, *KY, *KS, *KC, *ENDS, *R2, *X2, *W3;
     int *KX, *SEP, *misc, *WP;
@@ -1950,13 +2266,6 @@ struct SmallSmem {
 // so the chunk chains of the spline solve (lane p walks the knots of chunk p, 16 knots after
 // lane p-1's) read different banks.
 __host__ __device__ __forceinline__ int kp(int k) { return k + (k >> 4); }
-
-// Spline values written by chunk_interior into the padded knot array from knot `first` on.
-struct PadOut {
-    double* a;
-    int first;
-    __device__ __forceinline__ double& operator[](int k) const { return a[kp(first + k)]; }
-};
 
 // Layout of the dynamic shared memory for rows of n samples (doubles first, 16-byte aligned).
 __host__ __device__ inline size_t small_layout(int n, SmallSmem* L, unsigned char* base) {
@@ -2007,6 +2316,13 @@ __host__ __device__ inline size_t small_layout(int n, SmallSmem* L, unsigned cha
     }
     return off;
 }
+
+// Padded knot array slots from knot `first` on.
+struct PadSlots {
+    double* a;
+    int first;
+    __device__ __forceinline__ double& operator()(int k) const { return a[kp(first + k)]; }
+};
 
 // Spline row of knot g from the knot arrays (the slopes of segments g-1 and g).
 struct KnotRowFn {
@@ -2126,7 +2442,8 @@ __device__ __noinline__ int small_knots(const SmallSmem& S, int n, int e) {
     return K;
 }
 
-// The canonical tile-aligned spline solve of the K knots in KX/KY: spline values to KC.
+// The canonical tile-aligned spline solve of the K knots in KX/KY: spline values to KC (KS, the
+// slopes, is spent: the interior sweeps leave their factors there).
 __device__ __noinline__ void small_spline(const SmallSmem& S, int n, int K) {
     const int ntiles = (n + kTileSamples - 1) / kTileSamples;
     int* toff = S.misc;        // [ntiles+1] first knot of each tile
@@ -2164,7 +2481,9 @@ __device__ __noinline__ void small_spline(const SmallSmem& S, int n, int K) {
         ChunkEnds ce;
         const int len = p > soff[t] ? gs - S.SEP[p - 1] - 1 : 0;
         if (len > 0) {
-            ce = chunk_ends(len, KnotRowFn{S.KX, S.KS, S.SEP[p - 1]});
+            // the sweep's reciprocals wait in the rows' spline values
+            const int gb = S.SEP[p - 1];
+            ce = chunk_ends(len, KnotRowFn{S.KX, S.KS, gb}, PadSlots{S.KC, gb + 1});
         } else {
             ce.ga = 0.0; ce.aa = 0.0; ce.ba = 1.0;
             ce.gb = 0.0; ce.ab = 1.0; ce.bb = 0.0;
@@ -2206,7 +2525,8 @@ __device__ __noinline__ void small_spline(const SmallSmem& S, int n, int K) {
     // the separator system, partitioned as k_reduced_solve does
     const PlaneRowFn R2{SROW, S.pcap, 0};
     if (P <= kChunk) {
-        if (threadIdx.x == 0) thomas_small(P, R2, S.X2, 1);
+        if (threadIdx.x == 0)
+            thomas_rolled(P, R2, Slots{S.X2}, Slots{SROW + 2 * S.pcap});
     } else {
         const int Q = (P - 1) / kChunk;
         double* ends = S.W3;
@@ -2218,7 +2538,7 @@ __device__ __noinline__ void small_spline(const SmallSmem& S, int n, int K) {
             const int first = q * kChunk;
             const int len = (q < Q) ? kChunk - 1 : P - first;
             const PlaneRowFn fn{SROW, S.pcap, first};
-            const ChunkEnds ce = chunk_ends(len, fn);
+            const ChunkEnds ce = chunk_ends(len, fn, Slots{S.X2 + first});
             ends[6 * q + 0] = ce.ga;
             ends[6 * q + 1] = ce.aa;
             ends[6 * q + 2] = ce.ba;
@@ -2255,7 +2575,8 @@ __device__ __noinline__ void small_spline(const SmallSmem& S, int n, int K) {
             const int len = (q < Q) ? kChunk - 1 : P - first;
             const double xl = (q > 0) ? x3[q - 1] : 0.0;
             const double xr = (q < Q) ? x3[q] : 0.0;
-            chunk_interior(len, PlaneRowFn{SROW, S.pcap, first}, xl, xr, S.X2 + first, 1);
+            chunk_interior_iw(len, PlaneRowFn{SROW, S.pcap, first}, xl, xr, Slots{S.X2 + first},
+                              Slots{SROW + 2 * S.pcap + first});
             if (q < Q) S.X2[first + kChunk - 1] = xr;
         }
     }
@@ -2270,8 +2591,8 @@ __device__ __noinline__ void small_spline(const SmallSmem& S, int n, int K) {
             const int gb = S.SEP[p - 1];
             const int len = gs - gb - 1;
             if (len > 0)
-                chunk_interior(len, KnotRowFn{S.KX, S.KS, gb}, S.X2[p - 1], S.X2[p],
-                               PadOut{S.KC, gb + 1}, 1);
+                chunk_interior_iw(len, KnotRowFn{S.KX, S.KS, gb}, S.X2[p - 1], S.X2[p],
+                                  PadSlots{S.KC, gb + 1}, PadSlots{S.KS, gb});
         }
     }
     __syncthreads();

@@ -280,7 +280,8 @@ k_stage_end(SiftArgs a, BatchArgs b) {
             if (i >= n) return;
             const ChanState& cs = a.cs[c];
             const int s = cs.stage;
-            const double* hf = a.h[cs.iter & 1] + ch.samp0 + i;
+            // the realizations that finished in the last iteration: their mode is h
+            const size_t so = (size_t)ch.samp0 + i, ld = (size_t)row_ld(n);
             const size_t rn = (size_t)n;
             if (s < M) {
                 double* Ei = b.E + (size_t)s * b.S + ch.samp0 + i;
@@ -289,7 +290,7 @@ k_stage_end(SiftArgs a, BatchArgs b) {
                     const size_t o = (size_t)r * rn;
                     double m;
                     if (a.mark[row0 + r] == 0) {
-                        m = hf[o];
+                        m = a.h[a.par[row0 + r]][so + r * ld];
                         Ei[o] = m;
                     } else {
                         m = Ei[o];
@@ -310,7 +311,7 @@ k_stage_end(SiftArgs a, BatchArgs b) {
                 const double inr = 1.0 / (double)nr;
                 for (int r = 0; r < nr; ++r) {
                     const size_t o = (size_t)r * rn;
-                    const double m = a.mark[row0 + r] == 0 ? hf[o] : md[o];
+                    const double m = a.mark[row0 + r] == 0 ? a.h[a.par[row0 + r]][so + r * ld] : md[o];
                     t = fma(inr, h0[o] - m, t);
                 }
                 *fn = t;
@@ -318,7 +319,7 @@ k_stage_end(SiftArgs a, BatchArgs b) {
             } else {
                 for (int r = 0; r < nr; ++r) {
                     const size_t o = (size_t)r * rn;
-                    const double m = a.mark[row0 + r] == 0 ? hf[o] : md[o];
+                    const double m = a.mark[row0 + r] == 0 ? a.h[a.par[row0 + r]][so + r * ld] : md[o];
                     t = t + (h0[o] - m);
                 }
                 const double avg = t / (double)nr;
@@ -391,10 +392,11 @@ k_stage_begin(SiftArgs a, BatchArgs b) {
             if (i >= n) return;
             const int ns = a.cs[c].stage + 1;
             const size_t rn = (size_t)n;
+            const size_t ld = (size_t)row_ld(n);
             double* h = a.h[0] + ch.samp0 + i;
             if (ns < M) {
                 const double* w = b.W + ch.samp0 + i;
-                for (int r = 0; r < nr; ++r) h[(size_t)r * rn] = w[(size_t)r * rn];
+                for (int r = 0; r < nr; ++r) h[(size_t)r * ld] = w[(size_t)r * rn];
                 return;
             }
             const int k = ns - M;
@@ -411,7 +413,7 @@ k_stage_begin(SiftArgs a, BatchArgs b) {
                     const double esc = 1.0 / sqrt(b.evar[ch.row0 + r]);
                     const double v = fma(nstd * E[o], esc, xv);
                     h0[o] = v;
-                    h[o] = v;
+                    h[(size_t)r * ld] = v;
                 }
             } else {
                 const double sq = sqrt(b.svar[c]);
@@ -420,7 +422,7 @@ k_stage_begin(SiftArgs a, BatchArgs b) {
                     const size_t o = (size_t)r * rn;
                     const double v = fma(nstd * E[o], sq, rv);
                     h0[o] = v;
-                    h[o] = v;
+                    h[(size_t)r * ld] = v;
                 }
             }
         });
@@ -442,6 +444,9 @@ k_commit_plan(SiftArgs a, BatchArgs b) {
             for (int r = threadIdx.x; r < ch.nr; r += blockDim.x) {
                 a.mark[ch.row0 + r] = -1;
                 a.finish[ch.row0 + r] = 0;
+                a.par[ch.row0 + r] = 0;
+                a.cnt[ch.row0 + r] = 0u;
+                a.any[ch.row0 + r] = 0;
             }
         __syncthreads();  // every thread has read cs before thread 0 changes it
         if (threadIdx.x == 0) {
