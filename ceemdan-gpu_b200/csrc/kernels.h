@@ -288,10 +288,10 @@ size_t small_sift_smem(int n);
 __global__ void k_sift_small(SiftArgs a, SmallArgs sa);
 
 // k_spline_solve: threads per CTA, chunks swept per pass over the staged rows, dynamic shared
-// memory (the stage of 87,080 bytes and the level-3 workspace; two CTAs per SM).
+// memory (the stage of 87,088 bytes and the level-3 workspace; two CTAs per SM).
 constexpr int kSolveThreads = 256;
 constexpr int kSolveChunks = 128;
-constexpr int kSolveStage = 87080;
+constexpr int kSolveStage = 87088;
 constexpr int kSolveSmem = 111600;
 
 // stage kernels (stage_kernels.cu)

@@ -1214,184 +1214,352 @@ constexpr int kSolvePass = kSolveChunks * kChunk;                 // level-2 row
 constexpr int kSolveSlots = kSolvePass + (kSolvePass >> 4) + 1;  // padded
 constexpr int kTabTiles = 256;  // rows of up to this many tiles keep their tables in shared memory
 
-// Level-2 rows staged in shared memory (4 padded planes).
-struct RedStage {
-    double l[kSolveSlots], m[kSolveSlots], u[kSolveSlots], r[kSolveSlots];
-    double x[kSolveSlots];  // reciprocal pivots, then the solution
+// Rows of a system with one pad slot per 16 (row i at kq(i)): a chunk's rows are consecutive, and
+// the lanes that sweep neighbouring chunks read different banks.
+struct alignas(16) SepRow {
+    double l, m, u, r;
 };
-struct StageSlots {
-    double* p;
-    int first;
-    __device__ __forceinline__ double& operator()(int k) const { return p[kq(first + k)]; }
-};
+__device__ __forceinline__ SepRow load_row(const SepRow* p) {
+    const double2 a = reinterpret_cast<const double2*>(p)[0];
+    const double2 b = reinterpret_cast<const double2*>(p)[1];
+    return SepRow{a.x, a.y, b.x, b.y};
+}
+__device__ __forceinline__ SepRow sep_row(const Row& w) { return SepRow{w.l, w.m, w.u, w.r}; }
+// padded length of n rows
+__host__ __device__ __forceinline__ int padded(int n) { return n + (n >> 4) + 1; }
 
+// Level-2 rows staged in shared memory.
+struct RedStage {
+    SepRow row[kSolveSlots];
+    double x[kSolveSlots + 1];  // reciprocal pivots, then the solution
+};
 static_assert(sizeof(RedStage) == kSolveStage, "the host sizes the workspace after it");
 
-struct StageRowFn {
-    const RedStage* st;
-    int first;  // local row of chunk row 0
-    __device__ __forceinline__ Row operator()(int k) const {
-        const int j = kq(first + k);
-        Row w;
-        w.l = st->l[j];
-        w.m = st->m[j];
-        w.u = st->u[j];
-        w.r = st->r[j];
-        return w;
+// chunk_ends (same operations, same order) of len consecutive rows; the top-down sweep's
+// reciprocals to iw (kIw).  Rows are read one ahead of their use.
+template <bool kIw, class Pivot>
+__device__ __forceinline__ ChunkEnds ends_sweep(Pivot& pv, const SepRow* r, int len, double* iw) {
+    SepRow w = load_row(r), v = load_row(r + len - 1);
+    const double lf = w.l, ul = v.u;
+    double iu = pv.inv(w.m), iv = pv.inv(v.m);
+    double cp = w.u * iu, gp = w.r * iu, ap = -w.l * iu;
+    double cq = v.l * iv, gq = v.r * iv, bq = -v.u * iv;
+    if (kIw) iw[0] = iu;
+    if (len > 1) {
+        w = load_row(r + 1);
+        v = load_row(r + len - 2);
     }
-};
+#pragma unroll 1
+    for (int k = 1; k < len; ++k) {
+        const SepRow a = w, b = v;
+        if (k + 1 < len) {
+            w = load_row(r + k + 1);
+            v = load_row(r + len - 2 - k);
+        }
+        iu = pv.inv(fma(-a.l, cp, a.m));
+        iv = pv.inv(fma(-b.u, cq, b.m));
+        cp = a.u * iu;
+        gp = fma(-a.l, gp, a.r) * iu;
+        ap = (-a.l * ap) * iu;
+        cq = b.l * iv;
+        gq = fma(-b.u, gq, b.r) * iv;
+        bq = (-b.u * bq) * iv;
+        if (kIw) iw[k] = iu;
+    }
+    return ChunkEnds{gq, -lf * iv, bq, gp, ap, -ul * iu};
+}
+template <bool kIw>
+__device__ __noinline__ void ends_rows_checked(const SepRow* r, int len, double* iw,
+                                               ChunkEnds& e) {
+    CheckedPivot pv;
+    e = ends_sweep<kIw>(pv, r, len, iw);
+}
+// ... to out[0..5] = ga, aa, ba, gb, ab, bb
+template <bool kIw>
+__device__ __forceinline__ void ends_rows(const SepRow* r, int len, double* iw, double* out) {
+    RawPivot pv;
+    ChunkEnds e = ends_sweep<kIw>(pv, r, len, iw);
+    if (pv.ones) {
+        ChunkEnds c;
+        ends_rows_checked<kIw>(r, len, iw, c);
+        e = c;
+    }
+    out[0] = e.ga;
+    out[1] = e.aa;
+    out[2] = e.ba;
+    out[3] = e.gb;
+    out[4] = e.ab;
+    out[5] = e.bb;
+}
 
-// Rows of a spline's separator system, in their tiles' slots: separator p is separator
-// p - soff[t] of tile t, the last tile with soff[t] <= p.
-struct SepRows {
-    const double* rows;  // the spline's first tile's slots
-    const int* soff;
-    int ntiles;
-    __device__ __forceinline__ Row operator()(int p) const {
-        int lo = 0, hi = ntiles - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (soff[mid] <= p) lo = mid;
+// Row p of the next level: separator row s between the chunks with end relations e (left) and
+// e + 6 (right).
+__device__ __forceinline__ SepRow next_row(const SepRow& s, const double* e) {
+    return sep_row(reduced_row(Row{s.l, s.m, s.u, s.r}, e[3], e[4], e[5], e[6], e[7], e[8]));
+}
+
+// Back substitution x[k] <- x[k] - fac(k) x[k+1], row k's factor in its u.
+__device__ __forceinline__ void back_rows(const SepRow* r, double* x, int len, double xv) {
+    double f = 0.0, g = 0.0;
+    if (len > 1) {
+        f = r[len - 2].u;
+        g = x[len - 2];
+    }
+#pragma unroll 1
+    for (int k = len - 2; k >= 0; --k) {
+        const double fc = f, gc = g;
+        if (k > 0) {
+            f = r[k - 1].u;
+            g = x[k - 1];
+        }
+        xv = fma(-fc, xv, gc);
+        x[k] = xv;
+    }
+}
+
+// chunk_interior_iw of len consecutive rows: x holds the reciprocals, then the solution; the rows'
+// u is overwritten.
+__device__ __forceinline__ void interior_rows(SepRow* r, int len, double xl, double xr,
+                                              double* x) {
+    SepRow w = load_row(r);
+    double iw = x[0], gp = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < len; ++k) {
+        const SepRow a = w;
+        const double ic = iw;
+        if (k + 1 < len) {
+            w = load_row(r + k + 1);
+            iw = x[k + 1];
+        }
+        double ri = a.r;
+        if (k == 0) ri = fma(-a.l, xl, ri);
+        if (k == len - 1) ri = fma(-a.u, xr, ri);
+        gp = (k == 0 ? ri : fma(-a.l, gp, ri)) * ic;
+        r[k].u = a.u * ic;
+        x[k] = gp;
+    }
+    back_rows(r, x, len, gp);
+}
+
+// Canonical Thomas of n rows (kCoupled: a chunk between xl and xr), reciprocals formed here.
+template <bool kCoupled>
+__device__ __forceinline__ void thomas_rows(SepRow* r, int n, double xl, double xr, double* x) {
+    SepRow w = load_row(r);
+    double cp = 0.0, gp = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) {
+        const SepRow a = w;
+        if (k + 1 < n) w = load_row(r + k + 1);
+        double ri = a.r;
+        if (kCoupled && k == 0) ri = fma(-a.l, xl, ri);
+        if (kCoupled && k == n - 1) ri = fma(-a.u, xr, ri);
+        const double iw = pivot_inv(k == 0 ? a.m : fma(-a.l, cp, a.m));
+        gp = (k == 0 ? ri : fma(-a.l, gp, ri)) * iw;
+        cp = a.u * iw;
+        r[k].u = cp;
+        x[k] = gp;
+    }
+    back_rows(r, x, n, gp);
+}
+
+// cta_partitioned<SplinePivot> on padded rows: n rows at `rows` (u overwritten), solution to the
+// padded x; ws: 5 padded(n/16) + 6 (n/16 + 1) doubles and as much again for what is below, at
+// most 0.75 n + 64.  Every thread of the CTA calls it.
+struct RowsLevel {
+    SepRow* r;
+    double* x;
+    int n;
+};
+__device__ __forceinline__ RowsLevel rows_level(int k, int depth, int n, SepRow* rows, double* x,
+                                                double* ws) {
+    if (k == 0) return RowsLevel{rows, x, n};
+    int ro = 0, xo = 0, size = n, mine = 0, mr = 0, mx = 0;
+    for (int i = 1; i <= depth; ++i) {
+        size = (size - 1) / kChunk;
+        if (i == k) {
+            mine = size;
+            mr = ro;
+            mx = xo;
+        }
+        ro += 4 * padded(size);
+        xo += padded(size);
+    }
+    return RowsLevel{reinterpret_cast<SepRow*>(ws + mr), ws + ro + mx, mine};
+}
+
+__device__ void partition_rows(int n, SepRow* rows, double* x, double* ws) {
+    int depth = 0, all = 0;
+    for (int size = n; size > kChunk && depth < 7; ++depth) {
+        size = (size - 1) / kChunk;
+        all += 5 * padded(size);
+    }
+    double* ends = ws + all;
+#pragma unroll 1
+    for (int k = 0; k < depth; ++k) {
+        const RowsLevel v = rows_level(k, depth, n, rows, x, ws);
+        const RowsLevel o = rows_level(k + 1, depth, n, rows, x, ws);
+        for (int q = threadIdx.x; q <= o.n; q += blockDim.x) {
+            const int first = q * kChunk;
+            const int len = (q < o.n) ? kChunk - 1 : v.n - first;
+            ends_rows<true>(v.r + kq(first), len, v.x + kq(first), ends + 6 * q);
+        }
+        __syncthreads();
+        for (int p = threadIdx.x; p < o.n; p += blockDim.x)
+            o.r[kq(p)] = next_row(load_row(v.r + kq(p * kChunk + kChunk - 1)), ends + 6 * p);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        const RowsLevel v = rows_level(depth, depth, n, rows, x, ws);
+        thomas_rows<false>(v.r, v.n, 0.0, 0.0, v.x);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int k = depth - 1; k >= 0; --k) {
+        const RowsLevel v = rows_level(k, depth, n, rows, x, ws);
+        const RowsLevel o = rows_level(k + 1, depth, n, rows, x, ws);
+        for (int q = threadIdx.x; q <= o.n; q += blockDim.x) {
+            const int first = q * kChunk;
+            const int len = (q < o.n) ? kChunk - 1 : v.n - first;
+            const double xl = (q > 0) ? o.x[kq(q - 1)] : 0.0;
+            const double xr = (q < o.n) ? o.x[kq(q)] : 0.0;
+            interior_rows(v.r + kq(first), len, xl, xr, v.x + kq(first));
+            if (q < o.n) v.x[kq(first + kChunk - 1)] = xr;
+        }
+        __syncthreads();
+    }
+}
+
+// Asynchronous copies of the rows p0 .. p0 + kSolvePass - 1 of a spline's separator system from
+// their tiles' slots (separator p is separator p - soff[t] of tile t) into the stage: eight
+// threads per tile.  kInner: without the tiles' first and last rows.
+template <bool kInner>
+__device__ __forceinline__ void stage_rows(RedStage& st, const double* rows, const int* soff,
+                                           int ntiles, int p0) {
+    int t = 0;
+    if (p0 > 0) {  // the tile of row p0: the last one with soff[t] <= p0
+        int hi = ntiles - 1;
+        while (t < hi) {
+            const int mid = (t + hi + 1) >> 1;
+            if (soff[mid] <= p0) t = mid;
             else hi = mid - 1;
         }
-        const double2* s = reinterpret_cast<const double2*>(
-            rows + ((size_t)lo * kRowSlots + (size_t)(p - soff[lo])) * 4);
-        const double2 a = s[0], b = s[1];
-        Row w;
-        w.l = a.x;
-        w.m = a.y;
-        w.u = b.x;
-        w.r = b.y;
-        return w;
     }
-};
-
-__device__ __forceinline__ void stage_level2(RedStage& st, const SepRows& src, int p0, int P) {
-    const int rows = min(kSolvePass, P - p0);
-    constexpr int kB = 4;  // rows per thread whose loads are in flight together
-    for (int j0 = threadIdx.x; j0 < rows; j0 += kB * kSolveThreads) {
-        Row w[kB];
-#pragma unroll
-        for (int t = 0; t < kB; ++t) {
-            const int j = j0 + t * kSolveThreads;
-            if (j < rows) w[t] = src(p0 + j);
-        }
-#pragma unroll
-        for (int t = 0; t < kB; ++t) {
-            const int j = j0 + t * kSolveThreads;
-            if (j < rows) {
-                const int q = kq(j);
-                st.l[q] = w[t].l;
-                st.m[q] = w[t].m;
-                st.u[q] = w[t].u;
-                st.r[q] = w[t].r;
-            }
+    const int end = p0 + kSolvePass;
+    for (t += threadIdx.x >> 3; t < ntiles && soff[t] < end; t += kSolveThreads >> 3) {
+        const int s0 = soff[t];
+        const int a = max(s0 + (kInner ? 1 : 0), p0), b = min(soff[t + 1] - (kInner ? 1 : 0), end);
+        const double* src = rows + ((size_t)t * kRowSlots - s0) * 4;
+        for (int p = a + (threadIdx.x & 7); p < b; p += 8) {
+            SepRow* dst = st.row + kq(p - p0);
+            cp_async16(dst, src + (size_t)p * 4);
+            cp_async16(&dst->u, src + (size_t)p * 4 + 2);
         }
     }
 }
 
-// The separator system of one spline (P rows), solution to X.  wg: global workspace, used when
-// the level-3 system does not fit the wcap doubles of shared memory after the stage.  Every
-// thread of the CTA calls it.
-__device__ __forceinline__ void solve_separators(unsigned char* dyn_smem, int wcap,
-                                                 const SepRows& src, int P, double* X,
+// The separator system of one spline (P rows), solution to X.  One pass (P <= kSolvePass): the
+// rows are staged already.  wg: global workspace, used when the level-3 system does not fit the
+// wcap doubles of shared memory after the stage.  Every thread of the CTA calls it, after a
+// barrier.
+__device__ __forceinline__ void solve_separators(RedStage& st, int wcap, const double* rows,
+                                                 const int* soff, int ntiles, int P, double* X,
                                                  double* wg) {
-    RedStage& st = *reinterpret_cast<RedStage*>(dyn_smem);
+    const bool one = P <= kSolvePass;
     if (P <= kChunk) {
-        stage_level2(st, src, 0, P);
+        if (threadIdx.x == 0) thomas_rows<false>(st.row, P, 0.0, 0.0, st.x);
         __syncthreads();
-        if (threadIdx.x == 0)
-            thomas_rolled(P, StageRowFn{&st, 0}, Slots{X}, StageSlots{st.u, 0});
+        if (threadIdx.x < P) X[threadIdx.x] = st.x[threadIdx.x];
         return;
     }
     const int Q = (P - 1) / kChunk;  // level-3 size
-    const bool one = P <= kSolvePass;
-    // End relations and separator rows outlive the passes over the stage.  One pass: the level-3
-    // workspace follows the stage.  More: the stage is filled again for the second sweep, so its
-    // x plane (the reciprocals would not last) holds them with what follows the stage, and the
-    // rest of the level-3 workspace takes the staged rows' place in between.
-    const bool fits = one ? 16 * (size_t)Q + 74 <= (size_t)wcap
-                          : 10 * (size_t)(Q + 1) <= (size_t)wcap + kSolveSlots &&
-                                6 * (size_t)Q + 64 <= 4 * (size_t)kSolveSlots;
-    double* ends = !fits ? wg
-                         : (one ? reinterpret_cast<double*>(dyn_smem + sizeof(RedStage)) : st.x);
-    double* sep = ends + 6 * (size_t)(Q + 1);
-    double* L3 = (fits && !one) ? reinterpret_cast<double*>(dyn_smem) : sep + 4 * (size_t)(Q + 1);
-    double* x3 = L3 + 4 * (size_t)Q;
-    double* ws3 = x3 + Q;  // deeper levels
+    // One pass: the level-3 workspace follows the stage.  More: the stage is filled again for the
+    // second sweep, so its x plane (the reciprocals would not last) and what follows the stage
+    // hold the end relations and separator rows, and the level-3 system takes the staged rows'
+    // place in between.
+    const int deep = 5 * padded(Q) + Q + 64;  // level-3 rows, solution and below
+    const bool fits = one ? 6 * (Q + 1) + deep <= wcap
+                          : 10 * (Q + 1) <= wcap + kSolveSlots && deep <= 4 * kSolveSlots;
+    double* ends = !fits ? wg : (one ? reinterpret_cast<double*>(&st + 1) : st.x);
+    SepRow* sep = reinterpret_cast<SepRow*>(ends + 6 * (size_t)(Q + 1));  // (several passes)
+    SepRow* r3 = one ? sep : (fits ? st.row : sep + (Q + 1));
+    double* x3 = reinterpret_cast<double*>(r3 + padded(Q));
+    double* ws3 = x3 + ((padded(Q) + 1) & ~1);  // deeper levels
     for (int p0 = 0; p0 < P; p0 += kSolvePass) {
-        __syncthreads();
-        stage_level2(st, src, p0, P);
-        __syncthreads();
-        const int q = p0 / kChunk + threadIdx.x;
-        if (threadIdx.x < kSolveChunks && q <= Q) {
-            const int first = q * kChunk;
-            const int len = (q < Q) ? kChunk - 1 : P - first;
-            const StageRowFn fn{&st, first - p0};
-            // one pass: the reciprocals stay in the stage
-            const ChunkEnds ce = one ? chunk_ends(len, fn, StageSlots{st.x, first})
-                                     : chunk_ends(len, fn, NoIw());
-            ends[6 * q + 0] = ce.ga;
-            ends[6 * q + 1] = ce.aa;
-            ends[6 * q + 2] = ce.ba;
-            ends[6 * q + 3] = ce.gb;
-            ends[6 * q + 4] = ce.ab;
-            ends[6 * q + 5] = ce.bb;
-            if (q < Q) {
-                const Row s2 = fn(kChunk - 1);
-                sep[4 * q + 0] = s2.l;
-                sep[4 * q + 1] = s2.m;
-                sep[4 * q + 2] = s2.u;
-                sep[4 * q + 3] = s2.r;
-            }
+        if (!one) {
+            __syncthreads();
+            stage_rows<false>(st, rows, soff, ntiles, p0);
+            cp_async_wait_all();
+            __syncthreads();
         }
-    }
-    __syncthreads();
-    for (int p = threadIdx.x; p < Q; p += kSolveThreads) {
-        Row s2;
-        s2.l = sep[4 * p + 0];
-        s2.m = sep[4 * p + 1];
-        s2.u = sep[4 * p + 2];
-        s2.r = sep[4 * p + 3];
-        const Row w = reduced_row(s2, ends[6 * p + 3], ends[6 * p + 4], ends[6 * p + 5],
-                                  ends[6 * (p + 1) + 0], ends[6 * (p + 1) + 1],
-                                  ends[6 * (p + 1) + 2]);
-        L3[p] = w.l;
-        L3[Q + p] = w.m;
-        L3[2 * Q + p] = w.u;
-        L3[3 * Q + p] = w.r;
-    }
-    __syncthreads();
-    cta_partitioned<SplinePivot>(Q, L3, Q, x3, ws3);
-    double* xq = x3;
-    if (fits && !one) {  // the stage is filled again: the level-3 solution moves out of it
-        xq = ends;
-        for (int p = threadIdx.x; p < Q; p += kSolveThreads) xq[p] = x3[p];
-    }
-    for (int p0 = 0; p0 < P; p0 += kSolvePass) {
-        __syncthreads();
-        if (!one) stage_level2(st, src, p0, P);  // else: still staged from pass one
-        __syncthreads();
         const int q = p0 / kChunk + threadIdx.x;
         if (threadIdx.x < kSolveChunks && q <= Q) {
             const int first = q * kChunk;
             const int len = (q < Q) ? kChunk - 1 : P - first;
-            const double xl = (q > 0) ? xq[q - 1] : 0.0;
-            const double xr = (q < Q) ? xq[q] : 0.0;
-            const StageRowFn fn{&st, first - p0};
-            const StageSlots fac{st.u, first - p0};
+            const int i = kq(first - p0);
             if (one) {
-                chunk_interior_iw(len, fn, xl, xr, StageSlots{st.x, first}, fac);
-                if (q < Q) st.x[kq(first + kChunk - 1)] = xr;
+                ends_rows<true>(st.row + i, len, st.x + i, ends + 6 * q);
             } else {
-                chunk_interior_rolled(len, fn, xl, xr, StageSlots{st.r, first - p0}, fac);
-                if (q < Q) st.r[kq(first + kChunk - 1 - p0)] = xr;
+                ends_rows<false>(st.row + i, len, nullptr, ends + 6 * q);
+                if (q < Q) sep[q] = load_row(st.row + i + kChunk - 1);
             }
         }
+    }
+    __syncthreads();
+    for (int p = threadIdx.x; p < Q; p += kSolveThreads)
+        r3[kq(p)] = next_row(load_row(one ? st.row + kq(p * kChunk + kChunk - 1) : sep + p),
+                             ends + 6 * p);
+    __syncthreads();
+    partition_rows(Q, r3, x3, ws3);
+    if (fits && !one) {  // the stage is filled again: the level-3 solution moves out of it
+        for (int p = threadIdx.x; p < Q; p += kSolveThreads) ends[kq(p)] = x3[kq(p)];
+        x3 = ends;
+    }
+    for (int p0 = 0; p0 < P; p0 += kSolvePass) {
+        if (!one) {
+            __syncthreads();
+            stage_rows<false>(st, rows, soff, ntiles, p0);
+            cp_async_wait_all();
+            __syncthreads();
+        }
+        const int q = p0 / kChunk + threadIdx.x;
+        if (threadIdx.x < kSolveChunks && q <= Q) {
+            const int first = q * kChunk;
+            const int len = (q < Q) ? kChunk - 1 : P - first;
+            const double xl = (q > 0) ? x3[kq(q - 1)] : 0.0;
+            const double xr = (q < Q) ? x3[kq(q)] : 0.0;
+            SepRow* r = st.row + kq(first - p0);
+            if (one) {
+                double* x = st.x + kq(first);
+                interior_rows(r, len, xl, xr, x);
+                if (q < Q) x[kChunk - 1] = xr;
+            } else {  // the x plane is taken: the solution goes straight to X, row by row
+                double cp = 0.0, gp = 0.0;
+#pragma unroll 1
+                for (int k = 0; k < len; ++k) {
+                    const SepRow a = load_row(r + k);
+                    double ri = a.r;
+                    if (k == 0) ri = fma(-a.l, xl, ri);
+                    if (k == len - 1) ri = fma(-a.u, xr, ri);
+                    const double iw = pivot_inv(k == 0 ? a.m : fma(-a.l, cp, a.m));
+                    gp = (k == 0 ? ri : fma(-a.l, gp, ri)) * iw;
+                    cp = a.u * iw;
+                    r[k].u = cp;
+                    r[k].r = gp;
+                }
+                double xv = gp;
+                X[first + len - 1] = xv;
+#pragma unroll 1
+                for (int k = len - 2; k >= 0; --k) {
+                    xv = fma(-r[k].u, xv, r[k].r);
+                    X[first + k] = xv;
+                }
+                if (q < Q) X[first + kChunk - 1] = xr;
+            }
+        }
+    }
+    if (one) {
         __syncthreads();
-        const double* sol = one ? st.x : st.r;
-        for (int j = threadIdx.x; j < min(kSolvePass, P - p0); j += kSolveThreads)
-            X[p0 + j] = sol[kq(j)];
+        for (int p = threadIdx.x; p < P; p += kSolveThreads) X[p] = st.x[kq(p)];
     }
 }
 
@@ -1470,13 +1638,18 @@ k_spline_solve(const __grid_constant__ SiftArgs a) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     __shared__ int s_tab[3][kTabTiles + 1];
     __shared__ int s_scan[kSolveThreads / 32], s_k[kSolveThreads / 32], s_m[kSolveThreads / 32];
-    const int ra = active_rows(a);
+    RedStage& st = *reinterpret_cast<RedStage*>(dyn_smem);
     const int vs = blockIdx.x;
+    // one channel: the grid is its splines, and every load below is under way before the
+    // channel's done word is looked at
+    const int ra = a.nchan == 1 ? a.nr1 : active_rows(a);
     if (vs >= 2 * ra) return;
     int e;
     const Geo q = spline_geo(a, vs, ra, e);
-    if (a.mark[q.g] == 0) return;  // the row repeats its last iteration (k_tile_sift)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int done = a.nchan == 1 ? a.cs[0].done : 0, mark = a.mark[q.g];
+    const int c_first = tid < q.ntiles ? a.tile_cnt[tix(a, e, q, 0) + tid] : 0;
+    if (done || mark == 0) return;  // (0: the row repeats its last iteration, k_tile_sift)
     const int sp = spline_id(a, e, q);
     const int ntiles = q.ntiles;
     const size_t te0 = tix(a, e, q, 0);
@@ -1491,7 +1664,7 @@ k_spline_solve(const __grid_constant__ SiftArgs a) {
     int P = 0, NE = 0, K = 0, cm = 0;
     for (int t0 = 0; t0 < ntiles; t0 += kSolveThreads) {
         const int t = t0 + tid;
-        const int c = t < ntiles ? cnt[t] : 0;
+        const int c = t0 == 0 ? c_first : (t < ntiles ? cnt[t] : 0);
         const int own = tile_seps(c) | (c > 0 ? 0x10000 : 0);  // both sums stay below 2^16
         int incl = own;
 #pragma unroll
@@ -1531,6 +1704,8 @@ k_spline_solve(const __grid_constant__ SiftArgs a) {
         a.cmax[sp] = cm;
     }
     __syncthreads();
+    const bool one = P <= kSolvePass;
+    if (one) stage_rows<true>(st, rows, soff, ntiles, 0);
     // the first tile holds sample 0 and the last one sample n-1, so both have knots
     if (K > 5) {
         const bool l = cnt[0] < 6, r = cnt[ntiles - 1] < 6;
@@ -1555,33 +1730,34 @@ k_spline_solve(const __grid_constant__ SiftArgs a) {
         TileHdr hp, hn;
         if (i > 0) hp = hd[ne[i - 1]];
         if (i + 1 < NE) hn = hd[ne[i + 1]];
-        double2* row = reinterpret_cast<double2*>(rows + (size_t)t * (kRowSlots * 4));
+        const int k = tile_seps(c) - 1;
+        // (one pass: straight into the stage)
+        SepRow* row0 = one ? st.row + kq(soff[t])
+                           : reinterpret_cast<SepRow*>(rows) + (size_t)t * kRowSlots;
+        SepRow* row1 = one ? st.row + kq(soff[t] + k) : row0 + k;
         Row sr = identity_row();
         if (i > 0 && (c > 1 || i + 1 < NE)) {
             const int xp = c > 1 ? h.x1 : hn.x0;
             const double yp = c > 1 ? h.y1 : hn.y0;
-            sr = spline_row(hp.xb, h.x0, xp, seg_slope(hp.xb, h.x0, hp.yb, h.y0),
-                            seg_slope(h.x0, xp, h.y0, yp));
+            sr = spline_row(hp.xb, h.x0, xp, div_int(h.y0 - hp.yb, (double)(h.x0 - hp.xb)),
+                            div_int(yp - h.y0, (double)(xp - h.x0)));
         }
         Row o = c > 1 ? reduced_row(sr, 0.0, 1.0, 0.0, h.ga, h.aa, h.ba)
                       : reduced_row(sr, 0.0, 1.0, 0.0, 0.0, 0.0, 1.0);
-        row[0] = make_double2(o.l, o.m);
-        row[1] = make_double2(o.u, o.r);
+        *row0 = sep_row(o);
         if (c > 1) {
             sr = identity_row();
             if (i + 1 < NE)
-                sr = spline_row(h.xa, h.xb, hn.x0, seg_slope(h.xa, h.xb, h.ya, h.yb),
-                                seg_slope(h.xb, hn.x0, h.yb, hn.y0));
+                sr = spline_row(h.xa, h.xb, hn.x0, div_int(h.yb - h.ya, (double)(h.xb - h.xa)),
+                                div_int(hn.y0 - h.yb, (double)(hn.x0 - h.xb)));
             o = reduced_row(sr, h.gb, h.ab, h.bb, 0.0, 0.0, 1.0);
-            const int k = tile_seps(c) - 1;
-            row[2 * k] = make_double2(o.l, o.m);
-            row[2 * k + 1] = make_double2(o.u, o.r);
+            *row1 = sep_row(o);
         }
     }
+    if (one) cp_async_wait_all();
     __syncthreads();
     double* X = a.xsep + rec_base(a, e, q);
-    solve_separators(dyn_smem, a.solve_wcap, SepRows{rows, soff, ntiles}, P, X,
-                     a.red + red_base(a, e, q));
+    solve_separators(st, a.solve_wcap, rows, soff, ntiles, P, X, a.red + red_base(a, e, q));
     __syncthreads();
     // the knots just before and after every tile
     TileEdge* ed = a.edge + te0;
