@@ -159,19 +159,81 @@ k_adj_knots(const unsigned char* slot, TapeLayout L, int cap, int32_t* kx) {
 }
 
 // Segment sums of eb * t^p (p = 0..3) over segment s = (x_s, x_{s+1}] (sample 0 in segment 0),
-// in sample order; one thread per segment.  S: 4 planes of [2*nr][cap].
-__device__ __forceinline__ void adj_segsum_one(const Slot& v, const TapeLayout& L, int n, int cap,
-                                               const int32_t* kx, const double* eb, double* S,
-                                               int sp, int s) {
-    const int r = sp % L.nr;
-    if (s >= knots(v, sp, cap) - 1) return;
+// in sample order.  S: 4 planes of [2*nr][cap].  One thread per segment; when the spline has no
+// more segments than the grid has warps for it (segments of 64 samples and more on average), one
+// warp per segment: the lanes form the products of 32 samples, then four lanes, one per power,
+// add them in order.  The additions of a segment are one serial chain, so a long segment costs
+// its length times the time of a step: 34 cycles when one thread also forms the products, about
+// 10 as a lane's load and add (N = 8192: longest segments 242 us a launch, 55 as a warp).
+struct SegRange {
+    int x0, first, last;  // knot, samples first .. last (first > last: none)
+};
+__device__ __forceinline__ SegRange seg_range(const Slot& v, int n, int cap, const int32_t* kx,
+                                              int sp, int s) {
+    SegRange g{0, 1, 0};
+    if (s >= knots(v, sp, cap) - 1) return g;
     const int32_t* x = kx + (size_t)sp * cap;
-    const double* e = eb + (size_t)r * n;
     const int x0 = x[s], x1 = x[s + 1];
-    if (x0 < 0 || x1 >= n || x1 <= x0) return;  // knots increase inside 0..n-1
+    if (x0 < 0 || x1 >= n || x1 <= x0) return g;  // knots increase inside 0..n-1
+    g.x0 = x0;
+    g.first = s == 0 ? x0 : x0 + 1;
+    g.last = x1;
+    return g;
+}
+
+__global__ void __launch_bounds__(kAdjThreads)
+k_adj_segsums(const unsigned char* slot, TapeLayout L, int n, int cap, const int32_t* kx,
+              const double* eb, double* S) {
+    __shared__ double s_p[kAdjThreads / 32][4][34];
+    const Slot v = view(slot, L);
+    const int sp = blockIdx.y;
+    const int r = sp % L.nr;
+    if (!updated(v, L.nr, r)) return;
+    const double* e = eb + (size_t)r * n;
+    const size_t plane = (size_t)2 * L.nr * cap;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nseg = knots(v, sp, cap) - 1;
+    if (nseg <= (int)gridDim.x * (kAdjThreads / 32)) {
+        const int s = blockIdx.x * (kAdjThreads / 32) + warp;
+        const SegRange g = seg_range(v, n, cap, kx, sp, s);
+        if (g.first > g.last) return;
+        double(*p)[34] = s_p[warp];
+        double acc = 0.0;
+        double ev = g.first + lane <= g.last ? e[g.first + lane] : 0.0;
+        for (int i0 = g.first; i0 <= g.last; i0 += 32) {
+            const double t = (double)(i0 + lane - g.x0);
+            const double p1 = ev * t, p2 = p1 * t, p3 = p2 * t;
+            p[0][lane] = ev;
+            p[1][lane] = p1;
+            p[2][lane] = p2;
+            p[3][lane] = p3;
+            __syncwarp();
+            if (i0 + 32 + lane <= g.last) ev = e[i0 + 32 + lane];
+            if (lane < 4) {
+                const double2* q = reinterpret_cast<const double2*>(p[lane]);
+                const int m = min(32, g.last - i0 + 1);
+                if (m == 32) {
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) {
+                        const double2 w = q[k];
+                        acc = acc + w.x;
+                        acc = acc + w.y;
+                    }
+                } else {
+                    for (int k = 0; k < m; ++k) acc = acc + p[lane][k];
+                }
+            }
+            __syncwarp();
+        }
+        if (lane < 4) S[lane * plane + (size_t)sp * cap + s] = acc;
+        return;
+    }
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const SegRange g = seg_range(v, n, cap, kx, sp, s);
+    if (g.first > g.last) return;
     double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    for (int i = s == 0 ? x0 : x0 + 1; i <= x1; ++i) {
-        const double t = (double)(i - x0);
+    for (int i = g.first; i <= g.last; ++i) {
+        const double t = (double)(i - g.x0);
         const double ev = e[i];
         const double p1 = ev * t, p2 = p1 * t, p3 = p2 * t;
         a0 = a0 + ev;
@@ -179,21 +241,11 @@ __device__ __forceinline__ void adj_segsum_one(const Slot& v, const TapeLayout& 
         a2 = a2 + p2;
         a3 = a3 + p3;
     }
-    const size_t plane = (size_t)2 * L.nr * cap;
     double* o = S + (size_t)sp * cap + s;
     o[0] = a0;
     o[plane] = a1;
     o[2 * plane] = a2;
     o[3 * plane] = a3;
-}
-
-__global__ void __launch_bounds__(kAdjThreads)
-k_adj_segsums(const unsigned char* slot, TapeLayout L, int n, int cap, const int32_t* kx,
-              const double* eb, double* S) {
-    const Slot v = view(slot, L);
-    const int sp = blockIdx.y;
-    if (!updated(v, L.nr, sp % L.nr)) return;
-    adj_segsum_one(v, L, n, cap, kx, eb, S, sp, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // Transposed coefficient maps (a = y_s, b = (y_{s+1}-y_s)/h - h(2c_s+c_{s+1})/3, c = c_s,
@@ -257,7 +309,7 @@ k_adj_rows(const unsigned char* slot, TapeLayout L, int cap, const int32_t* kx, 
 
 // Transposed spline solve: one CTA per spline, the canonical partitioned solve.
 __global__ void __launch_bounds__(kAdjThreads)
-k_adj_solve(const unsigned char* slot, TapeLayout L, int cap, double* sys, double* z,
+k_adj_solve(const unsigned char* slot, TapeLayout L, int cap, const double* sys, double* z,
             double* ws, size_t ws_stride) {
     const Slot v = view(slot, L);
     const int sp = blockIdx.x;

@@ -590,8 +590,13 @@ ceemdan_status backward_impl(const ceemdan_tape& T, const double* g, double* gy,
         if (std::strcmp(e, "grid") == 0) grid_solve = true;
         if (std::strcmp(e, "cta") == 0) grid_solve = false;
     }
+    // a spline's system in one CTA's shared memory when it fits (n up to about 16,000)
+    const bool smem_solve = !grid_solve && adj_solve_smem(cap) <= kAdjSolveSmem;
+    if (smem_solve)
+        CK(cudaFuncSetAttribute(k_adj_solve_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)kAdjSolveSmem));
     int* nrows = nullptr;
-    if (grid_solve) CKS(ws.alloc_n(&nrows, (size_t)nsp));
+    if (grid_solve || smem_solve) CKS(ws.alloc_n(&nrows, (size_t)nsp));
     CK(cudaMemsetAsync(gm, 0, rn * sizeof(double), st));
     CK(cudaMemsetAsync(scal, 0, 8 * sizeof(double), st));
     CK(cudaMemcpyAsync(fbar, g + ns * T.n, T.n * sizeof(double), cudaMemcpyDeviceToDevice, st));
@@ -680,6 +685,9 @@ ceemdan_status backward_impl(const ceemdan_tape& T, const double* g, double* gy,
                     CK(psolve_launch(bsp, cap, nrows, sys, cap, z, wsp, ws_stride, st, &nl,
                                      kx));
                     g_launches += (uint64_t)nl - 1;
+                } else if (smem_solve) {
+                    k_adj_solve_smem<<<(unsigned)bsp, kThreads, adj_solve_smem(cap), st>>>(
+                        nrows, cap, kx, sys + 3 * (size_t)cap, 4 * (size_t)cap, z);
                 } else {
                     k_adj_solve<<<(unsigned)bsp, kThreads, 0, st>>>(slot, L, cap, sys, z, wsp,
                                                                     ws_stride);

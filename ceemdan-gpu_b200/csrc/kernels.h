@@ -248,17 +248,22 @@ __global__ void k_tridiag_batched(int n, const double* l, const double* m, const
                                   const double* r, double* x, double* sys, double* ws,
                                   size_t ws_stride);
 // In-CTA canonical partitioned solve (sift_kernels.cu): system in 4 planes of `plane` doubles
-// (l, m, u, r) at sys (u is overwritten), solution to x, workspace ws of >= 0.75*n + 16 doubles; every thread of
+// (l, m, u, r) at sys, solution to x, workspace ws of >= 0.75*n + 16 doubles; every thread of
 // the CTA calls it.
-__device__ void cta_tridiag(int n, double* sys, int plane, double* x, double* ws);
+__device__ void cta_tridiag(int n, const double* sys, int plane, double* x, double* ws);
 // the same solve of a spline system (pivots in pivot_inv's range)
-__device__ void cta_spline_tridiag(int n, double* sys, int plane, double* x, double* ws);
+__device__ void cta_spline_tridiag(int n, const double* sys, int plane, double* x, double* ws);
 // cta_spline_tridiag's solve for nsys systems at once, one level per launch (sift_kernels.cu)
 cudaError_t psolve_launch(int nsys, int max_rows, const int* nrows, const double* sys, int plane,
                           double* x, double* ws, size_t ws_stride, cudaStream_t st,
                           int* launches, const int32_t* kx);
 
-// reverse pass (adjoint.cu)
+// reverse pass (adjoint.cu; k_adj_solve_smem: sift_kernels.cu)
+// shared memory of k_adj_solve_smem for splines of up to cap knots, and the most it may take
+size_t adj_solve_smem(int cap);
+constexpr size_t kAdjSolveSmem = (size_t)227 * 1024;
+__global__ void k_adj_solve_smem(const int* nrows, int cap, const int32_t* kx, const double* rhs,
+                                 size_t stride, double* z);
 __global__ void k_tape_record(SiftArgs a, TapeLayout L, unsigned char* slot);
 __global__ void k_adj_seed(const unsigned char* slot, TapeLayout L, int n, double* gh,
                            double* gm, double* eb, const double* abar, double inr);
@@ -267,7 +272,7 @@ __global__ void k_adj_segsums(const unsigned char* slot, TapeLayout L, int n, in
                               const int32_t* kx, const double* eb, double* S);
 __global__ void k_adj_rows(const unsigned char* slot, TapeLayout L, int cap, const int32_t* kx,
                            const double* S, double* yb, double* sys, int* nrows);
-__global__ void k_adj_solve(const unsigned char* slot, TapeLayout L, int cap, double* sys,
+__global__ void k_adj_solve(const unsigned char* slot, TapeLayout L, int cap, const double* sys,
                             double* z, double* ws, size_t ws_stride);
 __global__ void k_adj_rhs(const unsigned char* slot, TapeLayout L, int cap, const int32_t* kx,
                           const double* yb, const double* z, double* y2);

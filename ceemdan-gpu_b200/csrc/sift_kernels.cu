@@ -206,6 +206,26 @@ __device__ __forceinline__ ChunkEnds chunk_ends(int len, const RowFn& row, const
     return e;
 }
 
+// x(k) <- x(k) - fac(k) x(k+1) from row len-2 down, x(len-1) = xv; loads one row ahead.
+template <class X, class Fac>
+__device__ __forceinline__ void back_sweep(int len, double xv, const X& x, const Fac& fac) {
+    double f = 0.0, g = 0.0;
+    if (len > 1) {
+        f = fac(len - 2);
+        g = x(len - 2);
+    }
+#pragma unroll 1
+    for (int k = len - 2; k >= 0; --k) {
+        const double fc = f, gc = g;
+        if (k > 0) {
+            f = fac(k - 1);
+            g = x(k - 1);
+        }
+        xv = fma(-fc, xv, gc);
+        x(k) = xv;
+    }
+}
+
 // Interior of a chunk whose end relations chunk_ends formed: coupling terms to the right-hand
 // side, then canonical Thomas with the reciprocals left in x(k); x(k) receives the solution,
 // fac(k) the factors meanwhile (fac(k) may be row k's own u or a slot of it that rows after k do
@@ -230,12 +250,7 @@ __device__ __forceinline__ void chunk_interior_iw(int len, const RowFn& row, dou
         fac(k) = wc.u * ic;
         x(k) = gp;
     }
-    double xv = gp;
-#pragma unroll 1
-    for (int k = len - 2; k >= 0; --k) {
-        xv = fma(-fac(k), xv, x(k));
-        x(k) = xv;
-    }
+    back_sweep(len, gp, x, fac);
 }
 
 // Canonical Thomas on n <= kChunk rows, solution to x(k), factors to fac(k) meanwhile.
@@ -254,39 +269,7 @@ __device__ __forceinline__ void thomas_rolled(int n, const RowFn& row, const X& 
         fac(k) = cp;
         x(k) = gp;
     }
-    double xv = gp;
-#pragma unroll 1
-    for (int k = n - 2; k >= 0; --k) {
-        xv = fma(-fac(k), xv, x(k));
-        x(k) = xv;
-    }
-}
-
-// chunk_interior_iw without stored reciprocals (the same values, formed again).
-template <class RowFn, class X, class Fac>
-__device__ __forceinline__ void chunk_interior_rolled(int len, const RowFn& row, double xl,
-                                                      double xr, const X& x, const Fac& fac) {
-    Row w = row(0);
-    double cp = 0.0, gp = 0.0;
-#pragma unroll 1
-    for (int k = 0; k < len; ++k) {
-        const Row wc = w;
-        if (k + 1 < len) w = row(k + 1);
-        double ri = wc.r;
-        if (k == 0) ri = fma(-wc.l, xl, ri);
-        if (k == len - 1) ri = fma(-wc.u, xr, ri);
-        const double iw = pivot_inv(k == 0 ? wc.m : fma(-wc.l, cp, wc.m));
-        gp = k == 0 ? ri * iw : fma(-wc.l, gp, ri) * iw;
-        cp = wc.u * iw;
-        fac(k) = cp;
-        x(k) = gp;
-    }
-    double xv = gp;
-#pragma unroll 1
-    for (int k = len - 2; k >= 0; --k) {
-        xv = fma(-fac(k), xv, x(k));
-        x(k) = xv;
-    }
+    back_sweep(n, gp, x, fac);
 }
 
 // Consecutive doubles as a row-indexed destination; NoIw drops what it is given.
@@ -988,13 +971,104 @@ __device__ void cta_partitioned(int n, double* sys, int plane, double* x, double
     }
 }
 
+// In-CTA canonical partitioned solve of an explicit system in global memory (its sweeps keep their
+// factors in registers: a factor read back from memory would cost a round trip a row) stored at sys (4 planes of
+// `plane` doubles: l, m, u, r), solution to x.  ws: workspace for the deeper levels
+// (<= 0.75*n + 16 doubles).  All threads of the CTA must call it.
+template <class Pivot>
+__device__ void cta_partitioned_global(int n, const double* sys, int plane, double* x, double* ws) {
+    int sizes[8];
+    int depth = 0;
+    sizes[0] = n;
+    while (sizes[depth] > kChunk && depth < 7) {
+        sizes[depth + 1] = (sizes[depth] - 1) / kChunk;
+        ++depth;
+    }
+    const double* lv[8];
+    double* xv[8];
+    int off = 0;
+    lv[0] = sys;
+    for (int k = 1; k <= depth; ++k) {
+        lv[k] = ws + off;
+        off += 4 * sizes[k];
+    }
+    xv[0] = x;
+    for (int k = 1; k <= depth; ++k) {
+        xv[k] = ws + off;
+        off += sizes[k];
+    }
+    double* ends = ws + off;  // 6 * (chunks of the widest level)
+    for (int k = 0; k < depth; ++k) {
+        const int nk = sizes[k];
+        const int P = sizes[k + 1];
+        const int pl = (k == 0) ? plane : nk;
+        const double* L = lv[k];
+        for (int q = threadIdx.x; q <= P; q += blockDim.x) {
+            const int first = q * kChunk;
+            const int len = (q < P) ? kChunk - 1 : nk - first;
+            GlobalRowFn fn{L, L + pl, L + 2 * pl, L + 3 * pl, first};
+            const ChunkEnds ce = chunk_ends<Pivot>(len, fn, NoIw());
+            ends[6 * q + 0] = ce.ga;
+            ends[6 * q + 1] = ce.aa;
+            ends[6 * q + 2] = ce.ba;
+            ends[6 * q + 3] = ce.gb;
+            ends[6 * q + 4] = ce.ab;
+            ends[6 * q + 5] = ce.bb;
+        }
+        __syncthreads();
+        double* R = const_cast<double*>(lv[k + 1]);
+        for (int p = threadIdx.x; p < P; p += blockDim.x) {
+            const int s = p * kChunk + kChunk - 1;
+            Row sr;
+            sr.l = L[s];
+            sr.m = L[pl + s];
+            sr.u = L[2 * pl + s];
+            sr.r = L[3 * pl + s];
+            const Row o = reduced_row(sr, ends[6 * p + 3], ends[6 * p + 4], ends[6 * p + 5],
+                                      ends[6 * (p + 1) + 0], ends[6 * (p + 1) + 1],
+                                      ends[6 * (p + 1) + 2]);
+            R[p] = o.l;
+            R[P + p] = o.m;
+            R[2 * P + p] = o.u;
+            R[3 * P + p] = o.r;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        const int nb = sizes[depth];
+        const int pl = (depth == 0) ? plane : nb;
+        const double* L = lv[depth];
+        GlobalRowFn fn{L, L + pl, L + 2 * pl, L + 3 * pl, 0};
+        thomas_small<Pivot>(nb, fn, xv[depth], 1);
+    }
+    __syncthreads();
+    for (int k = depth - 1; k >= 0; --k) {
+        const int nk = sizes[k];
+        const int P = sizes[k + 1];
+        const int pl = (k == 0) ? plane : nk;
+        const double* L = lv[k];
+        const double* Xs = xv[k + 1];
+        double* xo = xv[k];
+        for (int q = threadIdx.x; q <= P; q += blockDim.x) {
+            const int first = q * kChunk;
+            const int len = (q < P) ? kChunk - 1 : nk - first;
+            GlobalRowFn fn{L, L + pl, L + 2 * pl, L + 3 * pl, first};
+            const double xl = (q > 0) ? Xs[q - 1] : 0.0;
+            const double xr = (q < P) ? Xs[q] : 0.0;
+            chunk_interior<true, Pivot>(len, fn, xl, xr, xo + first, 1);
+            if (q < P) xo[first + kChunk - 1] = xr;
+        }
+        __syncthreads();
+    }
+}
+
 }  // namespace
 
-__device__ void cta_tridiag(int n, double* sys, int plane, double* x, double* ws) {
-    cta_partitioned<AnyPivot>(n, sys, plane, x, ws);
+__device__ void cta_tridiag(int n, const double* sys, int plane, double* x, double* ws) {
+    cta_partitioned_global<AnyPivot>(n, sys, plane, x, ws);
 }
-__device__ void cta_spline_tridiag(int n, double* sys, int plane, double* x, double* ws) {
-    cta_partitioned<SplinePivot>(n, sys, plane, x, ws);
+__device__ void cta_spline_tridiag(int n, const double* sys, int plane, double* x, double* ws) {
+    cta_partitioned_global<SplinePivot>(n, sys, plane, x, ws);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1429,6 +1503,30 @@ __device__ void partition_rows(int n, SepRow* rows, double* x, double* ws) {
     }
 }
 
+// Rows of a spline's transposed system from its knot positions and right-hand side in padded
+// shared memory (KnotSysRows' values).
+struct StagedKnotRows {
+    const int* x;
+    const double* r;
+    int K, first;
+    __device__ __forceinline__ Row operator()(int k) const {
+        const int i = first + k;
+        if (i == 0 || i == K - 1) return identity_row();
+        const int x0 = x[kq(i)], dl = x0 - x[kq(i - 1)], du = x[kq(i + 1)] - x0;
+        Row w;
+        w.l = (double)dl;
+        w.m = (double)(2 * (dl + du));
+        w.u = (double)du;
+        w.r = r[kq(i)];
+        return w;
+    }
+};
+struct PadSlots17 {
+    double* p;  // padded array
+    int first;
+    __device__ __forceinline__ double& operator()(int k) const { return p[kq(first + k)]; }
+};
+
 // Asynchronous copies of the rows p0 .. p0 + kSolvePass - 1 of a spline's separator system from
 // their tiles' slots (separator p is separator p - soff[t] of tile t) into the stage: eight
 // threads per tile.  kInner: without the tiles' first and last rows.
@@ -1562,6 +1660,79 @@ __device__ __forceinline__ void solve_separators(RedStage& st, int wcap, const d
         for (int p = threadIdx.x; p < P; p += kSolveThreads) X[p] = st.x[kq(p)];
     }
 }
+
+}  // namespace
+
+// Transposed spline solve of the reverse pass in shared memory, one CTA per spline of nrows[s]
+// knots (0: none): positions kx, right-hand side rhs (rows s of `stride` doubles), solution to z;
+// cta_partitioned's operations in the same order.  The global-memory form spent its time in
+// round trips of its sweeps (N = 8192, white noise: 37 us a solve against X here).
+size_t adj_solve_smem(int cap) {
+    const int P = cap / kChunk + 1;
+    return sizeof(double) * (2 * (size_t)padded(cap) + 5 * (size_t)padded(P) + 6 * (size_t)(P + 1) +
+                             (size_t)P + 80) +
+           sizeof(int) * ((size_t)padded(cap) + 4);
+}
+
+__global__ void __launch_bounds__(kThreads)
+k_adj_solve_smem(const int* nrows, int cap, const int32_t* kx, const double* rhs, size_t stride,
+                 double* z) {
+    extern __shared__ __align__(16) unsigned char dyn_smem[];
+    const int sp = blockIdx.x;
+    const int K = nrows[sp];
+    if (K <= 0) return;
+    const int P = (K - 1) / kChunk;
+    SepRow* r2 = reinterpret_cast<SepRow*>(dyn_smem);
+    const int cp2 = cap / kChunk + 1;
+    double* x2 = reinterpret_cast<double*>(r2 + padded(cp2));
+    double* ends = x2 + ((padded(cp2) + 1) & ~1);
+    double* ws = ends + 6 * (cp2 + 1);
+    double* R = ws + ((cp2 + 65) & ~1);
+    double* Z = R + padded(cap);
+    int* X = reinterpret_cast<int*>(Z + padded(cap));
+    const int32_t* x = kx + (size_t)sp * cap;
+    const double* r = rhs + (size_t)sp * stride;
+    for (int i = threadIdx.x; i < K; i += kThreads) {
+        X[kq(i)] = x[i];
+        R[kq(i)] = r[i];
+    }
+    __syncthreads();
+    if (K <= kChunk) {
+        if (threadIdx.x == 0)
+            thomas_rolled(K, StagedKnotRows{X, R, K, 0}, PadSlots17{Z, 0}, PadSlots17{R, 0});
+    } else {
+        for (int q = threadIdx.x; q <= P; q += kThreads) {
+            const int first = q * kChunk, len = (q < P) ? kChunk - 1 : K - first;
+            const ChunkEnds e =
+                chunk_ends(len, StagedKnotRows{X, R, K, first}, PadSlots17{Z, first});
+            double* o = ends + 6 * q;
+            o[0] = e.ga;
+            o[1] = e.aa;
+            o[2] = e.ba;
+            o[3] = e.gb;
+            o[4] = e.ab;
+            o[5] = e.bb;
+        }
+        __syncthreads();
+        for (int p = threadIdx.x; p < P; p += kThreads)
+            r2[kq(p)] = next_row(
+                sep_row(StagedKnotRows{X, R, K, 0}(p * kChunk + kChunk - 1)), ends + 6 * p);
+        __syncthreads();
+        partition_rows(P, r2, x2, ws);
+        for (int q = threadIdx.x; q <= P; q += kThreads) {
+            const int first = q * kChunk, len = (q < P) ? kChunk - 1 : K - first;
+            const double xl = (q > 0) ? x2[kq(q - 1)] : 0.0, xr = (q < P) ? x2[kq(q)] : 0.0;
+            chunk_interior_iw(len, StagedKnotRows{X, R, K, first}, xl, xr, PadSlots17{Z, first},
+                              PadSlots17{R, first});
+            if (q < P) Z[kq(first + kChunk - 1)] = xr;
+        }
+    }
+    __syncthreads();
+    double* out = z + (size_t)sp * cap;
+    for (int i = threadIdx.x; i < K; i += kThreads) out[i] = Z[kq(i)];
+}
+
+namespace {
 
 // The end rule of a spline whose first (side 0) or last (side 1) tile holds fewer than six
 // knots: the three end knots come from the tiles' headers, the tile's chunk is eliminated again
@@ -2408,7 +2579,7 @@ k_tridiag_batched(int n, const double* l, const double* m, const double* u, cons
         S[3 * n + i] = r[b * n + i];
     }
     __syncthreads();
-    cta_partitioned<AnyPivot>(n, S, n, x + b * n, ws + b * ws_stride);
+    cta_partitioned_global<AnyPivot>(n, S, n, x + b * n, ws + b * ws_stride);
 }
 
 // =======================================================================================
