@@ -38,23 +38,6 @@ static_assert(kErrTimeout == CEEMDAN_ERR_TIMEOUT, "the kernels' timeout code is 
 thread_local std::string g_last_error;
 std::atomic<uint64_t> g_launches{0};
 
-
-
-// RN(1/h) and RN(1/(3h)) for h = 0..kRcpMax (entry 0 unused): the reciprocals the evaluation
-// and spline kernels divide with (div_rcp gives correctly rounded quotients from them).
-const double* rcp_tables() {
-    // initialised once, thread-safe (concurrent decompositions from several host threads)
-    static const std::vector<double> tab = [] {
-        std::vector<double> t(2 * (kRcpMax + 1), 0.0);
-        for (int h = 1; h <= kRcpMax; ++h) {
-            t[h] = 1.0 / (double)h;
-            t[kRcpMax + 1 + h] = 1.0 / (3.0 * (double)h);
-        }
-        return t;
-    }();
-    return tab.data();
-}
-
 int sm_count() {
     static const int sms = [] {
         int dev = 0, n = 0;

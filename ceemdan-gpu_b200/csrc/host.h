@@ -47,7 +47,11 @@ template <bool kDense, bool kEnv>
 __global__ void k_tile_sift(const __grid_constant__ SiftArgs a);
 __global__ void k_spline_solve(const __grid_constant__ SiftArgs a);
 
-const double* rcp_tables();
+// the on-chip stage kernel, in one of its three forms
+template <int kMode>
+__global__ void k_sift_small(const __grid_constant__ SiftArgs a,
+                             const __grid_constant__ SmallArgs sa);
+
 int sm_count();
 cudaMemPool_t engine_pool();
 ceemdan_status pool_alloc(void** p, size_t bytes, cudaStream_t st);
@@ -280,12 +284,6 @@ struct SiftEngine {
         // (k_tile_sift copies a whole tile's slots from a tile's first separator on)
         CKS(ws.alloc_n(&a.xsep, 2 * (size_t)rec + kRowSlots));
         CKS(ws.alloc_n(&a.red, 2 * (size_t)red));
-        double* rcp = nullptr;
-        CKS(ws.alloc_n(&rcp, 2 * (size_t)(kRcpMax + 1)));
-        CK(cudaMemcpyAsync(rcp, rcp_tables(), sizeof(double) * 2 * (kRcpMax + 1),
-                           cudaMemcpyHostToDevice, ws.st));
-        a.rcp_h = rcp;
-        a.rcp_3h = rcp + (kRcpMax + 1);
         Chan* dchan = nullptr;
         CKS(ws.alloc_n(&dchan, (size_t)nchan));
         CK(cudaMemcpyAsync(dchan, hchan.data(), sizeof(Chan) * nchan, cudaMemcpyHostToDevice,
@@ -476,37 +474,77 @@ struct SiftEngine {
     // a stage runs as one cooperative launch of k_sift_small instead of groups of iterations.
     bool small = false;
     SmallArgs sa{};
-    size_t small_smem = 0;
+    int small_mode = -1;
+
+    // Launch configuration of the on-chip kernel in form `mode` (attributes in `at`).
+    cudaLaunchConfig_t small_config(int mode, cudaLaunchAttribute* at, cudaStream_t st) const {
+        cudaLaunchConfig_t c{};
+        c.gridDim = dim3((unsigned)(mode == kSmallPair ? 2 * nr : nr));
+        c.blockDim = dim3(kSmallThreads);
+        // the CTAs are latency-bound: when the launch has at most one CTA per SM, ask for more
+        // than half an SM's shared memory so that no two of them share an SM
+        c.dynamicSmemBytes = small_sift_smem(n, mode);
+        if ((int)c.gridDim.x <= sm_count())
+            c.dynamicSmemBytes = std::max(c.dynamicSmemBytes, (size_t)kSmallSpreadSmem);
+        c.stream = st;
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        at[1].id = cudaLaunchAttributeClusterDimension;
+        at[1].val.clusterDim.x = 2;
+        at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+        c.attrs = at;
+        c.numAttrs = mode == kSmallPair ? 2 : 1;
+        return c;
+    }
+    static const void* small_kernel(int mode) {
+        return mode == kSmallPair   ? (const void*)k_sift_small<kSmallPair>
+               : mode == kSmallDual ? (const void*)k_sift_small<kSmallDual>
+                                    : (const void*)k_sift_small<kSmallSingle>;
+    }
 
     ceemdan_status enable_small(Workspace& ws, int max_cap, int spin_limit) {
         if (a.nchan != 1 || n > kSmallMaxN) return CEEMDAN_OK;
         if (const char* e = std::getenv("CEEMDAN_SMALL"))
             if (e[0] == '0') return CEEMDAN_OK;
-        int dev = 0, coop = 0, sms = 0, per = 0;
+        int dev = 0, coop = 0, most = 0, per = 0;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        CK(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
         if (!coop) return CEEMDAN_OK;
-        small_smem = small_sift_smem(n);
-        CK(cudaFuncSetAttribute(k_sift_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)small_sift_smem(kSmallMaxN)));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sift_small, kSmallThreads,
-                                                         small_smem));
-        if (per < 1 || nr > per * sms) return CEEMDAN_OK;
-        // two CTAs per realization when they fit one per SM (CEEMDAN_SMALL_PAIR=0: one CTA)
-        sa.pair = 2 * nr <= sms ? 1 : 0;
-        if (const char* e = std::getenv("CEEMDAN_SMALL_PAIR"))
-            if (e[0] == '0') sa.pair = 0;
-        // the CTAs are latency-bound: when the launch has at most one CTA per SM, ask for more
-        // than half an SM's shared memory so that no two of them share an SM
-        if ((sa.pair ? 2 * nr : nr) <= sms)
-            small_smem = std::max(small_smem, (size_t)kSmallSpreadSmem);
-        CKS(ws.alloc_n(&sa.ready, (size_t)nr));
-        CKS(ws.alloc_n(&sa.pair_kmax, (size_t)nr));
-        CKS(ws.alloc_n(&sa.pair_mark, (size_t)nr));
-        CKS(ws.alloc_n(&sa.arrive, 1));
-        CKS(ws.alloc_n(&sa.nfin, (size_t)std::max(1, max_cap)));
-        CKS(ws.alloc_n(&sa.up, (size_t)nr * row_ld(n)));
+        // The statically declared shared memory counts too; the attribute is the same for every
+        // size, so that concurrent calls of other sizes agree on it.
+        const size_t room = (size_t)most - 4096;
+        for (int m : {kSmallPair, kSmallDual, kSmallSingle})
+            CK(cudaFuncSetAttribute(small_kernel(m), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)room));
+        // Two CTAs per realization when they fit one per SM as clusters (CEEMDAN_SMALL_PAIR=0:
+        // one CTA); else both envelopes side by side in one CTA when the shared memory holds
+        // them (rows of up to about 5000 samples), else one after the other.
+        small_mode = -1;
+        const char* pe = std::getenv("CEEMDAN_SMALL_PAIR");
+        cudaLaunchAttribute at[2];
+        if (2 * nr <= sm_count() && !(pe && pe[0] == '0') &&
+            small_sift_smem(n, kSmallPair) <= room) {
+            cudaLaunchConfig_t c = small_config(kSmallPair, at, nullptr);
+            c.attrs = at + 1;  // the cluster dimension alone
+            c.numAttrs = 1;
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, small_kernel(kSmallPair), &c) ==
+                    cudaSuccess &&
+                clusters >= nr)
+                small_mode = kSmallPair;
+            cudaGetLastError();
+        }
+        for (int m : {kSmallDual, kSmallSingle}) {
+            if (small_mode >= 0 || small_sift_smem(n, m) > room) continue;
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                &per, small_kernel(m), kSmallThreads,
+                small_config(m, at, nullptr).dynamicSmemBytes));
+            if (per >= 1 && nr <= per * sm_count()) small_mode = m;
+        }
+        if (small_mode < 0) return CEEMDAN_OK;
+        CKS(ws.alloc_n(&sa.arrive, (size_t)std::max(1, max_cap)));
+        if (small_mode == kSmallSingle) CKS(ws.alloc_n(&sa.up, (size_t)nr * row_ld(n)));
         // device copy of a taped stage's block table (blocks of kTapeBlockSlots slots)
         CKS(ws.alloc_n(&tblocks_dev, (size_t)(std::max(1, max_cap) + kTapeBlockSlots - 1) /
                                          kTapeBlockSlots));
@@ -537,15 +575,14 @@ struct SiftEngine {
         }
         k_begin_stage<<<1, kThreads, 0, st>>>(a, 0, cap, mode_out);
         ++g_launches;
-        CK(cudaMemsetAsync(sa.arrive, 0, sizeof(unsigned), st));
-        CK(cudaMemsetAsync(sa.ready, 0, sizeof(unsigned) * (size_t)nr, st));
-        CK(cudaMemsetAsync(sa.nfin, 0, sizeof(int) * (size_t)std::min(cap, small_cap), st));
+        CK(cudaMemsetAsync(sa.arrive, 0, sizeof(*sa.arrive) * (size_t)std::min(cap, small_cap),
+                           st));
         void* args[] = {(void*)&a, (void*)&sa};
         cudaEvent_t* sev = kernel_ms ? &ev[ev.size() - 2] : nullptr;
         if (sev) CK(cudaEventRecord(sev[0], st));
-        CK(cudaLaunchCooperativeKernel((const void*)k_sift_small,
-                                       dim3((unsigned)(sa.pair ? 2 * nr : nr)),
-                                       dim3(kSmallThreads), args, small_smem, st));
+        cudaLaunchAttribute at[2];
+        const cudaLaunchConfig_t cfg = small_config(small_mode, at, st);
+        CK(cudaLaunchKernelExC(&cfg, small_kernel(small_mode), args));
         ++g_launches;
         if (sev) CK(cudaEventRecord(sev[1], st));
         CK(cudaMemcpyAsync(hstate, state, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -10,7 +10,6 @@ namespace ceemdan {
 constexpr int kTileSamples = 2048;  // samples per extrema / evaluation tile
 constexpr int kRowSlots = 66;       // separator rows per tile and envelope (at most 65)
 constexpr int kEndKnots = 6;        // knots kept of a sparse end tile (at most 5)
-constexpr int kRcpMax = 4096;       // reciprocal tables cover knot spacings 1..kRcpMax
 
 // Stride of a row of n samples in the engine's own planes (h, mean envelope): a multiple of four
 // samples, so that every thread's groups of four are 32-byte aligned whatever n is.
@@ -130,8 +129,6 @@ struct SiftArgs {
     // knots of a spline's first and last tile when they are fewer than six [2*nrows][2][kEndKnots]
     int* end_x;
     double* end_y;
-    const double* rcp_h;   // [kRcpMax+1] RN(1/h)
-    const double* rcp_3h;  // [kRcpMax+1] RN(1/(3h))
     double* xsep;          // [2*rec_total] spline values at the separators
     double* red;           // [2*red_total] reduced-solve workspace
     double* dbg_upper;     // optional envelope outputs (stage-level entry point, one channel)
@@ -169,12 +166,17 @@ struct BatchArgs {
     int* finished;             // channels that have finished every stage
 };
 
-// Short rows: the whole lock-step sift of a stage in one cooperative launch, one CTA per
-// realization of channel 0 (k_sift_small).  Grid-wide state of the launch, zeroed per stage.
+// Short rows: the whole lock-step sift of a stage in one cooperative launch (sift_small.cu), in one
+// of three forms.
 constexpr int kSmallMaxN = 8192;       // longest row the on-chip path takes
 constexpr int kSmallThreads = 512;
-constexpr int kSmallPre = 8;  // samples per thread whose global loads k_sift_small issues at once
+constexpr int kSmallPair = 0, kSmallDual = 1, kSmallSingle = 2;
 constexpr int kSmallSpreadSmem = 120 * 1024;  // dynamic shared memory that fits one CTA per SM
+// samples of a row that the first CTA of a pair combines
+__host__ __device__ inline int small_half(int n) {
+    const int h = ((n + 1) / 2 + 31) & ~31;
+    return h < n ? h : n;
+}
 constexpr int kErrTimeout = 5;         // CEEMDAN_ERR_TIMEOUT, written to ChanState.err
 // Per-spline stride of the reduced-solve workspace.
 __host__ __device__ inline long long red_stride_of(int rec_stride) {
@@ -202,23 +204,17 @@ inline TapeLayout tape_layout(int nr, int ntiles) {
 
 // The on-chip stage kernel's own arguments (k_sift_small).
 struct SmallArgs {
-    unsigned* arrive;      // [1] CTAs arrived at the stop test, all iterations of the stage
-    int* nfin;             // [cap] realizations finished after each iteration
-    double* up;            // [nrows*n] upper envelope of the current iteration
-    int spin_limit;        // polls of the stop-test barrier before giving up (CEEMDAN_ERR_TIMEOUT)
-    unsigned extra;        // arrivals the barrier waits for beyond the launch's CTAs: 0, or 1 to
-                           // make every wait give up (the timeout path's test)
+    // [cap] per iteration: realizations arrived at the stop test, and in the high word those of
+    // them that have finished; zeroed per stage
+    unsigned long long* arrive;
+    double* up;            // [nrows*row_ld(n)] upper envelope of the iteration (kSmallSingle)
+    int spin_limit;        // polls of the stop test before giving up (CEEMDAN_ERR_TIMEOUT)
+    unsigned extra;        // arrivals the test waits for beyond the realizations: 0, or 1 to make
+                           // every wait give up (the timeout path's test)
     // taped forward: the stage's tape blocks (slot j at tblocks[j / kTapeBlockSlots] +
     // (j % kTapeBlockSlots) * tl.stride), null otherwise
     unsigned char* const* tblocks;
     TapeLayout tl;
-    // two CTAs per realization (upper / lower envelope) when the launch has room for them:
-    // per realization the iteration whose upper envelope is ready, its knot count, and the
-    // stop decision's mark for the upper CTA
-    int pair;
-    unsigned* ready;
-    int* pair_kmax;
-    int* pair_mark;
 };
 constexpr int kTapeBlockSlots = 32;  // tape slots per allocation block
 
@@ -289,8 +285,7 @@ __global__ void k_adj_out(int stage, const double* g, const double* hs, const do
                           double inv_n);
 
 // dynamic shared memory of k_sift_small for rows of n samples
-size_t small_sift_smem(int n);
-__global__ void k_sift_small(SiftArgs a, SmallArgs sa);
+size_t small_sift_smem(int n, int mode);
 
 // k_spline_solve: threads per CTA, chunks swept per pass over the staged rows, dynamic shared
 // memory (the stage of 87,088 bytes and the level-3 workspace; two CTAs per SM).

@@ -18,13 +18,13 @@
 // knots from its samples and bitmap.  An iteration moves 8 N bytes in k_tile_knots and 24 N in
 // k_tile_sift (h, next h, mean envelope) plus N/2 of bitmaps and about 6 bytes per knot of
 // separator rows.  Line numbers refer to the reference's cudaICEEMDAN.cu.
-#include <cuda/atomic>
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
 #include "canon.cuh"
 #include "kernels.h"
+#include "spline_device.cuh"
 
 namespace ceemdan {
 
@@ -147,195 +147,9 @@ __device__ __forceinline__ size_t red_base(const SiftArgs& a, int e, const Geo& 
            (size_t)q.r * (size_t)red_stride_of(__ldg(&ch->rec_stride));
 }
 
-// Exact division by a tabled reciprocal: div_rcp's quotient (Markstein's correction, correctly
-// rounded in its range); `slow` marks operands outside that range, which take the division.
-__device__ __forceinline__ double rcp_fast(double a, double d, double y, bool& slow) {
-    const double q0 = a * y;
-    const double r = fma(-q0, d, a);
-    const double q1 = fma(r, y, q0);
-    slow = !(fabs(a) > 0x1p-960) || !(fabs(q1) < 0x1p+1000);
-    return q1;
-}
-
-// ---------------------------------------------------------------------------------------
-// chunk primitives of the canonical partitioned solve (rows produced by a functor)
-// ---------------------------------------------------------------------------------------
-struct ChunkEnds {
-    double ga, aa, ba, gb, ab, bb;
-};
-
-// End relations of a chunk of `len` rows: top-down elimination gives the last row
-// x_b = gb + ab*xL + bb*xR, bottom-up elimination the first row x_a = ga + aa*xL + ba*xR.
-// The two sweeps are independent chains and run interleaved.  The pivot reciprocals of the
-// top-down sweep are those of the interior's sweep: row k's goes to iw_out(k), where
-// chunk_interior_iw takes it from.  (Loops stay rolled: a CTA passes here once, and unrolled
-// sweeps spent most of their time fetching instructions, up to 1000 cycles a row.)
-template <class Pivot = SplinePivot, class RowFn, class IwOut>
-__device__ __forceinline__ ChunkEnds chunk_ends(int len, const RowFn& row, const IwOut& iw_out) {
-    const Row wa = row(0), wb = row(len - 1);
-    double iw = Pivot::inv(wa.m);
-    double iv = Pivot::inv(wb.m);
-    double cp = wa.u * iw, gp = wa.r * iw, ap = -wa.l * iw;
-    double cq = wb.l * iv, gq = wb.r * iv, bq = -wb.u * iv;
-    iw_out(0) = iw;
-    Row w = len > 1 ? row(1) : wa, v = len > 1 ? row(len - 2) : wb;
-#pragma unroll 1
-    for (int k = 1; k < len; ++k) {
-        const Row wc = w, vc = v;
-        if (k + 1 < len) {  // the next rows load while this row's reciprocals form
-            w = row(k + 1);
-            v = row(len - 2 - k);
-        }
-        iw = Pivot::inv(fma(-wc.l, cp, wc.m));
-        iv = Pivot::inv(fma(-vc.u, cq, vc.m));
-        cp = wc.u * iw;
-        gp = fma(-wc.l, gp, wc.r) * iw;
-        ap = (-wc.l * ap) * iw;
-        cq = vc.l * iv;
-        gq = fma(-vc.u, gq, vc.r) * iv;
-        bq = (-vc.u * bq) * iv;
-        iw_out(k) = iw;
-    }
-    ChunkEnds e;
-    e.gb = gp;
-    e.ab = ap;
-    e.bb = -wb.u * iw;
-    e.ga = gq;
-    e.ba = bq;
-    e.aa = -wa.l * iv;
-    return e;
-}
-
-// x(k) <- x(k) - fac(k) x(k+1) from row len-2 down, x(len-1) = xv; loads one row ahead.
-template <class X, class Fac>
-__device__ __forceinline__ void back_sweep(int len, double xv, const X& x, const Fac& fac) {
-    double f = 0.0, g = 0.0;
-    if (len > 1) {
-        f = fac(len - 2);
-        g = x(len - 2);
-    }
-#pragma unroll 1
-    for (int k = len - 2; k >= 0; --k) {
-        const double fc = f, gc = g;
-        if (k > 0) {
-            f = fac(k - 1);
-            g = x(k - 1);
-        }
-        xv = fma(-fc, xv, gc);
-        x(k) = xv;
-    }
-}
-
-// Interior of a chunk whose end relations chunk_ends formed: coupling terms to the right-hand
-// side, then canonical Thomas with the reciprocals left in x(k); x(k) receives the solution,
-// fac(k) the factors meanwhile (fac(k) may be row k's own u or a slot of it that rows after k do
-// not read).
-template <class RowFn, class X, class Fac>
-__device__ __forceinline__ void chunk_interior_iw(int len, const RowFn& row, double xl, double xr,
-                                                  const X& x, const Fac& fac) {
-    Row w = row(0);
-    double iw = x(0), gp = 0.0;
-#pragma unroll 1
-    for (int k = 0; k < len; ++k) {
-        const Row wc = w;
-        const double ic = iw;
-        if (k + 1 < len) {
-            w = row(k + 1);
-            iw = x(k + 1);
-        }
-        double ri = wc.r;
-        if (k == 0) ri = fma(-wc.l, xl, ri);
-        if (k == len - 1) ri = fma(-wc.u, xr, ri);
-        gp = k == 0 ? ri * ic : fma(-wc.l, gp, ri) * ic;
-        fac(k) = wc.u * ic;
-        x(k) = gp;
-    }
-    back_sweep(len, gp, x, fac);
-}
-
-// Canonical Thomas on n <= kChunk rows, solution to x(k), factors to fac(k) meanwhile.
-template <class Pivot = SplinePivot, class RowFn, class X, class Fac>
-__device__ __forceinline__ void thomas_rolled(int n, const RowFn& row, const X& x,
-                                              const Fac& fac) {
-    Row w = row(0);
-    double cp = 0.0, gp = 0.0;
-#pragma unroll 1
-    for (int k = 0; k < n; ++k) {
-        const Row wc = w;
-        if (k + 1 < n) w = row(k + 1);
-        const double iw = Pivot::inv(k == 0 ? wc.m : fma(-wc.l, cp, wc.m));
-        gp = k == 0 ? wc.r * iw : fma(-wc.l, gp, wc.r) * iw;
-        cp = wc.u * iw;
-        fac(k) = cp;
-        x(k) = gp;
-    }
-    back_sweep(n, gp, x, fac);
-}
-
-// Consecutive doubles as a row-indexed destination; NoIw drops what it is given.
-struct Slots {
-    double* p;
-    __device__ __forceinline__ double& operator()(int k) const { return p[k]; }
-};
-struct NoIw {
-    struct Sink {
-        __device__ __forceinline__ void operator=(double) const {}
-    };
-    __device__ __forceinline__ Sink operator()(int) const { return Sink(); }
-};
-
-// Interior of a chunk of `len` rows once its separator values xl, xr are known: coupling
-// terms move to the right-hand side, then canonical Thomas; x_k written to out[k*stride].
-// kCoupled = false is the plain canonical Thomas (no coupling terms at all).
-template <bool kCoupled = true, class Pivot = SplinePivot, class RowFn, class Out>
-__device__ __forceinline__ void chunk_interior(int len, const RowFn& row, double xl, double xr,
-                                               Out out, int stride) {
-    double cp[kChunk], gp[kChunk];
-#pragma unroll
-    for (int k = 0; k < kChunk; ++k) {
-        if (k < len) {
-            const Row w = row(k);
-            double ri = w.r;
-            if (kCoupled && k == 0) ri = fma(-w.l, xl, ri);
-            if (kCoupled && k == len - 1) ri = fma(-w.u, xr, ri);
-            if (k == 0) {
-                const double iw = Pivot::inv(w.m);
-                cp[0] = w.u * iw;
-                gp[0] = ri * iw;
-            } else {
-                const double iw = Pivot::inv(fma(-w.l, cp[k - 1], w.m));
-                cp[k] = w.u * iw;
-                gp[k] = fma(-w.l, gp[k - 1], ri) * iw;
-            }
-        }
-    }
-    double xv = 0.0;
-#pragma unroll
-    for (int k = kChunk - 1; k >= 0; --k) {
-        if (k < len) {
-            xv = (k == len - 1) ? gp[k] : fma(-cp[k], xv, gp[k]);
-            out[k * stride] = xv;
-        }
-    }
-}
-
-// Canonical Thomas on n <= kChunk rows (base case), x written with stride.
-template <class Pivot = SplinePivot, class RowFn>
-__device__ __forceinline__ void thomas_small(int n, const RowFn& row, double* x, int stride) {
-    chunk_interior<false, Pivot>(n, row, 0.0, 0.0, x, stride);
-}
-
-// Rows of a tile, knots of a spline: the padded position of in-tile knot m in the shared-memory
-// knot arrays, one pad slot after every 16 knots, so that the chunk sweeps (lane p walks the
-// knots of chunk p, 16 knots after lane p-1's) read different banks.
-__device__ __forceinline__ int kq(int m) { return m + (m >> 4); }
-
 // Entry of k_tile_sift's arrays where the segment of a sample with r knots before it in the tile
 // starts: the knot before the tile at 0, in-tile knot m at 2 + kq(m).
 __device__ __forceinline__ int seg_at(int r) { return r + ((r + 15) >> 4); }
-
-// separators of a tile with c knots (local 0, 16, 32, ... and the last one)
-__device__ __forceinline__ int tile_seps(int c) { return c > 0 ? (c + kChunk - 2) / kChunk + 1 : 0; }
 
 // Four doubles to a 32-byte aligned address, as one access.
 __device__ __forceinline__ void store4(double* p, const double* v) {
@@ -343,22 +157,6 @@ __device__ __forceinline__ void store4(double* p, const double* v) {
                  "d"(v[2]), "d"(v[3])
                  : "memory");
 }
-
-// Asynchronous global -> shared copies.
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-// all but the newest group
-__device__ __forceinline__ void cp_async_wait_but_one() {
-    asm volatile("cp.async.wait_group 1;\n" ::);
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::); }
 
 // The tile kernels run as persistent CTAs: CTA b works on the b-th of gridDim.x contiguous ranges
 // of the active tiles, and copies the next tile's samples to shared memory while it computes on
@@ -436,141 +234,6 @@ __device__ __forceinline__ void unstage_tile(double* h, const double2* st, int m
         for (int i = 0; i < kPerThread; ++i)
             if (kPerThread * tid + i >= m) h[i] = 0.0;
     }
-}
-
-// The quotient a / d by the division itself, kept out of line of the fast path (a plain
-// division in a branch is evaluated unconditionally by the compiler).
-__device__ __forceinline__ double div_cold(double a, double d) {
-    double q;
-    asm volatile("div.rn.f64 %0, %1, %2;" : "=d"(q) : "d"(a), "d"(d));
-    return q;
-}
-
-// a / d for an integer-valued d in [1, 2^40], from its reciprocal (Markstein's correction as in
-// div_rcp; operands outside its range take the division).  The reciprocal is pivot_inv's without
-// the check for the all-ones significand, which an integer below 2^52 does not have; measured
-// against a table of 1/d in global memory it saves the load and its bounds.
-__device__ __forceinline__ double div_int(double a, double d) {
-    bool slow;
-    double q = rcp_fast(a, d, rcp_raw(d), slow);
-    if (slow) q = div_cold(a, d);
-    return q;
-}
-
-// seg_coeffs' b and d from the segment's length, slope and spline values.
-__device__ __forceinline__ void seg_coeffs_int(double h, double slope, double c0, double c1,
-                                               double& b, double& d) {
-    const double hq = h * fma(2.0, c0, c1);
-    bool slow;
-    double qb = rcp_fast(hq, 3.0, kRcp3, slow);
-    if (slow) qb = div_cold(hq, 3.0);
-    d = div_int(c1 - c0, 3.0 * h);
-    b = slope - qb;
-}
-
-// Pivots of one chunk inverted by rcp_raw, with one look for the all-ones significand at the end
-// (low word -1; once in 2^32 pivots the caller repeats the chunk with pivot_inv).
-struct RawPivot {
-    bool ones = false;
-    __device__ __forceinline__ double inv(double x) {
-        ones |= __double2loint(x) == -1;
-        return rcp_raw(x);
-    }
-};
-struct CheckedPivot {
-    bool ones = false;
-    __device__ __forceinline__ double inv(double x) { return pivot_inv(x); }
-};
-
-// End relations (chunk_ends: same operations, same order) of the chunk whose knots 0..len+1 sit
-// in the padded arrays x, s from the chunk's base on (s[i]: slope of segment i -> i+1).  Each
-// sweep loads one new knot and slope per row, a row ahead of its use.
-template <class Pivot, class XT>
-__device__ __forceinline__ ChunkEnds chunk_ends_sweep(Pivot& pv, const XT* x, const double* s,
-                                                      int len) {
-    int xt = x[2], xb = x[len - 1];
-    // top-down row 0 and bottom-up row len-1
-    double lt = (double)(x[1] - x[0]), ut = (double)(xt - x[1]);
-    double ub = (double)(x[kq(len + 1)] - x[len]), lb = (double)(x[len] - xb);
-    double st = s[1], sb = s[len - 1];
-    const double wr0 = 3.0 * (st - s[0]), vr0 = 3.0 * (s[len] - sb);
-    const double lf = lt, ul = ub;
-    double un = 0.0, lp = 0.0, sn = 0.0, sp = 0.0;  // the next row's
-    if (len > 1) {
-        const int xn = x[kq(3)], xp = x[len - 2];
-        un = (double)(xn - xt);
-        xt = xn;
-        lp = (double)(xb - xp);
-        xb = xp;
-        sn = s[2];
-        sp = s[len - 2];
-    }
-    double iw = pv.inv(2.0 * (lt + ut));
-    double iv = pv.inv(2.0 * (lb + ub));
-    double cp = ut * iw, gp = wr0 * iw, ap = -lt * iw;
-    double cq = lb * iv, gq = vr0 * iv, bq = -ub * iv;
-#pragma unroll 2
-    for (int k = 1; k < len; ++k) {
-        lt = ut;
-        ut = un;
-        ub = lb;
-        lb = lp;
-        const double wr = 3.0 * (sn - st), vr = 3.0 * (sb - sp);
-        st = sn;
-        sb = sp;
-        if (k + 1 < len) {
-            const int xn = x[kq(k + 3)], xp = x[len - 2 - k];
-            un = (double)(xn - xt);
-            xt = xn;
-            lp = (double)(xb - xp);
-            xb = xp;
-            sn = s[k + 2];
-            sp = s[len - 2 - k];
-        }
-        iw = pv.inv(fma(-lt, cp, 2.0 * (lt + ut)));
-        iv = pv.inv(fma(-ub, cq, 2.0 * (lb + ub)));
-        cp = ut * iw;
-        gp = fma(-lt, gp, wr) * iw;
-        ap = (-lt * ap) * iw;
-        cq = lb * iv;
-        gq = fma(-ub, gq, vr) * iv;
-        bq = (-ub * bq) * iv;
-    }
-    ChunkEnds e;
-    e.gb = gp;
-    e.ab = ap;
-    e.bb = -ul * iw;
-    e.ga = gq;
-    e.ba = bq;
-    e.aa = -lf * iv;
-    return e;
-}
-template <class XT>
-__device__ __noinline__ void chunk_ends_checked(ChunkEnds& e, const XT* x, const double* s,
-                                                int len) {
-    CheckedPivot pv;
-    e = chunk_ends_sweep(pv, x, s, len);
-}
-template <class XT>
-__device__ __forceinline__ ChunkEnds chunk_ends_knots(const XT* x, const double* s, int len) {
-    RawPivot pv;
-    ChunkEnds e = chunk_ends_sweep(pv, x, s, len);
-    if (pv.ones) {
-        ChunkEnds c;
-        chunk_ends_checked(c, x, s, len);
-        e = c;
-    }
-    return e;
-}
-
-// Inclusive prefix of v over the warp's lanes.
-__device__ __forceinline__ int warp_scan(int v, int lane) {
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += t;
-    }
-    return v;
 }
 
 // The chunk a thread sweeps, given the separators of the tile's two envelopes: the chunks of
@@ -874,102 +537,6 @@ struct GlobalRowFn {
         return w;
     }
 };
-
-// In-CTA canonical partitioned solve of an explicit system stored at sys (4 planes of
-// `plane` doubles: l, m, u, r; the u plane is overwritten), solution to x.  ws: workspace for the
-// deeper levels (<= 0.75*n + 16 doubles).  All threads of the CTA must call it.
-struct PartLevel {
-    double *L, *x;  // rows (4 planes of pl doubles), solution
-    int n, pl;
-};
-// level k of a system of n rows: its size, and where its rows and solution start in the workspace
-// (all levels' rows, then all levels' solutions, then the end relations)
-__device__ __forceinline__ PartLevel part_level(int k, int depth, int n, double* sys, int plane,
-                                                double* x, double* ws) {
-    if (k == 0) return PartLevel{sys, x, n, plane};
-    int rows = 0, sols = 0, size = n, mine = 0, mrow = 0, msol = 0;
-    for (int i = 1; i <= depth; ++i) {
-        size = (size - 1) / kChunk;
-        if (i == k) {
-            mine = size;
-            mrow = rows;
-            msol = sols;
-        }
-        rows += 4 * size;
-        sols += size;
-    }
-    return PartLevel{ws + mrow, ws + rows + msol, mine, mine};
-}
-
-template <class Pivot>
-__device__ void cta_partitioned(int n, double* sys, int plane, double* x, double* ws) {
-    int depth = 0, all = 0;  // all: rows and solutions of the levels below the first
-    for (int size = n; size > kChunk && depth < 7; ++depth) {
-        size = (size - 1) / kChunk;
-        all += 5 * size;
-    }
-    double* ends = ws + all;  // 6 * (chunks of the widest level)
-#pragma unroll 1
-    for (int k = 0; k < depth; ++k) {
-        const PartLevel v = part_level(k, depth, n, sys, plane, x, ws);
-        const PartLevel o = part_level(k + 1, depth, n, sys, plane, x, ws);
-        const int P = o.n, pl = v.pl;
-        const double* L = v.L;
-        for (int q = threadIdx.x; q <= P; q += blockDim.x) {
-            const int first = q * kChunk;
-            const int len = (q < P) ? kChunk - 1 : v.n - first;
-            GlobalRowFn fn{L, L + pl, L + 2 * pl, L + 3 * pl, first};
-            const ChunkEnds ce = chunk_ends<Pivot>(len, fn, Slots{v.x + first});
-            ends[6 * q + 0] = ce.ga;
-            ends[6 * q + 1] = ce.aa;
-            ends[6 * q + 2] = ce.ba;
-            ends[6 * q + 3] = ce.gb;
-            ends[6 * q + 4] = ce.ab;
-            ends[6 * q + 5] = ce.bb;
-        }
-        __syncthreads();
-        double* R = o.L;
-        for (int p = threadIdx.x; p < P; p += blockDim.x) {
-            const int s = p * kChunk + kChunk - 1;
-            Row sr;
-            sr.l = L[s];
-            sr.m = L[pl + s];
-            sr.u = L[2 * pl + s];
-            sr.r = L[3 * pl + s];
-            const Row w = reduced_row(sr, ends[6 * p + 3], ends[6 * p + 4], ends[6 * p + 5],
-                                      ends[6 * (p + 1) + 0], ends[6 * (p + 1) + 1],
-                                      ends[6 * (p + 1) + 2]);
-            R[p] = w.l;
-            R[P + p] = w.m;
-            R[2 * P + p] = w.u;
-            R[3 * P + p] = w.r;
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        const PartLevel v = part_level(depth, depth, n, sys, plane, x, ws);
-        GlobalRowFn fn{v.L, v.L + v.pl, v.L + 2 * v.pl, v.L + 3 * v.pl, 0};
-        thomas_rolled<Pivot>(v.n, fn, Slots{v.x}, Slots{v.L + 2 * v.pl});
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int k = depth - 1; k >= 0; --k) {
-        const PartLevel v = part_level(k, depth, n, sys, plane, x, ws);
-        const PartLevel o = part_level(k + 1, depth, n, sys, plane, x, ws);
-        const int P = o.n, pl = v.pl;
-        double* L = v.L;
-        for (int q = threadIdx.x; q <= P; q += blockDim.x) {
-            const int first = q * kChunk;
-            const int len = (q < P) ? kChunk - 1 : v.n - first;
-            GlobalRowFn fn{L, L + pl, L + 2 * pl, L + 3 * pl, first};
-            const double xl = (q > 0) ? o.x[q - 1] : 0.0;
-            const double xr = (q < P) ? o.x[q] : 0.0;
-            chunk_interior_iw(len, fn, xl, xr, Slots{v.x + first}, Slots{L + 2 * pl + first});
-            if (q < P) v.x[first + kChunk - 1] = xr;
-        }
-        __syncthreads();
-    }
-}
 
 // In-CTA canonical partitioned solve of an explicit system in global memory (its sweeps keep their
 // factors in registers: a factor read back from memory would cost a round trip a row) stored at sys (4 planes of
@@ -1288,220 +855,12 @@ constexpr int kSolvePass = kSolveChunks * kChunk;                 // level-2 row
 constexpr int kSolveSlots = kSolvePass + (kSolvePass >> 4) + 1;  // padded
 constexpr int kTabTiles = 256;  // rows of up to this many tiles keep their tables in shared memory
 
-// Rows of a system with one pad slot per 16 (row i at kq(i)): a chunk's rows are consecutive, and
-// the lanes that sweep neighbouring chunks read different banks.
-struct alignas(16) SepRow {
-    double l, m, u, r;
-};
-__device__ __forceinline__ SepRow load_row(const SepRow* p) {
-    const double2 a = reinterpret_cast<const double2*>(p)[0];
-    const double2 b = reinterpret_cast<const double2*>(p)[1];
-    return SepRow{a.x, a.y, b.x, b.y};
-}
-__device__ __forceinline__ SepRow sep_row(const Row& w) { return SepRow{w.l, w.m, w.u, w.r}; }
-// padded length of n rows
-__host__ __device__ __forceinline__ int padded(int n) { return n + (n >> 4) + 1; }
-
 // Level-2 rows staged in shared memory.
 struct RedStage {
     SepRow row[kSolveSlots];
     double x[kSolveSlots + 1];  // reciprocal pivots, then the solution
 };
 static_assert(sizeof(RedStage) == kSolveStage, "the host sizes the workspace after it");
-
-// chunk_ends (same operations, same order) of len consecutive rows; the top-down sweep's
-// reciprocals to iw (kIw).  Rows are read one ahead of their use.
-template <bool kIw, class Pivot>
-__device__ __forceinline__ ChunkEnds ends_sweep(Pivot& pv, const SepRow* r, int len, double* iw) {
-    SepRow w = load_row(r), v = load_row(r + len - 1);
-    const double lf = w.l, ul = v.u;
-    double iu = pv.inv(w.m), iv = pv.inv(v.m);
-    double cp = w.u * iu, gp = w.r * iu, ap = -w.l * iu;
-    double cq = v.l * iv, gq = v.r * iv, bq = -v.u * iv;
-    if (kIw) iw[0] = iu;
-    if (len > 1) {
-        w = load_row(r + 1);
-        v = load_row(r + len - 2);
-    }
-#pragma unroll 1
-    for (int k = 1; k < len; ++k) {
-        const SepRow a = w, b = v;
-        if (k + 1 < len) {
-            w = load_row(r + k + 1);
-            v = load_row(r + len - 2 - k);
-        }
-        iu = pv.inv(fma(-a.l, cp, a.m));
-        iv = pv.inv(fma(-b.u, cq, b.m));
-        cp = a.u * iu;
-        gp = fma(-a.l, gp, a.r) * iu;
-        ap = (-a.l * ap) * iu;
-        cq = b.l * iv;
-        gq = fma(-b.u, gq, b.r) * iv;
-        bq = (-b.u * bq) * iv;
-        if (kIw) iw[k] = iu;
-    }
-    return ChunkEnds{gq, -lf * iv, bq, gp, ap, -ul * iu};
-}
-template <bool kIw>
-__device__ __noinline__ void ends_rows_checked(const SepRow* r, int len, double* iw,
-                                               ChunkEnds& e) {
-    CheckedPivot pv;
-    e = ends_sweep<kIw>(pv, r, len, iw);
-}
-// ... to out[0..5] = ga, aa, ba, gb, ab, bb
-template <bool kIw>
-__device__ __forceinline__ void ends_rows(const SepRow* r, int len, double* iw, double* out) {
-    RawPivot pv;
-    ChunkEnds e = ends_sweep<kIw>(pv, r, len, iw);
-    if (pv.ones) {
-        ChunkEnds c;
-        ends_rows_checked<kIw>(r, len, iw, c);
-        e = c;
-    }
-    out[0] = e.ga;
-    out[1] = e.aa;
-    out[2] = e.ba;
-    out[3] = e.gb;
-    out[4] = e.ab;
-    out[5] = e.bb;
-}
-
-// Row p of the next level: separator row s between the chunks with end relations e (left) and
-// e + 6 (right).
-__device__ __forceinline__ SepRow next_row(const SepRow& s, const double* e) {
-    return sep_row(reduced_row(Row{s.l, s.m, s.u, s.r}, e[3], e[4], e[5], e[6], e[7], e[8]));
-}
-
-// Back substitution x[k] <- x[k] - fac(k) x[k+1], row k's factor in its u.
-__device__ __forceinline__ void back_rows(const SepRow* r, double* x, int len, double xv) {
-    double f = 0.0, g = 0.0;
-    if (len > 1) {
-        f = r[len - 2].u;
-        g = x[len - 2];
-    }
-#pragma unroll 1
-    for (int k = len - 2; k >= 0; --k) {
-        const double fc = f, gc = g;
-        if (k > 0) {
-            f = r[k - 1].u;
-            g = x[k - 1];
-        }
-        xv = fma(-fc, xv, gc);
-        x[k] = xv;
-    }
-}
-
-// chunk_interior_iw of len consecutive rows: x holds the reciprocals, then the solution; the rows'
-// u is overwritten.
-__device__ __forceinline__ void interior_rows(SepRow* r, int len, double xl, double xr,
-                                              double* x) {
-    SepRow w = load_row(r);
-    double iw = x[0], gp = 0.0;
-#pragma unroll 1
-    for (int k = 0; k < len; ++k) {
-        const SepRow a = w;
-        const double ic = iw;
-        if (k + 1 < len) {
-            w = load_row(r + k + 1);
-            iw = x[k + 1];
-        }
-        double ri = a.r;
-        if (k == 0) ri = fma(-a.l, xl, ri);
-        if (k == len - 1) ri = fma(-a.u, xr, ri);
-        gp = (k == 0 ? ri : fma(-a.l, gp, ri)) * ic;
-        r[k].u = a.u * ic;
-        x[k] = gp;
-    }
-    back_rows(r, x, len, gp);
-}
-
-// Canonical Thomas of n rows (kCoupled: a chunk between xl and xr), reciprocals formed here.
-template <bool kCoupled>
-__device__ __forceinline__ void thomas_rows(SepRow* r, int n, double xl, double xr, double* x) {
-    SepRow w = load_row(r);
-    double cp = 0.0, gp = 0.0;
-#pragma unroll 1
-    for (int k = 0; k < n; ++k) {
-        const SepRow a = w;
-        if (k + 1 < n) w = load_row(r + k + 1);
-        double ri = a.r;
-        if (kCoupled && k == 0) ri = fma(-a.l, xl, ri);
-        if (kCoupled && k == n - 1) ri = fma(-a.u, xr, ri);
-        const double iw = pivot_inv(k == 0 ? a.m : fma(-a.l, cp, a.m));
-        gp = (k == 0 ? ri : fma(-a.l, gp, ri)) * iw;
-        cp = a.u * iw;
-        r[k].u = cp;
-        x[k] = gp;
-    }
-    back_rows(r, x, n, gp);
-}
-
-// cta_partitioned<SplinePivot> on padded rows: n rows at `rows` (u overwritten), solution to the
-// padded x; ws: 5 padded(n/16) + 6 (n/16 + 1) doubles and as much again for what is below, at
-// most 0.75 n + 64.  Every thread of the CTA calls it.
-struct RowsLevel {
-    SepRow* r;
-    double* x;
-    int n;
-};
-__device__ __forceinline__ RowsLevel rows_level(int k, int depth, int n, SepRow* rows, double* x,
-                                                double* ws) {
-    if (k == 0) return RowsLevel{rows, x, n};
-    int ro = 0, xo = 0, size = n, mine = 0, mr = 0, mx = 0;
-    for (int i = 1; i <= depth; ++i) {
-        size = (size - 1) / kChunk;
-        if (i == k) {
-            mine = size;
-            mr = ro;
-            mx = xo;
-        }
-        ro += 4 * padded(size);
-        xo += padded(size);
-    }
-    return RowsLevel{reinterpret_cast<SepRow*>(ws + mr), ws + ro + mx, mine};
-}
-
-__device__ void partition_rows(int n, SepRow* rows, double* x, double* ws) {
-    int depth = 0, all = 0;
-    for (int size = n; size > kChunk && depth < 7; ++depth) {
-        size = (size - 1) / kChunk;
-        all += 5 * padded(size);
-    }
-    double* ends = ws + all;
-#pragma unroll 1
-    for (int k = 0; k < depth; ++k) {
-        const RowsLevel v = rows_level(k, depth, n, rows, x, ws);
-        const RowsLevel o = rows_level(k + 1, depth, n, rows, x, ws);
-        for (int q = threadIdx.x; q <= o.n; q += blockDim.x) {
-            const int first = q * kChunk;
-            const int len = (q < o.n) ? kChunk - 1 : v.n - first;
-            ends_rows<true>(v.r + kq(first), len, v.x + kq(first), ends + 6 * q);
-        }
-        __syncthreads();
-        for (int p = threadIdx.x; p < o.n; p += blockDim.x)
-            o.r[kq(p)] = next_row(load_row(v.r + kq(p * kChunk + kChunk - 1)), ends + 6 * p);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        const RowsLevel v = rows_level(depth, depth, n, rows, x, ws);
-        thomas_rows<false>(v.r, v.n, 0.0, 0.0, v.x);
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int k = depth - 1; k >= 0; --k) {
-        const RowsLevel v = rows_level(k, depth, n, rows, x, ws);
-        const RowsLevel o = rows_level(k + 1, depth, n, rows, x, ws);
-        for (int q = threadIdx.x; q <= o.n; q += blockDim.x) {
-            const int first = q * kChunk;
-            const int len = (q < o.n) ? kChunk - 1 : v.n - first;
-            const double xl = (q > 0) ? o.x[kq(q - 1)] : 0.0;
-            const double xr = (q < o.n) ? o.x[kq(q)] : 0.0;
-            interior_rows(v.r + kq(first), len, xl, xr, v.x + kq(first));
-            if (q < o.n) v.x[kq(first + kChunk - 1)] = xr;
-        }
-        __syncthreads();
-    }
-}
 
 // Rows of a spline's transposed system from its knot positions and right-hand side in padded
 // shared memory (KnotSysRows' values).
@@ -1607,7 +966,7 @@ __device__ __forceinline__ void solve_separators(RedStage& st, int wcap, const d
         r3[kq(p)] = next_row(load_row(one ? st.row + kq(p * kChunk + kChunk - 1) : sep + p),
                              ends + 6 * p);
     __syncthreads();
-    partition_rows(Q, r3, x3, ws3);
+    partition_rows(CtaGroup(), Q, r3, x3, ws3);
     if (fits && !one) {  // the stage is filled again: the level-3 solution moves out of it
         for (int p = threadIdx.x; p < Q; p += kSolveThreads) ends[kq(p)] = x3[kq(p)];
         x3 = ends;
@@ -1718,7 +1077,7 @@ k_adj_solve_smem(const int* nrows, int cap, const int32_t* kx, const double* rhs
             r2[kq(p)] = next_row(
                 sep_row(StagedKnotRows{X, R, K, 0}(p * kChunk + kChunk - 1)), ends + 6 * p);
         __syncthreads();
-        partition_rows(P, r2, x2, ws);
+        partition_rows(CtaGroup(), P, r2, x2, ws);
         for (int q = threadIdx.x; q <= P; q += kThreads) {
             const int first = q * kChunk, len = (q < P) ? kChunk - 1 : K - first;
             const double xl = (q > 0) ? x2[kq(q - 1)] : 0.0, xr = (q < P) ? x2[kq(q)] : 0.0;
@@ -2580,620 +1939,6 @@ k_tridiag_batched(int n, const double* l, const double* m, const double* u, cons
     }
     __syncthreads();
     cta_partitioned_global<AnyPivot>(n, S, n, x + b * n, ws + b * ws_stride);
-}
-
-// =======================================================================================
-// k_sift_small: the whole lock-step sift of one stage for rows of at most kSmallMaxN samples,
-// in one cooperative launch: CTA r holds realization r's h in shared memory and runs every
-// iteration on chip -- the deferred update, extrema and compaction, the end-knot rule, the
-// canonical tile-aligned spline solve (chunk end relations, separator rows, the separator
-// system by the same level-2/level-3 partition as k_reduced_solve, chunk interiors), segment
-// coefficients, both envelopes, the mean envelope, the sx statistics and the stop test -- and
-// meets the other CTAs once per iteration at the lock-step test (a counter polled at most
-// spin_limit times; when it runs out, the CTA sets CEEMDAN_ERR_TIMEOUT in the channel's error
-// word and returns).  Every operation is the one the multi-kernel iteration performs, in the
-// same order (canon.cuh; divisions taken as IEEE divisions, which the tabled-reciprocal fast
-// paths of the other kernels reproduce exactly), so the results are bit-identical.  Channel 0
-// only; the reference loop it replaces is cudaICEEMDAN.cu:1752-1867 (per iteration ~25
-// kernel launches and library calls, and a host round trip).
-// =======================================================================================
-namespace {
-
-__device__ __forceinline__ int sep_local(int k, int cnt) { return min(k * kChunk, cnt - 1); }
-
-struct SmallSmem {
-    double *H, *KY, *KS, *KC, *ENDS, *R2, *X2, *W3;
-    int *KX, *SEP, *misc, *WP;
-    unsigned* BM;
-    double* KD;  // segment d's, over the solve's workspace (ENDS .. W3) once the solve is done
-    int kcap, pcap, qcap, dcap;
-};
-
-// Knot k of the knot arrays KX, KY, KS, KC sits at kp(k): one pad slot after every 16 knots,
-// so the chunk chains of the spline solve (lane p walks the knots of chunk p, 16 knots after
-// lane p-1's) read different banks.
-__host__ __device__ __forceinline__ int kp(int k) { return k + (k >> 4); }
-
-// Layout of the dynamic shared memory for rows of n samples (doubles first, 16-byte aligned).
-__host__ __device__ inline size_t small_layout(int n, SmallSmem* L, unsigned char* base) {
-    const int ntiles = (n + kTileSamples - 1) / kTileSamples;
-    const int kcap = n / 2 + 2;
-    const int kpad = kp(kcap) + 1;  // knot arrays, one pad slot per 16 knots
-    const int pcap = kcap / kChunk + 2 * ntiles + 8;
-    const int qcap = pcap / kChunk + 1;
-    size_t off = 0;
-    auto take = [&](size_t bytes) {
-        const size_t o = off;
-        off += (bytes + 15) & ~(size_t)15;
-        return o;
-    };
-    const size_t oH = take(sizeof(double) * n);
-    const size_t oKY = take(sizeof(double) * kpad);
-    const size_t oKS = take(sizeof(double) * kpad);
-    const size_t oKC = take(sizeof(double) * kpad);
-    const size_t oE = take(sizeof(double) * 6 * pcap);
-    const size_t oR = take(sizeof(double) * 4 * pcap);
-    const size_t oX = take(sizeof(double) * pcap);
-    const size_t oW = take(sizeof(double) * (16 * (size_t)qcap + 74));
-    const size_t oKX = take(sizeof(int) * kpad);
-    const size_t oS = take(sizeof(int) * pcap);
-    const size_t oM = take(sizeof(int) * 64);
-    const int nw = (n + 31) >> 5;
-    const size_t oBM = take(sizeof(unsigned) * nw);
-    const size_t oWP = take(sizeof(int) * (nw + 1));
-    if (L && base) {
-        L->H = reinterpret_cast<double*>(base + oH);
-        L->KY = reinterpret_cast<double*>(base + oKY);
-        L->KS = reinterpret_cast<double*>(base + oKS);
-        L->KC = reinterpret_cast<double*>(base + oKC);
-        L->ENDS = reinterpret_cast<double*>(base + oE);
-        L->R2 = reinterpret_cast<double*>(base + oR);
-        L->X2 = reinterpret_cast<double*>(base + oX);
-        L->W3 = reinterpret_cast<double*>(base + oW);
-        L->KX = reinterpret_cast<int*>(base + oKX);
-        L->SEP = reinterpret_cast<int*>(base + oS);
-        L->misc = reinterpret_cast<int*>(base + oM);
-        L->BM = reinterpret_cast<unsigned*>(base + oBM);
-        L->WP = reinterpret_cast<int*>(base + oWP);
-        L->KD = L->ENDS;
-        L->kcap = kcap;
-        L->pcap = pcap;
-        L->qcap = qcap;
-        L->dcap = (int)((oKX - oE) / sizeof(double));
-    }
-    return off;
-}
-
-// Padded knot array slots from knot `first` on.
-struct PadSlots {
-    double* a;
-    int first;
-    __device__ __forceinline__ double& operator()(int k) const { return a[kp(first + k)]; }
-};
-
-// Spline row of knot g from the knot arrays (the slopes of segments g-1 and g).
-struct KnotRowFn {
-    const int* x;
-    const double* s;
-    int first;  // knot of row 0 minus 1 (the knot before the chunk)
-    __device__ __forceinline__ Row operator()(int k) const {
-        const int i = first + k;
-        return spline_row(x[kp(i)], x[kp(i + 1)], x[kp(i + 2)], s[kp(i)], s[kp(i + 1)]);
-    }
-};
-
-// Row p of a system stored as planes l, m, u, r of `plane` doubles.
-struct PlaneRowFn {
-    const double* L;
-    int plane, first;
-    __device__ __forceinline__ Row operator()(int k) const {
-        const int i = first + k;
-        Row w;
-        w.l = L[i];
-        w.m = L[plane + i];
-        w.u = L[2 * plane + i];
-        w.r = L[3 * plane + i];
-        return w;
-    }
-};
-
-// Exclusive prefix of v over the CTA's threads in thread order; *total = the sum.  scratch:
-// 2 * (kSmallThreads / 32) ints.
-__device__ __forceinline__ int block_excl_scan(int v, int* scratch, int* total) {
-    constexpr int kW = kSmallThreads / 32;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += u;
-    }
-    if (lane == 31) scratch[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        int w = lane < kW ? scratch[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += u;
-        }
-        if (lane < kW) scratch[kW + lane] = w;
-    }
-    __syncthreads();
-    const int before = warp > 0 ? scratch[kW + warp - 1] : 0;
-    *total = scratch[2 * kW - 1];
-    __syncthreads();
-    return before + incl - v;
-}
-
-static_assert(kSmallMaxN / 32 <= kSmallThreads, "one bitmap word per thread in the knot scan");
-static_assert(16 + 2 * (kSmallThreads / 32) <= 64, "scan scratch inside the misc ints");
-
-// Knots of envelope e of h[0..n) (its maxima or minima, and both end samples): the bitmap BM
-// (bit j of word w: sample 32w + j, one warp ballot per word), the knots before each word WP
-// (WP[nw] = K), and the knots in order in KX/KY with the end rule applied; returns K.
-__device__ __noinline__ int small_knots(const SmallSmem& S, int n, int e) {
-    const double* H = S.H;
-    const int nw = (n + 31) >> 5;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int w = warp; w < nw; w += kSmallThreads / 32) {
-        const int i = (w << 5) + lane;
-        bool k = false;
-        if (i < n) {
-            if (i == 0 || i == n - 1) {
-                k = true;
-            } else {
-                const double v = H[i], vl = H[i - 1], vr = H[i + 1];
-                k = e == 0 ? (v > vl && v > vr) : (v < vl && v < vr);
-            }
-        }
-        const unsigned b = __ballot_sync(0xffffffffu, k);
-        if (lane == 0) S.BM[w] = b;
-    }
-    __syncthreads();
-    int K;
-    const int c = (int)threadIdx.x < nw ? __popc(S.BM[threadIdx.x]) : 0;
-    const int ex = block_excl_scan(c, S.misc + 16, &K);
-    if ((int)threadIdx.x < nw) S.WP[threadIdx.x] = ex;
-    if (threadIdx.x == 0) S.WP[nw] = K;
-    __syncthreads();
-    for (int w = warp; w < nw; w += kSmallThreads / 32) {
-        const unsigned b = S.BM[w];
-        if (b >> lane & 1u) {
-            const int pos = kp(S.WP[w] + __popc(b & ((1u << lane) - 1u)));
-            const int i = (w << 5) + lane;
-            S.KX[pos] = i;
-            S.KY[pos] = H[i];
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {  // setBoundaryMax/Min, from the original values
-        int flags = 0;
-        if (K - 1 > 4) {
-            const int L = K - 1;
-            const int a0 = kp(0), a1 = kp(1), a2 = kp(2);
-            const int b0 = kp(L - 2), b1 = kp(L - 1), b2 = kp(L);
-            const double y0 =
-                boundary_left(e, S.KX[a0], S.KX[a1], S.KX[a2], S.KY[a0], S.KY[a1], S.KY[a2]);
-            const double yL =
-                boundary_right(e, S.KX[b0], S.KX[b1], S.KX[b2], S.KY[b0], S.KY[b1], S.KY[b2]);
-            // the tape's end-rule flags (as k_scan_boundary): a replaced value differs in bits
-            flags = (__double_as_longlong(y0) != __double_as_longlong(S.KY[a0]) ? 1 : 0) |
-                    (__double_as_longlong(yL) != __double_as_longlong(S.KY[b2]) ? 2 : 0);
-            S.KY[a0] = y0;
-            S.KY[b2] = yL;
-        }
-        S.misc[12] = flags;
-    }
-    __syncthreads();
-    return K;
-}
-
-// The canonical tile-aligned spline solve of the K knots in KX/KY: spline values to KC (KS, the
-// slopes, is spent: the interior sweeps leave their factors there).
-__device__ __noinline__ void small_spline(const SmallSmem& S, int n, int K) {
-    const int ntiles = (n + kTileSamples - 1) / kTileSamples;
-    int* toff = S.misc;        // [ntiles+1] first knot of each tile
-    int* soff = S.misc + 6;    // [ntiles+1] first separator of each tile
-    if (threadIdx.x == 0) {
-        // knots before each tile, from the bitmap scan (a tile is a whole number of words)
-        for (int t = 0; t < ntiles; ++t) toff[t] = S.WP[t * (kTileSamples / 32)];
-        toff[ntiles] = K;
-        soff[0] = 0;
-        for (int u = 0; u < ntiles; ++u) {
-            const int c = toff[u + 1] - toff[u];
-            soff[u + 1] = soff[u] + (c > 0 ? (c + kChunk - 2) / kChunk + 1 : 0);
-        }
-    }
-    // slopes of the segments (the exact quotients)
-    for (int i = threadIdx.x; i + 1 < K; i += kSmallThreads)
-        S.KS[kp(i)] = seg_slope(S.KX[kp(i)], S.KX[kp(i + 1)], S.KY[kp(i)], S.KY[kp(i + 1)]);
-    __syncthreads();
-    const int P = soff[ntiles];
-    // separators: local knots 0, 16, 32, ... and the last of every tile with knots
-    for (int p = threadIdx.x; p < P; p += kSmallThreads) {
-        int t = 0;
-        while (soff[t + 1] <= p) ++t;
-        const int c = toff[t + 1] - toff[t];
-        S.SEP[p] = toff[t] + sep_local(p - soff[t], c);
-    }
-    __syncthreads();
-    // chunk end relations (the chunk left of each separator; empty left of a tile's first
-    // knot) and the separator rows
-    double* SROW = S.R2;
-    for (int p = threadIdx.x; p < P; p += kSmallThreads) {
-        const int gs = S.SEP[p];
-        int t = 0;
-        while (soff[t + 1] <= p) ++t;
-        ChunkEnds ce;
-        const int len = p > soff[t] ? gs - S.SEP[p - 1] - 1 : 0;
-        if (len > 0) {
-            // the sweep's reciprocals wait in the rows' spline values
-            const int gb = S.SEP[p - 1];
-            ce = chunk_ends(len, KnotRowFn{S.KX, S.KS, gb}, PadSlots{S.KC, gb + 1});
-        } else {
-            ce.ga = 0.0; ce.aa = 0.0; ce.ba = 1.0;
-            ce.gb = 0.0; ce.ab = 1.0; ce.bb = 0.0;
-        }
-        double* en = S.ENDS + 6 * p;
-        en[0] = ce.ga; en[1] = ce.aa; en[2] = ce.ba;
-        en[3] = ce.gb; en[4] = ce.ab; en[5] = ce.bb;
-        const Row sr = (gs == 0 || gs == K - 1)
-                           ? identity_row()
-                           : spline_row(S.KX[kp(gs - 1)], S.KX[kp(gs)], S.KX[kp(gs + 1)],
-                                        S.KS[kp(gs - 1)], S.KS[kp(gs)]);
-        SROW[p] = sr.l;
-        SROW[S.pcap + p] = sr.m;
-        SROW[2 * S.pcap + p] = sr.u;
-        SROW[3 * S.pcap + p] = sr.r;
-    }
-    __syncthreads();
-    // level-2 rows: the separator rows with the neighbouring chunks eliminated
-    for (int p = threadIdx.x; p < P; p += kSmallThreads) {
-        Row sr;
-        sr.l = SROW[p];
-        sr.m = SROW[S.pcap + p];
-        sr.u = SROW[2 * S.pcap + p];
-        sr.r = SROW[3 * S.pcap + p];
-        const double* en = S.ENDS + 6 * p;
-        double ga = 0.0, aa = 0.0, ba = 1.0;
-        if (p + 1 < P) {
-            ga = S.ENDS[6 * (p + 1) + 0];
-            aa = S.ENDS[6 * (p + 1) + 1];
-            ba = S.ENDS[6 * (p + 1) + 2];
-        }
-        const Row w = reduced_row(sr, en[3], en[4], en[5], ga, aa, ba);
-        SROW[p] = w.l;
-        SROW[S.pcap + p] = w.m;
-        SROW[2 * S.pcap + p] = w.u;
-        SROW[3 * S.pcap + p] = w.r;
-    }
-    __syncthreads();
-    // the separator system, partitioned as k_reduced_solve does
-    const PlaneRowFn R2{SROW, S.pcap, 0};
-    if (P <= kChunk) {
-        if (threadIdx.x == 0)
-            thomas_rolled(P, R2, Slots{S.X2}, Slots{SROW + 2 * S.pcap});
-    } else {
-        const int Q = (P - 1) / kChunk;
-        double* ends = S.W3;
-        double* sep = ends + 6 * (size_t)(Q + 1);
-        double* L3 = sep + 4 * (size_t)(Q + 1);
-        double* x3 = L3 + 4 * (size_t)Q;
-        double* ws3 = x3 + Q;
-        for (int q = threadIdx.x; q <= Q; q += kSmallThreads) {
-            const int first = q * kChunk;
-            const int len = (q < Q) ? kChunk - 1 : P - first;
-            const PlaneRowFn fn{SROW, S.pcap, first};
-            const ChunkEnds ce = chunk_ends(len, fn, Slots{S.X2 + first});
-            ends[6 * q + 0] = ce.ga;
-            ends[6 * q + 1] = ce.aa;
-            ends[6 * q + 2] = ce.ba;
-            ends[6 * q + 3] = ce.gb;
-            ends[6 * q + 4] = ce.ab;
-            ends[6 * q + 5] = ce.bb;
-            if (q < Q) {
-                const Row s2 = fn(kChunk - 1);
-                sep[4 * q + 0] = s2.l;
-                sep[4 * q + 1] = s2.m;
-                sep[4 * q + 2] = s2.u;
-                sep[4 * q + 3] = s2.r;
-            }
-        }
-        __syncthreads();
-        for (int p = threadIdx.x; p < Q; p += kSmallThreads) {
-            Row s2;
-            s2.l = sep[4 * p + 0];
-            s2.m = sep[4 * p + 1];
-            s2.u = sep[4 * p + 2];
-            s2.r = sep[4 * p + 3];
-            const Row w = reduced_row(s2, ends[6 * p + 3], ends[6 * p + 4], ends[6 * p + 5],
-                                      ends[6 * (p + 1) + 0], ends[6 * (p + 1) + 1],
-                                      ends[6 * (p + 1) + 2]);
-            L3[p] = w.l;
-            L3[Q + p] = w.m;
-            L3[2 * Q + p] = w.u;
-            L3[3 * Q + p] = w.r;
-        }
-        __syncthreads();
-        cta_partitioned<SplinePivot>(Q, L3, Q, x3, ws3);
-        for (int q = threadIdx.x; q <= Q; q += kSmallThreads) {
-            const int first = q * kChunk;
-            const int len = (q < Q) ? kChunk - 1 : P - first;
-            const double xl = (q > 0) ? x3[q - 1] : 0.0;
-            const double xr = (q < Q) ? x3[q] : 0.0;
-            chunk_interior_iw(len, PlaneRowFn{SROW, S.pcap, first}, xl, xr, Slots{S.X2 + first},
-                              Slots{SROW + 2 * S.pcap + first});
-            if (q < Q) S.X2[first + kChunk - 1] = xr;
-        }
-    }
-    __syncthreads();
-    // spline values: the separators', then the chunk interiors between them
-    for (int p = threadIdx.x; p < P; p += kSmallThreads) {
-        const int gs = S.SEP[p];
-        S.KC[kp(gs)] = S.X2[p];
-        int t = 0;
-        while (soff[t + 1] <= p) ++t;
-        if (p > soff[t]) {
-            const int gb = S.SEP[p - 1];
-            const int len = gs - gb - 1;
-            if (len > 0)
-                chunk_interior_iw(len, KnotRowFn{S.KX, S.KS, gb}, S.X2[p - 1], S.X2[p],
-                                  PadSlots{S.KC, gb + 1}, PadSlots{S.KS, gb});
-        }
-    }
-    __syncthreads();
-}
-
-// Tape of envelope e of realization r at iteration j (taped forward): the knot bitmap in the
-// multi-kernel layout (64 words per tile, zero past the row), the knot count and the end-rule
-// flags -- what k_tape_record copies from the multi-kernel iteration.
-__device__ __forceinline__ void small_tape_knots(const SmallSmem& S, const SmallArgs& sa, int j,
-                                                 int r, int n, int e, int K) {
-    const TapeLayout& L = sa.tl;
-    unsigned char* slot =
-        sa.tblocks[j / kTapeBlockSlots] + (size_t)(j % kTapeBlockSlots) * L.stride;
-    const int words = L.ntiles * (kTileSamples / 32);
-    const int nw = (n + 31) >> 5;
-    unsigned* bits = reinterpret_cast<unsigned*>(slot) + (size_t)(e * L.nr + r) * words;
-    for (int w = threadIdx.x; w < words; w += kSmallThreads) bits[w] = w < nw ? S.BM[w] : 0u;
-    if (threadIdx.x == 0) {
-        reinterpret_cast<int*>(slot + L.off_kc)[e * L.nr + r] = K;
-        (slot + L.off_bf)[e * L.nr + r] = (unsigned char)S.misc[12];
-    }
-}
-
-// Segment coefficients after the solve: b of segment i into KS[i] (the slopes are spent) and,
-// when the K - 1 segments fit the solve's workspace, d into KD[i]; returns whether d is stored.
-__device__ __noinline__ bool small_coeffs(const SmallSmem& S, int K) {
-    const bool dk = K - 1 <= S.dcap;
-    for (int i = threadIdx.x; i + 1 < K; i += kSmallThreads) {
-        const int i0 = kp(i), i1 = kp(i + 1);
-        double b, d;
-        seg_coeffs(S.KX[i0], S.KX[i1], S.KY[i0], S.KY[i1], S.KC[i0], S.KC[i1], b, d);
-        S.KS[i0] = b;
-        if (dk) S.KD[i] = d;
-    }
-    __syncthreads();
-    return dk;
-}
-
-// Envelope at sample s: segment i holds x_i < s <= x_{i+1} (segment 0 also s = 0), i.e. i is
-// the number of knots before s, less one -- a rank in the knot bitmap.  d as seg_coeffs forms
-// it when it is not stored.
-__device__ __forceinline__ double small_env_at(const SmallSmem& S, int s, bool dk) {
-    const int w = s >> 5;
-    const int before = S.WP[w] + __popc(S.BM[w] & ((1u << (s & 31)) - 1u));
-    const int i = s > 0 ? before - 1 : 0;
-    const int i0 = kp(i), i1 = kp(i + 1);
-    const int x0 = S.KX[i0];
-    const double c0 = S.KC[i0];
-    const double d = dk ? S.KD[i] : (S.KC[i1] - c0) / (3.0 * (double)(S.KX[i1] - x0));
-    return seg_eval(S.KY[i0], S.KS[i0], c0, d, (double)(s - x0));
-}
-
-}  // namespace
-
-size_t small_sift_smem(int n) { return small_layout(n, nullptr, nullptr); }
-
-// Bounded wait of one thread until *word >= target (acquire); false when it gave up.
-__device__ __forceinline__ bool small_wait(unsigned* word, unsigned target, int limit) {
-    cuda::atomic_ref<unsigned, cuda::thread_scope_device> w(*word);
-    int spins = 0;
-    while (w.load(cuda::memory_order_acquire) < target) {
-        if (++spins > limit) return false;
-        __nanosleep(64);
-    }
-    return true;
-}
-
-__global__ void __launch_bounds__(kSmallThreads, 1)
-k_sift_small(SiftArgs a, SmallArgs sa) {
-    extern __shared__ __align__(16) unsigned char small_smem[];
-    __shared__ int s_red[2][kSmallThreads / 32];
-    __shared__ int s_ctl[5];  // mark, finish, all finished, error, the upper knot count
-    // Realization r; role 2: one CTA does both envelopes.  Paired (two CTAs per realization):
-    // role 0 builds the upper envelope and hands it over through global memory, role 1 the
-    // lower one, then the mean, the statistics and the stop decision.  Both keep h.
-    const bool pair = sa.pair != 0;
-    const int r = pair ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
-    const int role = pair ? (int)(blockIdx.x & 1) : 2;
-    const int nreal = pair ? (int)(gridDim.x >> 1) : (int)gridDim.x;
-    const Geo q = geo(a, 0, r);
-    const int n = q.n;
-    SmallSmem S;
-    small_layout(n, &S, small_smem);
-    ChanState& cst = a.cs[0];
-    const int cap = cst.cap;
-    double* mode = cst.mode_out + (size_t)q.r * n;
-    double* menv = a.menv + q.base;
-    double* up = sa.up + q.base;
-    const double* hin = a.h[0] + q.base;  // the stage input
-    const double inv_n = 1.0 / (double)n;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < n; i += kSmallThreads) S.H[i] = hin[i];
-    if (threadIdx.x == 0) {
-        s_ctl[0] = -1;
-        s_ctl[1] = 0;
-    }
-    __syncthreads();
-    int j = 0;
-    for (; j < cap; ++j) {
-        // deferred update of the previous iteration (updateRealizations); the mean envelope
-        // and the upper envelope are read through L2 (the paired CTA wrote them)
-        const int mk = s_ctl[0];
-        if (mk == 1) {
-            // the mean envelope's loads of a round are all issued before the subtractions
-            for (int i0 = 0; i0 < n; i0 += kSmallPre * kSmallThreads) {
-                double mv[kSmallPre];
-#pragma unroll
-                for (int k = 0; k < kSmallPre; ++k) {
-                    const int i = i0 + k * kSmallThreads + threadIdx.x;
-                    mv[k] = i < n ? __ldcg(menv + i) : 0.0;
-                }
-#pragma unroll
-                for (int k = 0; k < kSmallPre; ++k) {
-                    const int i = i0 + k * kSmallThreads + threadIdx.x;
-                    if (i < n) S.H[i] = S.H[i] - mv[k];
-                }
-            }
-        } else if (mk == 0 && role != 0)
-            for (int i = threadIdx.x; i < n; i += kSmallThreads) mode[i] = S.H[i];
-        __syncthreads();
-        int kmax = 0, kmin = 0;
-        if (role != 1) {
-            kmax = small_knots(S, n, 0);
-            if (sa.tblocks) small_tape_knots(S, sa, j, q.r, n, 0, kmax);
-            small_spline(S, n, kmax);
-            const bool dmax = small_coeffs(S, kmax);
-            for (int s = threadIdx.x; s < n; s += kSmallThreads) up[s] = small_env_at(S, s, dmax);
-            __syncthreads();
-            if (role == 0 && threadIdx.x == 0) {  // hand the upper envelope over
-                sa.pair_kmax[r] = kmax;
-                __threadfence();
-                cuda::atomic_ref<unsigned, cuda::thread_scope_device> rd(sa.ready[r]);
-                rd.store((unsigned)(j + 1), cuda::memory_order_release);
-            }
-        }
-        if (role != 0) {
-            kmin = small_knots(S, n, 1);
-            if (sa.tblocks) small_tape_knots(S, sa, j, q.r, n, 1, kmin);
-            small_spline(S, n, kmin);
-            const bool dmin = small_coeffs(S, kmin);
-            if (role == 1) {  // the upper envelope of this iteration from the paired CTA
-                if (threadIdx.x == 0) {
-                    const bool ok = small_wait(sa.ready + r, (unsigned)(j + 1), sa.spin_limit);
-                    if (!ok) atomicExch(&cst.err, kErrTimeout);
-                    s_ctl[3] = ok ? 0 : 1;
-                    s_ctl[4] = ok ? __ldcg(sa.pair_kmax + r) : 0;
-                }
-                __syncthreads();
-                if (s_ctl[3]) return;
-                kmax = s_ctl[4];
-            }
-            const bool write_mean = kmax > 3 && kmin > 3;
-            int cnt = 0, any = 0;
-            // the upper envelope's loads of a round are all issued first (the mean envelope's
-            // stores would otherwise hold each load back behind the previous sample's store)
-            for (int s0 = 0; s0 < n; s0 += kSmallPre * kSmallThreads) {
-                double uv[kSmallPre];
-#pragma unroll
-                for (int k = 0; k < kSmallPre; ++k) {
-                    const int s = s0 + k * kSmallThreads + threadIdx.x;
-                    uv[k] = s < n ? __ldcg(up + s) : 0.0;
-                }
-#pragma unroll
-                for (int k = 0; k < kSmallPre; ++k) {
-                    const int s = s0 + k * kSmallThreads + threadIdx.x;
-                    if (s < n) {
-                        const double v = small_env_at(S, s, dmin);
-                        const double u = uv[k];
-                        if (write_mean) menv[s] = (u + v) / 2.0;
-                        any |= sx_greater(u, v, a.sd2) ? 1 : 0;
-                        cnt += sx_greater(u, v, a.sd) ? 1 : 0;
-                    }
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-                any |= __shfl_xor_sync(0xffffffffu, any, o);
-            }
-            if (lane == 0) {
-                s_red[0][warp] = cnt;
-                s_red[1][warp] = any;
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                int c = 0, y = 0;
-                for (int w = 0; w < kSmallThreads / 32; ++w) {
-                    c += s_red[0][w];
-                    y |= s_red[1][w];
-                }
-                // the sifting-fraction carry and siftingCriterion (as k_criterion)
-                const double fr = (a.frac[q.g] + (double)c) * inv_n;
-                a.frac[q.g] = fr;
-                const bool crit = fr > a.tol || (y != 0 && (kmax + kmin) > 6);
-                int fin = s_ctl[1];
-                int mark;
-                if (crit) {
-                    mark = 1;
-                    if (fin == 0 && j == cap - 1) {
-                        mark = 0;
-                        fin = 1;
-                    }
-                } else {
-                    if (fin == 0) {
-                        mark = 0;
-                        fin = 1;
-                    } else {
-                        mark = 1;
-                    }
-                }
-                s_ctl[0] = mark;
-                s_ctl[1] = fin;
-                if (pair) sa.pair_mark[r] = mark;
-                if (sa.tblocks)
-                    reinterpret_cast<signed char*>(sa.tblocks[j / kTapeBlockSlots] +
-                                                   (size_t)(j % kTapeBlockSlots) * sa.tl.stride +
-                                                   sa.tl.off_mark)[q.r] = (signed char)mark;
-                atomicAdd(&cst.knots, (unsigned long long)(kmax + kmin));
-                // the lock-step test: every realization's finish flag of this iteration
-                if (fin) atomicAdd(sa.nfin + j, 1);
-            }
-        }
-        // every CTA meets the others once per iteration (the stop test's lock step)
-        if (threadIdx.x == 0) {
-            // the fence orders this CTA's writes before its arrival; the arrival is a
-            // reduction that does not wait for the counter's old value (the wait below
-            // acquires)
-            __threadfence();
-            atomicAdd(sa.arrive, 1u);
-            const unsigned target = (unsigned)(j + 1) * gridDim.x + sa.extra;
-            const bool ok = small_wait(sa.arrive, target, sa.spin_limit);
-            if (!ok) atomicExch(&cst.err, kErrTimeout);
-            cuda::atomic_ref<int, cuda::thread_scope_device> nf(sa.nfin[j]);
-            s_ctl[2] = a.forced > 0 ? (j + 1 >= a.forced ? 1 : 0)
-                                    : (nf.load(cuda::memory_order_acquire) == nreal ? 1 : 0);
-            s_ctl[3] = ok ? 0 : 1;
-            if (role == 0) s_ctl[0] = __ldcg(sa.pair_mark + r);  // the next update's mark
-        }
-        __syncthreads();
-        if (s_ctl[3]) return;  // a wait gave up: the host reports CEEMDAN_ERR_TIMEOUT
-        if (s_ctl[2]) {
-            ++j;
-            break;
-        }
-    }
-    if (j > cap) j = cap;
-    // realizations that finished in the last iteration export h (k_export_final)
-    if (s_ctl[0] == 0 && role != 0)
-        for (int i = threadIdx.x; i < n; i += kSmallThreads) mode[i] = S.H[i];
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        cst.iter = j;
-        cst.iters += (unsigned long long)j;
-        cst.done = 1;
-    }
 }
 
 }  // namespace ceemdan

@@ -1,0 +1,574 @@
+// Device primitives of the canonical spline solve shared by the kernels' translation units: exact
+// integer-divisor quotients, chunk sweeps over rows and knots, and the partitioned solve of padded
+// rows.  Arithmetic order: canon.cuh.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "canon.cuh"
+#include "kernels.h"
+
+namespace ceemdan {
+namespace {
+
+// Exact division by a tabled reciprocal: div_rcp's quotient (Markstein's correction, correctly
+// rounded in its range); `slow` marks operands outside that range, which take the division.
+__device__ __forceinline__ double rcp_fast(double a, double d, double y, bool& slow) {
+    const double q0 = a * y;
+    const double r = fma(-q0, d, a);
+    const double q1 = fma(r, y, q0);
+    slow = !(fabs(a) > 0x1p-960) || !(fabs(q1) < 0x1p+1000);
+    return q1;
+}
+
+// ---------------------------------------------------------------------------------------
+// chunk primitives of the canonical partitioned solve (rows produced by a functor)
+// ---------------------------------------------------------------------------------------
+struct ChunkEnds {
+    double ga, aa, ba, gb, ab, bb;
+};
+
+// End relations of a chunk of `len` rows: top-down elimination gives the last row
+// x_b = gb + ab*xL + bb*xR, bottom-up elimination the first row x_a = ga + aa*xL + ba*xR.
+// The two sweeps are independent chains and run interleaved.  The pivot reciprocals of the
+// top-down sweep are those of the interior's sweep: row k's goes to iw_out(k), where
+// chunk_interior_iw takes it from.  (Loops stay rolled: a CTA passes here once, and unrolled
+// sweeps spent most of their time fetching instructions, up to 1000 cycles a row.)
+template <class Pivot = SplinePivot, class RowFn, class IwOut>
+__device__ __forceinline__ ChunkEnds chunk_ends(int len, const RowFn& row, const IwOut& iw_out) {
+    const Row wa = row(0), wb = row(len - 1);
+    double iw = Pivot::inv(wa.m);
+    double iv = Pivot::inv(wb.m);
+    double cp = wa.u * iw, gp = wa.r * iw, ap = -wa.l * iw;
+    double cq = wb.l * iv, gq = wb.r * iv, bq = -wb.u * iv;
+    iw_out(0) = iw;
+    Row w = len > 1 ? row(1) : wa, v = len > 1 ? row(len - 2) : wb;
+#pragma unroll 1
+    for (int k = 1; k < len; ++k) {
+        const Row wc = w, vc = v;
+        if (k + 1 < len) {  // the next rows load while this row's reciprocals form
+            w = row(k + 1);
+            v = row(len - 2 - k);
+        }
+        iw = Pivot::inv(fma(-wc.l, cp, wc.m));
+        iv = Pivot::inv(fma(-vc.u, cq, vc.m));
+        cp = wc.u * iw;
+        gp = fma(-wc.l, gp, wc.r) * iw;
+        ap = (-wc.l * ap) * iw;
+        cq = vc.l * iv;
+        gq = fma(-vc.u, gq, vc.r) * iv;
+        bq = (-vc.u * bq) * iv;
+        iw_out(k) = iw;
+    }
+    ChunkEnds e;
+    e.gb = gp;
+    e.ab = ap;
+    e.bb = -wb.u * iw;
+    e.ga = gq;
+    e.ba = bq;
+    e.aa = -wa.l * iv;
+    return e;
+}
+
+// x(k) <- x(k) - fac(k) x(k+1) from row len-2 down, x(len-1) = xv; loads one row ahead.
+template <class X, class Fac>
+__device__ __forceinline__ void back_sweep(int len, double xv, const X& x, const Fac& fac) {
+    double f = 0.0, g = 0.0;
+    if (len > 1) {
+        f = fac(len - 2);
+        g = x(len - 2);
+    }
+#pragma unroll 1
+    for (int k = len - 2; k >= 0; --k) {
+        const double fc = f, gc = g;
+        if (k > 0) {
+            f = fac(k - 1);
+            g = x(k - 1);
+        }
+        xv = fma(-fc, xv, gc);
+        x(k) = xv;
+    }
+}
+
+// Interior of a chunk whose end relations chunk_ends formed: coupling terms to the right-hand
+// side, then canonical Thomas with the reciprocals left in x(k); x(k) receives the solution,
+// fac(k) the factors meanwhile (fac(k) may be row k's own u or a slot of it that rows after k do
+// not read).
+template <class RowFn, class X, class Fac>
+__device__ __forceinline__ void chunk_interior_iw(int len, const RowFn& row, double xl, double xr,
+                                                  const X& x, const Fac& fac) {
+    Row w = row(0);
+    double iw = x(0), gp = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < len; ++k) {
+        const Row wc = w;
+        const double ic = iw;
+        if (k + 1 < len) {
+            w = row(k + 1);
+            iw = x(k + 1);
+        }
+        double ri = wc.r;
+        if (k == 0) ri = fma(-wc.l, xl, ri);
+        if (k == len - 1) ri = fma(-wc.u, xr, ri);
+        gp = k == 0 ? ri * ic : fma(-wc.l, gp, ri) * ic;
+        fac(k) = wc.u * ic;
+        x(k) = gp;
+    }
+    back_sweep(len, gp, x, fac);
+}
+
+// Canonical Thomas on n <= kChunk rows, solution to x(k), factors to fac(k) meanwhile.
+template <class Pivot = SplinePivot, class RowFn, class X, class Fac>
+__device__ __forceinline__ void thomas_rolled(int n, const RowFn& row, const X& x,
+                                              const Fac& fac) {
+    Row w = row(0);
+    double cp = 0.0, gp = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) {
+        const Row wc = w;
+        if (k + 1 < n) w = row(k + 1);
+        const double iw = Pivot::inv(k == 0 ? wc.m : fma(-wc.l, cp, wc.m));
+        gp = k == 0 ? wc.r * iw : fma(-wc.l, gp, wc.r) * iw;
+        cp = wc.u * iw;
+        fac(k) = cp;
+        x(k) = gp;
+    }
+    back_sweep(n, gp, x, fac);
+}
+
+// Consecutive doubles as a row-indexed destination; NoIw drops what it is given.
+struct Slots {
+    double* p;
+    __device__ __forceinline__ double& operator()(int k) const { return p[k]; }
+};
+struct NoIw {
+    struct Sink {
+        __device__ __forceinline__ void operator=(double) const {}
+    };
+    __device__ __forceinline__ Sink operator()(int) const { return Sink(); }
+};
+
+// Interior of a chunk of `len` rows once its separator values xl, xr are known: coupling
+// terms move to the right-hand side, then canonical Thomas; x_k written to out[k*stride].
+// kCoupled = false is the plain canonical Thomas (no coupling terms at all).
+template <bool kCoupled = true, class Pivot = SplinePivot, class RowFn, class Out>
+__device__ __forceinline__ void chunk_interior(int len, const RowFn& row, double xl, double xr,
+                                               Out out, int stride) {
+    double cp[kChunk], gp[kChunk];
+#pragma unroll
+    for (int k = 0; k < kChunk; ++k) {
+        if (k < len) {
+            const Row w = row(k);
+            double ri = w.r;
+            if (kCoupled && k == 0) ri = fma(-w.l, xl, ri);
+            if (kCoupled && k == len - 1) ri = fma(-w.u, xr, ri);
+            if (k == 0) {
+                const double iw = Pivot::inv(w.m);
+                cp[0] = w.u * iw;
+                gp[0] = ri * iw;
+            } else {
+                const double iw = Pivot::inv(fma(-w.l, cp[k - 1], w.m));
+                cp[k] = w.u * iw;
+                gp[k] = fma(-w.l, gp[k - 1], ri) * iw;
+            }
+        }
+    }
+    double xv = 0.0;
+#pragma unroll
+    for (int k = kChunk - 1; k >= 0; --k) {
+        if (k < len) {
+            xv = (k == len - 1) ? gp[k] : fma(-cp[k], xv, gp[k]);
+            out[k * stride] = xv;
+        }
+    }
+}
+
+// Canonical Thomas on n <= kChunk rows (base case), x written with stride.
+template <class Pivot = SplinePivot, class RowFn>
+__device__ __forceinline__ void thomas_small(int n, const RowFn& row, double* x, int stride) {
+    chunk_interior<false, Pivot>(n, row, 0.0, 0.0, x, stride);
+}
+
+// Rows of a tile, knots of a spline: the padded position of in-tile knot m in the shared-memory
+// knot arrays, one pad slot after every 16 knots, so that the chunk sweeps (lane p walks the
+// knots of chunk p, 16 knots after lane p-1's) read different banks.
+__device__ __forceinline__ int kq(int m) { return m + (m >> 4); }
+
+// separators of a tile with c knots (local 0, 16, 32, ... and the last one)
+__device__ __forceinline__ int tile_seps(int c) { return c > 0 ? (c + kChunk - 2) / kChunk + 1 : 0; }
+
+// Asynchronous global -> shared copies.
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+// all but the newest group
+__device__ __forceinline__ void cp_async_wait_but_one() {
+    asm volatile("cp.async.wait_group 1;\n" ::);
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::); }
+
+// The quotient a / d by the division itself, kept out of line of the fast path (a plain
+// division in a branch is evaluated unconditionally by the compiler).
+__device__ __forceinline__ double div_cold(double a, double d) {
+    double q;
+    asm volatile("div.rn.f64 %0, %1, %2;" : "=d"(q) : "d"(a), "d"(d));
+    return q;
+}
+
+// a / d for an integer-valued d in [1, 2^40], from its reciprocal (Markstein's correction as in
+// div_rcp; operands outside its range take the division).  The reciprocal is pivot_inv's without
+// the check for the all-ones significand, which an integer below 2^52 does not have; measured
+// against a table of 1/d in global memory it saves the load and its bounds.
+__device__ __forceinline__ double div_int(double a, double d) {
+    bool slow;
+    double q = rcp_fast(a, d, rcp_raw(d), slow);
+    if (slow) q = div_cold(a, d);
+    return q;
+}
+
+// seg_coeffs' b and d from the segment's length, slope and spline values.
+__device__ __forceinline__ void seg_coeffs_int(double h, double slope, double c0, double c1,
+                                               double& b, double& d) {
+    const double hq = h * fma(2.0, c0, c1);
+    bool slow;
+    double qb = rcp_fast(hq, 3.0, kRcp3, slow);
+    if (slow) qb = div_cold(hq, 3.0);
+    d = div_int(c1 - c0, 3.0 * h);
+    b = slope - qb;
+}
+
+// Pivots of one chunk inverted by rcp_raw, with one look for the all-ones significand at the end
+// (low word -1; once in 2^32 pivots the caller repeats the chunk with pivot_inv).
+struct RawPivot {
+    bool ones = false;
+    __device__ __forceinline__ double inv(double x) {
+        ones |= __double2loint(x) == -1;
+        return rcp_raw(x);
+    }
+};
+struct CheckedPivot {
+    bool ones = false;
+    __device__ __forceinline__ double inv(double x) { return pivot_inv(x); }
+};
+
+// End relations (chunk_ends: same operations, same order) of the chunk whose knots 0..len+1 sit
+// in the padded arrays x, s from the chunk's base on (s[i]: slope of segment i -> i+1).  Each
+// sweep loads one new knot and slope per row, a row ahead of its use.
+template <bool kIw, class Pivot, class XT>
+__device__ __forceinline__ ChunkEnds chunk_ends_sweep(Pivot& pv, const XT* x, const double* s,
+                                                      int len, double* iwo) {
+    int xt = x[2], xb = x[len - 1];
+    // top-down row 0 and bottom-up row len-1
+    double lt = (double)(x[1] - x[0]), ut = (double)(xt - x[1]);
+    double ub = (double)(x[kq(len + 1)] - x[len]), lb = (double)(x[len] - xb);
+    double st = s[1], sb = s[len - 1];
+    const double wr0 = 3.0 * (st - s[0]), vr0 = 3.0 * (s[len] - sb);
+    const double lf = lt, ul = ub;
+    double un = 0.0, lp = 0.0, sn = 0.0, sp = 0.0;  // the next row's
+    if (len > 1) {
+        const int xn = x[kq(3)], xp = x[len - 2];
+        un = (double)(xn - xt);
+        xt = xn;
+        lp = (double)(xb - xp);
+        xb = xp;
+        sn = s[2];
+        sp = s[len - 2];
+    }
+    double iw = pv.inv(2.0 * (lt + ut));
+    double iv = pv.inv(2.0 * (lb + ub));
+    if (kIw) iwo[0] = iw;
+    double cp = ut * iw, gp = wr0 * iw, ap = -lt * iw;
+    double cq = lb * iv, gq = vr0 * iv, bq = -ub * iv;
+#pragma unroll 2
+    for (int k = 1; k < len; ++k) {
+        lt = ut;
+        ut = un;
+        ub = lb;
+        lb = lp;
+        const double wr = 3.0 * (sn - st), vr = 3.0 * (sb - sp);
+        st = sn;
+        sb = sp;
+        if (k + 1 < len) {
+            const int xn = x[kq(k + 3)], xp = x[len - 2 - k];
+            un = (double)(xn - xt);
+            xt = xn;
+            lp = (double)(xb - xp);
+            xb = xp;
+            sn = s[k + 2];
+            sp = s[len - 2 - k];
+        }
+        iw = pv.inv(fma(-lt, cp, 2.0 * (lt + ut)));
+        iv = pv.inv(fma(-ub, cq, 2.0 * (lb + ub)));
+        cp = ut * iw;
+        gp = fma(-lt, gp, wr) * iw;
+        ap = (-lt * ap) * iw;
+        cq = lb * iv;
+        gq = fma(-ub, gq, vr) * iv;
+        bq = (-ub * bq) * iv;
+        if (kIw) iwo[k] = iw;
+    }
+    ChunkEnds e;
+    e.gb = gp;
+    e.ab = ap;
+    e.bb = -ul * iw;
+    e.ga = gq;
+    e.ba = bq;
+    e.aa = -lf * iv;
+    return e;
+}
+template <bool kIw, class XT>
+__device__ __noinline__ void chunk_ends_checked(ChunkEnds& e, const XT* x, const double* s,
+                                                int len, double* iwo) {
+    CheckedPivot pv;
+    e = chunk_ends_sweep<kIw>(pv, x, s, len, iwo);
+}
+// kIw: the top-down sweep's reciprocals to iwo[0 .. len-1]
+template <bool kIw = false, class XT>
+__device__ __forceinline__ ChunkEnds chunk_ends_knots(const XT* x, const double* s, int len,
+                                                      double* iwo = nullptr) {
+    RawPivot pv;
+    ChunkEnds e = chunk_ends_sweep<kIw>(pv, x, s, len, iwo);
+    if (pv.ones) {
+        ChunkEnds c;
+        chunk_ends_checked<kIw>(c, x, s, len, iwo);
+        e = c;
+    }
+    return e;
+}
+
+// Inclusive prefix of v over the warp's lanes.
+__device__ __forceinline__ int warp_scan(int v, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += t;
+    }
+    return v;
+}
+
+// Rows of a system with one pad slot per 16 (row i at kq(i)): a chunk's rows are consecutive, and
+// the lanes that sweep neighbouring chunks read different banks.
+struct alignas(16) SepRow {
+    double l, m, u, r;
+};
+__device__ __forceinline__ SepRow load_row(const SepRow* p) {
+    const double2 a = reinterpret_cast<const double2*>(p)[0];
+    const double2 b = reinterpret_cast<const double2*>(p)[1];
+    return SepRow{a.x, a.y, b.x, b.y};
+}
+__device__ __forceinline__ SepRow sep_row(const Row& w) { return SepRow{w.l, w.m, w.u, w.r}; }
+// padded length of n rows
+__host__ __device__ __forceinline__ int padded(int n) { return n + (n >> 4) + 1; }
+
+// chunk_ends (same operations, same order) of len consecutive rows; the top-down sweep's
+// reciprocals to iw (kIw).  Rows are read one ahead of their use.
+template <bool kIw, class Pivot>
+__device__ __forceinline__ ChunkEnds ends_sweep(Pivot& pv, const SepRow* r, int len, double* iw) {
+    SepRow w = load_row(r), v = load_row(r + len - 1);
+    const double lf = w.l, ul = v.u;
+    double iu = pv.inv(w.m), iv = pv.inv(v.m);
+    double cp = w.u * iu, gp = w.r * iu, ap = -w.l * iu;
+    double cq = v.l * iv, gq = v.r * iv, bq = -v.u * iv;
+    if (kIw) iw[0] = iu;
+    if (len > 1) {
+        w = load_row(r + 1);
+        v = load_row(r + len - 2);
+    }
+#pragma unroll 1
+    for (int k = 1; k < len; ++k) {
+        const SepRow a = w, b = v;
+        if (k + 1 < len) {
+            w = load_row(r + k + 1);
+            v = load_row(r + len - 2 - k);
+        }
+        iu = pv.inv(fma(-a.l, cp, a.m));
+        iv = pv.inv(fma(-b.u, cq, b.m));
+        cp = a.u * iu;
+        gp = fma(-a.l, gp, a.r) * iu;
+        ap = (-a.l * ap) * iu;
+        cq = b.l * iv;
+        gq = fma(-b.u, gq, b.r) * iv;
+        bq = (-b.u * bq) * iv;
+        if (kIw) iw[k] = iu;
+    }
+    return ChunkEnds{gq, -lf * iv, bq, gp, ap, -ul * iu};
+}
+template <bool kIw>
+__device__ __noinline__ void ends_rows_checked(const SepRow* r, int len, double* iw,
+                                               ChunkEnds& e) {
+    CheckedPivot pv;
+    e = ends_sweep<kIw>(pv, r, len, iw);
+}
+// ... to out[0..5] = ga, aa, ba, gb, ab, bb
+template <bool kIw>
+__device__ __forceinline__ void ends_rows(const SepRow* r, int len, double* iw, double* out) {
+    RawPivot pv;
+    ChunkEnds e = ends_sweep<kIw>(pv, r, len, iw);
+    if (pv.ones) {
+        ChunkEnds c;
+        ends_rows_checked<kIw>(r, len, iw, c);
+        e = c;
+    }
+    out[0] = e.ga;
+    out[1] = e.aa;
+    out[2] = e.ba;
+    out[3] = e.gb;
+    out[4] = e.ab;
+    out[5] = e.bb;
+}
+
+// Row p of the next level: separator row s between the chunks with end relations e (left) and
+// e + 6 (right).
+__device__ __forceinline__ SepRow next_row(const SepRow& s, const double* e) {
+    return sep_row(reduced_row(Row{s.l, s.m, s.u, s.r}, e[3], e[4], e[5], e[6], e[7], e[8]));
+}
+
+// Back substitution x[k] <- x[k] - fac(k) x[k+1], row k's factor in its u.
+__device__ __forceinline__ void back_rows(const SepRow* r, double* x, int len, double xv) {
+    double f = 0.0, g = 0.0;
+    if (len > 1) {
+        f = r[len - 2].u;
+        g = x[len - 2];
+    }
+#pragma unroll 1
+    for (int k = len - 2; k >= 0; --k) {
+        const double fc = f, gc = g;
+        if (k > 0) {
+            f = r[k - 1].u;
+            g = x[k - 1];
+        }
+        xv = fma(-fc, xv, gc);
+        x[k] = xv;
+    }
+}
+
+// chunk_interior_iw of len consecutive rows: x holds the reciprocals, then the solution; the rows'
+// u is overwritten.
+__device__ __forceinline__ void interior_rows(SepRow* r, int len, double xl, double xr,
+                                              double* x) {
+    SepRow w = load_row(r);
+    double iw = x[0], gp = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < len; ++k) {
+        const SepRow a = w;
+        const double ic = iw;
+        if (k + 1 < len) {
+            w = load_row(r + k + 1);
+            iw = x[k + 1];
+        }
+        double ri = a.r;
+        if (k == 0) ri = fma(-a.l, xl, ri);
+        if (k == len - 1) ri = fma(-a.u, xr, ri);
+        gp = (k == 0 ? ri : fma(-a.l, gp, ri)) * ic;
+        r[k].u = a.u * ic;
+        x[k] = gp;
+    }
+    back_rows(r, x, len, gp);
+}
+
+// Canonical Thomas of n rows (kCoupled: a chunk between xl and xr), reciprocals formed here.
+template <bool kCoupled>
+__device__ __forceinline__ void thomas_rows(SepRow* r, int n, double xl, double xr, double* x) {
+    SepRow w = load_row(r);
+    double cp = 0.0, gp = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < n; ++k) {
+        const SepRow a = w;
+        if (k + 1 < n) w = load_row(r + k + 1);
+        double ri = a.r;
+        if (kCoupled && k == 0) ri = fma(-a.l, xl, ri);
+        if (kCoupled && k == n - 1) ri = fma(-a.u, xr, ri);
+        const double iw = pivot_inv(k == 0 ? a.m : fma(-a.l, cp, a.m));
+        gp = (k == 0 ? ri : fma(-a.l, gp, ri)) * iw;
+        cp = a.u * iw;
+        r[k].u = cp;
+        x[k] = gp;
+    }
+    back_rows(r, x, n, gp);
+}
+
+// cta_partitioned<SplinePivot> on padded rows: n rows at `rows` (u overwritten), solution to the
+// padded x; ws: 5 padded(n/16) + 6 (n/16 + 1) doubles and as much again for what is below, at
+// most 0.75 n + 64.  Every thread of the group calls it.
+struct RowsLevel {
+    SepRow* r;
+    double* x;
+    int n;
+};
+__device__ __forceinline__ RowsLevel rows_level(int k, int depth, int n, SepRow* rows, double* x,
+                                                double* ws) {
+    if (k == 0) return RowsLevel{rows, x, n};
+    int ro = 0, xo = 0, size = n, mine = 0, mr = 0, mx = 0;
+    for (int i = 1; i <= depth; ++i) {
+        size = (size - 1) / kChunk;
+        if (i == k) {
+            mine = size;
+            mr = ro;
+            mx = xo;
+        }
+        ro += 4 * padded(size);
+        xo += padded(size);
+    }
+    return RowsLevel{reinterpret_cast<SepRow*>(ws + mr), ws + ro + mx, mine};
+}
+
+// The threads that work on one system: a whole CTA, or half of one with a barrier of its own.
+struct CtaGroup {
+    __device__ __forceinline__ int tid() const { return threadIdx.x; }
+    __device__ __forceinline__ int size() const { return blockDim.x; }
+    __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+
+template <class Group>
+__device__ void partition_rows(const Group& grp, int n, SepRow* rows, double* x, double* ws) {
+    const int tid = grp.tid(), size_g = grp.size();
+    int depth = 0, all = 0;
+    for (int size = n; size > kChunk && depth < 7; ++depth) {
+        size = (size - 1) / kChunk;
+        all += 5 * padded(size);
+    }
+    double* ends = ws + all;
+#pragma unroll 1
+    for (int k = 0; k < depth; ++k) {
+        const RowsLevel v = rows_level(k, depth, n, rows, x, ws);
+        const RowsLevel o = rows_level(k + 1, depth, n, rows, x, ws);
+        for (int q = tid; q <= o.n; q += size_g) {
+            const int first = q * kChunk;
+            const int len = (q < o.n) ? kChunk - 1 : v.n - first;
+            ends_rows<true>(v.r + kq(first), len, v.x + kq(first), ends + 6 * q);
+        }
+        grp.sync();
+        for (int p = tid; p < o.n; p += size_g)
+            o.r[kq(p)] = next_row(load_row(v.r + kq(p * kChunk + kChunk - 1)), ends + 6 * p);
+        grp.sync();
+    }
+    if (tid == 0) {
+        const RowsLevel v = rows_level(depth, depth, n, rows, x, ws);
+        thomas_rows<false>(v.r, v.n, 0.0, 0.0, v.x);
+    }
+    grp.sync();
+#pragma unroll 1
+    for (int k = depth - 1; k >= 0; --k) {
+        const RowsLevel v = rows_level(k, depth, n, rows, x, ws);
+        const RowsLevel o = rows_level(k + 1, depth, n, rows, x, ws);
+        for (int q = tid; q <= o.n; q += size_g) {
+            const int first = q * kChunk;
+            const int len = (q < o.n) ? kChunk - 1 : v.n - first;
+            const double xl = (q > 0) ? o.x[kq(q - 1)] : 0.0;
+            const double xr = (q < o.n) ? o.x[kq(q)] : 0.0;
+            interior_rows(v.r + kq(first), len, xl, xr, v.x + kq(first));
+            if (q < o.n) v.x[kq(first + kChunk - 1)] = xr;
+        }
+        grp.sync();
+    }
+}
+
+}  // namespace
+}  // namespace ceemdan
