@@ -41,9 +41,10 @@ constexpr int kThreads = 256;
 
 // The tile kernels run as persistent CTAs over the active tiles.  kEnv: the envelopes of one
 // iteration to dbg_upper / dbg_lower, no update and no stop test.  kDense: shared memory for
-// kSiftDense entries (three CTAs per SM) or kSiftSparse (four).
+// kSiftDense entries (three CTAs per SM) or kSiftSparse (five).
 __global__ void k_tile_knots(const __grid_constant__ SiftArgs a);
-template <bool kDense, bool kEnv>
+// kSplit: of the rows of its class only.
+template <bool kDense, bool kSplit, bool kEnv>
 __global__ void k_tile_sift(const __grid_constant__ SiftArgs a);
 __global__ void k_spline_solve(const __grid_constant__ SiftArgs a);
 
@@ -268,10 +269,15 @@ struct SiftEngine {
         if (const char* e = std::getenv("CEEMDAN_SPLIT_COUNT"))
             if (e[0] == '1') a.count_bits = 0;
         CKS(ws.alloc_n(&a.cmax, 2 * R));
+        CKS(ws.alloc_n(&a.cls_count, 2));
+        CKS(ws.alloc_n(&a.cls_row, 2 * R));
+        CKS(ws.alloc_n(&a.cls_wait, R));
         CKS(ws.alloc_n(&a.tile_cnt, 2 * T));
         CKS(ws.alloc_n(&a.plan, 2 * (size_t)nchan + 2));
         CKS(ws.alloc_n(&a.bitmap, 2 * T * (kTileSamples / 32)));
         CKS(ws.alloc_n(&a.scan, T));
+        CKS(ws.alloc_n(&a.list_x, 2 * T * kListSlots));
+        CKS(ws.alloc_n(&a.list_s, 2 * T * kListSlots));
         CKS(ws.alloc_n(&a.hdr, 2 * T));
         CKS(ws.alloc_n(&a.edge, 2 * T));
         CKS(ws.alloc_n(&a.rows, 2 * T * kRowSlots * 4));
@@ -308,10 +314,11 @@ struct SiftEngine {
         a.solve_wcap = (kSolveSmem - kSolveStage) / (int)sizeof(double);
         CK(cudaFuncSetAttribute(k_spline_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSolveSmem));
-        for (auto k : {k_tile_sift<false, false>, k_tile_sift<false, true>})
+        for (auto k : {k_tile_sift<false, true, false>, k_tile_sift<false, true, true>})
             CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)tile_sift_smem(false)));
-        for (auto k : {k_tile_sift<true, false>, k_tile_sift<true, true>})
+        for (auto k : {k_tile_sift<true, false, false>, k_tile_sift<true, false, true>,
+                       k_tile_sift<true, true, false>, k_tile_sift<true, true, true>})
             CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)tile_sift_smem(true)));
         CK(cudaFuncSetAttribute(k_tile_knots, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -323,8 +330,8 @@ struct SiftEngine {
             return std::max(1, (int)std::min<size_t>(T, (size_t)std::max(1, per) * sm_count()));
         };
         knots_grid = grid((const void*)k_tile_knots, tile_knots_smem());
-        dense_grid = grid((const void*)k_tile_sift<true, false>, tile_sift_smem(true));
-        sift_grid = grid((const void*)k_tile_sift<false, false>, tile_sift_smem(false));
+        dense_grid = grid((const void*)k_tile_sift<true, true, false>, tile_sift_smem(true));
+        sift_grid = grid((const void*)k_tile_sift<false, true, false>, tile_sift_smem(false));
         CK(cudaGetLastError());
         // as many tiles as the dense form holds at once: one launch does for all rows
         a.sift_split = (size_t)dense_grid < T ? 1 : 0;
@@ -404,6 +411,7 @@ struct SiftEngine {
         CK(cudaMemsetAsync(a.any, 0, sizeof(int) * a.nrows, st));
         CK(cudaMemsetAsync(a.par, 0, sizeof(int) * a.nrows, st));
         CK(cudaMemsetAsync(a.acc, 0, sizeof(*a.acc) * a.nrows, st));
+        CK(cudaMemsetAsync(a.cls_wait, 0, sizeof(unsigned) * a.nrows, st));
         CK(cudaMemsetAsync(a.acc_wide, 0, sizeof(*a.acc_wide) * 2 * a.nrows, st));
         CK(cudaMemsetAsync(cs, 0, sizeof(ChanState) * a.nchan, st));
         return CEEMDAN_OK;
@@ -449,16 +457,21 @@ struct SiftEngine {
             ++g_launches;
         }
         mark_ev(2, 0);
-        if (a.dbg_upper) {
-            k_tile_sift<true, true><<<dense_grid, kTileThreads, tile_sift_smem(true), st>>>(a);
-            if (a.sift_split)
-                k_tile_sift<false, true><<<sift_grid, kTileThreads, tile_sift_smem(false), st>>>(a);
-        } else {
-            k_tile_sift<true, false><<<dense_grid, kTileThreads, tile_sift_smem(true), st>>>(a);
-            if (a.sift_split)
-                k_tile_sift<false, false><<<sift_grid, kTileThreads, tile_sift_smem(false), st>>>(
-                    a);
-        }
+        auto sift = [&](auto one, auto dense, auto sparse) {
+            const size_t sd = tile_sift_smem(true), ss = tile_sift_smem(false);
+            if (!a.sift_split) {
+                one<<<dense_grid, kTileThreads, sd, st>>>(a);
+                return;
+            }
+            dense<<<dense_grid, kTileThreads, sd, st>>>(a);
+            sparse<<<sift_grid, kTileThreads, ss, st>>>(a);
+        };
+        if (a.dbg_upper)
+            sift(k_tile_sift<true, false, true>, k_tile_sift<true, true, true>,
+                 k_tile_sift<false, true, true>);
+        else
+            sift(k_tile_sift<true, false, false>, k_tile_sift<true, true, false>,
+                 k_tile_sift<false, true, false>);
         mark_ev(2, 1);
         g_launches += sift_kernels();
         CK(cudaGetLastError());

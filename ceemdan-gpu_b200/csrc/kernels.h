@@ -67,6 +67,9 @@ struct TileEdge {
 // Threads per CTA of the tile kernels: a thread holds 16 consecutive samples.
 constexpr int kTileThreads = 128;
 
+// Slots of a tile's knots of one envelope: at most 1025, a pad slot after every sixteen.
+constexpr int kListSlots = 1096;
+
 // Knots of a tile (maxima in the low half words, minima in the high ones): before each warp's
 // samples, and in all.
 struct TileScan {
@@ -115,10 +118,18 @@ struct SiftArgs {
     int count_bits;
     int* kcount;           // [2*nrows] maxima counts, minima counts (by spline)
     int* cmax;             // [2*nrows] knots of a spline's densest tile
-    int sift_split;        // k_tile_sift runs as two launches (dense and sparse rows), else one
+    // k_tile_sift runs as two launches (sparse rows, class 0, and dense ones), else one: the rows
+    // (high word) and tiles of each class [2]; its rows: channel, row in it, first tile in the list
+    // [2][nrows]; a row's first knot count + 1 until the second comes [nrows]
+    int sift_split;
+    unsigned long long* cls_count;
+    int4* cls_row;
+    unsigned* cls_wait;
     int* tile_cnt;         // [2*ntot] knots found in each tile
     unsigned* bitmap;      // [2][ntot][64] knot flags of each tile (word j/32, bit j%32)
     TileScan* scan;        // [ntot]
+    short* list_x;         // [2*ntot][kListSlots] a tile's knots, padded (kq): positions in it,
+    double* list_s;        // and slopes of the segments from them (k_tile_knots -> k_tile_sift)
     TileHdr* hdr;          // [2*ntot]
     TileEdge* edge;        // [2*ntot]
     double* rows;          // [2*ntot][kRowSlots][4] rows (l, m, u, r) of the separator system
@@ -219,10 +230,10 @@ struct SmallArgs {
 constexpr int kTapeBlockSlots = 32;  // tape slots per allocation block
 
 __global__ void k_gather_knots(SiftArgs a, int e, int32_t* kx, double* ky);
-// Shared-memory entries of k_tile_sift.  Dense: both envelopes of a tile of up to about 1860 knots
+// Shared-memory entries of k_tile_sift.  Dense: both envelopes of a tile of up to about 1780 knots
 // at once (white noise has 1370, sifted a thousand times 1490), one after the other above.
-// Sparse: up to about 1260 knots a tile, every stage after the first of white noise.
-constexpr int kSiftDense = 1984, kSiftSparse = 1344;
+// Sparse: up to about 660 knots a tile, the stages after the second of white noise.
+constexpr int kSiftDense = 1928, kSiftSparse = 736;
 size_t tile_sift_smem(bool dense);
 size_t tile_knots_smem();
 

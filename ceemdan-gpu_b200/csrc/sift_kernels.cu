@@ -148,8 +148,17 @@ __device__ __forceinline__ size_t red_base(const SiftArgs& a, int e, const Geo& 
 }
 
 // Entry of k_tile_sift's arrays where the segment of a sample with r knots before it in the tile
-// starts: the knot before the tile at 0, in-tile knot m at 2 + kq(m).
+// starts: the knot before the tile at 0, in-tile knot m at 2 + kq(m).  An envelope's entries start
+// kLead past a multiple of eight, so that its list of in-tile knots starts at one (the 16-byte
+// copies of the positions).
 __device__ __forceinline__ int seg_at(int r) { return r + ((r + 15) >> 4); }
+constexpr int kLead = 6;
+// With both envelopes there: where envelope 1's entries start, and the entries that takes (the
+// copies round up to eight), given the most knots a tile of the row has.
+__device__ __forceinline__ int sift_base1(int cm0) { return kLead + ((seg_at(cm0 + 1) + 8) & ~7); }
+__device__ __forceinline__ int sift_need(int cm0, int cm1) {
+    return sift_base1(cm0) + seg_at(cm1 + 1) + 8;
+}
 
 // Four doubles to a 32-byte aligned address, as one access.
 __device__ __forceinline__ void store4(double* p, const double* v) {
@@ -161,39 +170,75 @@ __device__ __forceinline__ void store4(double* p, const double* v) {
 // The tile kernels run as persistent CTAs: CTA b works on the b-th of gridDim.x contiguous ranges
 // of the active tiles, and copies the next tile's samples to shared memory while it computes on
 // the current one.  TileIter walks the range; mark and par are the row's (loaded once a row).
+// kList: the rows of k_tile_sift's class cls, as k_spline_solve listed them (contiguous ranges of
+// all rows would leave most CTAs idle while a few work on the rows of the other class).
+template <bool kList, int cls>
 struct TileIter {
     int v, end;  // active tile, end of the range
-    int tile, mark, par;
-    // averageUppperLower: the mean envelope keeps its previous value unless both envelopes have
-    // more than 3 knots
-    bool mean;
-    int need;  // shared-memory entries of k_tile_sift the row's tiles need at most
+    int tile;
+    int cm;      // knots of the row's densest tile (of the envelope whose list the thread fetches)
+    int base1;   // k_tile_sift: envelope 1's entries when both envelopes are there at once
+    unsigned flags;  // above four bits of the row: its position in the list (kList)
     Geo q;
     __device__ __forceinline__ void row(const SiftArgs& a) {
-        q = tile_geo(a, v, tile);
-        mark = a.mark[q.g];
-        par = a.par[q.g];
-        mean = min(a.kcount[q.g], a.kcount[a.nrows + q.g]) > 3;
-        need = seg_at(a.cmax[q.g] + 1) + seg_at(a.cmax[a.nrows + q.g] + 1) + 2;
+        if (kList) {
+            const int4 w = a.cls_row[(size_t)cls * a.nrows + (flags >> 4)];
+            q = geo(a, w.x, w.y);
+            tile = v - w.z;
+        } else {
+            q = tile_geo(a, v, tile);
+        }
+        const int cm0 = a.cmax[q.g], cm1 = a.cmax[a.nrows + q.g];
+        cm = threadIdx.x < kTileThreads / 2 ? cm0 : cm1;
+        base1 = sift_base1(cm0);
+        const int need = sift_need(cm0, cm1);
+        flags = (flags & ~15u) | (a.par[q.g] != 0 ? 1u : 0u) | (a.mark[q.g] != 0 ? 2u : 0u) |
+                (min(a.kcount[q.g], a.kcount[a.nrows + q.g]) > 3 ? 4u : 0u) |
+                (need > kSiftDense ? 8u : 0u);
     }
     __device__ __forceinline__ explicit TileIter(const SiftArgs& a) {
-        const int total = active_tiles(a);
+        const unsigned long long word = kList ? a.cls_count[cls] : 0ull;
+        const int total = kList ? (int)(word & 0xffffffffull) : active_tiles(a);
         v = (int)((long long)total * blockIdx.x / gridDim.x);
         end = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
-        tile = mark = par = need = 0;
-        mean = false;
-        if (v < end) row(a);
+        tile = cm = base1 = 0;
+        flags = 0u;
+        if (v >= end) return;
+        if (kList) {  // the last row that starts at v or before: 32 of them a look
+            const int lane = threadIdx.x & 31;
+            int pos = 0;
+            for (int n = (int)(word >> 32); n > 1;) {
+                const int step = (n + 31) >> 5, i = lane * step;
+                const bool le = i < n && a.cls_row[(size_t)cls * a.nrows + pos + i].z <= v;
+                const int last = (31 - __clz(__ballot_sync(0xffffffffu, le))) * step;
+                pos += last;
+                n = min(step, n - last);
+            }
+            flags = (unsigned)pos << 4;
+        }
+        row(a);
     }
+    __device__ __forceinline__ int par() const { return (int)(flags & 1u); }
+    __device__ __forceinline__ bool live() const { return flags & 2u; }  // else: repeats
+    // averageUppperLower: the mean envelope keeps its previous value unless both envelopes have
+    // more than 3 knots
+    __device__ __forceinline__ bool mean() const { return flags & 4u; }
+    // k_tile_sift: more entries than the dense form has
+    __device__ __forceinline__ bool two() const { return flags & 8u; }
     __device__ __forceinline__ bool more() const { return v < end; }
     __device__ __forceinline__ void next(const SiftArgs& a) {
         ++v;
-        if (++tile == q.ntiles && v < end) row(a);
+        if (++tile == q.ntiles) {
+            if (kList) flags += 16u;
+            if (v < end) row(a);
+        }
     }
     // past the rest of the row while it does not satisfy pred
     template <class Pred>
     __device__ __forceinline__ void to_row(const SiftArgs& a, Pred pred) {
         while (v < end && !pred(*this)) {
             v += q.ntiles - tile;
+            if (kList) flags += 16u;
             if (v < end) row(a);
         }
     }
@@ -206,26 +251,33 @@ __device__ __forceinline__ int stage_piece(int u) { return u ^ ((u >> 3) & 7); }
 
 __device__ __forceinline__ void stage_tile(double2* st, const double* h, int m, int tid) {
     const int u0 = (tid & ~31) * (kPerThread / 2) + (tid & 31);
+    // 32 pieces on, the swizzle changes in its third bit only
+    double2* const s0 = st + stage_piece(u0);
+    double2* const s1 = st + (stage_piece(u0) ^ 4);
+    const double* src = h + 2 * u0;
     if (m == kTileSamples) {
 #pragma unroll
-        for (int g = 0; g < kPerThread / 2; ++g) cp_async16(st + stage_piece(u0 + 32 * g), h + 2 * (u0 + 32 * g));
+        for (int g = 0; g < kPerThread / 2; ++g) cp_async16((g & 1 ? s1 : s0) + 32 * g, src + 64 * g);
     } else {
         const int m4 = (m + 3) & ~3;  // rows are padded to a multiple of four samples
 #pragma unroll
         for (int g = 0; g < kPerThread / 2; ++g)
-            if (2 * (u0 + 32 * g) < m4)
-                cp_async16(st + stage_piece(u0 + 32 * g), h + 2 * (u0 + 32 * g));
+            if (2 * (u0 + 32 * g) < m4) cp_async16((g & 1 ? s1 : s0) + 32 * g, src + 64 * g);
     }
+}
+// piece g of the thread's own samples (g < 8)
+__device__ __forceinline__ double2* own_piece(double2* st, int tid, int g) {
+    return st + ((kPerThread / 2 * tid + (tid & 7)) ^ g);
 }
 // sample j of the tile
 __device__ __forceinline__ double staged(const double2* st, int j) {
     return reinterpret_cast<const double*>(st + stage_piece(j >> 1))[j & 1];
 }
 // the thread's samples (zeros past the row)
-__device__ __forceinline__ void unstage_tile(double* h, const double2* st, int m, int tid) {
+__device__ __forceinline__ void unstage_tile(double* h, double2* st, int m, int tid) {
 #pragma unroll
     for (int g = 0; g < kPerThread / 2; ++g) {
-        const double2 w = st[stage_piece(kPerThread / 2 * tid + g)];
+        const double2 w = *own_piece(st, tid, g);
         h[2 * g] = w.x;
         h[2 * g + 1] = w.y;
     }
@@ -249,15 +301,17 @@ __device__ __forceinline__ bool sweep_lane(int tid, int ns0, int ns1, int& e, in
 // Shared memory of k_tile_knots: per envelope the knots' positions within the tile and the slopes
 // of the segments starting at them (padded positions kq), and the tile's samples.  41.5 KB: five
 // CTAs per SM.
-constexpr int kKnotCap = kTileSamples / 2 + 1 + (kTileSamples / 2 + 1) / kChunk + 1;
 struct KnotSmem {
-    double s[2][kKnotCap];
+    double s[2][kListSlots];
     double ex[2][3][kRowSlots];       // first-row end relations of chunk k
     double2 stage[kTileSamples / 2];  // the samples
     double halo[kTileWarps][2];       // each warp's neighbours
     double yend[2][2];                // the row's end values
-    short x[2][kKnotCap];
+    alignas(16) short x[2][kListSlots];
 };
+static_assert(kListSlots % 8 == 0 &&
+                  kListSlots >= kTileSamples / 2 + 1 + (kTileSamples / 2 + 1) / kChunk + 1,
+              "a tile's knots of one envelope, padded, in 16-byte pieces");
 
 }  // namespace
 
@@ -278,12 +332,14 @@ k_tile_knots(const __grid_constant__ SiftArgs a) {
     KnotSmem& S = *reinterpret_cast<KnotSmem*>(dyn_smem);
     __shared__ int s_w[kTileWarps];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    TileIter it(a);
-    auto live = [](const TileIter& t) { return t.mark != 0; };  // else: repeats (k_tile_sift)
+    if (blockIdx.x == 0 && threadIdx.x < 2) a.cls_count[threadIdx.x] = 0ull;  // (k_spline_solve)
+    using Iter = TileIter<false, 0>;
+    Iter it(a);
+    auto live = [](const Iter& t) { return t.live(); };
     auto prefetch = [&]() {
         if (!it.more()) return;
         const int n0 = it.tile * kTileSamples, left = it.q.n - n0;
-        const double* h = a.h[it.par] + it.q.base + n0;
+        const double* h = a.h[it.par()] + it.q.base + n0;
         stage_tile(S.stage, h, min(kTileSamples, left), tid);
         const int j = warp * kWarpSamples;  // the neighbours of the warp's samples
         if (lane == 0 && n0 + j > 0 && j <= left) cp_async8(&S.halo[warp][0], h + j - 1);
@@ -358,15 +414,13 @@ k_tile_knots(const __grid_constant__ SiftArgs a) {
     {
         const int ex = wb + incl - own;
         int p0 = ex & 0xffff, p1 = ex >> 16;
-        const unsigned any = __reduce_or_sync(0xffffffffu, b0 | b1);
-#pragma unroll
-        for (int i0 = 0; i0 < kPerThread; i0 += 4) {
-            if (!(any >> i0 & 15u)) continue;  // no knots at these samples in the whole warp
-#pragma unroll
-            for (int i = i0; i < i0 + 4; ++i) {
-                if (b0 >> i & 1u) S.x[0][kq(p0++)] = (short)(j0 + i);
-                if (b1 >> i & 1u) S.x[1][kq(p1++)] = (short)(j0 + i);
-            }
+        // one knot of each envelope a turn: as many turns as the warp's fullest thread has knots
+        unsigned w0 = b0, w1 = b1;
+        while (w0 | w1) {
+            if (w0) S.x[0][kq(p0++)] = (short)(j0 + __ffs(w0) - 1);
+            if (w1) S.x[1][kq(p1++)] = (short)(j0 + __ffs(w1) - 1);
+            w0 &= w0 - 1u;
+            w1 &= w1 - 1u;
         }
     }
     __syncthreads();
@@ -440,9 +494,20 @@ k_tile_knots(const __grid_constant__ SiftArgs a) {
     }
     __syncthreads();
     // the samples are done with: the next tile's land during the sweeps
+    const size_t sl0 = tix(a, 0, q, tile) * kListSlots, sl1 = tix(a, 1, q, tile) * kListSlots;
     it.next(a);
     it.to_row(a, live);
     prefetch();
+    {  // the knots' positions and slopes for k_tile_sift, as they lie here
+        const int e = warp >> 1, c = e ? c1 : c0, n = c > 0 ? kq(c - 1) + 1 : 0;
+        const size_t sl = e ? sl1 : sl0;
+        const int4* xs = reinterpret_cast<const int4*>(S.x[e]);
+        const double2* ss = reinterpret_cast<const double2*>(S.s[e]);
+        int4* xo = reinterpret_cast<int4*>(a.list_x + sl);
+        double2* so = reinterpret_cast<double2*>(a.list_s + sl);
+        for (int i = tid & 63; i < (n + 7) >> 3; i += kTileThreads / 2) xo[i] = xs[i];
+        for (int i = tid & 63; i < (n + 1) >> 1; i += kTileThreads / 2) so[i] = ss[i];
+    }
     int e, k;
     const bool act = sweep_lane(tid, tile_seps(c0), tile_seps(c1), e, k);
     const int c = e ? c1 : c0;
@@ -1140,10 +1205,14 @@ __device__ __noinline__ void end_rule_sparse(const SiftArgs& a, int e, int sp, i
         if (c == 1) h0.y0 = v;
         if (c == 2) h0.y1 = v;
     }
-    if (c < 3) return;  // no rows between the tile's separators
     y[side == 0 ? 0 : c - 1] = v;
     double s[4];
     for (int i = 0; i + 1 < c; ++i) s[i] = seg_slope(x[i], x[i + 1], y[i], y[i + 1]);
+    if (c > 1) {  // k_tile_sift's slope of the end segment
+        const int i = side == 0 ? 0 : c - 2;
+        a.list_s[(size_t)(&h0 - a.hdr) * kListSlots + i] = s[i];
+    }
+    if (c < 3) return;  // no rows between the tile's separators
     const ChunkEnds ce = chunk_ends_knots(x, s, c - 2);
     h0.ga = ce.ga;
     h0.aa = ce.aa;
@@ -1179,7 +1248,18 @@ k_spline_solve(const __grid_constant__ SiftArgs a) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int done = a.nchan == 1 ? a.cs[0].done : 0, mark = a.mark[q.g];
     const int c_first = tid < q.ntiles ? a.tile_cnt[tix(a, e, q, 0) + tid] : 0;
-    if (done || mark == 0) return;  // (0: the row repeats its last iteration, k_tile_sift)
+    if (done) return;
+    // the row to the list of its class of k_tile_sift
+    auto list_row = [&](int cls) {
+        const unsigned long long w =
+            atomicAdd(&a.cls_count[cls], 1ull << 32 | (unsigned long long)q.ntiles);
+        a.cls_row[(size_t)cls * a.nrows + (size_t)(w >> 32)] =
+            make_int4(q.c, q.r, (int)(w & 0xffffffffull), 0);
+    };
+    if (mark == 0) {  // the row repeats its last iteration (k_tile_sift)
+        if (e == 0 && tid == 0 && a.sift_split) list_row(0);
+        return;
+    }
     const int sp = spline_id(a, e, q);
     const int ntiles = q.ntiles;
     const size_t te0 = tix(a, e, q, 0);
@@ -1232,6 +1312,14 @@ k_spline_solve(const __grid_constant__ SiftArgs a) {
         soff[ntiles] = P;
         a.kcount[sp] = K;
         a.cmax[sp] = cm;
+        if (a.sift_split) {  // the spline that comes second knows both counts
+            const unsigned other = atomicExch(&a.cls_wait[q.g], (unsigned)cm + 1u);
+            if (other != 0u) {
+                a.cls_wait[q.g] = 0u;
+                const int co = (int)other - 1;
+                list_row(sift_need(e ? co : cm, e ? cm : co) > kSiftSparse ? 1 : 0);
+            }
+        }
     }
     __syncthreads();
     const bool one = P <= kSolvePass;
@@ -1316,26 +1404,37 @@ k_spline_solve(const __grid_constant__ SiftArgs a) {
 }
 
 // =======================================================================================
-// k_tile_sift: one CTA per tile: the spline values of the tile's knots (chunk interiors, one
-// thread per chunk), the segment coefficients in shared memory, both envelopes at every sample,
-// the mean envelope, the sx statistics, and the sample's next value h - m written to the other h
-// plane.  The stop decision comes after a row's last tile (criterion below); it either takes the
+// k_tile_sift: persistent CTAs over the tiles: the spline values of the tile's knots (chunk
+// interiors, one thread per chunk), the segment coefficients in shared memory, both envelopes at
+// every sample, the mean envelope, the sx statistics, and the sample's next value h - m written to
+// the other h plane.  The stop decision comes after a row's last tile (criterion below); it either takes the
 // new plane as the row's h (mark 1) or keeps the old one (mark 0, the realization has finished:
 // its mode is h).  A row marked 0 repeats its iteration: h, knots and envelopes are the same, so
 // the next launch only exports the mode and counts the iteration; the new plane is already what
 // that iteration's update gives.  The knots of both envelopes fit the shared-memory arrays at
-// white-noise density (about 1440 a tile); denser tiles take one envelope after the other.
+// white-noise density (about 1440 a tile); denser rows take one envelope after the other.
+//
+// Bound by latency: a tile is a chain of short phases between barriers, so what counts is how many
+// CTAs an SM holds.  Registers are kept under 96 (flags and counts read anew in the rare paths,
+// two samples at a time, row words packed): five CTAs per SM with room for 736 knots, three with
+// room for 1928; a row goes by its densest tile.  Knots and slopes come from k_tile_knots' lists
+// instead of being found again, a row's counts are added once per CTA, not per tile, and both
+// planes are stored coalesced out of shared memory (a thread's 32 bytes in a line each took 32
+// cycles of the load/store unit, half of all it did).  B200, N=244032 NR=100, K/N = 0.18: 262 ->
+// 208 us (2.8 TB/s of its 24 N bytes); K/N = 0.001: 167 -> 145 us; white noise: 381 -> 321 us.
+// Four CTAs with room for 1184: 225, 153 and 321 us.  Each class's launch takes the tiles of its
+// own rows in even shares: with rows of both classes (K/N = 0.23) 398 -> 234 us.
 // =======================================================================================
 namespace {
 
 // The row's stop decision after an iteration (sifting fraction carry, siftingCriterion,
 // checkBreak), by one thread once all its tiles are counted (cn samples with sx > sd, any: some
 // sx > sd2); the channel's last row closes the channel's iteration.
-__device__ __noinline__ void row_criterion(const SiftArgs& a, const Geo& q, ChanState& cst,
+__device__ __noinline__ void row_criterion(const SiftArgs& a, int c, int g, int r, int n,
                                            unsigned cn, int any) {
-    const int g = q.g;
-    const int nr = a.nchan == 1 ? a.nr1 : __ldg(&a.chan[q.c].nr);
-    const double inv_n = 1.0 / (double)q.n;
+    ChanState& cst = a.cs[c];
+    const int nr = a.nchan == 1 ? a.nr1 : __ldg(&a.chan[c].nr);
+    const double inv_n = 1.0 / (double)n;
     const int j = cst.iter, cap = cst.cap;
     const int kk = a.kcount[g] + a.kcount[a.nrows + g];
     const double fr = (a.frac[g] + (double)cn) * inv_n;
@@ -1349,7 +1448,7 @@ __device__ __noinline__ void row_criterion(const SiftArgs& a, const Geo& q, Chan
     }
     a.mark[g] = mark;
     a.finish[g] = fin;
-    if (a.tape_mark) a.tape_mark[q.r] = (signed char)mark;
+    if (a.tape_mark) a.tape_mark[r] = (signed char)mark;
     if (mark == 1) {
         a.par[g] ^= 1;
     } else {  // the row's repeated iteration has the same counts
@@ -1369,19 +1468,19 @@ __device__ __noinline__ void row_criterion(const SiftArgs& a, const Geo& q, Chan
     }
 }
 
-// Adds a tile's counts to its row's: one 64-bit sum of tiles, tiles with some sx > sd2, and
-// samples with sx > sd, so that the thread that completes the row has them all from its own
+// Adds the counts of some tiles (of one CTA's range) to their row's: one 64-bit sum of tiles,
+// additions with some sx > sd2, and samples with sx > sd, so that the thread that completes the row has them all from its own
 // addition, without a fence between counts and ticket (a fence here waits for the tile's stores:
 // about a microsecond of every CTA).  Rows of 2^17 tiles and more (2^28 samples) do not fit one
 // word: they are counted in separate words, ordered by fences.  Returns true to the thread that
 // completes the row.
-__device__ __forceinline__ bool count_tile(const SiftArgs& a, const Geo& q, unsigned& cn,
-                                           int& any) {
+__device__ __forceinline__ bool count_tiles(const SiftArgs& a, const Geo& q, unsigned tiles,
+                                            unsigned& cn, int& any) {
     const int bits = 32 - __clz(q.ntiles);
     if (bits <= a.count_bits) {
         const int s1 = bits + 12, s2 = s1 + bits;
         const unsigned long long add = (unsigned long long)cn | (unsigned long long)any << s1 |
-                                       1ull << s2;
+                                       (unsigned long long)tiles << s2;
         const unsigned long long sum = atomicAdd(&a.acc[q.g], add) + add;
         if ((int)(sum >> s2) != q.ntiles) return false;
         a.acc[q.g] = 0ull;
@@ -1393,7 +1492,7 @@ __device__ __forceinline__ bool count_tile(const SiftArgs& a, const Geo& q, unsi
     if (cn) atomicAdd(w, cn);
     if (any) atomicOr(w + 1, 1u);
     __threadfence();
-    if (atomicAdd(w + 2, 1u) != (unsigned)q.ntiles - 1u) return false;
+    if (atomicAdd(w + 2, tiles) + tiles != (unsigned)q.ntiles) return false;
     __threadfence();
     cn = atomicExch(w, 0u);
     any = (int)atomicExch(w + 1, 0u);
@@ -1402,26 +1501,40 @@ __device__ __forceinline__ bool count_tile(const SiftArgs& a, const Geo& q, unsi
 }
 
 // chunk_interior (same operations, same order) of the chunk whose knots 0..len+1 sit in the
-// padded arrays from the chunk's base on: s slopes, d segment lengths on entry; c receives the
-// spline values of knots 1..len, d[k] the factor of row k meanwhile.
+// padded arrays from the chunk's base on: x positions, s slopes; c receives the spline values of
+// knots 1..len, d[k] the factor of row k meanwhile.  One new knot and slope a row, read ahead.
 template <class Pivot>
-__device__ __forceinline__ void chunk_interior_sweep(Pivot& pv, const double* s, double* c,
-                                                     double* d, int len, double xl, double xr) {
-    // row k: lengths d[k], d[k+1], slopes s[k], s[k+1]; row 0 takes xl, row len-1 takes xr
-    double l = d[0], u = d[1], sn = s[1];
-    double ri = fma(-l, xl, 3.0 * (sn - s[0]));
+__device__ __forceinline__ void chunk_interior_sweep(Pivot& pv, const short* x, const double* s,
+                                                     double* c, double* d, int len, double xl,
+                                                     double xr) {
+    // row k: lengths x[k+1] - x[k], x[k+2] - x[k+1], slopes s[k], s[k+1]; row 0 takes xl, row
+    // len-1 takes xr
+    int xt = x[2];
+    double l = (double)(x[1] - x[0]), u = (double)(xt - x[1]), un = 0.0, st = s[1], sn = 0.0;
+    double ri = fma(-l, xl, 3.0 * (st - s[0]));
     if (len == 1) ri = fma(-u, xr, ri);
+    if (len > 1) {
+        const int xn = x[kq(3)];
+        un = (double)(xn - xt);
+        xt = xn;
+        sn = s[2];
+    }
     double iw = pv.inv(2.0 * (l + u));
     double cp = u * iw, gp = ri * iw;
     d[0] = cp;
 #pragma unroll 2
     for (int k = 1; k < len; ++k) {
         c[k] = gp;
-        const double sv = sn;
         l = u;
-        u = d[k + 1];
-        sn = s[k + 1];
-        ri = 3.0 * (sn - sv);
+        u = un;
+        ri = 3.0 * (sn - st);
+        st = sn;
+        if (k + 1 < len) {
+            const int xn = x[kq(k + 3)];
+            un = (double)(xn - xt);
+            xt = xn;
+            sn = s[k + 2];
+        }
         if (k == len - 1) ri = fma(-u, xr, ri);
         iw = pv.inv(fma(-l, cp, 2.0 * (l + u)));
         gp = fma(-l, gp, ri) * iw;
@@ -1436,33 +1549,31 @@ __device__ __forceinline__ void chunk_interior_sweep(Pivot& pv, const double* s,
         c[k + 1] = xv;
     }
 }
-// The factors of row k take the place of segment k's length, which rows after k do not read; the
-// rare repetition with checked pivots finds the lengths in the knots' positions.
 __device__ __noinline__ void chunk_interior_checked(const short* x, const double* s, double* c,
                                                     double* d, int len, double xl, double xr) {
-    for (int i = 0; i <= len; ++i) d[i] = (double)(x[kq(i + 1)] - x[i]);
     CheckedPivot pv;
-    chunk_interior_sweep(pv, s, c, d, len, xl, xr);
+    chunk_interior_sweep(pv, x, s, c, d, len, xl, xr);
 }
 __device__ __forceinline__ void chunk_interior_knots(const short* x, const double* s, double* c,
                                                      double* d, int len, double xl, double xr) {
     RawPivot pv;
-    chunk_interior_sweep(pv, s, c, d, len, xl, xr);
+    chunk_interior_sweep(pv, x, s, c, d, len, xl, xr);
     if (pv.ones) chunk_interior_checked(x, s, c, d, len, xl, xr);
 }
 
 // Shared memory of k_tile_sift: kCap entries each for the knots' positions and segments (seg_at;
 // envelope 1 after envelope 0; the knot after the tile where in-tile knot `count` would be), the
-// tile's samples, and small pieces.  d holds the segment lengths until the sweeps.
+// tile's samples, and small pieces.  b holds the slopes at first.
 template <int kCap>
 struct SiftSmem {
     double b[kCap], c[kCap], d[kCap];
-    double2 stage[kTileSamples / 2];  // the samples
-    TileEdge edge[2][2];              // this and the next tile's edges (envelopes 0, 1)
-    unsigned bits[2][2][kWords];      // and bitmaps
-    TileScan scan[2];                 // and knot counts
+    double2 stage[kTileSamples / 2];  // the samples, in the end their next values
+    double2 mean[kTileSamples / 4];   // half of every thread's mean envelope
+    TileEdge edge[2];                 // and edges (envelopes 0, 1)
+    unsigned bits[2][kWords];         // and bitmaps
+    TileScan scan;                    // and knot counts
     double xs[2][kRowSlots];          // the tile's separator values
-    short x[kCap];
+    alignas(16) short x[kCap];
 };
 
 }  // namespace
@@ -1471,86 +1582,94 @@ size_t tile_sift_smem(bool dense) {
     return dense ? sizeof(SiftSmem<kSiftDense>) : sizeof(SiftSmem<kSiftSparse>);
 }
 
-template <bool kDense, bool kEnv>
-__global__ void __launch_bounds__(kTileThreads, kDense ? 3 : 4)
+template <bool kDense, bool kSplit, bool kEnv>
+__global__ void __launch_bounds__(kTileThreads, kDense ? 3 : 5)
 k_tile_sift(const __grid_constant__ SiftArgs a) {
     constexpr int kCap = kDense ? kSiftDense : kSiftSparse;
     extern __shared__ __align__(16) unsigned char dyn_smem[];
     SiftSmem<kCap>& S = *reinterpret_cast<SiftSmem<kCap>*>(dyn_smem);
-    __shared__ int s_w[kTileWarps];
+    __shared__ int s_w[kTileWarps], s_begin;  // (s_begin: thread 0's own)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    TileIter it(a);
-    // the rows of this launch
-    auto mine = [&](const TileIter& t) {
-        return a.sift_split == 0 || (t.need > kSiftSparse) == kDense;
+    TileIter<kSplit, kDense ? 1 : 0> it(a);
+    // the knots' positions and slopes of envelope e of the tile, to the entries from base on
+    auto fetch_list = [&](int e, int cm, int base, int th, int wh) {
+        if (cm == 0) return;
+        const size_t sl = tix(a, e, it.q, it.tile) * kListSlots;
+        const int n = kq(cm - 1) + 1;  // (of the row's densest tile)
+        for (int i = th; i < (n + 7) >> 3; i += wh)
+            cp_async16(&S.x[base + 2 + 8 * i], a.list_x + sl + 8 * i);
+        for (int i = th; i < (n + 1) >> 1; i += wh)
+            cp_async16(&S.b[base + 2 + 2 * i], a.list_s + sl + 2 * i);
     };
-    int buf = 0;
-    auto prefetch = [&](int to) {
+    constexpr int kHalf = kTileThreads / 2;  // threads per envelope
+    int sep = 0;  // the tile's first separator (of the envelope the thread fetches)
+    // the tile's pieces, in two groups: what the sweeps read, then the samples
+    auto prefetch = [&]() {
         if (!it.more()) return;
+        if (it.live()) {
+            const int e = tid / kHalf, th = tid % kHalf;
+            const size_t te = tix(a, e, it.q, it.tile);
+            if (th < kWords / 4) cp_async16(&S.bits[e][4 * th], a.bitmap + te * kWords + 4 * th);
+            if (th >= 16 && th < 16 + (int)sizeof(TileEdge) / 16)
+                cp_async16(reinterpret_cast<char*>(&S.edge[e]) + 16 * (th - 16),
+                           reinterpret_cast<const char*>(a.edge + te) + 16 * (th - 16));
+            if (tid >= 24 && tid < 24 + (int)sizeof(TileScan) / 16)
+                cp_async16(reinterpret_cast<char*>(&S.scan) + 16 * (tid - 24),
+                           reinterpret_cast<const char*>(a.scan + it.q.tile0 + it.tile) +
+                               16 * (tid - 24));
+            if (e == 0 || !(kDense && it.two()))
+                fetch_list(e, it.cm, e ? it.base1 : kLead, th, kHalf);
+            const double* X = a.xsep + rec_base(a, e, it.q) + sep;
+            for (int i = th; i < kRowSlots; i += kHalf) cp_async8(&S.xs[e][i], X + i);
+        }
+        cp_async_commit();
         const int n0 = it.tile * kTileSamples;
-        stage_tile(S.stage, a.h[it.par] + it.q.base + n0, min(kTileSamples, it.q.n - n0), tid);
-        const int e = (tid >> 5) & 1;
-        const size_t te = tix(a, e, it.q, it.tile);
-        if (tid < 64 && lane < kWords / 4)
-            cp_async16(&S.bits[to][e][4 * lane], a.bitmap + te * kWords + 4 * lane);
-        if (tid < 64 && lane >= 16 && lane < 16 + (int)sizeof(TileEdge) / 16)
-            cp_async16(reinterpret_cast<char*>(&S.edge[to][e]) + 16 * (lane - 16),
-                       reinterpret_cast<const char*>(a.edge + te) + 16 * (lane - 16));
-        if (tid >= 24 && tid < 24 + (int)sizeof(TileScan) / 16)
-            cp_async16(reinterpret_cast<char*>(&S.scan[to]) + 16 * (tid - 24),
-                       reinterpret_cast<const char*>(a.scan + it.q.tile0 + it.tile) +
-                           16 * (tid - 24));
+        stage_tile(S.stage, a.h[it.par()] + it.q.base + n0, min(kTileSamples, it.q.n - n0), tid);
+        cp_async_commit();
     };
-    it.to_row(a, mine);
-    prefetch(0);
+    if (tid == 0) s_begin = it.v;
+    if (it.more() && it.tile > 0) sep = a.edge[tix(a, tid / kHalf, it.q, it.tile)].sep0;
+    prefetch();
+    // samples with sx > sd of the row's tiles so far, and in the sign bit whether some sx > sd2
+    unsigned cnt_row = 0u;
     while (it.more()) {
     const Geo q = it.q;
     const int tile = it.tile;
-    const bool repeat = it.mark == 0, write_mean = it.mean;
+    const bool repeat = !it.live(), write_mean = it.mean();
     ChanState& cst = a.cs[q.c];
     const int n0 = tile * kTileSamples;
     const int m = min(kTileSamples, q.n - n0);  // samples of the tile
-    const double* __restrict__ hin = a.h[it.par] + q.base + n0;
-    double* __restrict__ hout = a.h[it.par ^ 1] + q.base + n0;
+    // the tile in the current plane and in the next one (kEnv: in the upper envelope)
+    auto hin = [&]() -> const double* { return a.h[it.par()] + q.base + n0; };
+    auto hout = [&]() -> double* {
+        return kEnv ? a.dbg_upper + (size_t)q.r * q.n + n0 : a.h[it.par() ^ 1] + q.base + n0;
+    };
     const int j0 = kPerThread * tid;
     const int lim = m - j0;  // the thread's samples in the row
-    cp_async_wait_all();
-    __syncthreads();  // also: the CTA's last tile is done with shared memory
+    if (repeat) cp_async_wait_all();
+    else cp_async_wait_but_one();  // (the samples are waited for after the sweeps)
+    __syncthreads();
     unsigned cnt = 0u;  // samples with sx > sd
     int any = 0;        // some sx > sd2
-    // once a warp is done with its staged samples the next tile's take their place
-    auto advance = [&]() {
-        __syncwarp();
-        it.next(a);
-        it.to_row(a, mine);
-        buf ^= 1;
-        prefetch(buf);
-    };
     if (repeat) {
         // repeated iteration of a finished row: its mode is h
         double* mo = cst.mode_out + (size_t)q.r * q.n + n0;
         const int w0 = warp * kWarpSamples;
         for (int j = w0 + lane; j < min(m, w0 + kWarpSamples); j += 32) mo[j] = staged(S.stage, j);
-        advance();
     } else {
-    const TileEdge* ed0 = &S.edge[buf][0];
-    const TileEdge* ed1 = &S.edge[buf][1];
-    // the tile's separator values land while its knots are compacted
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        const double* X = a.xsep + rec_base(a, e, q) + (e ? ed1 : ed0)->sep0;
-        if (tid < kRowSlots) cp_async8(&S.xs[e][tid], X + tid);
-    }
-    const unsigned b0 = reinterpret_cast<const TileBits*>(S.bits[buf][0])[tid];
-    const unsigned b1 = reinterpret_cast<const TileBits*>(S.bits[buf][1])[tid];
-    const int tot = S.scan[buf].total;
+    const TileEdge* ed0 = &S.edge[0];
+    const TileEdge* ed1 = &S.edge[1];
+    const unsigned b0 = reinterpret_cast<const TileBits*>(S.bits[0])[tid];
+    const unsigned b1 = reinterpret_cast<const TileBits*>(S.bits[1])[tid];
+    const int tot = S.scan.total;
     const int own = __popc(b0) | __popc(b1) << 16;
-    const int ex = S.scan[buf].before[warp] + warp_scan(own, lane) - own;
+    const int ex = S.scan.before[warp] + warp_scan(own, lane) - own;
     const bool first = tile == 0, last = tile == q.ntiles - 1;
     const int c0 = tot & 0xffff, c1 = tot >> 16;
-    // (only the densest tiles of the dense launch; the sparse launch's rows all fit)
-    const bool two = kDense && seg_at(c0 + 1) + seg_at(c1 + 1) + 2 > kCap;
-    const int base1 = two ? 0 : seg_at(c0 + 1) + 1;
+    // (only the densest rows of the dense launch)
+    const bool two = kDense && it.two();
+    const int base0 = kLead, base1 = two ? kLead : it.base1;
+    sep += tile_seps(tid < kHalf ? c0 : c1);  // the next tile's, unless a row starts there
     // knots before the thread's first sample (sample 0 of the row lies in the first segment)
     const bool origin = first && tid == 0;
     const int rA0 = origin ? 1 : ex & 0xffff, rA1 = origin ? 1 : ex >> 16;
@@ -1573,74 +1692,33 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
     };
     // envelope e at the thread's sample i, one at a time (the paths that are not the common one);
     // values from h itself: other warps may have refilled the stage
-    auto env_one = [&](int e, int i) -> double {
-        const unsigned b = (e ? b1 : b0) & ((1u << i) - 1u);
-        int r = (e ? ex >> 16 : ex & 0xffff) + __popc(b);
+    auto env_one = [&](int e, int i, unsigned flags, int before) -> double {
+        int r = (e ? before >> 16 : before & 0xffff) + __popc(flags & ((1u << i) - 1u));
         if (first && j0 + i == 0) r = 1;
-        const int p = (e ? base1 : 0) + seg_at(r);
+        const int p = (e ? base1 : base0) + seg_at(r);
         const int x = knot_x(e, r, p);
         double y;
         if (r == 0) y = (e ? ed1 : ed0)->py;
         else if (first && r == 1) y = a.yend[2 * (e * a.nrows + q.g)];
-        else y = hin[x];
+        else y = hin()[x];
         return seg_eval(y, S.b[p], S.c[p], S.d[p], (double)(j0 + i - x));
     };
-    double yu = 0.0, yv = 0.0;  // values of the knots the thread's first segments start at
-    int xu = 0, xv = 0;         // and their positions
+    // the thread's first segments: their first knots' values (read before the first next samples
+    // replace them), and the first sample's place in them
+    double yu = 0.0, yv = 0.0, tu = 0.0, tv = 0.0;
     for (int pass = 0; pass < (two ? 2 : 1); ++pass) {
         if (pass) {  // the upper envelope waits in the tile's part of the output plane
-            double* up = kEnv ? a.dbg_upper + (size_t)q.r * q.n + n0 : hout;
-            for (int i = 0; i < kPerThread && i < lim; ++i) up[j0 + i] = env_one(0, i);
+            double* up = hout();
+            for (int i = 0; i < kPerThread && i < lim; ++i) up[j0 + i] = env_one(0, i, b0, ex);
+            __syncthreads();
+            fetch_list(1, a.cmax[a.nrows + q.g], base1, tid, kTileThreads);
+            cp_async_wait_all();
             __syncthreads();
         }
-        {
-            const unsigned w0 = two && pass ? 0u : b0, w1 = two && !pass ? 0u : b1;
-            const unsigned wb = __reduce_or_sync(0xffffffffu, w0 | w1);
-            int p0 = ex & 0xffff, p1 = ex >> 16;
-#pragma unroll
-            for (int i0 = 0; i0 < kPerThread; i0 += 4) {
-                if (!(wb >> i0 & 15u)) continue;  // no knots at these samples in the whole warp
-#pragma unroll
-                for (int i = i0; i < i0 + 4; ++i) {
-                    if (w0 >> i & 1u) S.x[2 + kq(p0++)] = (short)(j0 + i);
-                    if (w1 >> i & 1u) S.x[base1 + 2 + kq(p1++)] = (short)(j0 + i);
-                }
-            }
-        }
-        constexpr int kHalf = kTileThreads / 2;  // threads per envelope
         const int eh = two ? pass : tid / kHalf, th = two ? tid : tid % kHalf;
         const int wh = two ? kTileThreads : kHalf;
-        const int ch = eh ? c1 : c0, bh = eh ? base1 : 0;
-        __syncthreads();
-        if (!two) {
-            xu = knot_x(0, rA0, seg_at(rA0));
-            yu = knot_y(0, rA0, xu);
-            xv = knot_x(1, rA1, base1 + seg_at(rA1));
-            yv = knot_y(1, rA1, xv);
-        }
-        // slopes and lengths; segment r starts at seg_at(r) (r = 0: it enters the tile,
-        // r = count: it leaves)
-        const int r0 = first ? 1 : 0, r1 = last ? ch - 1 : ch;
+        const int ch = eh ? c1 : c0, bh = eh ? base1 : base0;
         const int step = kq(wh);  // seg_at advances by 17 for 16 segments
-        // the segments with a knot outside the tile or at an end of the row: the first and last
-        const bool outer = th >= wh - 2;
-        const int ro = th == wh - 1 ? r0 : r1, io = bh + seg_at(ro), io1 = bh + seg_at(ro + 1);
-        for (int r = r0 + 1 + th, i0 = bh + seg_at(r), i1 = bh + seg_at(r + 1); r < r1;
-             r += wh, i0 += step, i1 += step) {
-            const int x0 = S.x[i0], x1 = S.x[i1];
-            const double len = (double)(x1 - x0);
-            S.b[i0] = div_int(staged(S.stage, x1) - staged(S.stage, x0), len);
-            S.d[i0] = len;
-        }
-        double lo = 0.0;
-        if (outer) {
-            const int x0 = knot_x(eh, ro, io), x1 = knot_x(eh, ro + 1, io1);
-            lo = (double)(x1 - x0);
-            S.b[io] = div_int(knot_y(eh, ro + 1, x1) - knot_y(eh, ro, x0), lo);
-            S.d[io] = lo;
-        }
-        if (!pass) cp_async_wait_all();  // the separator values
-        __syncthreads();
         {
             const int ns0 = two && pass ? 0 : tile_seps(c0);
             const int ns1 = two && !pass ? 0 : tile_seps(c1);
@@ -1648,7 +1726,7 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
             if (sweep_lane(tid, ns0, ns1, e, k)) {
                 const double xl = S.xs[e][k - 1], xr = S.xs[e][k];
                 const int jb = (k - 1) * kChunk, js = min(k * kChunk, (e ? c1 : c0) - 1);
-                const int base = (e ? base1 : 0) + 2, i = base + kq(jb);
+                const int base = (e ? base1 : base0) + 2, i = base + kq(jb);
                 if (js - jb > 1)
                     chunk_interior_knots(S.x + i, S.b + i, S.c + i, S.d + i, js - jb - 1, xl,
                                          xr);
@@ -1660,28 +1738,46 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
             if (th == wh - 2) S.c[bh + 2 + kq(ch)] = ed->nc;
             if (th == wh - 3 && ch == 1) S.c[bh + 2] = S.xs[eh][0];
         }
+        if (!pass) cp_async_wait_all();  // the samples
         __syncthreads();
-        for (int r = r0 + 1 + th, i0 = bh + seg_at(r), i1 = bh + seg_at(r + 1); r < r1;
+        // segment r starts at seg_at(r)
+        for (int r = 1 + th, i0 = bh + seg_at(r), i1 = bh + seg_at(r + 1); r < ch;
              r += wh, i0 += step, i1 += step) {
             double b, d;
             seg_coeffs_int((double)(S.x[i1] - S.x[i0]), S.b[i0], S.c[i0], S.c[i1], b, d);
             S.b[i0] = b;
             S.d[i0] = d;
         }
-        // (one of the two threads when the first segment is the last)
-        if (outer && (r0 != r1 || th == wh - 1)) {
+        // the segments that enter and leave the tile (one and the same without a knot in it)
+        if (th == wh - 1 ? !first : th == wh - 2 && !last && ch > 0) {
+            const int r = th == wh - 1 ? 0 : ch, i0 = bh + seg_at(r), i1 = bh + seg_at(r + 1);
+            const int x0 = knot_x(eh, r, i0), x1 = knot_x(eh, r + 1, i1);
+            const double len = (double)(x1 - x0);
             double b, d;
-            seg_coeffs_int(lo, S.b[io], S.c[io], S.c[io1], b, d);
-            S.b[io] = b;
-            S.d[io] = d;
+            seg_coeffs_int(len, div_int(knot_y(eh, r + 1, x1) - knot_y(eh, r, x0), len), S.c[i0],
+                           S.c[i1], b, d);
+            S.b[i0] = b;
+            S.d[i0] = d;
+        }
+        if (!two) {
+            const int xu = rA0 == 0 ? ed0->px - n0 : S.x[base0 + seg_at(rA0)];
+            const int xv = rA1 == 0 ? ed1->px - n0 : S.x[base1 + seg_at(rA1)];
+            yu = rA0 == 0 ? ed0->py : staged(S.stage, xu);
+            yv = rA1 == 0 ? ed1->py : staged(S.stage, xv);
+            if (first) {  // the end value (the last segment starts before the other one)
+                if (rA0 == 1) yu = a.yend[2 * q.g];
+                if (rA1 == 1) yv = a.yend[2 * (a.nrows + q.g)];
+            }
+            tu = (double)(j0 - xu);
+            tv = (double)(j0 - xv);
         }
         __syncthreads();
     }
     // kEnv: the envelopes themselves go to the caller's arrays in place of the next h and the
     // mean envelope (contiguous rows, aligned to 32 bytes or not)
-    const size_t o = kEnv ? (size_t)q.r * q.n + n0 + j0 : q.base + n0 + j0;
-    double* __restrict__ me = (kEnv ? a.dbg_lower : a.menv) + o;
-    hout = kEnv ? a.dbg_upper + o : hout + j0;
+    auto mean = [&]() -> double* {
+        return kEnv ? a.dbg_lower + (size_t)q.r * q.n + n0 : a.menv + q.base + n0;
+    };
     const bool wide = !kEnv || (((size_t)a.dbg_upper | (size_t)a.dbg_lower) & 31) == 0 &&
                                    (q.n & 3) == 0;
     bool redo = false;
@@ -1692,91 +1788,138 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
         // samples pass its first knot (whose value is that sample's).  sx > t is decided by the
         // signs of p - q t for bounds t around the threshold (sx_bounds; one fma rounds to zero or
         // to the exact sign, over- and underflow included); a thread with an undecided sample
-        // or a NaN redoes its samples with the division.
+        // or a NaN redoes its samples with the division.  Once the warp has seen some sx > sd2 in
+        // the row it only counts.
+        const bool known = __any_sync(0xffffffffu, cnt_row >> 31 != 0u);
         int ru = rA0, rv = rA1;
-        int pu = seg_at(ru), pv = base1 + seg_at(rv);
-        double bu = S.b[pu], cu = S.c[pu], du = S.d[pu], tu = (double)(j0 - xu);
-        double bv = S.b[pv], cv = S.c[pv], dv = S.d[pv], tv = (double)(j0 - xv);
+        double bu, cu, du, bv, cv, dv;
+        auto load_u = [&]() {
+            const int p = base0 + seg_at(ru);
+            bu = S.b[p];
+            cu = S.c[p];
+            du = S.d[p];
+        };
+        auto load_v = [&]() {
+            const int p = base1 + seg_at(rv);
+            bv = S.b[p];
+            cv = S.c[p];
+            dv = S.d[p];
+        };
+        load_u();
+        load_v();
         const unsigned f0 = origin ? b0 & ~1u : b0, f1 = origin ? b1 & ~1u : b1;
         const unsigned wf = __reduce_or_sync(0xffffffffu, f0 | f1);
-        int und = 0, amax = 0;
-        // four samples at a time: without a knot among them in the whole warp one set of
-        // coefficients serves all four, and nothing splits the block's instruction stream
+        int und = 0, smax = 0, amax = -1, bmax = -1;
+        double2* mean_w = S.mean + warp * (kTileSamples / 4 / kTileWarps);
+        // two samples at a time: without a knot among them in the whole warp one set of
+        // coefficients serves both, and nothing splits the instruction stream
 #pragma unroll 1
         for (int i0 = 0; i0 < kPerThread; i0 += 4) {
-            const double2 ha = S.stage[stage_piece(kPerThread / 2 * tid + i0 / 2)];
-            const double2 hb = S.stage[stage_piece(kPerThread / 2 * tid + i0 / 2 + 1)];
-            const double h[4] = {ha.x, ha.y, hb.x, hb.y};
-            double eu[4], ev[4];
-            if (!(wf >> i0 & 15u)) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+            for (int k = 0; k < 4; k += 2) {
+            double2* const pa = own_piece(S.stage, tid, (i0 + k) / 2);
+            double eu[2], ev[2];
+            if (!(wf >> (i0 + k) & 3u)) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
                     eu[i] = seg_eval(yu, bu, cu, du, tu + (double)i);
                     ev[i] = seg_eval(yv, bv, cv, dv, tv + (double)i);
                 }
-                tu += 4.0;
-                tv += 4.0;
+                tu += 2.0;
+                tv += 2.0;
             } else {
+                const double2 hk = *pa;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+                for (int i = 0; i < 2; ++i) {
                     eu[i] = seg_eval(yu, bu, cu, du, tu);
                     ev[i] = seg_eval(yv, bv, cv, dv, tv);
                     tu += 1.0;
                     tv += 1.0;
-                    if (f0 >> (i0 + i) & 1u) {
+                    if (f0 >> (i0 + k + i) & 1u) {
                         ++ru;
-                        pu = seg_at(ru);
-                        yu = h[i];
-                        bu = S.b[pu];
-                        cu = S.c[pu];
-                        du = S.d[pu];
+                        load_u();
+                        yu = i ? hk.y : hk.x;
                         tu = 1.0;
                     }
-                    if (f1 >> (i0 + i) & 1u) {
+                    if (f1 >> (i0 + k + i) & 1u) {
                         ++rv;
-                        pv = base1 + seg_at(rv);
-                        yv = h[i];
-                        bv = S.b[pv];
-                        cv = S.c[pv];
-                        dv = S.d[pv];
+                        load_v();
+                        yv = i ? hk.y : hk.x;
                         tv = 1.0;
                     }
                 }
             }
             if (kEnv) {
-                store4(hout + i0, eu);
-                store4(me + i0, ev);
+                *reinterpret_cast<double2*>(hout() + j0 + i0 + k) = make_double2(eu[0], eu[1]);
+                *reinterpret_cast<double2*>(mean() + j0 + i0 + k) = make_double2(ev[0], ev[1]);
                 continue;
             }
-            double mv[4], hn[4];
+            const double2 hk = *pa;
+            double mv[2], hn[2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < 2; ++i) {
                 const double s = eu[i] + ev[i], p = fabs(s), w = fabs(eu[i] - ev[i]);
                 mv[i] = s / 2.0;
-                hn[i] = h[i] - mv[i];
+                hn[i] = (i ? hk.y : hk.x) - mv[i];
                 const int s1 = __double2hiint(fma(-a.sd_hi, w, p));
                 const int s0 = __double2hiint(fma(-a.sd_lo, w, p));
-                const int t1 = __double2hiint(fma(-a.sd2_hi, w, p));
-                const int t0 = __double2hiint(fma(-a.sd2_lo, w, p));
-                und |= ((s1 - 1) & ~s0) | ((t1 - 1) & ~t0);  // sign bit: neither bound decides
+                und |= (s1 - 1) & ~s0;  // sign bit: neither bound decides
                 cnt += 1u - ((unsigned)s0 >> 31);  // (when decided, not below means above)
-                amax = max(amax, t1);
+                smax = max(smax, s1);
+                if (!known) {
+                    amax = max(amax, __double2hiint(fma(-a.sd2_hi, w, p)));
+                    bmax = max(bmax, __double2hiint(fma(-a.sd2_lo, w, p)));
+                }
             }
-            store4(hout + i0, hn);
-            store4(me + i0, mv);
+            *pa = make_double2(hn[0], hn[1]);
+            mean_w[stage_piece(4 * lane) ^ ((i0 + k) / 2 & 3)] = make_double2(mv[0], mv[1]);
+            }
+            if (kEnv) continue;
+            if (i0 & 4) {  // 64 bytes of every lane's samples
+                __syncwarp();
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+                    const int j = lane + 32 * g;
+                    const int u = stage_piece(2 * j);
+                    const double2 p0 = mean_w[u], p1 = mean_w[u ^ 1];
+                    const double w[4] = {p0.x, p0.y, p1.x, p1.y};
+                    store4(mean() + warp * kWarpSamples + kPerThread * (j >> 1) + (i0 & 8) +
+                               4 * (j & 1), w);
+                }
+                __syncwarp();
+            }
+        }
+        if (!kEnv) {
+#pragma unroll
+            for (int g = 0; g < kPerThread / 4; ++g) {
+                const int u = (tid & ~31) * (kPerThread / 2) + 2 * (lane + 32 * g);
+                const double2 p0 = S.stage[stage_piece(u)], p1 = S.stage[stage_piece(u) ^ 1];
+                const double w[4] = {p0.x, p0.y, p1.x, p1.y};
+                store4(hout() + 2 * u, w);
+            }
         }
         any = amax > 0 ? 1 : 0;
-        redo = und < 0 || amax > 0x7ff00000;  // (a NaN)
+        // undecided, a NaN, or no sample surely above sd2 and not all surely below
+        redo = und < 0 || smax > 0x7ff00000 || (amax <= 0 && bmax >= 0);
     }
-    if (!common || (redo && !kEnv)) {
+    if (__any_sync(0xffffffffu, !common || (redo && !kEnv))) {
+        // (the flags and counts anew: kept, they would cost the common path registers)
+        const unsigned f0 = reinterpret_cast<const TileBits*>(S.bits[0])[tid];
+        const unsigned f1 = reinterpret_cast<const TileBits*>(S.bits[1])[tid];
+        const int mine = __popc(f0) | __popc(f1) << 16;
+        const int before = S.scan.before[warp] + warp_scan(mine, lane) - mine;
+        if (!common || redo) {
         cnt = 0u;
         any = 0;
+        double* ho = hout() + j0;
+        double* me = mean() + j0;
+        const double* hi = hin() + j0;
 #pragma unroll 1
         for (int i = 0; i < kPerThread && i < lim; ++i) {
-            const double u = two ? hout[i] : env_one(0, i);
-            const double v = env_one(1, i);
+            const double u = two ? ho[i] : env_one(0, i, f0, before);
+            const double v = env_one(1, i, f1, before);
             if (kEnv) {
-                hout[i] = u;
+                ho[i] = u;
                 me[i] = v;
                 continue;
             }
@@ -1784,20 +1927,30 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
                 double mv = (u + v) / 2.0;
                 if (write_mean) me[i] = mv;
                 else mv = me[i];
-                hout[i] = hin[j0 + i] - mv;
+                ho[i] = hi[i] - mv;
             }
             any |= sx_greater(u, v, a.sd2) ? 1 : 0;
             cnt += sx_greater(u, v, a.sd) ? 1 : 0;
         }
+        }
     }
-    advance();
     }
-    if (!kEnv) {
-        // the counts of the warps, then the row's
-        any = __any_sync(0xffffffffu, any != 0) ? 1 : 0;
-        cnt = __reduce_add_sync(0xffffffffu, cnt);
-        if (lane == 0) s_w[warp] = (int)(cnt | (unsigned)any << 30);
-        __syncthreads();
+    cnt_row = ((cnt_row & 0x7fffffffu) + cnt) | (cnt_row & 0x80000000u) |
+              (any != 0 ? 0x80000000u : 0u);
+    const int v = it.v;
+    it.next(a);
+    // the CTA's last tile of the row: the counts of the warps, then the row's
+    const bool leave = !kEnv && (!it.more() || it.q.g != q.g);
+    if (leave) {
+        const bool y = __any_sync(0xffffffffu, cnt_row >> 31 != 0u);
+        cnt_row = __reduce_add_sync(0xffffffffu, cnt_row & 0x7fffffffu);
+        if (lane == 0) s_w[warp] = (int)(cnt_row | (y ? 1u << 30 : 0u));
+    }
+    __syncthreads();
+    // every warp is done with the tile: the next one's pieces take its place
+    if (it.tile == 0) sep = 0;
+    prefetch();
+    if (leave) {
         if (tid == 0) {
             unsigned t = 0u;
             int y = 0;
@@ -1806,22 +1959,27 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
                 t += (unsigned)s_w[w] & 0x3fffffffu;
                 y |= s_w[w] >> 30;
             }
-            if (count_tile(a, q, t, y)) {
+            // (since the start of the row or of the CTA's range)
+            const int tiles = v + 1 - max(v - tile, s_begin);
+            if (count_tiles(a, q, (unsigned)tiles, t, y)) {
                 if (repeat) {
                     t = a.cnt[q.g];
                     y = a.any[q.g];
                 }
-                row_criterion(a, q, cst, t, y);
+                row_criterion(a, q.c, q.g, q.r, q.n, t, y);
             }
         }
+        cnt_row = 0u;
     }
     }
 }
 
-template __global__ void k_tile_sift<true, false>(const __grid_constant__ SiftArgs a);
-template __global__ void k_tile_sift<false, false>(const __grid_constant__ SiftArgs a);
-template __global__ void k_tile_sift<true, true>(const __grid_constant__ SiftArgs a);
-template __global__ void k_tile_sift<false, true>(const __grid_constant__ SiftArgs a);
+template __global__ void k_tile_sift<true, false, false>(const __grid_constant__ SiftArgs a);
+template __global__ void k_tile_sift<true, true, false>(const __grid_constant__ SiftArgs a);
+template __global__ void k_tile_sift<false, true, false>(const __grid_constant__ SiftArgs a);
+template __global__ void k_tile_sift<true, false, true>(const __grid_constant__ SiftArgs a);
+template __global__ void k_tile_sift<true, true, true>(const __grid_constant__ SiftArgs a);
+template __global__ void k_tile_sift<false, true, true>(const __grid_constant__ SiftArgs a);
 
 // Mode export of channel c's realizations that finished in the last executed iteration
 // (blockIdx.y = realization).
