@@ -76,12 +76,13 @@ WORKLOAD_ITERATIONS = 12487
 
 # algorithmic bytes per sift iteration per realization: coefficients of N and of K (knots of
 # both envelopes).  Kernel kinds follow include/ceemdan_b200.h.
-BYTES_PER_N = {"extrema": 24.25, "eval": 8.25,
-               # on-chip stage kernel: global bytes per sample-iteration (mean envelope read
-               # and written, upper envelope written and read back; h stays in shared memory)
-               "sift_small": 32.0}
-BYTES_PER_K = {"extrema": 12.0, "chunk_reduce": 17.0, "reduced_solve": 10.5,
-               "segments": 44.5, "eval": 36.0}
+# extrema: h read, bitmaps written; knots' positions and slopes, separator rows.  eval: h read,
+# next h and mean envelope written, bitmaps read; positions, slopes and separator values read.
+BYTES_PER_N = {"extrema": 8.25, "eval": 24.25,
+               # on-chip stage kernel: global bytes per sample-iteration (mean envelope written;
+               # h stays in shared memory)
+               "sift_small": 8.0}
+BYTES_PER_K = {"extrema": 12.0, "reduced_solve": 2.5, "eval": 10.5}
 
 
 def _peaks():
@@ -96,7 +97,8 @@ def _peaks():
 
 def _traffic_ratio(kernel):
     """DRAM bytes / algorithmic bytes of `kernel` from the committed ncu summary, if any."""
-    path = os.path.join(ROOT, "profiles", f"k_{kernel}_eeg244032.md")
+    name = {"extrema": "tile_knots", "eval": "tile_sift"}.get(kernel, kernel)
+    path = os.path.join(ROOT, "profiles", f"k_{name}_eeg244032.md")
     try:
         for line in open(path):
             if line.startswith("traffic_over_algorithmic:"):

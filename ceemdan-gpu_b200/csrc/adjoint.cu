@@ -2,7 +2,7 @@
 //
 // A taped forward call records, for every executed iteration of every signal stage, the knot
 // bitmaps and counts of both envelopes, the end-rule flags and the marks (k_tape_record,
-// k_scan_boundary, k_criterion).  With that structure fixed, one sift iteration of
+// k_spline_solve, k_tile_sift).  With that structure fixed, one sift iteration of
 // cudaICEEMDAN.cu:1752-2002 is linear in h:
 //   knots       y_i = h[x_i], end values replaced by the extrapolation of :210-291
 //   spline      natural cubic spline through (x_i, y_i) (:311-343, the cuSPARSE solve :1630)
@@ -71,7 +71,7 @@ __device__ double end_rule_adjoint(const int32_t* x, const double* y2, int K, in
 
 }  // namespace
 
-// One slot of the tape from the iteration just executed (launched before k_criterion, which
+// One slot of the tape from the iteration just executed (launched before k_tile_sift, which
 // writes the marks into the slot itself).  Iterations after the stop word record nothing.
 __global__ void k_tape_record(SiftArgs a, TapeLayout L, unsigned char* slot) {
     if (a.cs[0].done) return;  // the taped forward has one channel

@@ -13,20 +13,15 @@
 // at the next iteration, in the same launches as the others.  G iterations are captured once
 // in a CUDA graph (two copies, so that the host reads the finished-channel count of one while
 // the other runs) and replayed until every channel has finished; the host never launches
-// single kernels inside the loop.  The persistent grid sizes are chosen by a small autotuner
-// that times the first replays of the wave with each candidate (the candidates compute the
-// same results: only the assignment of tiles to CTAs differs) and keeps the fastest for later waves and calls of the same shape.
+// single kernels inside the loop.
 //
 // Channels that do not fit the device memory together are processed in waves, longest first.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdlib>
-#include <map>
-#include <mutex>
 #include <numeric>
 #include <string>
-#include <tuple>
 #include <vector>
 
 #include "host.h"

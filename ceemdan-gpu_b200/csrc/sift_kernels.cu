@@ -14,10 +14,10 @@
 //                    the update h -= m (updateRealizations :528-544), and after a row's last
 //                    tile its stop test (meanD/multiplyD on sx :1851, siftingCriterion :495-525,
 //                    checkBreak :547-580)
-// Knots, slopes and coefficients live in shared memory only; both tile kernels rebuild a tile's
-// knots from its samples and bitmap.  An iteration moves 8 N bytes in k_tile_knots and 24 N in
-// k_tile_sift (h, next h, mean envelope) plus N/2 of bitmaps and about 6 bytes per knot of
-// separator rows.  Line numbers refer to the reference's cudaICEEMDAN.cu.
+// Spline values and coefficients live in shared memory only; k_tile_knots hands the knots'
+// positions and slopes over.  An iteration moves 8 N bytes in k_tile_knots and 24 N in k_tile_sift
+// (h, next h, mean envelope) plus N/2 of bitmaps, and per knot 20 bytes of positions and slopes
+// and about 6 of separator rows.  Line numbers refer to the reference's cudaICEEMDAN.cu.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -318,13 +318,18 @@ static_assert(kListSlots % 8 == 0 &&
 size_t tile_knots_smem() { return sizeof(KnotSmem); }
 
 // =======================================================================================
-// k_tile_knots: one CTA per 2048-sample tile, both envelopes; thread t holds samples 16t..16t+15.
-// Strict extrema from the signs of neighbour differences, eight to a byte of the knot bitmaps; the
-// knots compacted into shared memory; the segment slopes; the end relations of the chunks between
-// separators (one thread per chunk) and from them the rows of the separator system inside the
-// tile.  What the tile's first and last separators need from other tiles goes into the tile's
-// header for k_spline_solve.  Issue bound: eight samples to a thread take half the instructions
-// of one sample to a lane (signs shared between neighbours, one scan step per thread).
+// k_tile_knots: persistent CTAs over the 2048-sample tiles, both envelopes; thread t holds samples
+// 16t..16t+15.  Strict extrema from the signs of neighbour differences, a bit each in the knot
+// bitmaps; the knots compacted into shared memory; the segment slopes; the end relations of the
+// chunks between separators (one thread per chunk) and from them the rows of the separator system
+// inside the tile.  What the tile's first and last separators need from other tiles goes into the
+// tile's header for k_spline_solve.
+//
+// Bound by instructions and the barriers between short phases (half of the issue slots used):
+// sixteen samples to a thread share signs between neighbours and one scan step, where one sample
+// to a lane took four times the instructions.  B200, N=244032 NR=100: 103 us at K/N = 0.18, 61 us
+// at 0.001 (3.2 TB/s of its 8 N bytes), where the separate extrema, end-rule and chunk kernels took
+// 178 us on average.  Six CTAs per SM instead of five change nothing.
 // =======================================================================================
 __global__ void __launch_bounds__(kTileThreads, 5)
 k_tile_knots(const __grid_constant__ SiftArgs a) {
@@ -1229,8 +1234,9 @@ __device__ __noinline__ void end_rule_sparse(const SiftArgs& a, int e, int sp, i
 // separators, tiles with knots), the end rule where one tile could not decide it, the rows of the
 // separators at the tiles' edges, the separator system (levels >= 2 of the canonical partitioned
 // solve), and for every tile the knots just outside it with their spline values.  The system's
-// rows are staged once when they fit a pass (2048 rows).  Latency bound: two CTAs per SM with
-// the level-3 system in shared memory.
+// rows are staged once when they fit a pass (2048 rows).  Latency bound (a chain of short sweeps
+// per CTA): two CTAs per SM with the level-3 system in shared memory.  B200, N=244032 NR=100: 24 us
+// at K/N = 0.18, 56 us for white noise; the two kernels before it took 42 us on average.
 // =======================================================================================
 __global__ void __launch_bounds__(kSolveThreads, 2)
 k_spline_solve(const __grid_constant__ SiftArgs a) {
@@ -1421,7 +1427,7 @@ k_spline_solve(const __grid_constant__ SiftArgs a) {
 // instead of being found again, a row's counts are added once per CTA, not per tile, and both
 // planes are stored coalesced out of shared memory (a thread's 32 bytes in a line each took 32
 // cycles of the load/store unit, half of all it did).  B200, N=244032 NR=100, K/N = 0.18: 262 ->
-// 208 us (2.8 TB/s of its 24 N bytes); K/N = 0.001: 167 -> 145 us; white noise: 381 -> 321 us.
+// 206 us (2.8 TB/s of its 24 N bytes); K/N = 0.001: 167 -> 142 us; white noise: 381 -> 314 us.
 // Four CTAs with room for 1184: 225, 153 and 321 us.  Each class's launch takes the tiles of its
 // own rows in even shares: with rows of both classes (K/N = 0.23) 398 -> 234 us.
 // =======================================================================================
@@ -1633,7 +1639,7 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
     // samples with sx > sd of the row's tiles so far, and in the sign bit whether some sx > sd2
     unsigned cnt_row = 0u;
     while (it.more()) {
-    const Geo q = it.q;
+    const Geo& q = it.q;
     const int tile = it.tile;
     const bool repeat = !it.live(), write_mean = it.mean();
     ChanState& cst = a.cs[q.c];
@@ -1937,19 +1943,14 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
     }
     cnt_row = ((cnt_row & 0x7fffffffu) + cnt) | (cnt_row & 0x80000000u) |
               (any != 0 ? 0x80000000u : 0u);
-    const int v = it.v;
-    it.next(a);
     // the CTA's last tile of the row: the counts of the warps, then the row's
-    const bool leave = !kEnv && (!it.more() || it.q.g != q.g);
+    const bool leave = !kEnv && (tile + 1 == q.ntiles || it.v + 1 == it.end);
     if (leave) {
         const bool y = __any_sync(0xffffffffu, cnt_row >> 31 != 0u);
         cnt_row = __reduce_add_sync(0xffffffffu, cnt_row & 0x7fffffffu);
         if (lane == 0) s_w[warp] = (int)(cnt_row | (y ? 1u << 30 : 0u));
     }
     __syncthreads();
-    // every warp is done with the tile: the next one's pieces take its place
-    if (it.tile == 0) sep = 0;
-    prefetch();
     if (leave) {
         if (tid == 0) {
             unsigned t = 0u;
@@ -1960,7 +1961,7 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
                 y |= s_w[w] >> 30;
             }
             // (since the start of the row or of the CTA's range)
-            const int tiles = v + 1 - max(v - tile, s_begin);
+            const int tiles = it.v + 1 - max(it.v - tile, s_begin);
             if (count_tiles(a, q, (unsigned)tiles, t, y)) {
                 if (repeat) {
                     t = a.cnt[q.g];
@@ -1971,6 +1972,10 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
         }
         cnt_row = 0u;
     }
+    // every warp is done with the tile: the next one's pieces take its place
+    it.next(a);
+    if (it.tile == 0) sep = 0;
+    prefetch();
     }
 }
 

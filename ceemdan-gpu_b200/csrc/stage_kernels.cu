@@ -228,7 +228,7 @@ __global__ void k_check_iota(const int32_t* x, size_t n, int* err) {
 
 // =======================================================================================
 // Batched engine: stage transitions.  A channel whose stage has finished (ChanState.done, set
-// by k_criterion) and that has stages left is "in transition" from the first of these kernels
+// by k_tile_sift) and that has stages left is "in transition" from the first of these kernels
 // to k_commit_plan, which opens its next stage; all four read the same states.
 // =======================================================================================
 namespace {

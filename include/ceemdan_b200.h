@@ -69,13 +69,14 @@ typedef struct ceemdan_options {
 
 /* Kernel kinds of h_kernel_ms. */
 enum {
-    CEEMDAN_K_EXTREMA = 0,       /* deferred update + extrema + compaction */
-    CEEMDAN_K_BOUNDARY = 1,      /* end-knot extrapolation */
-    CEEMDAN_K_CHUNK_REDUCE = 2,  /* chunk end relations of the spline solve + separator rows */
+    CEEMDAN_K_EXTREMA = 0,       /* extrema, end rule, slopes, chunk end relations */
+    CEEMDAN_K_BOUNDARY = 1,      /* 0: part of CEEMDAN_K_EXTREMA and CEEMDAN_K_REDUCED_SOLVE */
+    CEEMDAN_K_CHUNK_REDUCE = 2,  /* 0: part of CEEMDAN_K_EXTREMA */
     CEEMDAN_K_REDUCED_SOLVE = 3, /* per-spline separator solve */
-    CEEMDAN_K_SEGMENTS = 4,      /* chunk interiors -> segment coefficients b, c, d */
-    CEEMDAN_K_EVAL = 5,          /* envelopes, mean envelope, sx statistics */
-    CEEMDAN_K_CRITERION = 6,     /* stop test */
+    CEEMDAN_K_SEGMENTS = 4,      /* 0: part of CEEMDAN_K_EVAL */
+    CEEMDAN_K_EVAL = 5,          /* segment coefficients, envelopes, mean envelope, update, sx
+                                    statistics, stop test */
+    CEEMDAN_K_CRITERION = 6,     /* 0: part of CEEMDAN_K_EVAL */
     CEEMDAN_K_SIFT_SMALL = 7,    /* a whole stage on chip (rows of at most 8192 samples) */
     CEEMDAN_NUM_KERNEL_KINDS = 8
 };
@@ -178,8 +179,7 @@ ceemdan_status ceemdan_batch_f64(size_t channels, const size_t* lengths,
  * channel, replayed as a CUDA graph) moves each channel through its own stages, so channels
  * whose stages end at different iterations never wait for each other.  Channels that do not
  * fit together are run in waves, longest first, each wave within wave_bytes of device memory
- * (0 = 85% of the free memory).  Persistent grid sizes are autotuned on the first wave of a
- * shape (environment CEEMDAN_BATCH_TUNE=0: defaults).  opt->h_iters_out, when given, receives
+ * (0 = 85% of the free memory).  opt->h_iters_out, when given, receives
  * [channels][2*(num_imfs-1)] iteration counts (the channel's noise stages, then its CEEMDAN
  * stages); opt->h_kernel_ms and opt->h_counters accumulate as for the plain call (iterations =
  * iterations of the shared loop); opt->group = iterations per graph replay (0 = auto);
