@@ -930,6 +930,8 @@ struct RedStage {
     SepRow row[kSolveSlots];
     double x[kSolveSlots + 1];  // reciprocal pivots, then the solution
 };
+static_assert(2 * kSolveChunks == kSolveThreads && kSolveChunks % 32 == 0,
+              "a thread per chunk and direction");
 static_assert(sizeof(RedStage) == kSolveStage, "the host sizes the workspace after it");
 
 // Rows of a spline's transposed system from its knot positions and right-hand side in padded
@@ -1018,16 +1020,18 @@ __device__ __forceinline__ void solve_separators(RedStage& st, int wcap, const d
             cp_async_wait_all();
             __syncthreads();
         }
-        const int q = p0 / kChunk + threadIdx.x;
-        if (threadIdx.x < kSolveChunks && q <= Q) {
+        int lane_q;
+        const bool top = ends_item(threadIdx.x, kSolveChunks, lane_q);
+        const int q = p0 / kChunk + lane_q;
+        if (q <= Q) {
             const int first = q * kChunk;
             const int len = (q < Q) ? kChunk - 1 : P - first;
             const int i = kq(first - p0);
-            if (one) {
-                ends_rows<true>(st.row + i, len, st.x + i, ends + 6 * q);
-            } else {
+            if (!top) {
                 ends_rows<false>(st.row + i, len, nullptr, ends + 6 * q);
-                if (q < Q) sep[q] = load_row(st.row + i + kChunk - 1);
+                if (!one && q < Q) sep[q] = load_row(st.row + i + kChunk - 1);
+            } else {
+                ends_rows<true>(st.row + i, len, one ? st.x + i : nullptr, ends + 6 * q);
             }
         }
     }

@@ -25,8 +25,11 @@
 //
 // B200, one iteration of the first stages, the previous form (one kernel, unrolled sweeps, the
 // upper envelope handed over through L2, the stop test awaited at once) and this one: N=4096 NR=50
-// 37.6 -> 15.7 us, N=8192 NR=50 49.1 -> 21.1 (kPair); N=2501 NR=100 54.5 -> 19.5, N=5000 NR=100
-// 65.0 -> 27.8 (kDual); N=7680 NR=100 79.6 -> 35.6 (kSingle).
+// 37.6 -> 14.3 us, N=8192 NR=50 49.1 -> 19.2 (kPair); N=2501 NR=100 54.5 -> 14.7, N=5000 NR=100
+// 65.0 -> 20.5 (kDual); N=7680 NR=100 79.6 -> 33.2 (kSingle).  The code of an iteration has to stay
+// in the instruction cache: with a copy of build_envelope for each group kDual took 18.2 and 26.5.
+// At N=4096 NR=50 a quarter of the 28,000 cycles is the separator system (two sweeps of 15 rows at
+// 80 cycles a reciprocal, and their barriers), a quarter the evaluation and the exchange.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -132,41 +135,70 @@ __device__ __forceinline__ EnvSmem env_smem(const SmallLayout& L, unsigned char*
     return E;
 }
 
-// The interior of a chunk whose reciprocals the end relations left in c[1 .. len]
+// The interior of a chunk whose reciprocals the end relations left in c[1 .. len] (the chain is
+// 17 cycles a row forward and 9 back; a row a turn with its loads and tests took 180, four rows a
+// turn take 110)
 // (chunk_interior_knots' arrays): c receives the spline values, d the factors meanwhile.
 __device__ __forceinline__ void interior_known(const double* s, double* c, double* d, int len,
                                                double xl, double xr) {
-    double l = d[0], u = d[1], s0 = s[0], s1 = s[1], iw = c[1], gp = 0.0;
+    double l = d[0], u = d[1], s0 = s[1];
+    double ri = fma(-l, xl, 3.0 * (s0 - s[0]));
+    if (len == 1) ri = fma(-u, xr, ri);
+    double iw = c[1];
+    double gp = ri * iw;
+    d[0] = u * iw;
+    c[1] = gp;
+    int k = 1;
+    // four rows at a time, loaded before the first of them is needed
 #pragma unroll 1
-    for (int k = 0; k < len; ++k) {
-        const double uc = u, ic = iw;
-        double ri = 3.0 * (s1 - s0);
-        s0 = s1;
-        if (k + 1 < len) {  // a row ahead of its use
-            u = d[k + 2];
-            s1 = s[k + 2];
-            iw = c[k + 2];
+    for (; k + 4 < len; k += 4) {
+        double du[4], ds[4], dw[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            du[i] = d[k + 1 + i];
+            ds[i] = s[k + 1 + i];
+            dw[i] = c[k + 1 + i];
         }
-        if (k == 0) ri = fma(-l, xl, ri);
-        if (k == len - 1) ri = fma(-uc, xr, ri);
-        gp = (k == 0 ? ri : fma(-l, gp, ri)) * ic;
-        d[k] = uc * ic;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            gp = fma(-u, gp, 3.0 * (ds[i] - s0)) * dw[i];
+            s0 = ds[i];
+            u = du[i];
+            d[k + i] = u * dw[i];
+            c[k + 1 + i] = gp;
+        }
+    }
+#pragma unroll 1
+    for (; k < len; ++k) {
+        l = u;
+        u = d[k + 1];
+        ri = 3.0 * (s[k + 1] - s0);
+        s0 = s[k + 1];
+        if (k == len - 1) ri = fma(-u, xr, ri);
+        iw = c[k + 1];
+        gp = fma(-l, gp, ri) * iw;
+        d[k] = u * iw;
         c[k + 1] = gp;
-        l = uc;
     }
-    double xv = gp, f = 0.0, g = 0.0;
-    if (len > 1) {
-        f = d[len - 2];
-        g = c[len - 1];
+    double xv = gp;
+    k = len - 2;
+#pragma unroll 1
+    for (; k >= 3; k -= 4) {
+        double f[4], g[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            f[i] = d[k - i];
+            g[i] = c[k + 1 - i];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            xv = fma(-f[i], xv, g[i]);
+            c[k + 1 - i] = xv;
+        }
     }
 #pragma unroll 1
-    for (int k = len - 2; k >= 0; --k) {
-        const double fc = f, gc = g;
-        if (k > 0) {
-            f = d[k - 1];
-            g = c[k];
-        }
-        xv = fma(-fc, xv, gc);
+    for (; k >= 0; --k) {
+        xv = fma(-d[k], xv, c[k + 1]);
         c[k + 1] = xv;
     }
 }
@@ -272,17 +304,19 @@ __device__ void build_envelope(const Group& grp, const EnvSmem& E, int* warp_tot
         };
         if (tid == 0) {
             double y0 = H[0];
+            const bool near = I.cnt[0] > 2;  // the three knots lie in the first tile
+            const int p1 = near ? 1 : after(0);
             if (K - 1 > 4) {
-                const int p1 = after(0), p2 = after(p1);
+                const int p2 = near ? 2 : after(p1);
                 y0 = boundary_left(e, E.X[0], E.X[p1], E.X[p2], H[0], H[E.X[p1]], H[E.X[p2]]);
             }
             I.yend[0] = y0;
-            if (K > 2) segment(0, after(0), y0, H[E.X[after(0)]]);
+            if (K > 2) segment(0, p1, y0, H[E.X[p1]]);
             else segment(0, pl, y0, H[n - 1]);  // (two knots: no rule)
         } else {
             double yL = H[n - 1];
             if (K - 1 > 4) {
-                const int p2 = before(pl1);
+                const int c = I.cnt[tl], p2 = c > 2 ? I.base[tl] + kq(c - 3) : before(pl1);
                 yL = boundary_right(e, E.X[p2], E.X[pl1], E.X[pl], H[E.X[p2]], H[E.X[pl1]],
                                     H[n - 1]);
             }
@@ -315,28 +349,25 @@ __device__ void build_envelope(const Group& grp, const EnvSmem& E, int* warp_tot
         }
     }
     // end relations of the chunk left of each separator
-    for (int p = tid; p < P; p += G) {
-        int t, k;
+    for (int i = tid; i < ends_items(P); i += G) {
+        int p, t, k;
+        const bool top = ends_item(i, P, p);
+        if (p >= P) continue;
         sep_tile(I, ntiles, p, t, k);
         const int jb = (k - 1) * kChunk, js = min(k * kChunk, I.cnt[t] - 1);
         double* en = E.ends + 6 * p;
         if (k > 0 && js - jb > 1) {
             const int b = I.base[t] + kq(jb);
-            const ChunkEnds ce =
-                chunk_ends_knots<true>(E.X + b, E.S + b, js - jb - 1, E.C + b + 1);
-            en[0] = ce.ga;
-            en[1] = ce.aa;
-            en[2] = ce.ba;
-            en[3] = ce.gb;
-            en[4] = ce.ab;
-            en[5] = ce.bb;
+            if (top) chunk_ends_half<true>(E.X + b, E.S + b, js - jb - 1, en, E.C + b + 1);
+            else chunk_ends_half<false>(E.X + b, E.S + b, js - jb - 1, en, nullptr);
+        } else if (top) {
+            en[3] = 0.0;
+            en[4] = 1.0;
+            en[5] = 0.0;
         } else {
             en[0] = 0.0;
             en[1] = 0.0;
             en[2] = 1.0;
-            en[3] = 0.0;
-            en[4] = 1.0;
-            en[5] = 0.0;
         }
     }
     if (tid == G - 1) {
@@ -532,23 +563,27 @@ k_sift_small(const __grid_constant__ SiftArgs a, const __grid_constant__ SmallAr
             }
             if ((int)(v >> 32) == nreal) s_stop = 1;
         };
-        auto none = []() {};
+        // (one copy of build_envelope's code, for the instruction cache)
         if constexpr (kMode == kSmallSingle) {
-            build_envelope(grp, E0, warp_tot(0), H, s_g, s_l, n, 0, sa, j, r, wait);
-            __syncthreads();
-            if (tid == 0) s_kcnt[0] = E0.I->K;
+#pragma unroll 1
+            for (int e = 0; e < 2; ++e) {
+                build_envelope(grp, E0, warp_tot(0), H, s_g, s_l, n, e, sa, j, r, [&]() {
+                    if (e == 0) wait();
+                });
+                __syncthreads();
+                if (tid == 0) s_kcnt[e] = E0.I->K;
+                if (e == 0) {
 #pragma unroll 4
-            for (int s = tid; s < n; s += kSmallThreads) up[s] = env_at(E0, H, s);
-            __syncthreads();
-            build_envelope(grp, E0, warp_tot(0), H, s_g, s_l, n, 1, sa, j, r, none);
-            __syncthreads();
-            if (tid == 0) s_kcnt[1] = E0.I->K;
+                    for (int s = tid; s < n; s += kSmallThreads) up[s] = env_at(E0, H, s);
+                    __syncthreads();
+                }
+            }
         } else if constexpr (kMode == kSmallDual) {
-            if (group == 0)
-                build_envelope(grp, E0, warp_tot(0), H, s_g, s_l, n, 0, sa, j, r, wait);
-            else
-                build_envelope(grp, E1, warp_tot(1), H, s_g, s_l, n, 1, sa, j, r, none);
-            if (grp.tid() == 0) s_kcnt[group] = group ? E1.I->K : E0.I->K;
+            const EnvSmem E = env_smem(L, set0 + group * L.set);
+            build_envelope(grp, E, warp_tot(group), H, s_g, s_l, n, group, sa, j, r, [&]() {
+                if (group == 0) wait();
+            });
+            if (grp.tid() == 0) s_kcnt[group] = E.I->K;
             __syncthreads();
         } else {
             build_envelope(grp, E0, warp_tot(0), H, s_g, s_l, n, rank, sa, j, r, wait);
@@ -575,28 +610,54 @@ k_sift_small(const __grid_constant__ SiftArgs a, const __grid_constant__ SmallAr
         }
         const int kmax = s_kcnt[0], kmin = s_kcnt[1];
         const bool write_mean = kmax > 3 && kmin > 3;
-        int cnt = 0, any = 0;
+        // the envelopes at the thread's sample k
+        auto envelopes = [&](int k, int s, double& u, double& v) {
+            if constexpr (kPair) {
+                const double o = recv[s - own0];
+                u = rank == 0 ? ev[k] : o;
+                v = rank == 0 ? o : ev[k];
+            } else {
+                u = kMode == kSmallSingle ? up[s] : env_at(E0, H, s);
+                v = env_at(E1, H, s);
+            }
+        };
+        // sx > sd, sx > sd2 by the signs of p - q t for bounds t around the thresholds, as in
+        // k_tile_sift; a thread with an undecided sample or a NaN does its samples again
+        int cnt = 0, any = 0, und = 0, smax = 0, amax = -1, bmax = -1;
 #pragma unroll
         for (int k = 0; k < kOwn; ++k) {
             const int s = own0 + k * kSmallThreads + tid;
             if (s < own1) {
                 double u, v;
-                if constexpr (kPair) {
-                    const double o = recv[s - own0];
-                    u = rank == 0 ? ev[k] : o;
-                    v = rank == 0 ? o : ev[k];
-                } else {
-                    u = kMode == kSmallSingle ? up[s] : env_at(E0, H, s);
-                    v = env_at(E1, H, s);
-                }
+                envelopes(k, s, u, v);
+                const double sum = u + v, p = fabs(sum), w = fabs(u - v);
                 if (write_mean) {
-                    mean[k] = (u + v) / 2.0;
+                    mean[k] = sum / 2.0;
                     menv[s] = mean[k];
                 } else {
                     mean[k] = __ldcg(menv + s);
                 }
-                any |= sx_greater(u, v, a.sd2) ? 1 : 0;
-                cnt += sx_greater(u, v, a.sd) ? 1 : 0;
+                const int s1 = __double2hiint(fma(-a.sd_hi, w, p));
+                const int s0 = __double2hiint(fma(-a.sd_lo, w, p));
+                und |= (s1 - 1) & ~s0;
+                cnt += 1 - (int)((unsigned)s0 >> 31);
+                smax = max(smax, s1);
+                amax = max(amax, __double2hiint(fma(-a.sd2_hi, w, p)));
+                bmax = max(bmax, __double2hiint(fma(-a.sd2_lo, w, p)));
+            }
+        }
+        any = amax > 0 ? 1 : 0;
+        if (und < 0 || smax > 0x7ff00000 || (amax <= 0 && bmax >= 0)) {
+            cnt = any = 0;
+#pragma unroll (kPair ? kOwn : 1)
+            for (int k = 0; k < kOwn; ++k) {
+                const int s = own0 + k * kSmallThreads + tid;
+                if (s < own1) {
+                    double u, v;
+                    envelopes(k, s, u, v);
+                    any |= sx_greater(u, v, a.sd2) ? 1 : 0;
+                    cnt += sx_greater(u, v, a.sd) ? 1 : 0;
+                }
             }
         }
         any = __any_sync(0xffffffffu, any != 0) ? 1 : 0;

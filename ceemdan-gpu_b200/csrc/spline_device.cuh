@@ -261,9 +261,9 @@ struct CheckedPivot {
 // End relations (chunk_ends: same operations, same order) of the chunk whose knots 0..len+1 sit
 // in the padded arrays x, s from the chunk's base on (s[i]: slope of segment i -> i+1).  Each
 // sweep loads one new knot and slope per row, a row ahead of its use.
-template <bool kIw, class Pivot, class XT>
+template <class Pivot, class XT>
 __device__ __forceinline__ ChunkEnds chunk_ends_sweep(Pivot& pv, const XT* x, const double* s,
-                                                      int len, double* iwo) {
+                                                      int len) {
     int xt = x[2], xb = x[len - 1];
     // top-down row 0 and bottom-up row len-1
     double lt = (double)(x[1] - x[0]), ut = (double)(xt - x[1]);
@@ -283,7 +283,6 @@ __device__ __forceinline__ ChunkEnds chunk_ends_sweep(Pivot& pv, const XT* x, co
     }
     double iw = pv.inv(2.0 * (lt + ut));
     double iv = pv.inv(2.0 * (lb + ub));
-    if (kIw) iwo[0] = iw;
     double cp = ut * iw, gp = wr0 * iw, ap = -lt * iw;
     double cq = lb * iv, gq = vr0 * iv, bq = -ub * iv;
 #pragma unroll 2
@@ -312,7 +311,6 @@ __device__ __forceinline__ ChunkEnds chunk_ends_sweep(Pivot& pv, const XT* x, co
         cq = lb * iv;
         gq = fma(-ub, gq, vr) * iv;
         bq = (-ub * bq) * iv;
-        if (kIw) iwo[k] = iw;
     }
     ChunkEnds e;
     e.gb = gp;
@@ -323,24 +321,82 @@ __device__ __forceinline__ ChunkEnds chunk_ends_sweep(Pivot& pv, const XT* x, co
     e.aa = -lf * iv;
     return e;
 }
-template <bool kIw, class XT>
+template <class XT>
 __device__ __noinline__ void chunk_ends_checked(ChunkEnds& e, const XT* x, const double* s,
-                                                int len, double* iwo) {
+                                                int len) {
     CheckedPivot pv;
-    e = chunk_ends_sweep<kIw>(pv, x, s, len, iwo);
+    e = chunk_ends_sweep(pv, x, s, len);
 }
-// kIw: the top-down sweep's reciprocals to iwo[0 .. len-1]
-template <bool kIw = false, class XT>
-__device__ __forceinline__ ChunkEnds chunk_ends_knots(const XT* x, const double* s, int len,
-                                                      double* iwo = nullptr) {
+template <class XT>
+__device__ __forceinline__ ChunkEnds chunk_ends_knots(const XT* x, const double* s, int len) {
     RawPivot pv;
-    ChunkEnds e = chunk_ends_sweep<kIw>(pv, x, s, len, iwo);
+    ChunkEnds e = chunk_ends_sweep(pv, x, s, len);
     if (pv.ones) {
         ChunkEnds c;
-        chunk_ends_checked<kIw>(c, x, s, len, iwo);
+        chunk_ends_checked(c, x, s, len);
         e = c;
     }
     return e;
+}
+
+// One direction of chunk_ends_sweep (same operations, same order; see ends_sweep): top gb, ab, bb to
+// out[3..5] and the reciprocals to iwo, else ga, aa, ba to out[0..2].
+template <bool top, class Pivot, class XT>
+__device__ __forceinline__ void chunk_ends_one(Pivot& pv, const XT* x, const double* s, int len,
+                                               double* out, double* iwo) {
+    // knots and slopes in the sweep's direction
+    auto knot = [&](int i) -> int { return x[kq(top ? i : len + 1 - i)]; };
+    auto slope = [&](int i) -> double { return s[top ? i : len - i]; };
+    auto length = [](int from, int to) { return (double)(top ? to - from : from - to); };
+    auto rhs = [](double s0, double s1) { return 3.0 * (top ? s1 - s0 : s0 - s1); };
+    const int x1 = knot(1);
+    int xt = knot(2);
+    // row k: o the length towards the sweep's start, t towards its end
+    double o = length(knot(0), x1), t = length(x1, xt), st = slope(1), tn = 0.0, sn = 0.0;
+    const double r0 = rhs(slope(0), st);
+    if (len > 1) {
+        const int xn = knot(3);
+        tn = length(xt, xn);
+        xt = xn;
+        sn = slope(2);
+    }
+    double i = pv.inv(2.0 * (o + t));
+    if (top) iwo[0] = i;
+    double c = t * i, g = r0 * i, f = -o * i;
+#pragma unroll 2
+    for (int k = 1; k < len; ++k) {
+        o = t;
+        t = tn;
+        const double r = rhs(st, sn);
+        st = sn;
+        if (k + 1 < len) {
+            const int xn = knot(k + 3);
+            tn = length(xt, xn);
+            xt = xn;
+            sn = slope(k + 2);
+        }
+        i = pv.inv(fma(-o, c, 2.0 * (o + t)));
+        c = t * i;
+        g = fma(-o, g, r) * i;
+        f = (-o * f) * i;
+        if (top) iwo[k] = i;
+    }
+    out[top ? 3 : 0] = g;
+    out[top ? 4 : 2] = f;
+    out[top ? 5 : 1] = -t * i;
+}
+template <bool top, class XT>
+__device__ __noinline__ void chunk_ends_one_checked(const XT* x, const double* s, int len,
+                                                    double* out, double* iwo) {
+    CheckedPivot pv;
+    chunk_ends_one<top>(pv, x, s, len, out, iwo);
+}
+template <bool top, class XT>
+__device__ __forceinline__ void chunk_ends_half(const XT* x, const double* s, int len, double* out,
+                                                double* iwo) {
+    RawPivot pv;
+    chunk_ends_one<top>(pv, x, s, len, out, iwo);
+    if (pv.ones) chunk_ends_one_checked<top>(x, s, len, out, iwo);
 }
 
 // Inclusive prefix of v over the warp's lanes.
@@ -367,61 +423,60 @@ __device__ __forceinline__ SepRow sep_row(const Row& w) { return SepRow{w.l, w.m
 // padded length of n rows
 __host__ __device__ __forceinline__ int padded(int n) { return n + (n >> 4) + 1; }
 
-// chunk_ends (same operations, same order) of len consecutive rows; the top-down sweep's
-// reciprocals to iw (kIw).  Rows are read one ahead of their use.
-template <bool kIw, class Pivot>
-__device__ __forceinline__ ChunkEnds ends_sweep(Pivot& pv, const SepRow* r, int len, double* iw) {
-    SepRow w = load_row(r), v = load_row(r + len - 1);
-    const double lf = w.l, ul = v.u;
-    double iu = pv.inv(w.m), iv = pv.inv(v.m);
-    double cp = w.u * iu, gp = w.r * iu, ap = -w.l * iu;
-    double cq = v.l * iv, gq = v.r * iv, bq = -v.u * iv;
-    if (kIw) iw[0] = iu;
+// One direction of chunk_ends (same operations, same order) of len consecutive rows: top the
+// top-down sweep, gb, ab, bb to out[3..5] and its reciprocals to iw (unless null), else the bottom-up
+// one, ga, aa, ba to out[0..2].  The two directions are different warps' work: a thread that does
+// both waits for its own instructions while the warps beside it have nothing to do.
+template <bool top, class Pivot>
+__device__ __forceinline__ void ends_sweep(Pivot& pv, const SepRow* r, int len, double* iw,
+                                           double* out) {
+    const double* p = reinterpret_cast<const double*>(top ? r : r + len - 1);
+    constexpr int step = top ? 4 : -4;
+    // the row's coefficient towards the sweep's start and towards its end
+    constexpr int io = top ? 0 : 2, it = 2 - io;
+    double o = p[io], t = p[it], m = p[1], b = p[3];
+    double i = pv.inv(m);
+    double c = t * i, g = b * i, f = -o * i;
+    if (top && iw) iw[0] = i;
+    double on = 0.0, tn = 0.0, mn = 0.0, bn = 0.0;  // the next row's
     if (len > 1) {
-        w = load_row(r + 1);
-        v = load_row(r + len - 2);
+        p += step;
+        on = p[io], tn = p[it], mn = p[1], bn = p[3];
     }
-#pragma unroll 1
+#pragma unroll 2
     for (int k = 1; k < len; ++k) {
-        const SepRow a = w, b = v;
+        o = on, t = tn, m = mn, b = bn;
         if (k + 1 < len) {
-            w = load_row(r + k + 1);
-            v = load_row(r + len - 2 - k);
+            p += step;
+            on = p[io], tn = p[it], mn = p[1], bn = p[3];
         }
-        iu = pv.inv(fma(-a.l, cp, a.m));
-        iv = pv.inv(fma(-b.u, cq, b.m));
-        cp = a.u * iu;
-        gp = fma(-a.l, gp, a.r) * iu;
-        ap = (-a.l * ap) * iu;
-        cq = b.l * iv;
-        gq = fma(-b.u, gq, b.r) * iv;
-        bq = (-b.u * bq) * iv;
-        if (kIw) iw[k] = iu;
+        i = pv.inv(fma(-o, c, m));
+        c = t * i;
+        g = fma(-o, g, b) * i;
+        f = (-o * f) * i;
+        if (top && iw) iw[k] = i;
     }
-    return ChunkEnds{gq, -lf * iv, bq, gp, ap, -ul * iu};
+    out[top ? 3 : 0] = g;
+    out[top ? 4 : 2] = f;
+    out[top ? 5 : 1] = -t * i;
 }
-template <bool kIw>
-__device__ __noinline__ void ends_rows_checked(const SepRow* r, int len, double* iw,
-                                               ChunkEnds& e) {
+template <bool top>
+__device__ __noinline__ void ends_rows_checked(const SepRow* r, int len, double* iw, double* out) {
     CheckedPivot pv;
-    e = ends_sweep<kIw>(pv, r, len, iw);
+    ends_sweep<top>(pv, r, len, iw, out);
 }
-// ... to out[0..5] = ga, aa, ba, gb, ab, bb
-template <bool kIw>
+template <bool top>
 __device__ __forceinline__ void ends_rows(const SepRow* r, int len, double* iw, double* out) {
     RawPivot pv;
-    ChunkEnds e = ends_sweep<kIw>(pv, r, len, iw);
-    if (pv.ones) {
-        ChunkEnds c;
-        ends_rows_checked<kIw>(r, len, iw, c);
-        e = c;
-    }
-    out[0] = e.ga;
-    out[1] = e.aa;
-    out[2] = e.ba;
-    out[3] = e.gb;
-    out[4] = e.ab;
-    out[5] = e.bb;
+    ends_sweep<top>(pv, r, len, iw, out);
+    if (pv.ones) ends_rows_checked<top>(r, len, iw, out);
+}
+// Work item i of the two directions of n chunks: whole warps of one direction.
+__device__ __forceinline__ int ends_items(int n) { return 2 * ((n + 31) & ~31); }
+__device__ __forceinline__ bool ends_item(int i, int n, int& q) {
+    const int half = (n + 31) & ~31;
+    q = i < half ? i : i - half;
+    return i < half;
 }
 
 // Row p of the next level: separator row s between the chunks with end relations e (left) and
@@ -432,19 +487,24 @@ __device__ __forceinline__ SepRow next_row(const SepRow& s, const double* e) {
 
 // Back substitution x[k] <- x[k] - fac(k) x[k+1], row k's factor in its u.
 __device__ __forceinline__ void back_rows(const SepRow* r, double* x, int len, double xv) {
-    double f = 0.0, g = 0.0;
-    if (len > 1) {
-        f = r[len - 2].u;
-        g = x[len - 2];
+    int k = len - 2;
+#pragma unroll 1
+    for (; k >= 3; k -= 4) {  // four rows at a time, loaded before the first is needed
+        double f[4], g[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            f[i] = r[k - i].u;
+            g[i] = x[k - i];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            xv = fma(-f[i], xv, g[i]);
+            x[k - i] = xv;
+        }
     }
 #pragma unroll 1
-    for (int k = len - 2; k >= 0; --k) {
-        const double fc = f, gc = g;
-        if (k > 0) {
-            f = r[k - 1].u;
-            g = x[k - 1];
-        }
-        xv = fma(-fc, xv, gc);
+    for (; k >= 0; --k) {
+        xv = fma(-r[k].u, xv, x[k]);
         x[k] = xv;
     }
 }
@@ -454,20 +514,37 @@ __device__ __forceinline__ void back_rows(const SepRow* r, double* x, int len, d
 __device__ __forceinline__ void interior_rows(SepRow* r, int len, double xl, double xr,
                                               double* x) {
     SepRow w = load_row(r);
-    double iw = x[0], gp = 0.0;
+    double ri = fma(-w.l, xl, w.r);
+    if (len == 1) ri = fma(-w.u, xr, ri);
+    double gp = ri * x[0];
+    r[0].u = w.u * x[0];
+    x[0] = gp;
+    int k = 1;
 #pragma unroll 1
-    for (int k = 0; k < len; ++k) {
-        const SepRow a = w;
-        const double ic = iw;
-        if (k + 1 < len) {
-            w = load_row(r + k + 1);
-            iw = x[k + 1];
+    for (; k + 4 < len; k += 4) {  // four rows at a time, loaded before the first is needed
+        double l[4], u[4], b[4], iw[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            l[i] = r[k + i].l;
+            u[i] = r[k + i].u;
+            b[i] = r[k + i].r;
+            iw[i] = x[k + i];
         }
-        double ri = a.r;
-        if (k == 0) ri = fma(-a.l, xl, ri);
-        if (k == len - 1) ri = fma(-a.u, xr, ri);
-        gp = (k == 0 ? ri : fma(-a.l, gp, ri)) * ic;
-        r[k].u = a.u * ic;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            gp = fma(-l[i], gp, b[i]) * iw[i];
+            r[k + i].u = u[i] * iw[i];
+            x[k + i] = gp;
+        }
+    }
+#pragma unroll 1
+    for (; k < len; ++k) {
+        w = load_row(r + k);
+        ri = w.r;
+        if (k == len - 1) ri = fma(-w.u, xr, ri);
+        const double iw = x[k];
+        gp = fma(-w.l, gp, ri) * iw;
+        r[k].u = w.u * iw;
         x[k] = gp;
     }
     back_rows(r, x, len, gp);
@@ -539,10 +616,14 @@ __device__ void partition_rows(const Group& grp, int n, SepRow* rows, double* x,
     for (int k = 0; k < depth; ++k) {
         const RowsLevel v = rows_level(k, depth, n, rows, x, ws);
         const RowsLevel o = rows_level(k + 1, depth, n, rows, x, ws);
-        for (int q = tid; q <= o.n; q += size_g) {
+        for (int i = tid; i < ends_items(o.n + 1); i += size_g) {
+            int q;
+            const bool top = ends_item(i, o.n + 1, q);
+            if (q > o.n) continue;
             const int first = q * kChunk;
             const int len = (q < o.n) ? kChunk - 1 : v.n - first;
-            ends_rows<true>(v.r + kq(first), len, v.x + kq(first), ends + 6 * q);
+            if (top) ends_rows<true>(v.r + kq(first), len, v.x + kq(first), ends + 6 * q);
+            else ends_rows<false>(v.r + kq(first), len, nullptr, ends + 6 * q);
         }
         grp.sync();
         for (int p = tid; p < o.n; p += size_g)
