@@ -426,7 +426,8 @@ __host__ __device__ __forceinline__ int padded(int n) { return n + (n >> 4) + 1;
 // One direction of chunk_ends (same operations, same order) of len consecutive rows: top the
 // top-down sweep, gb, ab, bb to out[3..5] and its reciprocals to iw (unless null), else the bottom-up
 // one, ga, aa, ba to out[0..2].  The two directions are different warps' work: a thread that does
-// both waits for its own instructions while the warps beside it have nothing to do.
+// both waits for its own instructions while the warps beside it have nothing to do (on chip, N=2501
+// NR=100: 19.5 -> 18.2 us an iteration; as one code with the direction an argument 3 us slower).
 template <bool top, class Pivot>
 __device__ __forceinline__ void ends_sweep(Pivot& pv, const SepRow* r, int len, double* iw,
                                            double* out) {
