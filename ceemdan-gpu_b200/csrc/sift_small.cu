@@ -570,8 +570,9 @@ k_sift_small(const __grid_constant__ SiftArgs a, const __grid_constant__ SmallAr
                 build_envelope(grp, E0, warp_tot(0), H, s_g, s_l, n, e, sa, j, r, [&]() {
                     if (e == 0) wait();
                 });
-                __syncthreads();
+                // (before the barrier: every thread decides by both counts)
                 if (tid == 0) s_kcnt[e] = E0.I->K;
+                __syncthreads();
                 if (e == 0) {
 #pragma unroll 4
                     for (int s = tid; s < n; s += kSmallThreads) up[s] = env_at(E0, H, s);
