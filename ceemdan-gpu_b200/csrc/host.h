@@ -561,7 +561,8 @@ struct SiftEngine {
         // device copy of a taped stage's block table (blocks of kTapeBlockSlots slots)
         CKS(ws.alloc_n(&tblocks_dev, (size_t)(std::max(1, max_cap) + kTapeBlockSlots - 1) /
                                          kTapeBlockSlots));
-        // a negative limit -k: the test of the timeout path (every wait gives up after k polls)
+        // a negative limit -k: the test of the timeout path (the waits of every realization's
+        // first CTA give up after k polls, the other CTA's of a pair do not)
         sa.spin_limit = spin_limit > 0 ? spin_limit : (spin_limit < 0 ? -spin_limit : (1 << 22));
         sa.extra = spin_limit < 0 ? 1u : 0u;
         small_cap = std::max(1, max_cap);

@@ -220,8 +220,9 @@ struct SmallArgs {
     unsigned long long* arrive;
     double* up;            // [nrows*row_ld(n)] upper envelope of the iteration (kSmallSingle)
     int spin_limit;        // polls of the stop test before giving up (CEEMDAN_ERR_TIMEOUT)
-    unsigned extra;        // arrivals the test waits for beyond the realizations: 0, or 1 to make
-                           // every wait give up (the timeout path's test)
+    unsigned extra;        // arrivals that the first CTA of a realization waits for beyond the
+                           // realizations: 0, or 1 to make its waits give up (the timeout path's
+                           // test)
     // taped forward: the stage's tape blocks (slot j at tblocks[j / kTapeBlockSlots] +
     // (j % kTapeBlockSlots) * tl.stride), null otherwise
     unsigned char* const* tblocks;

@@ -49,6 +49,9 @@ constexpr int kMaxTiles = kSmallMaxN / kTileSamples;
 constexpr int kSmallWords = kSmallMaxN / 32;
 static_assert(kSmallMaxN % kTileSamples == 0 && kTileSamples == 64 * 32, "two warps of words a tile");
 
+// What a CTA's wait at the lock-step test came to.
+constexpr int kGoOn = 0, kStop = 1, kGaveUp = 2;
+
 // The threads that build one envelope: the whole CTA, or half of it with its own barrier.
 template <int kSize>
 struct SmallGroup {
@@ -448,7 +451,8 @@ k_sift_small(const __grid_constant__ SiftArgs a, const __grid_constant__ SmallAr
     __shared__ unsigned s_g[kSmallWords + 1], s_l[kSmallWords + 1];  // signs of h[i] - h[i+1]
     __shared__ int s_part[2 * kWarps];  // counts of every warp of the realization
     __shared__ int s_kcnt[2];           // knot counts, upper and lower
-    __shared__ int s_stop, s_err;       // the lock-step test of the last iteration
+    // how the last iteration's lock-step test ended, as each CTA of the realization saw it
+    __shared__ int s_end[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int r = kPair ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
     const int rank = kPair ? (int)(blockIdx.x & 1) : 0;
@@ -470,13 +474,13 @@ k_sift_small(const __grid_constant__ SiftArgs a, const __grid_constant__ SmallAr
     const int oth0 = kPair ? (rank == 0 ? half : 0) : 0, oth1 = kPair ? (rank == 0 ? n : half) : 0;
     double* recv = reinterpret_cast<double*>(set0 + L.recv);  // the other CTA's envelope, own half
     double* recv_peer = nullptr;
-    int *part_peer = nullptr, *kcnt_peer = nullptr, *err_peer = nullptr;
+    int *part_peer = nullptr, *kcnt_peer = nullptr, *end_peer = nullptr;
     if constexpr (kPair) {
         cg::cluster_group cl = cg::this_cluster();
         recv_peer = cl.map_shared_rank(recv, rank ^ 1);
         part_peer = cl.map_shared_rank(s_part, rank ^ 1);
         kcnt_peer = cl.map_shared_rank(s_kcnt, rank ^ 1);
-        err_peer = cl.map_shared_rank(&s_err, rank ^ 1);
+        end_peer = cl.map_shared_rank(s_end, rank ^ 1);
     }
     ChanState& cst = a.cs[0];
     const int cap = cst.cap;
@@ -489,7 +493,7 @@ k_sift_small(const __grid_constant__ SiftArgs a, const __grid_constant__ SmallAr
     for (int i = tid; i < n; i += kSmallThreads) H[i] = hin[i];
     if (tid == 0) {
         s_g[0] = s_l[0] = 0u;
-        s_stop = s_err = 0;
+        s_end[0] = s_end[1] = kGoOn;
     }
     // every thread carries the realization's state (the same values)
     double frac = a.frac[r];
@@ -531,7 +535,7 @@ k_sift_small(const __grid_constant__ SiftArgs a, const __grid_constant__ SmallAr
     };
 
     int j = 0;
-    bool ended = false;  // by the lock-step test: iteration j's work is discarded
+    int end = kGoOn;  // else by the lock-step test: iteration j's work is discarded
     for (; j < cap; ++j) {
         update();
         __syncthreads();
@@ -550,18 +554,18 @@ k_sift_small(const __grid_constant__ SiftArgs a, const __grid_constant__ SmallAr
         auto wait = [&]() {
             if (j == 0 || a.forced > 0) return;
             const volatile unsigned long long* word = sa.arrive + (j - 1);
-            const unsigned target = (unsigned)nreal + sa.extra;
+            const unsigned target = (unsigned)nreal + (rank == 0 ? sa.extra : 0u);
             int spins = 0;
             unsigned long long v = *word;
             while ((unsigned)v < target) {
                 if (++spins > sa.spin_limit) {
-                    s_err = 1;
+                    s_end[rank] = kGaveUp;
                     return;
                 }
                 __nanosleep(32);
                 v = *word;
             }
-            if ((int)(v >> 32) == nreal) s_stop = 1;
+            if ((int)(v >> 32) == nreal) s_end[rank] = kStop;
         };
         // (one copy of build_envelope's code, for the instruction cache)
         if constexpr (kMode == kSmallSingle) {
@@ -590,7 +594,10 @@ k_sift_small(const __grid_constant__ SiftArgs a, const __grid_constant__ SmallAr
             build_envelope(grp, E0, warp_tot(0), H, s_g, s_l, n, rank, sa, j, r, wait);
             // the solve's workspace (recv) is free in both CTAs, coefficients ready
             cg::this_cluster().sync();
-            if (tid == 0) s_kcnt[rank] = kcnt_peer[rank] = E0.I->K;
+            if (tid == 0) {
+                s_kcnt[rank] = kcnt_peer[rank] = E0.I->K;
+                end_peer[rank] = s_end[rank];
+            }
 #pragma unroll 4
             for (int s = oth0 + tid; s < oth1; s += kSmallThreads)
                 recv_peer[s - oth0] = env_at(E0, H, s);
@@ -605,10 +612,11 @@ k_sift_small(const __grid_constant__ SiftArgs a, const __grid_constant__ SmallAr
             }
             cg::this_cluster().barrier_wait();
         }
-        if (s_stop) {  // the previous iteration was the stage's last
-            ended = true;
-            break;
-        }
+        // The previous iteration was the stage's last, or a wait gave up.  Both CTAs of a pair know
+        // what either saw, so they leave together: one that went on alone would write to the
+        // other's shared memory after its exit.
+        end = kPair ? max(s_end[0], s_end[1]) : s_end[0];
+        if (end != kGoOn) break;
         const int kmax = s_kcnt[0], kmin = s_kcnt[1];
         const bool write_mean = kmax > 3 && kmin > 3;
         // the envelopes at the thread's sample k
@@ -669,12 +677,10 @@ k_sift_small(const __grid_constant__ SiftArgs a, const __grid_constant__ SmallAr
             if constexpr (kPair) part_peer[rank * kWarps + warp] = v;
         }
         if constexpr (kPair) {
-            if (tid == 0 && s_err) *err_peer = 1;
             cg::this_cluster().sync();
         } else {
             __syncthreads();
         }
-        if (s_err) break;  // (both CTAs of a pair see it)
         const int v = lane < (kPair ? 2 : 1) * kWarps ? s_part[lane] : 0;
         const int c = __reduce_add_sync(0xffffffffu, v & 0x3fffffff);
         const bool y = __any_sync(0xffffffffu, (v >> 30) != 0);
@@ -700,11 +706,11 @@ k_sift_small(const __grid_constant__ SiftArgs a, const __grid_constant__ SmallAr
             break;
         }
     }
-    if (s_err) {  // a wait gave up: the host reports CEEMDAN_ERR_TIMEOUT
+    if (end == kGaveUp) {  // the host reports CEEMDAN_ERR_TIMEOUT
         if (tid == 0) atomicExch(&cst.err, kErrTimeout);
         return;
     }
-    if (!ended && mark == 0) update();  // the modes of the last iteration
+    if (end == kGoOn && mark == 0) update();  // the modes of the last iteration
     if (tid == 0 && rank == 0) {
         a.frac[r] = frac;
         if (r == 0) {

@@ -49,9 +49,9 @@ typedef struct ceemdan_options {
     int32_t spin_limit;          /* polls of an in-kernel wait before it gives up and the call
                                     returns CEEMDAN_ERR_TIMEOUT (0 = auto, about a second): the
                                     lock-step stop test of the on-chip path for short rows.  A
-                                    negative value -k is a test of that failure path: the wait
-                                    expects one arrival more than the launch has, so it always
-                                    gives up after k polls */
+                                    negative value -k is a test of that failure path: the first
+                                    CTA of every realization expects one arrival more than the
+                                    launch has, so its wait always gives up after k polls */
     double* h_kernel_ms;         /* optional [CEEMDAN_NUM_KERNEL_KINDS]: accumulated device time
                                     per kernel kind (CUDA events around every launch) */
     uint64_t* h_counters;        /* optional [CEEMDAN_NUM_COUNTERS]: accumulated work counters */
