@@ -173,7 +173,10 @@ ceemdan_status check_coords(const int32_t* d_x, size_t n, int* d_err, cudaStream
 // cuRAND generators kept between calls, at most kKeptGenerators idle ones (creating and destroying
 // one, with its device memory, took 0.7 ms of every call: N=1024 NR=8, 5 IMFs 2.85 -> 2.16 ms).  A
 // generator is one caller's between take and give; the next one's stream waits for the last use
-// of its state, and seed and offset are set anew, so the numbers are a new generator's.
+// of its state, and seed and offset are set anew, so the numbers are a new generator's.  That wait
+// costs nothing by itself: cuRAND seeds a generator in its first generation, kept or new, and holds
+// the host there until the device has finished everything queued on it, other streams' work
+// included (measured: 306 ms behind a kernel of 306 ms on another stream).
 namespace {
 constexpr size_t kKeptGenerators = 4;
 struct Generator {
@@ -187,6 +190,13 @@ std::vector<Generator> g_gen_idle;
 void destroy_generator(Generator& g) {
     if (g.gen) curandDestroyGenerator(g.gen);
     if (g.used) cudaEventDestroy(g.used);
+    g = Generator();
+}
+
+bool set_generator(const Generator& g, uint64_t seed, cudaStream_t st) {
+    return curandSetStream(g.gen, st) == CURAND_STATUS_SUCCESS &&
+           curandSetPseudoRandomGeneratorSeed(g.gen, seed) == CURAND_STATUS_SUCCESS &&
+           curandSetGeneratorOffset(g.gen, 0) == CURAND_STATUS_SUCCESS;
 }
 
 bool take_generator(Generator& g, uint64_t seed, cudaStream_t st) {
@@ -201,18 +211,16 @@ bool take_generator(Generator& g, uint64_t seed, cudaStream_t st) {
                 break;
             }
     }
-    bool ok = true;
     if (g.gen) {
-        ok = cudaStreamWaitEvent(st, g.used, 0) == cudaSuccess;
-    } else {
-        g.dev = dev;
-        ok = cudaEventCreateWithFlags(&g.used, cudaEventDisableTiming) == cudaSuccess &&
-             curandCreateGenerator(&g.gen, CURAND_RNG_PSEUDO_DEFAULT) == CURAND_STATUS_SUCCESS;
+        if (cudaStreamWaitEvent(st, g.used, 0) == cudaSuccess && set_generator(g, seed, st))
+            return true;
+        cudaGetLastError();
+        destroy_generator(g);  // a new one serves
     }
-    ok = ok && curandSetStream(g.gen, st) == CURAND_STATUS_SUCCESS &&
-         curandSetPseudoRandomGeneratorSeed(g.gen, seed) == CURAND_STATUS_SUCCESS &&
-         curandSetGeneratorOffset(g.gen, 0) == CURAND_STATUS_SUCCESS;
-    return ok;
+    g.dev = dev;
+    return cudaEventCreateWithFlags(&g.used, cudaEventDisableTiming) == cudaSuccess &&
+           curandCreateGenerator(&g.gen, CURAND_RNG_PSEUDO_DEFAULT) == CURAND_STATUS_SUCCESS &&
+           set_generator(g, seed, st);
 }
 
 // ok: the generator's work is on st; otherwise it is not used again
