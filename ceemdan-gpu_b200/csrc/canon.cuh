@@ -99,21 +99,29 @@ CEEMDAN_HD Row identity_row() {
 }
 
 // 1/x, correctly rounded, for the pivots of spline systems: x in [1, 2^40] (the systems are
-// diagonally dominant with integer spacings; see the sweeps below).  The hardware's 20-bit
-// reciprocal estimate e0 is refined once cubically, y = e0(1 + e + e^2) with e = 1 - x e0
-// (|e| < 2^-19, so y is within one ulp), and rounded by Markstein's correction: r = 1 - x y is
-// exact in one fma, and RN(y + r y) = RN(1/x) for every x whose significand is not all ones
-// (P. Markstein, IBM J. Res. Dev. 34(1), 1990).  The all-ones significand x = 2^(k+1)(1-2^-53)
-// has RN(1/x) = 2^-(k+1) (1 + 2^-52), selected.  No branch: two independent sweeps interleave
-// where the general reciprocal's range branch makes them run one after the other (measured on
-// a B200, two reciprocal-and-fma chains side by side: 162 cycles a step with 1.0/x, 71 so).
+// diagonally dominant with integer spacings; see the sweeps below).  It starts from the estimate
+// y0 that PTX documents (of the operand's and to the result's leading 20 fraction bits), whose
+// e = 1 - x y0 is below 2^-18 (tests/pivot_estimate_check.cu: all 2^20 leading significands).  By
+// Goldschmidt's factors, 1/x = y0 / (1 - e) = y0 (1 + e)(1 + e^2)(1 + e^4)... (R. Goldschmidt,
+// Applications of Division by Convergence, MIT 1964; Anderson et al., IBM J. Res. Dev. 11(1), 1967):
+// y1 = y0 (1 + e) and e^2 form side by side, and y2 = y1 (1 + e^2) is 1/x to 2^-72 but for the two
+// roundings of y1 and y2, half an ulp each, so within one ulp.  Markstein's correction rounds it
+// (P. Markstein, IBM J. Res. Dev. 34(1), 1990): r = 1 - x y2 is exact in one fma and RN(y2 + r y2)
+// = RN(1/x) for every x whose significand is not all ones (tests/test_reciprocal_rounding.py: the
+// 33 significands whose reciprocals lie close enough to a midpoint, every start within an ulp).
+// The all-ones significand x = 2^(k+1)(1-2^-53) has RN(1/x) = 2^-(k+1) (1 + 2^-52), selected.  No
+// branch: two independent sweeps interleave where the general reciprocal's range branch makes them
+// run one after the other (measured on a B200, two reciprocal-and-fma chains side by side: 131
+// cycles a step with 1.0/x, 80 with rcp_raw, 105 with pivot_inv; one chain 71, 70, 84).
 // rcp_raw is the reciprocal without that selection, for x known to have another significand.
 CEEMDAN_HD double rcp_raw(double x) {
 #ifdef __CUDA_ARCH__
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double e = fma(-x, y, 1.0);
-    y = fma(y, fma(e, e, e), y);
+    const double e2 = e * e;
+    y = fma(y, e, y);
+    y = fma(y, e2, y);
     return fma(fma(-x, y, 1.0), y, y);
 #else
     return 1.0 / x;
