@@ -1768,6 +1768,14 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
                            S.c[i1], b, d);
             S.b[i0] = b;
             S.d[i0] = d;
+        } else if (th == wh - 2 && last) {
+            // The samples past the row, in the warp that holds its end: envelopes of opposite
+            // sign so large that the end knot's value vanishes in them, so sx = 0, which counts
+            // nowhere (where it would not vanish, NaN: its thread does its samples again).
+            const int i0 = bh + seg_at(ch);
+            const double big = fabs(staged(S.stage, m - 1)) < 0x1p+900 ? 0x1p+1000 : NAN;
+            S.b[i0] = eh ? -big : big;
+            S.d[i0] = 0.0;
         }
         if (!two) {
             const int xu = rA0 == 0 ? ed0->px - n0 : S.x[base0 + seg_at(rA0)];
@@ -1791,8 +1799,10 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
     const bool wide = !kEnv || (((size_t)a.dbg_upper | (size_t)a.dbg_lower) & 31) == 0 &&
                                    (q.n & 3) == 0;
     bool redo = false;
-    // (the warp's samples all in the row: warp-uniform)
-    const bool common = !two && (kEnv || write_mean) && wide && m - warp * kWarpSamples >= kWarpSamples;
+    // samples of the row in the warp's part of the tile (warp-uniform)
+    const int in_row = m - warp * kWarpSamples;
+    const bool full = in_row >= kWarpSamples;
+    const bool common = !two && (kEnv || write_mean) && wide && (full || (!kEnv && in_row > 0));
     if (common) {
         // Both envelopes along the thread's samples: a segment's coefficients are loaded when the
         // samples pass its first knot (whose value is that sample's).  sx > t is decided by the
@@ -1893,8 +1903,8 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
                     const int u = stage_piece(2 * j);
                     const double2 p0 = mean_w[u], p1 = mean_w[u ^ 1];
                     const double w[4] = {p0.x, p0.y, p1.x, p1.y};
-                    store4(mean() + warp * kWarpSamples + kPerThread * (j >> 1) + (i0 & 8) +
-                               4 * (j & 1), w);
+                    const int o = kPerThread * (j >> 1) + (i0 & 8) + 4 * (j & 1);
+                    if (full || o < in_row) store4(mean() + warp * kWarpSamples + o, w);
                 }
                 __syncwarp();
             }
@@ -1905,7 +1915,7 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
                 const int u = (tid & ~31) * (kPerThread / 2) + 2 * (lane + 32 * g);
                 const double2 p0 = S.stage[stage_piece(u)], p1 = S.stage[stage_piece(u) ^ 1];
                 const double w[4] = {p0.x, p0.y, p1.x, p1.y};
-                store4(hout() + 2 * u, w);
+                if (full || 2 * u < m) store4(hout() + 2 * u, w);  // (rows are padded to four)
             }
         }
         any = amax > 0 ? 1 : 0;
