@@ -1792,7 +1792,8 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
         __syncthreads();
     }
     // kEnv: the envelopes themselves go to the caller's arrays in place of the next h and the
-    // mean envelope (contiguous rows, aligned to 32 bytes or not)
+    // mean envelope (contiguous rows, aligned to 32 bytes or not: then a sample to a
+    // lane, and the padded copy of the rows in: 61441 x 50 281 us a call, 61440 x 50 260)
     auto mean = [&]() -> double* {
         return kEnv ? a.dbg_lower + (size_t)q.r * q.n + n0 : a.menv + q.base + n0;
     };
@@ -1802,7 +1803,7 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
     // samples of the row in the warp's part of the tile (warp-uniform)
     const int in_row = m - warp * kWarpSamples;
     const bool full = in_row >= kWarpSamples;
-    const bool common = !two && (kEnv || write_mean) && wide && (full || (!kEnv && in_row > 0));
+    const bool common = !two && (kEnv || write_mean) && in_row > 0;
     if (common) {
         // Both envelopes along the thread's samples: a segment's coefficients are loaded when the
         // samples pass its first knot (whose value is that sample's).  sx > t is decided by the
@@ -1869,9 +1870,10 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
                     }
                 }
             }
+            double2* const pm = mean_w + (stage_piece(4 * lane) ^ ((i0 + k) / 2 & 3));
             if (kEnv) {
-                *reinterpret_cast<double2*>(hout() + j0 + i0 + k) = make_double2(eu[0], eu[1]);
-                *reinterpret_cast<double2*>(mean() + j0 + i0 + k) = make_double2(ev[0], ev[1]);
+                *pa = make_double2(eu[0], eu[1]);
+                *pm = make_double2(ev[0], ev[1]);
                 continue;
             }
             const double2 hk = *pa;
@@ -1892,11 +1894,17 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
                 }
             }
             *pa = make_double2(hn[0], hn[1]);
-            mean_w[stage_piece(4 * lane) ^ ((i0 + k) / 2 & 3)] = make_double2(mv[0], mv[1]);
+            *pm = make_double2(mv[0], mv[1]);
             }
-            if (kEnv) continue;
             if (i0 & 4) {  // 64 bytes of every lane's samples
                 __syncwarp();
+                if (!wide) {
+                    double* const out = mean() + warp * kWarpSamples;
+                    for (int g = 0; g < 8; ++g) {
+                        const int i = lane + 32 * g, o = kPerThread * (i >> 3) + (i0 & 8) + (i & 7);
+                        if (o < in_row) out[o] = staged(mean_w, i);
+                    }
+                } else
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
                     const int j = lane + 32 * g;
@@ -1909,7 +1917,10 @@ k_tile_sift(const __grid_constant__ SiftArgs a) {
                 __syncwarp();
             }
         }
-        if (!kEnv) {
+        if (!wide) {
+            for (int i = lane; i < min(in_row, kWarpSamples); i += 32)
+                hout()[warp * kWarpSamples + i] = staged(S.stage, warp * kWarpSamples + i);
+        } else {
 #pragma unroll
             for (int g = 0; g < kPerThread / 4; ++g) {
                 const int u = (tid & ~31) * (kPerThread / 2) + 2 * (lane + 32 * g);

@@ -43,3 +43,29 @@ def test_many_short_rows(pkg, orc, wl, cuda, n, nr):
                              return_iters=True)
     assert list(it) == list(wit)
     assert np.array_equal(got.cpu().numpy(), want, equal_nan=True)
+
+
+@pytest.mark.parametrize("n", LENGTHS + [6144, 6147])
+@pytest.mark.parametrize("shift", [0, 1, 2, 5])
+def test_envelopes_into_any_alignment(pkg, orc, cuda, n, shift):
+    """Outputs that start `shift` doubles past a 256-byte boundary, rows of every length modulo
+    four; nothing around the output is touched."""
+    import ctypes
+    import torch
+    nr = 5
+    rng = np.random.default_rng(n)
+    rows = rng.standard_normal((nr, n))
+    rows[1] = np.cumsum(rows[1])
+    rows[2] = np.cos(2 * np.pi * 1.3 * np.arange(n) / n)
+    h = torch.tensor(rows, device=cuda)
+    bufs = [torch.full((nr * n + 16,), -7.5, dtype=torch.float64, device=cuda) for _ in range(2)]
+    p = lambda t, k=0: ctypes.c_void_p(t.data_ptr() + 8 * k)  # noqa: E731
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert pkg.lib().ceemdan_envelopes_f64(nr, n, p(h), p(bufs[0], shift), p(bufs[1], shift), None,
+                                           stream) == 0
+    for e, b in enumerate(bufs):
+        b = b.cpu().numpy()
+        got = b[shift:shift + nr * n].reshape(nr, n)
+        for r in range(nr):
+            assert np.array_equal(got[r], orc.envelope(rows[r], e, solver=1, chunk=16))
+        assert (b[:shift] == -7.5).all() and (b[shift + nr * n:] == -7.5).all()
