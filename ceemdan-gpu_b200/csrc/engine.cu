@@ -1065,7 +1065,7 @@ ceemdan_status ceemdan_envelopes_f64(size_t nr, size_t n, const double* d_h, dou
     Workspace ws(st);
     SiftEngine eng;
     CKS(eng.init(ws, (int)nr, (int)n, o));
-    CKS(eng.reset_carries(st));
+    CKS(eng.reset_carries(st, false));
     CK(cudaMemsetAsync(eng.a.mark, 0xff, sizeof(int) * nr, st));
     CKS(eng.rows_in(eng.h[0], d_h, nr, st));
     eng.a.dbg_upper = d_upper;
@@ -1094,15 +1094,14 @@ ceemdan_status ceemdan_extrema_f64(size_t nr, size_t n, const double* d_h, int32
     Workspace ws(st);
     SiftEngine eng;
     CKS(eng.init(ws, (int)nr, (int)n, o));
-    CKS(eng.reset_carries(st));
+    CKS(eng.reset_carries(st, false));
     CK(cudaMemsetAsync(eng.a.mark, 0xff, sizeof(int) * nr, st));
     CKS(eng.rows_in(eng.h[0], d_h, nr, st));
     SiftArgs& a = eng.a;
-    const dim3 grid_tiles((unsigned)eng.ntiles, (unsigned)nr);
-    k_tile_knots<<<eng.knots_grid, kTileThreads, tile_knots_smem(), st>>>(a);
-    k_spline_solve<<<eng.solve_grid, kSolveThreads, kSolveSmem, st>>>(a);
-    k_gather_knots<<<grid_tiles, kThreads, 0, st>>>(a, 0, d_kx_max, d_ky_max);
-    k_gather_knots<<<grid_tiles, kThreads, 0, st>>>(a, 1, d_kx_min, d_ky_min);
+    const dim3 grid_tiles((unsigned)eng.ntiles, (unsigned)nr, 2);
+    k_tile_knots<true><<<eng.knots_grid, kTileThreads, tile_knots_smem(), st>>>(a);
+    k_spline_solve<true><<<eng.solve_grid, kSolveThreads, 0, st>>>(a);
+    k_gather_knots<<<grid_tiles, kThreads, 0, st>>>(a, d_kx_max, d_ky_max, d_kx_min, d_ky_min);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(d_counts, a.kcount, 2 * nr * sizeof(int), cudaMemcpyDeviceToDevice, st));
     CK(cudaMemcpyAsync(eng.hstate, eng.state, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -42,10 +42,13 @@ constexpr int kThreads = 256;
 // The tile kernels run as persistent CTAs over the active tiles.  kEnv: the envelopes of one
 // iteration to dbg_upper / dbg_lower, no update and no stop test.  kDense: shared memory for
 // kSiftDense entries (three CTAs per SM) or kSiftSparse (five).
+// kExtrema: the knots alone.
+template <bool kExtrema>
 __global__ void k_tile_knots(const __grid_constant__ SiftArgs a);
 // kSplit: of the rows of its class only.
 template <bool kDense, bool kSplit, bool kEnv>
 __global__ void k_tile_sift(const __grid_constant__ SiftArgs a);
+template <bool kExtrema>
 __global__ void k_spline_solve(const __grid_constant__ SiftArgs a);
 
 // the on-chip stage kernel, in one of its three forms
@@ -312,7 +315,7 @@ struct SiftEngine {
             group = rn >= (size_t)(1 << 22) ? 4 : (rn >= (size_t)(1 << 18) ? 8 : 32);
         }
         a.solve_wcap = (kSolveSmem - kSolveStage) / (int)sizeof(double);
-        CK(cudaFuncSetAttribute(k_spline_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        CK(cudaFuncSetAttribute(k_spline_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 kSolveSmem));
         for (auto k : {k_tile_sift<false, true, false>, k_tile_sift<false, true, true>})
             CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -321,15 +324,16 @@ struct SiftEngine {
                        k_tile_sift<true, true, false>, k_tile_sift<true, true, true>})
             CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)tile_sift_smem(true)));
-        CK(cudaFuncSetAttribute(k_tile_knots, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)tile_knots_smem()));
+        for (auto k : {k_tile_knots<false>, k_tile_knots<true>})
+            CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)tile_knots_smem()));
         // persistent CTAs, as many as the GPU holds at once
         auto grid = [&](const void* k, size_t smem) {
             int per = 0;
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, kTileThreads, smem);
             return std::max(1, (int)std::min<size_t>(T, (size_t)std::max(1, per) * sm_count()));
         };
-        knots_grid = grid((const void*)k_tile_knots, tile_knots_smem());
+        knots_grid = grid((const void*)k_tile_knots<false>, tile_knots_smem());
         dense_grid = grid((const void*)k_tile_sift<true, true, false>, tile_sift_smem(true));
         sift_grid = grid((const void*)k_tile_sift<false, true, false>, tile_sift_smem(false));
         CK(cudaGetLastError());
@@ -401,11 +405,12 @@ struct SiftEngine {
     }
 
     // Zero the whole-call carries: mean envelope and sifting fraction accumulator, and the
-    // channels' states.
-    ceemdan_status reset_carries(cudaStream_t st) {
+    // channels' states.  mean false: without the mean envelope, for the stage-level entries that
+    // neither read nor write it.
+    ceemdan_status reset_carries(cudaStream_t st, bool mean = true) {
         const Chan& last = hchan.back();
         const size_t S = (size_t)last.samp0 + (size_t)last.nr * row_ld(last.n);
-        CK(cudaMemsetAsync(a.menv, 0, sizeof(double) * S, st));
+        if (mean) CK(cudaMemsetAsync(a.menv, 0, sizeof(double) * S, st));
         CK(cudaMemsetAsync(a.frac, 0, sizeof(double) * a.nrows, st));
         CK(cudaMemsetAsync(a.cnt, 0, sizeof(unsigned) * a.nrows, st));
         CK(cudaMemsetAsync(a.any, 0, sizeof(int) * a.nrows, st));
@@ -444,10 +449,10 @@ struct SiftEngine {
             ++g_launches;
         }
         mark_ev(0, 0);
-        k_tile_knots<<<knots_grid, kTileThreads, tile_knots_smem(), st>>>(a);
+        k_tile_knots<false><<<knots_grid, kTileThreads, tile_knots_smem(), st>>>(a);
         mark_ev(0, 1);
         mark_ev(1, 0);
-        k_spline_solve<<<solve_grid, kSolveThreads, kSolveSmem, st>>>(a);
+        k_spline_solve<false><<<solve_grid, kSolveThreads, kSolveSmem, st>>>(a);
         mark_ev(1, 1);
         if (slot) {
             const size_t pieces = tape->L.off_kc / 16;  // 16-byte pieces of the bitmaps

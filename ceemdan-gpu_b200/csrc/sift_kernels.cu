@@ -330,7 +330,11 @@ size_t tile_knots_smem() { return sizeof(KnotSmem); }
 // to a lane took four times the instructions.  B200, N=244032 NR=100: 103 us at K/N = 0.18, 61 us
 // at 0.001 (3.2 TB/s of its 8 N bytes), where the separate extrema, end-rule and chunk kernels took
 // 178 us on average.  Six CTAs per SM instead of five change nothing.
+//
+// kExtrema: the knots alone (bitmaps, counts, headers' knots, end values), their values in place of
+// the slopes in the lists, for the extrema entry.
 // =======================================================================================
+template <bool kExtrema>
 __global__ void __launch_bounds__(kTileThreads, 5)
 k_tile_knots(const __grid_constant__ SiftArgs a) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -468,14 +472,17 @@ k_tile_knots(const __grid_constant__ SiftArgs a) {
             if (last && i == c - 1) v = S.yend[e][1];
             return v;
         };
+        // (the knots' own values where the slopes go)
+        for (int i = tid % kHalf, p = kq(i); i < c && kExtrema; i += kHalf, p += kq(kHalf))
+            S.s[e][p] = staged(S.stage, x[p]);
         // 16 knots on, the padded positions advance by 17; the segments at the row's ends take
         // the end values
-        for (int i = tid % kHalf, p0 = kq(i), p1 = kq(i + 1); i + 1 < c;
+        for (int i = tid % kHalf, p0 = kq(i), p1 = kq(i + 1); i + 1 < c && !kExtrema;
              i += kHalf, p0 += kq(kHalf), p1 += kq(kHalf)) {
             const int x0 = x[p0], x1 = x[p1];
             S.s[e][p0] = div_int(staged(S.stage, x1) - staged(S.stage, x0), (double)(x1 - x0));
         }
-        for (int side = 0; side < 2; ++side) {
+        for (int side = 0; side < 2 && !kExtrema; ++side) {
             const int i = side == 0 ? 0 : c - 2;  // written by the same thread above
             if ((side == 0 ? first : last) && c > 1 && tid % kHalf == i % kHalf)
                 S.s[e][kq(i)] = div_int(y(i + 1, kq(i + 1)) - y(i, kq(i)),
@@ -513,6 +520,7 @@ k_tile_knots(const __grid_constant__ SiftArgs a) {
         for (int i = tid & 63; i < (n + 7) >> 3; i += kTileThreads / 2) xo[i] = xs[i];
         for (int i = tid & 63; i < (n + 1) >> 1; i += kTileThreads / 2) so[i] = ss[i];
     }
+    if (kExtrema) continue;  // (the next tile's first barrier separates these reads, too)
     int e, k;
     const bool act = sweep_lane(tid, tile_seps(c0), tile_seps(c1), e, k);
     const int c = e ? c1 : c0;
@@ -555,37 +563,39 @@ k_tile_knots(const __grid_constant__ SiftArgs a) {
     // (the next tile's first barrier separates these reads of s, x and ex from its writes)
     }
 }
+template __global__ void k_tile_knots<false>(const __grid_constant__ SiftArgs a);
+template __global__ void k_tile_knots<true>(const __grid_constant__ SiftArgs a);
 
-// Compacted copy of the knots of envelope e (stage-level entry point, one channel): row r's
-// knots to kx/ky[r*n + i], from the bitmaps, the samples and the end values.
+// Compacted copy of the knots (stage-level entry point, one channel; blockIdx.z: envelope): row r's
+// knots to kx/ky[r*n + i], from k_tile_knots<true>'s lists and the end values.  (From the bitmaps and
+// the samples it took 97 us at N=244032 NR=50, from the lists 62, and k_tile_knots 50 instead of
+// 35.)
 __global__ void __launch_bounds__(kThreads)
-k_gather_knots(SiftArgs a, int e, int32_t* kx, double* ky) {
-    __shared__ int2 s_wo[kWords];
-    __shared__ int s_before;
-    const int tile = blockIdx.x;
+k_gather_knots(const __grid_constant__ SiftArgs a, int32_t* kx_max, double* ky_max,
+               int32_t* kx_min, double* ky_min) {
+    __shared__ int s_before[kThreads / 32];
+    const int e = blockIdx.z, tile = blockIdx.x, tid = threadIdx.x;
     const Geo q = geo(a, 0, blockIdx.y);
-    if (threadIdx.x == 0) s_before = 0;
+    int before = 0;  // knots of the tiles before this one
+    for (int t = tid; t < tile; t += kThreads) before += a.tile_cnt[tix(a, e, q, t)];
+    before = __reduce_add_sync(0xffffffffu, before);
+    if ((tid & 31) == 0) s_before[tid >> 5] = before;
     __syncthreads();
-    int before = 0;
-    for (int t = threadIdx.x; t < tile; t += kThreads) before += a.tile_cnt[tix(a, e, q, t)];
-    if (before) atomicAdd(&s_before, before);
-    const unsigned* bm = a.bitmap + tix(a, e, q, tile) * kWords;
-    if (threadIdx.x < kWords) {
-        int w = 0;
-        for (int i = 0; i < (int)threadIdx.x; ++i) w += __popc(bm[i]);
-        s_wo[threadIdx.x] = make_int2((int)bm[threadIdx.x], w);
-    }
-    __syncthreads();
-    const int sp = spline_id(a, e, q);
-    const double* h = a.h[a.par[q.g]] + q.base;
-    for (int j = threadIdx.x; j < kTileSamples; j += kThreads) {
-        const int2 wo = s_wo[j >> 5];
-        if (!((unsigned)wo.x >> (j & 31) & 1u)) continue;
-        const size_t o =
-            (size_t)q.r * q.n + s_before + wo.y + __popc((unsigned)wo.x & ((1u << (j & 31)) - 1u));
-        const int s = tile * kTileSamples + j;
-        kx[o] = s;
-        ky[o] = s == 0 ? a.yend[2 * sp] : (s == q.n - 1 ? a.yend[2 * sp + 1] : h[s]);
+    before = 0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) before += s_before[w];
+    const int c = a.tile_cnt[tix(a, e, q, tile)], n0 = tile * kTileSamples;
+    const short* x = a.list_x + tix(a, e, q, tile) * kListSlots;
+    const double* y = a.list_s + tix(a, e, q, tile) * kListSlots;
+    const double* yend = a.yend + 2 * spline_id(a, e, q);
+    const size_t o = (size_t)q.r * q.n + before;
+    int32_t* const kx = (e ? kx_min : kx_max) + o;
+    double* const ky = (e ? ky_min : ky_max) + o;
+#pragma unroll 4
+    for (int m = tid; m < c; m += kThreads) {
+        const int s = n0 + x[kq(m)];
+        kx[m] = s;
+        ky[m] = s == 0 ? yend[0] : (s == q.n - 1 ? yend[1] : y[kq(m)]);
     }
 }
 
@@ -1170,7 +1180,8 @@ namespace {
 // The end rule of a spline whose first (side 0) or last (side 1) tile holds fewer than six
 // knots: the three end knots come from the tiles' headers, the tile's chunk is eliminated again
 // with the new end value.  ne: the tiles with knots, in order (NE of them); hd: the spline's
-// headers; cnt: the tiles' knot counts.
+// headers; cnt: the tiles' knot counts.  kExtrema: the end value alone.
+template <bool kExtrema>
 __device__ __noinline__ void end_rule_sparse(const SiftArgs& a, int e, int sp, int side,
                                              const int* ne, int NE, const int* cnt, TileHdr* hd) {
     const int te = ne[side == 0 ? 0 : NE - 1];
@@ -1205,6 +1216,7 @@ __device__ __noinline__ void end_rule_sparse(const SiftArgs& a, int e, int sp, i
     const double v = side == 0 ? boundary_left(e, ex[0], ex[1], ex[2], ey[0], ey[1], ey[2])
                                : boundary_right(e, ex[2], ex[1], ex[0], ey[2], ey[1], ey[0]);
     a.yend[2 * sp + side] = v;
+    if (kExtrema) return;
     if (side == 0) {
         h0.y0 = v;
         if (c == 1) h0.yb = v;
@@ -1241,7 +1253,11 @@ __device__ __noinline__ void end_rule_sparse(const SiftArgs& a, int e, int sp, i
 // rows are staged once when they fit a pass (2048 rows).  Latency bound (a chain of short sweeps
 // per CTA): two CTAs per SM with the level-3 system in shared memory.  B200, N=244032 NR=100: 23.5
 // us at K/N = 0.18, 55 us for white noise; the two kernels before it took 42 us on average.
+//
+// kExtrema: the counts and the end rule alone, for the extrema entry (no shared memory but the
+// tables).
 // =======================================================================================
+template <bool kExtrema>
 __global__ void __launch_bounds__(kSolveThreads, 2)
 k_spline_solve(const __grid_constant__ SiftArgs a) {
     extern __shared__ __align__(16) unsigned char dyn_smem[];
@@ -1322,7 +1338,7 @@ k_spline_solve(const __grid_constant__ SiftArgs a) {
         soff[ntiles] = P;
         a.kcount[sp] = K;
         a.cmax[sp] = cm;
-        if (a.sift_split) {  // the spline that comes second knows both counts
+        if (a.sift_split && !kExtrema) {  // the spline that comes second knows both counts
             const unsigned other = atomicExch(&a.cls_wait[q.g], (unsigned)cm + 1u);
             if (other != 0u) {
                 a.cls_wait[q.g] = 0u;
@@ -1333,16 +1349,17 @@ k_spline_solve(const __grid_constant__ SiftArgs a) {
     }
     __syncthreads();
     const bool one = P <= kSolvePass;
-    if (one) stage_rows<true>(st, rows, soff, ntiles, 0);
+    if (one && !kExtrema) stage_rows<true>(st, rows, soff, ntiles, 0);
     // the first tile holds sample 0 and the last one sample n-1, so both have knots
     if (K > 5) {
         const bool l = cnt[0] < 6, r = cnt[ntiles - 1] < 6;
         if (l || r) {
-            if (tid == 0 && l) end_rule_sparse(a, e, sp, 0, ne, NE, cnt, hd);
-            if (tid == 32 && r) end_rule_sparse(a, e, sp, 1, ne, NE, cnt, hd);
+            if (tid == 0 && l) end_rule_sparse<kExtrema>(a, e, sp, 0, ne, NE, cnt, hd);
+            if (tid == 32 && r) end_rule_sparse<kExtrema>(a, e, sp, 1, ne, NE, cnt, hd);
             __syncthreads();
         }
     }
+    if (kExtrema) return;
     if (a.bflags && tid == 0) {
         // a replaced end value differs from the sample in its bits (t > y or t < y)
         const double* h = a.h[a.par[q.g]] + q.base;
@@ -1412,6 +1429,8 @@ k_spline_solve(const __grid_constant__ SiftArgs a) {
         ed[t] = w;
     }
 }
+template __global__ void k_spline_solve<false>(const __grid_constant__ SiftArgs a);
+template __global__ void k_spline_solve<true>(const __grid_constant__ SiftArgs a);
 
 // =======================================================================================
 // k_tile_sift: persistent CTAs over the tiles: the spline values of the tile's knots (chunk
