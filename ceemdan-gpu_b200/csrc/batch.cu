@@ -41,14 +41,12 @@ struct BatchChannel {
 // transition kernels of one loop iteration
 constexpr int kTransKernels = 4;
 
-// Device bytes of one channel in a wave (sift state, noise modes, knots, records).
+// Device bytes of one channel in a wave: its part of the engine's arrays, and run_wave's own (the
+// planes W, E, H0 and MODE, the signal and the running mean, the statistics and counts).
 size_t channel_bytes(size_t n, size_t nr, size_t nimf) {
-    const size_t rn = nr * n;
-    const size_t tiles = nr * ((n + kTileSamples - 1) / kTileSamples);
-    const size_t planes = (nimf + 6) * rn * 8;          // h x2, menv, W, H0, MODE, E
-    const size_t knots = tiles * 1028 * (2 * 12 + 2 * 32);  // (a bound of the tiles' workspaces)
-    const size_t rec = nr * (n / 2 / kChunk + 64) * 8 * 2 * 17;  // chunk records, X, workspace
-    return planes + knots + rec + tiles * 1024;
+    const size_t plane = nr * (size_t)row_ld((int)n) + 32;
+    return SiftEngine::bytes_of(n, nr) +
+           sizeof(double) * ((nimf + 3) * plane + 2 * (n + 32) + 2 * nr) + 8 * nimf + 8192;
 }
 
 struct Wave {

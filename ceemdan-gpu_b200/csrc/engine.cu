@@ -572,18 +572,18 @@ int checkpoint_block(const ceemdan_tape& T) {
     const size_t slots = ((size_t)jmax + kTapeBlockSlots - 1) / kTapeBlockSlots * kTapeBlockSlots;
     const size_t tape_row = (size_t)2 * T.L.ntiles * (kTileSamples / 32) * sizeof(unsigned) + 16;
     // the reverse work arrays (eb; per spline knots, four segment sums, yb, the system, z, its
-    // workspace: a bound of 128 bytes per sample) and the rows of the two re-run engines (h,
-    // mean envelope, modes, knots, records, reduced workspaces: 160 bytes per sample each)
-    const size_t per_row = slots * tape_row + 128 * n + 2 * 160 * n;
+    // workspace: a bound of 128 bytes per sample), and a row of a re-run engine with its mode and,
+    // on chip, its upper envelope
+    const size_t row = slots * tape_row + 128 * n;
+    const size_t engine = SiftEngine::bytes_of(n, 1) + 2 * sizeof(double) * (n + 4);
     const size_t fixed = 2 * T.nr * n * sizeof(double) + ((size_t)64 << 20);  // gh, gm, margin
     const size_t usable = (size_t)(0.8 * (double)free_b);
-    const int most = usable <= fixed ? 1
-                                     : (int)std::max<size_t>(
-                                           1, std::min<size_t>((size_t)nr,
-                                                               (usable - fixed) / per_row));
-    // blocks of nearly equal size
-    const int blocks = (nr + most - 1) / most;
-    return (nr + blocks - 1) / blocks;
+    // the fewest blocks of nearly equal size (a shorter last one has an engine of its own)
+    for (int blocks = 1; blocks < nr; ++blocks) {
+        const size_t nb = (size_t)(nr + blocks - 1) / blocks, rem = (size_t)nr % nb;
+        if (fixed + nb * row + (nb + rem) * engine <= usable) return (int)nb;
+    }
+    return 1;
 }
 
 // Reverse pass (vector-Jacobian product) of a taped decomposition: gy = (d imfs/d y)^T g with

@@ -66,14 +66,22 @@ int grid_for(size_t count);
 ceemdan_status generate_noise(double* w, size_t count, uint64_t seed, cudaStream_t st);
 
 // Device allocations owned by one decomposition (or one stage-level call), stream-ordered on
-// the call's stream: freed after the work queued on it.
+// the call's stream: freed after the work queued on it.  A counting workspace allocates nothing
+// and only adds up what the pool would hand out (its granule is 512 bytes).
 struct Workspace {
     cudaStream_t st;
     std::vector<void*> blocks;
-    explicit Workspace(cudaStream_t s) : st(s) {}
+    bool counting = false;
+    size_t total = 0;
+    explicit Workspace(cudaStream_t s, bool count = false) : st(s), counting(count) {}
     Workspace(const Workspace&) = delete;
     Workspace& operator=(const Workspace&) = delete;
     ceemdan_status alloc(void** p, size_t bytes) {
+        total += (std::max<size_t>(bytes, 1) + 511) & ~(size_t)511;
+        if (counting) {
+            *p = nullptr;
+            return CEEMDAN_OK;
+        }
         const ceemdan_status s = pool_alloc(p, bytes, st);
         if (s == CEEMDAN_OK) blocks.push_back(*p);
         return s;
@@ -188,7 +196,9 @@ struct SiftEngine {
     int* state = nullptr;     // channel 0's (done, iter, err, cap) = the first words of cs[0]
     int* hstate = nullptr;    // pinned host mirror: two slots of (done, iter, err, cap)
     std::vector<Chan> hchan;  // host copy of the channel table
+    Chan* dchan = nullptr;
     int nr = 0, n = 0, ntiles = 0;  // channel 0
+    size_t samples = 0;             // of one plane (all channels' row blocks)
     cudaEvent_t group_ev[2] = {nullptr, nullptr};
     int group = 4;
     // persistent grids of the tile kernels, one CTA per spline
@@ -203,8 +213,23 @@ struct SiftEngine {
         return init(ws, std::vector<ChanSpec>{{n_, nr_}}, o);
     }
 
+    // Device bytes of an engine for nr rows of n samples (its arrays, without enable_small's).
+    static size_t bytes_of(size_t n_, size_t nr_) {
+        SiftEngine e;
+        Workspace count(nullptr, true);
+        if (e.layout({{(int)n_, (int)nr_}}) == CEEMDAN_OK) (void)e.arrays(count);
+        return count.total;
+    }
+
     ceemdan_status init(Workspace& ws, const std::vector<ChanSpec>& chans,
                         const ceemdan_options& o) {
+        CKS(layout(chans));
+        CKS(arrays(ws));
+        return start(ws, o);
+    }
+
+    // The rows' places in the arrays.
+    ceemdan_status layout(const std::vector<ChanSpec>& chans) {
         const int nchan = (int)chans.size();
         hchan.resize(chans.size());
         long long rows = 0, tiles = 0, samp = 0, rec = 0, red = 0;
@@ -246,13 +271,12 @@ struct SiftEngine {
         a.ntot = (int)tiles;
         a.rec_total = rec;
         a.red_total = red;
-        a.spin_limit = o.spin_limit > 0 ? o.spin_limit : (1 << 22);
-        a.sd = o.sd;
-        a.sd2 = o.sd2;
-        sx_bounds(o.sd, &a.sd_hi, &a.sd_lo);
-        sx_bounds(o.sd2, &a.sd2_hi, &a.sd2_lo);
-        a.tol = o.tol;
-        const size_t R = (size_t)rows, T = (size_t)tiles, S = (size_t)samp;
+        samples = (size_t)samp;
+        return CEEMDAN_OK;
+    }
+
+    ceemdan_status arrays(Workspace& ws) {
+        const size_t R = (size_t)a.nrows, T = (size_t)a.ntot, S = samples;
         CKS(ws.alloc_n(&h[0], S));
         CKS(ws.alloc_n(&h[1], S));
         a.h[0] = h[0];
@@ -267,16 +291,12 @@ struct SiftEngine {
         CKS(ws.alloc_n(&a.par, R));
         CKS(ws.alloc_n(&a.acc, R));
         CKS(ws.alloc_n(&a.acc_wide, 2 * R));
-        // counts of rows of up to 2^17 - 1 tiles fit one word (CEEMDAN_SPLIT_COUNT=1: never)
-        a.count_bits = 17;
-        if (const char* e = std::getenv("CEEMDAN_SPLIT_COUNT"))
-            if (e[0] == '1') a.count_bits = 0;
         CKS(ws.alloc_n(&a.cmax, 2 * R));
         CKS(ws.alloc_n(&a.cls_count, 2));
         CKS(ws.alloc_n(&a.cls_row, 2 * R));
         CKS(ws.alloc_n(&a.cls_wait, R));
         CKS(ws.alloc_n(&a.tile_cnt, 2 * T));
-        CKS(ws.alloc_n(&a.plan, 2 * (size_t)nchan + 2));
+        CKS(ws.alloc_n(&a.plan, 2 * (size_t)a.nchan + 2));
         CKS(ws.alloc_n(&a.bitmap, 2 * T * (kTileSamples / 32)));
         CKS(ws.alloc_n(&a.scan, T));
         CKS(ws.alloc_n(&a.list_x, 2 * T * kListSlots));
@@ -291,15 +311,30 @@ struct SiftEngine {
         CKS(ws.alloc_n(&a.end_x, 2 * R * 2 * kEndKnots));
         CKS(ws.alloc_n(&a.end_y, 2 * R * 2 * kEndKnots));
         // (k_tile_sift copies a whole tile's slots from a tile's first separator on)
-        CKS(ws.alloc_n(&a.xsep, 2 * (size_t)rec + kRowSlots));
-        CKS(ws.alloc_n(&a.red, 2 * (size_t)red));
-        Chan* dchan = nullptr;
-        CKS(ws.alloc_n(&dchan, (size_t)nchan));
-        CK(cudaMemcpyAsync(dchan, hchan.data(), sizeof(Chan) * nchan, cudaMemcpyHostToDevice,
-                           ws.st));
+        CKS(ws.alloc_n(&a.xsep, 2 * (size_t)a.rec_total + kRowSlots));
+        CKS(ws.alloc_n(&a.red, 2 * (size_t)a.red_total));
+        CKS(ws.alloc_n(&dchan, (size_t)a.nchan));
         a.chan = dchan;
-        CKS(ws.alloc_n(&cs, (size_t)nchan));
+        CKS(ws.alloc_n(&cs, (size_t)a.nchan));
         a.cs = cs;
+        return CEEMDAN_OK;
+    }
+
+    // The options, the channel table and the launch shapes.
+    ceemdan_status start(Workspace& ws, const ceemdan_options& o) {
+        const size_t R = (size_t)a.nrows, T = (size_t)a.ntot;
+        a.spin_limit = o.spin_limit > 0 ? o.spin_limit : (1 << 22);
+        a.sd = o.sd;
+        a.sd2 = o.sd2;
+        sx_bounds(o.sd, &a.sd_hi, &a.sd_lo);
+        sx_bounds(o.sd2, &a.sd2_hi, &a.sd2_lo);
+        a.tol = o.tol;
+        // counts of rows of up to 2^17 - 1 tiles fit one word (CEEMDAN_SPLIT_COUNT=1: never)
+        a.count_bits = 17;
+        if (const char* e = std::getenv("CEEMDAN_SPLIT_COUNT"))
+            if (e[0] == '1') a.count_bits = 0;
+        CK(cudaMemcpyAsync(dchan, hchan.data(), sizeof(Chan) * a.nchan, cudaMemcpyHostToDevice,
+                           ws.st));
         state = reinterpret_cast<int*>(cs);
         hstate = pinned_state();
         if (!hstate) {
@@ -308,7 +343,7 @@ struct SiftEngine {
         }
         CK(cudaEventCreateWithFlags(&group_ev[0], cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&group_ev[1], cudaEventDisableTiming));
-        const size_t rn = (size_t)samp;
+        const size_t rn = samples;
         if (o.group > 0) {
             group = o.group;
         } else {
