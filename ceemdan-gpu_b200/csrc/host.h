@@ -50,6 +50,8 @@ template <bool kDense, bool kSplit, bool kEnv>
 __global__ void k_tile_sift(const __grid_constant__ SiftArgs a);
 template <bool kExtrema>
 __global__ void k_spline_solve(const __grid_constant__ SiftArgs a);
+__global__ void k_gather_knots(const __grid_constant__ SiftArgs a, int32_t* kx_max,
+                               double* ky_max, int32_t* kx_min, double* ky_min);
 
 // the on-chip stage kernel, in one of its three forms
 template <int kMode>

@@ -230,8 +230,6 @@ struct SmallArgs {
 };
 constexpr int kTapeBlockSlots = 32;  // tape slots per allocation block
 
-__global__ void k_gather_knots(const __grid_constant__ SiftArgs a, int32_t* kx_max,
-                               double* ky_max, int32_t* kx_min, double* ky_min);
 // Shared-memory entries of k_tile_sift.  Dense: both envelopes of a tile of up to about 1780 knots
 // at once (white noise has 1370, sifted a thousand times 1490), one after the other above.
 // Sparse: up to about 660 knots a tile, the stages after the second of white noise.
