@@ -58,7 +58,8 @@ CEEMDAN_HD double boundary_right(int kind, int32_t xa, int32_t xb, int32_t xL,
 // Correctly rounded a / d from y = RN(1/d) (Markstein's theorem: q0 = RN(a*y) is within one
 // ulp of a/d, r = a - d*q0 is exact with one fma, RN(q0 + r*y) = RN(a/d)).  Three FP64 ops in
 // place of a division; zero, tiny and non-finite operands take the division (keeps the sign of
-// zero and stays clear of underflow, where the theorem's assumptions fail).
+// zero and stays clear of underflow, where the theorem's assumptions fail).  The kernels' form of it
+// is rcp_fast (spline_device.cuh); this one is what the host checks compare with the division.
 CEEMDAN_HD double div_plain(double a, double d) { return a / d; }
 
 CEEMDAN_HD double div_rcp(double a, double d, double y) {
@@ -157,15 +158,6 @@ CEEMDAN_HD Row reduced_row(const Row& s, double gb, double ab, double bb,
     o.u = s.u * ba;
     o.r = fma(-s.u, ga, fma(-s.l, gb, s.r));
     return o;
-}
-
-// Spline segment coefficients (spline_coefficients): b and d of segment [x0, x1].
-CEEMDAN_HD void seg_coeffs(int32_t x0, int32_t x1, double y0, double y1,
-                                           double c0, double c1, double& b, double& d) {
-    const double h = (double)(x1 - x0);
-    const double q = fma(2.0, c0, c1);
-    b = (y1 - y0) / h - (h * q) / 3.0;
-    d = (c1 - c0) / (3.0 * h);
 }
 
 // Horner evaluation a + t(b + t(c + t d)) as the reference's contracted form.

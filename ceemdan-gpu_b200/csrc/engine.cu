@@ -618,7 +618,7 @@ ceemdan_status backward_impl(const ceemdan_tape& T, const double* g, double* gy,
     CKS(ws.alloc_n(&sys, 4 * pc));
     CKS(ws.alloc_n(&z, pc));
     CKS(ws.alloc_n(&wsp, (size_t)nsp * ws_stride));
-    // the transposed spline solves: one CTA per spline (cta_tridiag), or for long splines the
+    // the transposed spline solves: one CTA per spline (k_adj_solve), or for long splines the
     // same solve level by level over the whole grid (psolve_launch); CEEMDAN_ADJ_SOLVE=cta or
     // grid chooses
     bool grid_solve = cap > 16384;

@@ -325,7 +325,6 @@ struct SiftEngine {
     // The options, the channel table and the launch shapes.
     ceemdan_status start(Workspace& ws, const ceemdan_options& o) {
         const size_t R = (size_t)a.nrows, T = (size_t)a.ntot;
-        a.spin_limit = o.spin_limit > 0 ? o.spin_limit : (1 << 22);
         a.sd = o.sd;
         a.sd2 = o.sd2;
         sx_bounds(o.sd, &a.sd_hi, &a.sd_lo);
@@ -536,11 +535,8 @@ struct SiftEngine {
         cudaLaunchConfig_t c{};
         c.gridDim = dim3((unsigned)(mode == kSmallPair ? 2 * nr : nr));
         c.blockDim = dim3(kSmallThreads);
-        // the CTAs are latency-bound: when the launch has at most one CTA per SM, ask for more
-        // than half an SM's shared memory so that no two of them share an SM
+        // (one CTA to an SM whatever its shared memory: 512 threads of more than 64 registers)
         c.dynamicSmemBytes = small_sift_smem(n, mode);
-        if ((int)c.gridDim.x <= sm_count())
-            c.dynamicSmemBytes = std::max(c.dynamicSmemBytes, (size_t)kSmallSpreadSmem);
         c.stream = st;
         at[0].id = cudaLaunchAttributeCooperative;
         at[0].val.cooperative = 1;

@@ -20,11 +20,12 @@ __host__ __device__ inline int row_ld(int n) { return (n + 3) & ~3; }
 // owns rows row0 .. row0+nr-1), and so are the 2048-sample tiles of the rows (row g of channel
 // c owns tiles tile0 + (g-row0)*ntiles + t).  Per-spline arrays are indexed by the spline
 // se = e*nrows + g (e = 0 maxima, 1 minima).  With one channel every array has the layout of a
-// single decomposition: row r at r*n, tile t of row r at r*ntiles + t.
+// single decomposition: row r at r*row_ld(n) of the engine's own planes (at r*n of the caller's),
+// tile t of row r at r*ntiles + t.
 struct Chan {
     int n, ntiles, nr, row0;
     int cap;               // knot capacity of a spline: n/2 + 2
-    int rec_stride;        // per-spline stride of chunk records / separator values
+    int rec_stride;        // per-spline stride of the separator values
     int tile0;             // first global tile
     int pad;
     long long samp0;       // first sample of row row0 in the row-major sample arrays
@@ -36,7 +37,7 @@ struct Chan {
 // iterations (done, iter, err, cap).
 struct ChanState {
     int done;              // the current stage has finished: the sift kernels skip the channel
-    int iter;              // executed iterations of the current stage (h[iter&1] is current)
+    int iter;              // executed iterations of the current stage
     int err;               // device error word (0 = none)
     int cap;               // sift cap of the current stage
     int stage;             // batched engine: current stage (2*(num_imfs-1) = all done)
@@ -90,7 +91,6 @@ struct SiftArgs {
     int solve_wcap;        // doubles of k_spline_solve's shared memory after the staged rows
     long long rec_total;   // record slots of one envelope (sum of the rows' rec_stride)
     long long red_total;   // reduced-workspace doubles of one envelope
-    int spin_limit;        // cap of in-kernel waits (reserved: no kernel waits today)
     double sd, sd2, tol;
     // margins of the division-free sx tests (sx_bounds): sx > t is true when |U+L| > |U-L|*t_hi
     // and false when |U+L| < |U-L|*t_lo, for |U-L| in (2^-800, 2^800)
@@ -112,7 +112,7 @@ struct SiftArgs {
     double* frac;          // sifting fraction accumulator, persists
     unsigned* cnt;         // [nrows] counts of a finished row's last iteration, for its repetition
     int* any;
-    // a row's counts of the current iteration (count_tile; back to 0 at its end): [nrows], or for
+    // a row's counts of the current iteration (count_tiles; back to 0 at its end): [nrows], or for
     // rows whose tile count has more than count_bits bits [nrows][2]
     unsigned long long *acc, *acc_wide;
     int count_bits;
@@ -182,7 +182,6 @@ struct BatchArgs {
 constexpr int kSmallMaxN = 8192;       // longest row the on-chip path takes
 constexpr int kSmallThreads = 512;
 constexpr int kSmallPair = 0, kSmallDual = 1, kSmallSingle = 2;
-constexpr int kSmallSpreadSmem = 120 * 1024;  // dynamic shared memory that fits one CTA per SM
 // samples of a row that the first CTA of a pair combines
 __host__ __device__ inline int small_half(int n) {
     const int h = ((n + 1) / 2 + 31) & ~31;
@@ -255,10 +254,8 @@ __global__ void k_tridiag_batched(int n, const double* l, const double* m, const
                                   const double* r, double* x, double* sys, double* ws,
                                   size_t ws_stride);
 // In-CTA canonical partitioned solve (sift_kernels.cu): system in 4 planes of `plane` doubles
-// (l, m, u, r) at sys, solution to x, workspace ws of >= 0.75*n + 16 doubles; every thread of
-// the CTA calls it.
-__device__ void cta_tridiag(int n, const double* sys, int plane, double* x, double* ws);
-// the same solve of a spline system (pivots in pivot_inv's range)
+// (l, m, u, r) at sys, solution to x, workspace ws of >= 0.75*n + 16 doubles, of a spline system
+// (pivots in pivot_inv's range); every thread of the CTA calls it.
 __device__ void cta_spline_tridiag(int n, const double* sys, int plane, double* x, double* ws);
 // cta_spline_tridiag's solve for nsys systems at once, one level per launch (sift_kernels.cu)
 cudaError_t psolve_launch(int nsys, int max_rows, const int* nrows, const double* sys, int plane,

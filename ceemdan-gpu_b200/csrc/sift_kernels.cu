@@ -121,8 +121,9 @@ __device__ __forceinline__ Geo spline_geo(const SiftArgs& a, int v, int ra, int&
     return row_geo(a, v - e * ra);
 }
 
-// Index of tile t of row q's spline e in the per-tile arrays (tile_cnt, bitmap words / 64,
-// nbr pairs / 2) and in the per-tile-plus-one arrays (tile_off, sep_off).
+// Index of tile t of row q's spline e in the per-tile arrays (tile_cnt, bitmap words / 64, lists,
+// headers, edges, separator rows), and of the row's first tile in the arrays with one entry more a
+// row (sep_off, tile_rank, tile_list).
 __device__ __forceinline__ size_t tix(const SiftArgs& a, int e, const Geo& q, int t) {
     return (size_t)e * a.ntot + (size_t)(q.tile0 + t);
 }
@@ -619,8 +620,8 @@ struct GlobalRowFn {
 };
 
 // In-CTA canonical partitioned solve of an explicit system in global memory (its sweeps keep their
-// factors in registers: a factor read back from memory would cost a round trip a row) stored at sys (4 planes of
-// `plane` doubles: l, m, u, r), solution to x.  ws: workspace for the deeper levels
+// factors in registers: a factor read back from memory would cost a round trip a row) stored at sys
+// (4 planes of `plane` doubles: l, m, u, r), solution to x.  ws: workspace for the deeper levels
 // (<= 0.75*n + 16 doubles).  All threads of the CTA must call it.
 template <class Pivot>
 __device__ void cta_partitioned_global(int n, const double* sys, int plane, double* x, double* ws) {
@@ -711,9 +712,6 @@ __device__ void cta_partitioned_global(int n, const double* sys, int plane, doub
 
 }  // namespace
 
-__device__ void cta_tridiag(int n, const double* sys, int plane, double* x, double* ws) {
-    cta_partitioned_global<AnyPivot>(n, sys, plane, x, ws);
-}
 __device__ void cta_spline_tridiag(int n, const double* sys, int plane, double* x, double* ws) {
     cta_partitioned_global<SplinePivot>(n, sys, plane, x, ws);
 }
@@ -722,9 +720,9 @@ __device__ void cta_spline_tridiag(int n, const double* sys, int plane, double* 
 // The same canonical partitioned solve for many systems at once, one level per launch, the
 // chunks of every system spread over the grid (blockIdx.y = system, x = chunk): system s has
 // nrows[s] rows (0: skipped) at sys + 4*plane*s (planes l, m, u, r), solution to
-// x + plane*s, deeper levels in ws + ws_stride*s with cta_partitioned's layout.  Every chunk
-// performs cta_partitioned's operations in the same order, so the solution is identical to
-// cta_tridiag's; the launches replace its in-CTA barriers.  For long systems whose one CTA
+// x + plane*s, deeper levels in ws + ws_stride*s with cta_partitioned_global's layout.  Every
+// chunk performs its operations in the same order, so the solution is identical to
+// cta_spline_tridiag's; the launches replace its in-CTA barriers.  For long systems whose one CTA
 // would otherwise walk thousands of chunks.
 // ---------------------------------------------------------------------------------------
 namespace {
@@ -1005,7 +1003,7 @@ __device__ __forceinline__ void solve_separators(RedStage& st, int wcap, const d
                                                  double* wg) {
     const bool one = P <= kSolvePass;
     if (P <= kChunk) {
-        if (threadIdx.x == 0) thomas_rows<false>(st.row, P, 0.0, 0.0, st.x);
+        if (threadIdx.x == 0) thomas_rows(st.row, P, st.x);
         __syncthreads();
         if (threadIdx.x < P) X[threadIdx.x] = st.x[threadIdx.x];
         return;
@@ -1108,7 +1106,7 @@ __device__ __forceinline__ void solve_separators(RedStage& st, int wcap, const d
 
 // Transposed spline solve of the reverse pass in shared memory, one CTA per spline of nrows[s]
 // knots (0: none): positions kx, right-hand side rhs (rows s of `stride` doubles), solution to z;
-// cta_partitioned's operations in the same order.  The global-memory form spent its time in
+// cta_partitioned_global's operations in the same order.  The global-memory form spent its time in
 // round trips of its sweeps (N = 8192, white noise: 37 us a solve against X here).
 size_t adj_solve_smem(int cap) {
     const int P = cap / kChunk + 1;
@@ -1498,8 +1496,8 @@ __device__ __noinline__ void row_criterion(const SiftArgs& a, int c, int g, int 
 }
 
 // Adds the counts of some tiles (of one CTA's range) to their row's: one 64-bit sum of tiles,
-// additions with some sx > sd2, and samples with sx > sd, so that the thread that completes the row has them all from its own
-// addition, without a fence between counts and ticket (a fence here waits for the tile's stores:
+// additions with some sx > sd2, and samples with sx > sd, so that the thread that completes the row
+// has them all from its own addition, without a fence between counts and ticket (a fence here waits for the tile's stores:
 // about a microsecond of every CTA).  Rows of 2^17 tiles and more (2^28 samples) do not fit one
 // word: they are counted in separate words, ordered by fences.  Returns true to the thread that
 // completes the row.

@@ -77,7 +77,7 @@ struct EnvSmem {
         int cnt[kMaxTiles], base[kMaxTiles];   // knots, first slot
         int soff[kMaxTiles + 1];               // separators before the tile
         int prev[kMaxTiles], next[kMaxTiles];  // slots of the last knot before / first after it
-        int K, flags;
+        int K;
         double yend[2];
     }* I;
 };
@@ -140,8 +140,7 @@ __device__ __forceinline__ EnvSmem env_smem(const SmallLayout& L, unsigned char*
 
 // The interior of a chunk whose reciprocals the end relations left in c[1 .. len] (the chain is
 // 17 cycles a row forward and 9 back; a row a turn with its loads and tests took 180, four rows a
-// turn take 110)
-// (chunk_interior_knots' arrays): c receives the spline values, d the factors meanwhile.
+// turn take 110), in chunk_interior_knots' arrays: c receives the spline values, d the factors meanwhile.
 __device__ __forceinline__ void interior_known(const double* s, double* c, double* d, int len,
                                                double xl, double xr) {
     double l = d[0], u = d[1], s0 = s[1];

@@ -12,8 +12,9 @@
 namespace ceemdan {
 namespace {
 
-// Exact division by a tabled reciprocal: div_rcp's quotient (Markstein's correction, correctly
-// rounded in its range); `slow` marks operands outside that range, which take the division.
+// Division by a divisor d with y = RN(1/d): div_rcp's quotient (Markstein's correction, correctly
+// rounded in its range; tests/spline_div_check.cu); `slow` marks operands outside that range, which
+// take the division.
 __device__ __forceinline__ double rcp_fast(double a, double d, double y, bool& slow) {
     const double q0 = a * y;
     const double r = fma(-q0, d, a);
@@ -137,11 +138,7 @@ __device__ __forceinline__ void thomas_rolled(int n, const RowFn& row, const X& 
     back_sweep(n, gp, x, fac);
 }
 
-// Consecutive doubles as a row-indexed destination; NoIw drops what it is given.
-struct Slots {
-    double* p;
-    __device__ __forceinline__ double& operator()(int k) const { return p[k]; }
-};
+// Drops the reciprocals it is given.
 struct NoIw {
     struct Sink {
         __device__ __forceinline__ void operator=(double) const {}
@@ -233,7 +230,8 @@ __device__ __forceinline__ double div_int(double a, double d) {
     return q;
 }
 
-// seg_coeffs' b and d from the segment's length, slope and spline values.
+// A segment's coefficients (spline_coefficients) from its length, slope and spline values:
+// b = slope - h (2 c0 + c1) / 3, d = (c1 - c0) / (3h).
 __device__ __forceinline__ void seg_coeffs_int(double h, double slope, double c0, double c1,
                                                double& b, double& d) {
     const double hq = h * fma(2.0, c0, c1);
@@ -552,20 +550,16 @@ __device__ __forceinline__ void interior_rows(SepRow* r, int len, double xl, dou
     back_rows(r, x, len, gp);
 }
 
-// Canonical Thomas of n rows (kCoupled: a chunk between xl and xr), reciprocals formed here.
-template <bool kCoupled>
-__device__ __forceinline__ void thomas_rows(SepRow* r, int n, double xl, double xr, double* x) {
+// Canonical Thomas of n rows, reciprocals formed here.
+__device__ __forceinline__ void thomas_rows(SepRow* r, int n, double* x) {
     SepRow w = load_row(r);
     double cp = 0.0, gp = 0.0;
 #pragma unroll 1
     for (int k = 0; k < n; ++k) {
         const SepRow a = w;
         if (k + 1 < n) w = load_row(r + k + 1);
-        double ri = a.r;
-        if (kCoupled && k == 0) ri = fma(-a.l, xl, ri);
-        if (kCoupled && k == n - 1) ri = fma(-a.u, xr, ri);
         const double iw = pivot_inv(k == 0 ? a.m : fma(-a.l, cp, a.m));
-        gp = (k == 0 ? ri : fma(-a.l, gp, ri)) * iw;
+        gp = (k == 0 ? a.r : fma(-a.l, gp, a.r)) * iw;
         cp = a.u * iw;
         r[k].u = cp;
         x[k] = gp;
@@ -573,7 +567,7 @@ __device__ __forceinline__ void thomas_rows(SepRow* r, int n, double xl, double 
     back_rows(r, x, n, gp);
 }
 
-// cta_partitioned<SplinePivot> on padded rows: n rows at `rows` (u overwritten), solution to the
+// cta_partitioned_global<SplinePivot>'s solve on padded rows: n rows at `rows` (u overwritten), solution to the
 // padded x; ws: 5 padded(n/16) + 6 (n/16 + 1) doubles and as much again for what is below, at
 // most 0.75 n + 64.  Every thread of the group calls it.
 struct RowsLevel {
@@ -634,7 +628,7 @@ __device__ void partition_rows(const Group& grp, int n, SepRow* rows, double* x,
     }
     if (tid == 0) {
         const RowsLevel v = rows_level(depth, depth, n, rows, x, ws);
-        thomas_rows<false>(v.r, v.n, 0.0, 0.0, v.x);
+        thomas_rows(v.r, v.n, v.x);
     }
     grp.sync();
 #pragma unroll 1
