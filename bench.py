@@ -79,9 +79,11 @@ WORKLOAD_ITERATIONS = 12487
 # extrema: h read, bitmaps written; knots' positions and slopes, separator rows.  eval: h read,
 # next h and mean envelope written, bitmaps read; positions, slopes and separator values read.
 BYTES_PER_N = {"extrema": 8.25, "eval": 24.25,
-               # on-chip stage kernel: global bytes per sample-iteration (mean envelope written;
-               # h stays in shared memory)
-               "sift_small": 8.0}
+               # on-chip stage kernel, two CTAs a realization (the form of every short-row workload
+               # here): global bytes per sample-iteration, the mean envelope written and read back by
+               # the other CTA; h stays in shared memory.  (One CTA with both envelopes side by
+               # side moves 8, one after the other 24.)
+               "sift_small": 16.0}
 BYTES_PER_K = {"extrema": 12.0, "reduced_solve": 2.5, "eval": 10.5}
 
 

@@ -328,7 +328,7 @@ size_t tile_knots_smem() { return sizeof(KnotSmem); }
 //
 // Bound by instructions and the barriers between short phases (half of the issue slots used):
 // sixteen samples to a thread share signs between neighbours and one scan step, where one sample
-// to a lane took four times the instructions.  B200, N=244032 NR=100: 103 us at K/N = 0.18, 61 us
+// to a lane took four times the instructions.  B200, N=244032 NR=100: 104 us at K/N = 0.18, 61 us
 // at 0.001 (3.2 TB/s of its 8 N bytes), where the separate extrema, end-rule and chunk kernels took
 // 178 us on average.  Six CTAs per SM instead of five change nothing.
 //
@@ -1106,8 +1106,9 @@ __device__ __forceinline__ void solve_separators(RedStage& st, int wcap, const d
 
 // Transposed spline solve of the reverse pass in shared memory, one CTA per spline of nrows[s]
 // knots (0: none): positions kx, right-hand side rhs (rows s of `stride` doubles), solution to z;
-// cta_partitioned_global's operations in the same order.  The global-memory form spent its time in
-// round trips of its sweeps (N = 8192, white noise: 37 us a solve against X here).
+// cta_partitioned_global's operations in the same order.  The global-memory form spends its time in
+// round trips of its sweeps (N = 8192, NR = 50: 45 us a launch in the first stage and 23 in the
+// eighth, 15 and 9 here).
 size_t adj_solve_smem(int cap) {
     const int P = cap / kChunk + 1;
     return sizeof(double) * (2 * (size_t)padded(cap) + 5 * (size_t)padded(P) + 6 * (size_t)(P + 1) +
@@ -1448,8 +1449,8 @@ template __global__ void k_spline_solve<true>(const __grid_constant__ SiftArgs a
 // instead of being found again, a row's counts are added once per CTA, not per tile, and both
 // planes are stored coalesced out of shared memory (a thread's 32 bytes in a line each took 32
 // cycles of the load/store unit, half of all it did).  B200, N=244032 NR=100, K/N = 0.18: 262 ->
-// 206 us (2.8 TB/s of its 24 N bytes); K/N = 0.001: 167 -> 142 us; white noise: 381 -> 314 us.
-// Four CTAs with room for 1184: 225, 153 and 321 us.  Each class's launch takes the tiles of its
+// 205 us (2.9 TB/s of its 24 N bytes); K/N = 0.001: 167 -> 138 us; white noise: 381 -> 312 us.
+// Four CTAs with room for 1184 were 225, 153 and 321 us where five were 206, 142 and 314.  Each class's launch takes the tiles of its
 // own rows in even shares: with rows of both classes (K/N = 0.23) 398 -> 234 us.
 // =======================================================================================
 namespace {
