@@ -1250,7 +1250,7 @@ __device__ __noinline__ void end_rule_sparse(const SiftArgs& a, int e, int sp, i
 // separators at the tiles' edges, the separator system (levels >= 2 of the canonical partitioned
 // solve), and for every tile the knots just outside it with their spline values.  The system's
 // rows are staged once when they fit a pass (2048 rows).  Latency bound (a chain of short sweeps
-// per CTA): two CTAs per SM with the level-3 system in shared memory.  B200, N=244032 NR=100: 23.5
+// per CTA): two CTAs per SM with the level-3 system in shared memory.  B200, N=244032 NR=100: 24
 // us at K/N = 0.18, 55 us for white noise; the two kernels before it took 42 us on average.
 //
 // kExtrema: the counts and the end rule alone, for the extrema entry (no shared memory but the

@@ -25,8 +25,8 @@
 //
 // B200, one iteration of the first stages, the previous form (one kernel, unrolled sweeps, the
 // upper envelope handed over through L2, the stop test awaited at once) and this one: N=4096 NR=50
-// 37.6 -> 14.3 us, N=8192 NR=50 49.1 -> 19.2 (kPair); N=2501 NR=100 54.5 -> 14.7, N=5000 NR=100
-// 65.0 -> 20.5 (kDual); N=7680 NR=100 79.6 -> 33.2 (kSingle).  The code of an iteration has to stay
+// 37.6 -> 14.2 us, N=8192 NR=50 49.1 -> 19.2 (kPair); N=2501 NR=100 54.5 -> 14.9, N=5000 NR=100
+// 65.0 -> 20.8 (kDual); N=7680 NR=100 79.6 -> 33.7 (kSingle).  The code of an iteration has to stay
 // in the instruction cache: with a copy of build_envelope for each group kDual took 18.2 and 26.5.
 // At N=4096 NR=50 a quarter of the 28,000 cycles is the separator system (two sweeps of 15 rows at
 // 80 cycles a reciprocal, and their barriers), a quarter the evaluation and the exchange.
